@@ -175,13 +175,15 @@ def _params(case, nx, ny, problem=None, d=None, walls="reflect"):
 
 
 def _solves(case, seed):
-    """The solves of a batch: half blasts, half four-quadrant problems, sides log-uniform, each with its own end time."""
-    r = random.Random(seed * 7919 + 17)
+    """The solves of a batch: half blasts, half four-quadrant problems, sides log-uniform and an end time each, as the
+    case says; their initial states from the seed."""
+    shape = random.Random(1009 * case["count"] + 31 * case["side_min"] + case["side_max"])
+    r = random.Random(seed)
     out = []
     for k in range(case["count"]):
         problem = ("blast", "quadrants")[k % 2]
-        nx, ny = (_log_uniform(r, case["side_min"], case["side_max"]) for _ in range(2))
-        out.append({"problem": problem, "nx": nx, "ny": ny, "t_end": r.uniform(0.02, 0.05),
+        nx, ny = (_log_uniform(shape, case["side_min"], case["side_max"]) for _ in range(2))
+        out.append({"problem": problem, "nx": nx, "ny": ny, "t_end": shape.uniform(0.02, 0.05),
                     "walls": ("reflect", "absorb")[k % 2], "drawn": _drawn(problem, r.randrange(1 << 30))})
     return out
 
