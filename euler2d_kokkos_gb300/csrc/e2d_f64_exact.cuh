@@ -1,8 +1,8 @@
 // e2d_f64_exact.cuh -- exact FP64 operations carried out on the integer
 // pipe.
 //
-// GB300 issues FP64 arithmetic at ~1.7 operations per SM per clock, about
-// 1/70 of its FP32 rate.  Comparisons, min/max against known signs, sign
+// GB300 issues FP64 arithmetic at 1.7 to 2 operations per SM per clock, about
+// 1/64 of its FP32 rate.  Comparisons, min/max against known signs, sign
 // tests and multiplications by 0.5 or 2 do not need the FP64 unit: on the
 // bit patterns of IEEE-754 doubles they are integer operations that give the
 // same bits as the FP64 instructions.  Each helper states the inputs for which
@@ -12,8 +12,53 @@
 
 #include <cuda_runtime.h>
 
+#include "e2d_f64_intdiv.h"
+
 namespace e2d {
 namespace f64x {
+
+// Additions and products as fused multiply-adds of three registers.  The FP64
+// pipe takes 16 clocks per SM for a warp's DFMA whose operands are all
+// registers and 19 for a DADD, a DMUL or any form with a constant or uniform
+// operand (measured: 625 against 527 G operations/s), so x + y is issued as
+// x * 1 + y and x * y as x * y + (-0): the same roundings and the same signs
+// of zero.  1 and -0 have to sit in registers the compiler knows nothing of;
+// each lane loads them from its own address.
+static __device__ double2 g_unit[32] = {
+#define E2D_U4 {1.0, -0.0}, {1.0, -0.0}, {1.0, -0.0}, {1.0, -0.0}
+    E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4
+#undef E2D_U4
+};
+struct Fp {
+  double one, mzero;
+  __device__ __forceinline__ Fp() {
+    const double2 *p = g_unit + (threadIdx.x & 31);
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(one), "=d"(mzero) : "l"(p));
+  }
+  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return fma(a, one, -b); }
+  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, mzero); }
+};
+
+// a / b and sqrt(x) as the IEEE operations give them, on the integer pipes
+// (e2d_f64_intdiv.h); operands outside their range run the operation itself.
+static __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
+static __device__ __noinline__ double sqrt_slow(double x) { return sqrt(x); }
+using f64i::Divisor;
+using f64i::divisor;
+__device__ __forceinline__ double quot(double a, const Divisor &d) {
+  bool ok;
+  double q = f64i::quotient(a, d, ok);
+  if (!ok) q = div_slow(a, __hiloint2double((int)d.hi, (int)d.lo));
+  return q;
+}
+__device__ __forceinline__ double quot(double a, double b) { return quot(a, divisor(b)); }
+__device__ __forceinline__ double root(double x) {
+  bool ok;
+  double s = f64i::root(x, ok);
+  if (!ok) s = sqrt_slow(x);
+  return s;
+}
 
 constexpr unsigned long long kMag = 0x7fffffffffffffffull;
 constexpr unsigned long long kSign = 0x8000000000000000ull;
@@ -52,6 +97,10 @@ __device__ __forceinline__ double max_any(double a, double b) { return okey(a) >
 // Sign tests for non-NaN x.
 __device__ __forceinline__ bool gt0(double x) { return sbits(x) > 0; }   // x > 0.0
 __device__ __forceinline__ bool le0(double x) { return sbits(x) <= 0; }  // x <= 0.0
+__device__ __forceinline__ bool lt0(double x) { return (ubits(x) > kSign) & (sbits(x) < 0); }  // x < 0.0
+__device__ __forceinline__ bool is_nan(double x) { return (ubits(x) & kMag) > 0x7ff0000000000000ull; }
+// x > c for x >= 0 and c > 0 (a NaN x gives false)
+__device__ __forceinline__ bool gt_pos(double x, double c) { return sbits(x) > sbits(c) && !is_nan(x); }
 
 // 0.5 * x: decrement the exponent of normal numbers with a biased exponent in
 // [2, 2046]; zeros are unchanged; subnormal results need rounding and use the
@@ -87,10 +136,10 @@ static __device__ __noinline__ bool product_le0_slow(double a, double b) { retur
 // test dlft*drgt <= 0 equals "a zero or opposite signs" unless the product
 // underflows to zero, which needs both magnitudes below 2^-511: that case is
 // decided by the FP64 product itself.
-__device__ __forceinline__ double slope_limited(bool st2, double q, double qp, double qm) {
-  const double d1 = q - qm;
-  const double d2 = qp - q;
-  const double dc = qp - qm;
+__device__ __forceinline__ double slope_limited(const Fp &f, bool st2, double q, double qp, double qm) {
+  const double d1 = f.sub(q, qm);
+  const double d2 = f.sub(qp, q);
+  const double dc = f.sub(qp, qm);
   const long long b1 = sbits(d1), b2 = sbits(d2);
   const unsigned long long a1 = (unsigned long long)b1 & kMag;
   const unsigned long long a2 = (unsigned long long)b2 & kMag;

@@ -89,8 +89,10 @@ __device__ __forceinline__ void fill_cell(const KParams64 &kp, double *__restric
     }
   }
   if (mode & (FILL_WRITE_Q | FILL_DT)) {
+    const Fp f;
     double dd, p, ux, uy;
-    primitives(ph, rho, e, mx, my, dd, p, ux, uy);
+    Divisor dv;
+    primitives(f, ph, rho, e, mx, my, dd, p, ux, uy, dv);
     if (mode & FILL_WRITE_Q) {
       q[d] = dd;
       q[d + g.plane] = p;
@@ -98,7 +100,7 @@ __device__ __forceinline__ void fill_cell(const KParams64 &kp, double *__restric
       q[d + 3 * g.plane] = uy;
     }
     if ((mode & FILL_DT) && !ghost) {
-      term = cfl_term(ph, dd, p, ux, uy);
+      term = cfl_term(f, ph, dv, p, ux, uy);
       flags |= state_flags(rho, e, mx, my);
     }
   }
@@ -110,7 +112,7 @@ __device__ __forceinline__ void fill_cell(const KParams64 &kp, double *__restric
 __device__ __forceinline__ void fill_reduce(double term, unsigned int flags, unsigned long long *acc,
                                             unsigned int *status) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) term = fmax(term, __shfl_xor_sync(0xffffffffu, term, off));
+  for (int off = 16; off > 0; off >>= 1) term = fmax_any(term, __shfl_xor_sync(0xffffffffu, term, off));
   flags = __reduce_or_sync(0xffffffffu, flags);
   __shared__ double wmax[FILL_BX * FILL_BY / 32];
   __shared__ unsigned int wflags[FILL_BX * FILL_BY / 32];
@@ -124,10 +126,10 @@ __device__ __forceinline__ void fill_reduce(double term, unsigned int flags, uns
     double m = wmax[0];
     unsigned int f = wflags[0];
     for (int w = 1; w < FILL_BX * FILL_BY / 32; ++w) {
-      m = fmax(m, wmax[w]);
+      m = fmax_any(m, wmax[w]);
       f |= wflags[w];
     }
-    if (m > 0.0) atomicMax(acc, (unsigned long long)__double_as_longlong(m));
+    if (gt0(m)) atomicMax(acc, (unsigned long long)__double_as_longlong(m));
     if (f) atomicOr(status, f);
   }
 }
@@ -228,7 +230,7 @@ __device__ __forceinline__ void gather_qtile(const KGeom &g, const double *__res
 // On return (after a block barrier) sXm holds the x-fluxes scaled by dt/dx
 // and sYm the y-fluxes scaled by dt/dy.
 template <int RS, int TX, int TY, int NT, bool FAST = false>
-__device__ __forceinline__ void tile_fluxes(const KPhys<double> &ph, const double dtdx, const double dtdy,
+__device__ __forceinline__ void tile_fluxes(const Fp &fp64, const KPhys<double> &ph, const double dtdx, const double dtdy,
                                             double *smem) {
   using T = TileSmem<TX, TY>;
   constexpr int QW = T::QW, QH = T::QH, XW = T::XW, YH = T::YH;
@@ -266,23 +268,23 @@ __device__ __forceinline__ void tile_fluxes(const KPhys<double> &ph, const doubl
     for (int v = 0; v < 4; ++v) {
       const double *P = sQ + v * QH * QW;
       qc[v] = P[c];
-      dqx[v] = slope(st_kind, qc[v], P[c + 1], P[c - 1]);
-      dqy[v] = slope(st_kind, qc[v], P[c + QW], P[c - QW]);
+      dqx[v] = slope(fp64, st_kind, qc[v], P[c + 1], P[c - 1]);
+      dqy[v] = slope(fp64, st_kind, qc[v], P[c + QW], P[c - QW]);
     }
     double s0[4];
     if (FAST)
-      trace_sources_fast(ph, qc, dqx, dqy, s0);
+      trace_sources_fast(fp64, ph, qc, dqx, dqy, s0);
     else
-      trace_sources(ph, qc, dqx, dqy, s0);
+      trace_sources(fp64, ph, qc, dqx, dqy, s0);
     if (yin) {
       const int o = (yy - 1) * XW + xx;
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         double fm, fp;
         if (FAST)
-          face_pair_fast(ph, v, qc[v], dqx[v], s0[v], 0.5 * dtdx, fm, fp);
+          face_pair_fast(fp64, ph, v, qc[v], dqx[v], s0[v], 0.5 * dtdx, fm, fp);
         else
-          face_pair(ph, v, qc[v], dqx[v], s0[v], dtdx, fm, fp);
+          face_pair(fp64, ph, v, qc[v], dqx[v], s0[v], dtdx, fm, fp);
         if (xx >= 1) sXm[v * TY * XW + o] = fm;
         if (xx <= TX) sXp[v * TY * XW + o] = fp;
       }
@@ -293,9 +295,9 @@ __device__ __forceinline__ void tile_fluxes(const KPhys<double> &ph, const doubl
       for (int v = 0; v < 4; ++v) {
         double fm, fp;
         if (FAST)
-          face_pair_fast(ph, v, qc[v], dqy[v], s0[v], 0.5 * dtdy, fm, fp);
+          face_pair_fast(fp64, ph, v, qc[v], dqy[v], s0[v], 0.5 * dtdy, fm, fp);
         else
-          face_pair(ph, v, qc[v], dqy[v], s0[v], dtdy, fm, fp);
+          face_pair(fp64, ph, v, qc[v], dqy[v], s0[v], dtdy, fm, fp);
         if (yy >= 1) sYm[v * YH * TX + o] = fm;
         if (yy <= TY) sYp[v * YH * TX + o] = fp;
       }
@@ -317,9 +319,9 @@ __device__ __forceinline__ void tile_fluxes(const KPhys<double> &ph, const doubl
         ql[v] = sXp[v * TY * XW + ol];
         qr[v] = sXm[v * TY * XW + orr];
       }
-      riemann_sel<RS, FAST>(ph, ql, qr, f);
+      riemann_sel<RS, FAST>(fp64, ph, ql, qr, f);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sXm[v * TY * XW + orr] = f[v] * dtdx;
+      for (int v = 0; v < 4; ++v) sXm[v * TY * XW + orr] = fp64.mul(f[v], dtdx);
     } else {
       const int kk = k - NXF;
       const int fy = kk / TX, x = kk - fy * TX;
@@ -331,11 +333,11 @@ __device__ __forceinline__ void tile_fluxes(const KPhys<double> &ph, const doubl
         ql[vs] = sYp[v * YH * TX + ol];
         qr[vs] = sYm[v * YH * TX + orr];
       }
-      riemann_sel<RS, FAST>(ph, ql, qr, f);
+      riemann_sel<RS, FAST>(fp64, ph, ql, qr, f);
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         const int vs = (v == E2D_IU) ? E2D_IV : (v == E2D_IV) ? E2D_IU : v;
-        sYm[v * YH * TX + orr] = f[vs] * dtdy;
+        sYm[v * YH * TX + orr] = fp64.mul(f[vs], dtdy);
       }
     }
   }
@@ -345,12 +347,13 @@ __device__ __forceinline__ void tile_fluxes(const KPhys<double> &ph, const doubl
 // The conservative update of cell (x, y) of a tile in the reference's order
 // (src/HydroRunFunctors.h:691-713): +Fx(i) -Fx(i+1) +Fy(j) -Fy(j+1).
 template <int TX, int TY>
-__device__ __forceinline__ double update_var(const TileSmem<TX, TY> &sm, int v, int x, int y, double uu) {
+__device__ __forceinline__ double update_var(const Fp &f, const TileSmem<TX, TY> &sm, int v, int x, int y,
+                                             double uu) {
   using T = TileSmem<TX, TY>;
-  uu = uu + sm.sXm[v * TY * T::XW + y * T::XW + x + 1];
-  uu = uu - sm.sXm[v * TY * T::XW + y * T::XW + x + 2];
-  uu = uu + sm.sYm[v * T::YH * TX + (y + 1) * TX + x];
-  uu = uu - sm.sYm[v * T::YH * TX + (y + 2) * TX + x];
+  uu = f.add(uu, sm.sXm[v * TY * T::XW + y * T::XW + x + 1]);
+  uu = f.sub(uu, sm.sXm[v * TY * T::XW + y * T::XW + x + 2]);
+  uu = f.add(uu, sm.sYm[v * T::YH * TX + (y + 1) * TX + x]);
+  uu = f.sub(uu, sm.sYm[v * T::YH * TX + (y + 2) * TX + x]);
   return uu;
 }
 
@@ -364,9 +367,10 @@ __device__ __forceinline__ void flux_tile(const KParams64 &kp, const double *__r
   const KGeom &g = kp.g;
   const int i0 = bx * TX;  // array column of the tile's first halo cell
   const int j0 = by * TY;
+  const Fp f;
   load_qtile<TX, TY, NT>(g, q, i0, j0, smem);
   __syncthreads();
-  tile_fluxes<RS, TX, TY, NT>(kp.ph, dtdx, dtdy, smem);
+  tile_fluxes<RS, TX, TY, NT>(f, kp.ph, dtdx, dtdy, smem);
   const TileSmem<TX, TY> sm(smem);
   // stage 4: conservative update
   for (int k = threadIdx.x; k < TX * TY; k += NT) {
@@ -375,7 +379,7 @@ __device__ __forceinline__ void flux_tile(const KParams64 &kp, const double *__r
     if (gi < g.nx + 2 && gj < g.ny + 2) {
       const size_t s = (size_t)gi + (size_t)g.isize * gj;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) u_out[s + v * g.plane] = update_var<TX, TY>(sm, v, x, y, u_in[s + v * g.plane]);
+      for (int v = 0; v < 4; ++v) u_out[s + v * g.plane] = update_var<TX, TY>(f, sm, v, x, y, u_in[s + v * g.plane]);
     }
   }
 }
@@ -401,8 +405,8 @@ __global__ void __launch_bounds__(NT, MINB)
       dt = step_dt(ph, clk->invdt_bits, clk->t, clk->t_end);
     }
     s_dt[0] = dt;
-    s_dt[1] = dt / ph.dx;
-    s_dt[2] = dt / ph.dy;
+    s_dt[1] = quot(dt, ph.dx);
+    s_dt[2] = quot(dt, ph.dy);
     s_run = run;
   }
   __syncthreads();
@@ -441,7 +445,7 @@ template <int NT>
 __device__ __forceinline__ void block_fold(double term, unsigned int flags, unsigned long long *acc,
                                            unsigned int *status) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) term = fmax(term, __shfl_xor_sync(0xffffffffu, term, off));
+  for (int off = 16; off > 0; off >>= 1) term = fmax_any(term, __shfl_xor_sync(0xffffffffu, term, off));
   flags = __reduce_or_sync(0xffffffffu, flags);
   __shared__ double wmax[NT / 32];
   __shared__ unsigned int wflags[NT / 32];
@@ -456,10 +460,10 @@ __device__ __forceinline__ void block_fold(double term, unsigned int flags, unsi
     unsigned int f = wflags[0];
 #pragma unroll
     for (int w = 1; w < NT / 32; ++w) {
-      m = fmax(m, wmax[w]);
+      m = fmax_any(m, wmax[w]);
       f |= wflags[w];
     }
-    if (m > 0.0) atomicMax(acc, (unsigned long long)__double_as_longlong(m));
+    if (gt0(m)) atomicMax(acc, (unsigned long long)__double_as_longlong(m));
     if (f) atomicOr(status, f);
   }
 }
@@ -468,7 +472,7 @@ __device__ __forceinline__ void block_fold(double term, unsigned int flags, unsi
 // shared memory: the conservative update into u_out, the primitives of the
 // new cells into q_out and the running maximum of their CFL terms and flags.
 template <int TX, int TY, int NT, bool FAST>
-__device__ __forceinline__ void step_epilogue(const KParams64 &kp, const double *__restrict__ u_in,
+__device__ __forceinline__ void step_epilogue(const Fp &f, const KParams64 &kp, const double *__restrict__ u_in,
                                               double *__restrict__ u_out, double *__restrict__ q_out, int i0,
                                               int j0, double *smem, double &term, unsigned int &flags) {
   const KGeom &g = kp.g;
@@ -482,19 +486,20 @@ __device__ __forceinline__ void step_epilogue(const KParams64 &kp, const double 
       double un[4];
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        un[v] = update_var<TX, TY>(sm, v, x, y, u_in[s + v * g.plane]);
+        un[v] = update_var<TX, TY>(f, sm, v, x, y, u_in[s + v * g.plane]);
         u_out[s + v * g.plane] = un[v];
       }
-      double dd, p, ux, uy, rd = 0.0;
+      double dd, p, ux, uy;
+      Divisor dv;
       if (FAST)
-        primitives_fast(ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, rd);
+        primitives_fast(f, ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, dv);
       else
-        primitives(ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy);
+        primitives(f, ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, dv);
       q_out[s] = dd;
       q_out[s + g.plane] = p;
       q_out[s + 2 * g.plane] = ux;
       q_out[s + 3 * g.plane] = uy;
-      term = fmax(term, FAST ? cfl_term_fast(ph, rd, p, ux, uy) : cfl_term(ph, dd, p, ux, uy));
+      term = fmax_any(term, FAST ? cfl_term_fast(f, ph, dv, p, ux, uy) : cfl_term(f, ph, dv, p, ux, uy));
       flags |= state_flags(un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV]);
     }
   }
@@ -572,8 +577,8 @@ __global__ void __launch_bounds__(NT, MINB)
     const int par = clk->nstep & 1;
     const double dt = step_dt(ph, clk->acc[par], clk->t, clk->t_end);
     s_dt[0] = dt;
-    s_dt[1] = dt / ph.dx;
-    s_dt[2] = dt / ph.dy;
+    s_dt[1] = quot(dt, ph.dx);
+    s_dt[2] = quot(dt, ph.dy);
     s_run = run;
     s_par = par;
     if (run && tma_tile) {
@@ -604,11 +609,12 @@ __global__ void __launch_bounds__(NT, MINB)
     __syncthreads();
   }
 
+  const Fp f;
   double term = 0.0;
   unsigned int flags = 0;
   if (ok) {
-    tile_fluxes<RS, TX, TY, NT, FAST>(ph, s_dt[1], s_dt[2], smem);
-    step_epilogue<TX, TY, NT, FAST>(kp, u_in, u_out, q_out, i0, j0, smem, term, flags);
+    tile_fluxes<RS, TX, TY, NT, FAST>(f, ph, s_dt[1], s_dt[2], smem);
+    step_epilogue<TX, TY, NT, FAST>(f, kp, u_in, u_out, q_out, i0, j0, smem, term, flags);
   }
   ghost_fill_tile<TX, TY, NT>(g, u_in, u_out, i0, j0, bx == 0, bx == (int)gridDim.x - 1, by == 0,
                               by == (int)gridDim.y - 1);
@@ -675,6 +681,7 @@ __global__ void __launch_bounds__(512, 1)
   double *smem = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   __shared__ double s_dt[3];
   const int tid = threadIdx.x;
+  const Fp f;
   for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
     const int k = list_entry(tile_begin, n_inst, w);
     BatchInst64 &I = insts[list_slots[k]];
@@ -684,8 +691,8 @@ __global__ void __launch_bounds__(512, 1)
     if (tid == 0) {
       const double dt = step_dt(kp.ph, I.acc[par], I.t, I.t_end);
       s_dt[0] = dt;
-      s_dt[1] = dt / kp.ph.dx;
-      s_dt[2] = dt / kp.ph.dy;
+      s_dt[1] = quot(dt, kp.ph.dx);
+      s_dt[2] = quot(dt, kp.ph.dy);
     }
     const int b = w - tile_begin[k];
     const int by = b / I.ntx, bx = b - by * I.ntx;
@@ -695,8 +702,8 @@ __global__ void __launch_bounds__(512, 1)
     __syncthreads();
     double term = 0.0;
     unsigned int flags = 0;
-    tile_fluxes<RS, 32, 32, 512>(kp.ph, s_dt[1], s_dt[2], smem);
-    step_epilogue<32, 32, 512, false>(kp, I.u[par], I.u[par ^ 1], I.q[par ^ 1], i0, j0, smem, term, flags);
+    tile_fluxes<RS, 32, 32, 512>(f, kp.ph, s_dt[1], s_dt[2], smem);
+    step_epilogue<32, 32, 512, false>(f, kp, I.u[par], I.u[par ^ 1], I.q[par ^ 1], i0, j0, smem, term, flags);
     ghost_fill_tile<32, 32, 512>(kp.g, I.u[par], I.u[par ^ 1], i0, j0, bx == 0, bx == I.ntx - 1, by == 0,
                                  by == nty - 1);
     block_fold<512>(term, flags, &I.acc[par ^ 1], &I.status);
@@ -731,46 +738,48 @@ __global__ void k_eval_f64(const KParams64 kp, const int what, const int n,
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const KPhys<double> &ph = kp.ph;
+  const Fp f;
   const int st_kind = (ph.slope_type == 2.0) ? 2 : (ph.slope_type == 1.0) ? 1 : 0;
   if (what == E2D_EVAL_PRIMITIVES) {
     const double *u = in + 4 * k;
     double d, p, ux, uy;
-    primitives(ph, u[E2D_ID], u[E2D_IP], u[E2D_IU], u[E2D_IV], d, p, ux, uy);
+    Divisor dv;
+    primitives(f, ph, u[E2D_ID], u[E2D_IP], u[E2D_IU], u[E2D_IV], d, p, ux, uy, dv);
     double *o = out + 5 * k;
     o[E2D_ID] = d;
     o[E2D_IP] = p;
     o[E2D_IU] = ux;
     o[E2D_IV] = uy;
-    o[4] = sqrt(ph.gamma0 * p / d);
+    o[4] = root(quot(f.mul(ph.gamma0, p), dv));
   } else if (what == E2D_EVAL_SLOPES) {
     const double *s = in + 20 * k;  // q, q(+x), q(-x), q(+y), q(-y)
     double *o = out + 8 * k;
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-      o[v] = slope(st_kind, s[v], s[4 + v], s[8 + v]);
-      o[4 + v] = slope(st_kind, s[v], s[12 + v], s[16 + v]);
+      o[v] = slope(f, st_kind, s[v], s[4 + v], s[8 + v]);
+      o[4 + v] = slope(f, st_kind, s[v], s[12 + v], s[16 + v]);
     }
   } else if (what >= E2D_EVAL_TRACE_XMIN && what <= E2D_EVAL_TRACE_YMAX) {
     const double *s = in + 12 * k;  // q, dqx, dqy
     double s0[4];
-    trace_sources(ph, s, s + 4, s + 8, s0);
+    trace_sources(f, ph, s, s + 4, s + 8, s0);
     const int face = what - E2D_EVAL_TRACE_XMIN;
     const bool xdir = face < 2;
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       double fm, fp;
-      face_pair(ph, v, s[v], xdir ? s[4 + v] : s[8 + v], s0[v], xdir ? dtdx : dtdy, fm, fp);
+      face_pair(f, ph, v, s[v], xdir ? s[4 + v] : s[8 + v], s0[v], xdir ? dtdx : dtdy, fm, fp);
       out[4 * k + v] = (face == 0 || face == 2) ? fm : fp;
     }
   } else {
     const double *s = in + 8 * k;  // qleft, qright
     double *o = out + 4 * k;
     if (what == E2D_EVAL_RIEMANN_HLLC)
-      riemann_hllc(ph, s, s + 4, o);
+      riemann_hllc(f, ph, s, s + 4, o);
     else if (what == E2D_EVAL_RIEMANN_HLL)
-      riemann_hll(ph, s, s + 4, o);
+      riemann_hll(f, ph, s, s + 4, o);
     else
-      riemann_approx(ph, s, s + 4, o);
+      riemann_approx(f, ph, s, s + 4, o);
   }
 }
 

@@ -26,45 +26,65 @@ __device__ __forceinline__ int src_lo_hi(int i, int n, int bc_lo, int bc_hi, boo
 __device__ __forceinline__ bool nonfinite(double x) { return nonfinite64(x); }
 
 // ------------------------------------------------------------ numerics
+using f64x::divisor;
+using f64x::Divisor;
+using f64x::Fp;
+using f64x::quot;
+using f64x::root;
+
+// max(p, d * smallp), d > 0.  High words of positive doubles grow like 2^20
+// times their logarithm (within 0.09 2^20), so p exceeds the product for
+// certain when they differ by more than smallp's exponent plus two; only then
+// is the product not formed (one FP64 instruction of the two each face state
+// would take; every cell of an ordinary flow).
+__device__ __forceinline__ double floor_pressure(const Fp &f, const KPhys<double> &ph, double p, double d) {
+  const int lim = (__double2hiint(ph.smallp) & 0x7ff00000) - (1020 << 20);  // (exponent + 3) 2^20
+  if (__double2hiint(p) >= 0x00100000 && __double2hiint(p) - __double2hiint(d) > lim) return p;
+  return max_pos(p, f.mul(d, ph.smallp));
+}
+
 // src/HydroBaseFunctor.h:76-102 (computePrimitives) without the sound speed.
-__device__ __forceinline__ void primitives(const KPhys<double> &ph, double rho, double e, double mx,
-                                           double my, double &d, double &p, double &ux, double &uy) {
+// `dv`: the density, ready as a divisor.
+__device__ __forceinline__ void primitives(const Fp &f, const KPhys<double> &ph, double rho, double e, double mx,
+                                           double my, double &d, double &p, double &ux, double &uy, Divisor &dv) {
   d = max_pos(rho, ph.smallr);
-  ux = mx / d;
-  uy = my / d;
-  const double eken = half(ux * ux + uy * uy);
-  const double ei = e / d - eken;
-  p = max_pos(ph.gm1 * d * ei, d * ph.smallp);
+  dv = divisor(d);
+  ux = quot(mx, dv);
+  uy = quot(my, dv);
+  const double eken = half(f.add(f.mul(ux, ux), f.mul(uy, uy)));
+  const double ei = f.sub(quot(e, dv), eken);
+  p = floor_pressure(f, ph, f.mul(f.mul(ph.gm1, d), ei), d);
 }
 
 // src/HydroBaseFunctor.h:475-516 for one variable and direction: slope_type
 // 0 gives a zero slope, 1 and 2 the limited slope.
-__device__ __forceinline__ double slope(int st_kind, double q, double qp, double qm) {
+__device__ __forceinline__ double slope(const Fp &f, int st_kind, double q, double qp, double qm) {
   if (st_kind == 0) return 0.0;
-  return f64x::slope_limited(st_kind == 2, q, qp, qm);
+  return f64x::slope_limited(f, st_kind == 2, q, qp, qm);
 }
 
 // Sources of trace_unsplit_2d_along_dir (src/HydroBaseFunctor.h:246-249).
-__device__ __forceinline__ void trace_sources(const KPhys<double> &ph, const double q[4],
+__device__ __forceinline__ void trace_sources(const Fp &f, const KPhys<double> &ph, const double q[4],
                                               const double dqx[4], const double dqy[4], double s0[4]) {
   const double r = q[E2D_ID], p = q[E2D_IP], u = q[E2D_IU], v = q[E2D_IV];
-  const double drx = dqx[E2D_ID], dpx = dqx[E2D_IP], dux = dqx[E2D_IU], dvx = dqx[E2D_IV];
-  const double dry = dqy[E2D_ID], dpy = dqy[E2D_IP], duy = dqy[E2D_IU], dvy = dqy[E2D_IV];
-  s0[E2D_ID] = -u * drx - v * dry - (dux + dvy) * r;
-  s0[E2D_IP] = -u * dpx - v * dpy - (dux + dvy) * ph.gamma0 * p;
-  s0[E2D_IU] = -u * dux - v * duy - (dpx) / r;
-  s0[E2D_IV] = -u * dvx - v * dvy - (dpy) / r;
+  const Divisor dr = divisor(r);
+  const double div = f.add(dqx[E2D_IU], dqy[E2D_IV]);
+  auto advect = [&](int k) { return f.sub(f.mul(-u, dqx[k]), f.mul(v, dqy[k])); };  // -u*dqx - v*dqy
+  s0[E2D_ID] = f.sub(advect(E2D_ID), f.mul(div, r));
+  s0[E2D_IP] = f.sub(advect(E2D_IP), f.mul(f.mul(div, ph.gamma0), p));
+  s0[E2D_IU] = f.sub(advect(E2D_IU), quot(dqx[E2D_IP], dr));
+  s0[E2D_IV] = f.sub(advect(E2D_IV), quot(dqy[E2D_IP], dr));
 }
 
 // The two face states of one direction (src/HydroBaseFunctor.h:251-289):
 // minus face q - dq/2 + s0*dtd/2, plus face q + dq/2 + s0*dtd/2, density
 // clamped at smallr.
-__device__ __forceinline__ void face_pair(const KPhys<double> &ph, int v, double q, double dq,
+__device__ __forceinline__ void face_pair(const Fp &f, const KPhys<double> &ph, int v, double q, double dq,
                                           double s0, double dtd, double &fm, double &fp) {
   const double h = half(dq);
-  const double sx = half(s0 * dtd);
-  fm = q - h + sx;
-  fp = q + h + sx;
+  const double sx = half(f.mul(s0, dtd));
+  fm = f.add(f.sub(q, h), sx);
+  fp = f.add(f.add(q, h), sx);
   if (v == E2D_ID) {
     fm = max_pos(fm, ph.smallr);
     fp = max_pos(fp, ph.smallr);
@@ -72,133 +92,144 @@ __device__ __forceinline__ void face_pair(const KPhys<double> &ph, int v, double
 }
 
 // src/HydroBaseFunctor.h:523-547.
-__device__ __forceinline__ void cmpflx(const KPhys<double> &ph, const double g[4], double f[4]) {
-  f[E2D_ID] = g[E2D_ID] * g[E2D_IU];
-  f[E2D_IU] = f[E2D_ID] * g[E2D_IU] + g[E2D_IP];
-  f[E2D_IV] = f[E2D_ID] * g[E2D_IV];
-  const double ekin = 0.5 * g[E2D_ID] * (g[E2D_IU] * g[E2D_IU] + g[E2D_IV] * g[E2D_IV]);
-  const double etot = g[E2D_IP] * ph.entho + ekin;
-  f[E2D_IP] = g[E2D_IU] * (etot + g[E2D_IP]);
+__device__ __forceinline__ void cmpflx(const Fp &o, const KPhys<double> &ph, const double g[4], double f[4]) {
+  f[E2D_ID] = o.mul(g[E2D_ID], g[E2D_IU]);
+  f[E2D_IU] = o.add(o.mul(f[E2D_ID], g[E2D_IU]), g[E2D_IP]);
+  f[E2D_IV] = o.mul(f[E2D_ID], g[E2D_IV]);
+  const double ekin = o.mul(half(g[E2D_ID]), o.add(o.mul(g[E2D_IU], g[E2D_IU]), o.mul(g[E2D_IV], g[E2D_IV])));
+  const double etot = o.add(o.mul(g[E2D_IP], ph.entho), ekin);
+  f[E2D_IP] = o.mul(g[E2D_IU], o.add(etot, g[E2D_IP]));
+}
+
+// fmax of any two doubles, NaN dropped as fmax drops it, on the integer pipe.
+__device__ __forceinline__ double fmax_any(double a, double b) {
+  return f64x::is_nan(a) ? b : f64x::is_nan(b) ? a : max_any(a, b);
 }
 
 // src/HydroBaseFunctor.h:558-693 (riemann_approx).
-__device__ __noinline__ void riemann_approx(const KPhys<double> &ph, const double *ql,
+__device__ __noinline__ void riemann_approx(const Fp &f, const KPhys<double> &ph, const double *ql,
                                             const double *qr, double *flux) {
   const double gamma0 = ph.gamma0, gamma6 = ph.gamma6;
-  const double rl = fmax(ql[E2D_ID], ph.smallr), ul = ql[E2D_IU];
-  const double pl = fmax(ql[E2D_IP], rl * ph.smallp);
-  const double rr = fmax(qr[E2D_ID], ph.smallr), ur = qr[E2D_IU];
-  const double pr = fmax(qr[E2D_IP], rr * ph.smallp);
-  const double cl = gamma0 * pl * rl;
-  const double cr = gamma0 * pr * rr;
-  double wl = sqrt(cl);
-  double wr = sqrt(cr);
-  double pstar = fmax(((wr * pl + wl * pr) + wl * wr * (ul - ur)) / (wl + wr), 0.0);
+  const double rl = fmax_any(ql[E2D_ID], ph.smallr), ul = ql[E2D_IU];
+  const double pl = fmax_any(ql[E2D_IP], f.mul(rl, ph.smallp));
+  const double rr = fmax_any(qr[E2D_ID], ph.smallr), ur = qr[E2D_IU];
+  const double pr = fmax_any(qr[E2D_IP], f.mul(rr, ph.smallp));
+  const double cl = f.mul(f.mul(gamma0, pl), rl);
+  const double cr = f.mul(f.mul(gamma0, pr), rr);
+  const Divisor dpl = divisor(pl), dpr = divisor(pr);
+  // sqrt(c * (1 + gamma6 * (p - ps) / ps))
+  auto wave = [&](double c, double p, double ps, const Divisor &dps) {
+    return root(f.mul(c, f.add(f.one, quot(f.mul(gamma6, f.sub(p, ps)), dps))));
+  };
+  double wl = root(cl);
+  double wr = root(cr);
+  double pstar = fmax_any(quot(f.add(f.add(f.mul(wr, pl), f.mul(wl, pr)), f.mul(f.mul(wl, wr), f.sub(ul, ur))),
+                               f.add(wl, wr)),
+                          0.0);
   double pold = pstar;
   double conv = 1.0;
-  for (int iter = 0; (iter < 10) && (conv > 1e-6); ++iter) {
-    const double wwl = sqrt(cl * (1.0 + gamma6 * (pold - pl) / pl));
-    const double wwr = sqrt(cr * (1.0 + gamma6 * (pold - pr) / pr));
-    const double qxl = 2.0 * wwl * wwl * wwl / (wwl * wwl + cl);
-    const double qxr = 2.0 * wwr * wwr * wwr / (wwr * wwr + cr);
-    const double usl = ul - (pold - pl) / wwl;
-    const double usr = ur + (pold - pr) / wwr;
-    const double delp = fmax(qxr * qxl / (qxr + qxl) * (usl - usr), -pold);
-    pold = pold + delp;
-    conv = fabs(delp / (pold + ph.smallpp));
+  for (int iter = 0; (iter < 10) && f64x::gt_pos(conv, 1e-6); ++iter) {
+    const double wwl = wave(cl, pold, pl, dpl);
+    const double wwr = wave(cr, pold, pr, dpr);
+    const double w2l = f.mul(wwl, wwl), w2r = f.mul(wwr, wwr);
+    // 2 w w w: the doubling is exact wherever it is applied (no overflow here)
+    const double qxl = quot(f.mul(f.mul(f64x::twice(wwl), wwl), wwl), f.add(w2l, cl));
+    const double qxr = quot(f.mul(f.mul(f64x::twice(wwr), wwr), wwr), f.add(w2r, cr));
+    const double usl = f.sub(ul, quot(f.sub(pold, pl), wwl));
+    const double usr = f.add(ur, quot(f.sub(pold, pr), wwr));
+    const double delp = fmax_any(f.mul(quot(f.mul(qxr, qxl), f.add(qxr, qxl)), f.sub(usl, usr)), -pold);
+    pold = f.add(pold, delp);
+    conv = fabs(quot(delp, f.add(pold, ph.smallpp)));
   }
   pstar = pold;
-  wl = sqrt(cl * (1.0 + gamma6 * (pstar - pl) / pl));
-  wr = sqrt(cr * (1.0 + gamma6 * (pstar - pr) / pr));
-  const double ustar = 0.5 * (ul + (pl - pstar) / wl + ur - (pr - pstar) / wr);
-  const double sgnm = copysign(1.0, ustar);
-  const bool lft = sgnm > 0.0;
+  wl = wave(cl, pstar, pl, dpl);
+  wr = wave(cr, pstar, pr, dpr);
+  const double ustar =
+      half(f.sub(f.add(f.add(ul, quot(f.sub(pl, pstar), wl)), ur), quot(f.sub(pr, pstar), wr)));
+  const bool lft = f64x::sbits(ustar) >= 0;  // copysign(1, ustar) > 0
+  auto signed_by = [&](double x) { return lft ? x : -x; };  // sgnm * x
   const double ro = lft ? rl : rr, uo = lft ? ul : ur, po = lft ? pl : pr, wo = lft ? wl : wr;
-  const double co = fmax(ph.smallc, sqrt(fabs(gamma0 * po / ro)));
-  const double rstar = fmax((ro / (1.0 + ro * (po - pstar) / (wo * wo))), ph.smallr);
-  const double cstar = fmax(ph.smallc, sqrt(fabs(gamma0 * pstar / rstar)));
-  double spout = co - sgnm * uo;
-  double spin = cstar - sgnm * ustar;
-  const double ushock = wo / ro - sgnm * uo;
-  if (pstar >= po) {
+  const Divisor dro = divisor(ro);
+  const double co = fmax_any(ph.smallc, root(fabs(quot(f.mul(gamma0, po), dro))));
+  const double rstar = fmax_any(
+      quot(ro, f.add(f.one, quot(f.mul(ro, f.sub(po, pstar)), f.mul(wo, wo)))), ph.smallr);
+  const double cstar = fmax_any(ph.smallc, root(fabs(quot(f.mul(gamma0, pstar), rstar))));
+  double spout = f.sub(co, signed_by(uo));
+  double spin = f.sub(cstar, signed_by(ustar));
+  const double ushock = f.sub(quot(wo, dro), signed_by(uo));
+  if (f64x::okey(pstar) >= f64x::okey(po)) {
     spin = ushock;
     spout = ushock;
   }
-  const double scr = fmax(spout - spin, ph.smallc + fabs(spout + spin));
-  double frac = 0.5 * (1.0 + (spout + spin) / scr);
-  if (frac != frac)
+  const double spsum = f.add(spout, spin);
+  const double scr = fmax_any(f.sub(spout, spin), f.add(ph.smallc, fabs(spsum)));
+  double frac = half(f.add(f.one, quot(spsum, scr)));
+  if (f64x::is_nan(frac))
     frac = 0.0;
   else
-    frac = frac >= 1.0 ? 1.0 : frac <= 0.0 ? 0.0 : frac;
+    frac = f64x::sbits(frac) >= f64x::sbits(1.0) ? 1.0 : f64x::le0(frac) ? 0.0 : frac;
+  const double rest = f.sub(f.one, frac);
   double g[4];
-  g[E2D_ID] = frac * rstar + (1.0 - frac) * ro;
-  g[E2D_IU] = frac * ustar + (1.0 - frac) * uo;
-  g[E2D_IP] = frac * pstar + (1.0 - frac) * po;
-  if (spout < 0.0) {
+  g[E2D_ID] = f.add(f.mul(frac, rstar), f.mul(rest, ro));
+  g[E2D_IU] = f.add(f.mul(frac, ustar), f.mul(rest, uo));
+  g[E2D_IP] = f.add(f.mul(frac, pstar), f.mul(rest, po));
+  if (f64x::lt0(spout)) {
     g[E2D_ID] = ro;
     g[E2D_IU] = uo;
     g[E2D_IP] = po;
   }
-  if (spin > 0.0) {
+  if (gt0(spin)) {
     g[E2D_ID] = rstar;
     g[E2D_IU] = ustar;
     g[E2D_IP] = pstar;
   }
   g[E2D_IV] = lft ? ql[E2D_IV] : qr[E2D_IV];
-  cmpflx(ph, g, flux);
+  cmpflx(f, ph, g, flux);
 }
 
 // src/HydroBaseFunctor.h:704-809 (riemann_hllc).  The reference builds the
-// star states of both sides and keeps one; here only the star state of the
-// side the contact selects (ustar > 0: left) is built, which yields the same
-// value.  Cut-offs,
-// maxima, the 0.5 factors and the sign tests use the exact integer forms of
-// e2d_f64_exact.cuh.
-__device__ __forceinline__ void riemann_hllc(const KPhys<double> &ph, const double *ql,
+// star states of both sides and keeps one; here only the total energy and the
+// star state of the side that is read are built (SL > 0 reads the left state,
+// else the contact selects), and the larger sound speed is the root of the
+// larger square (a correctly rounded root is monotonic): the same values.
+// Cut-offs, maxima, the 0.5 factors and the sign tests use the exact integer
+// forms of e2d_f64_exact.cuh.
+__device__ __forceinline__ void riemann_hllc(const Fp &f, const KPhys<double> &ph, const double *ql,
                                              const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
-  const double pl = max_pos(ql[E2D_IP], rl * ph.smallp);
+  const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
   const double ul = ql[E2D_IU];
-  const double hrl = half(rl);
-  double ecinl = hrl * ul * ul;
-  ecinl = ecinl + hrl * ql[E2D_IV] * ql[E2D_IV];
-  const double etotl = pl * ph.entho + ecinl;
   const double rr = max_pos(qr[E2D_ID], ph.smallr);
-  const double pr = max_pos(qr[E2D_IP], rr * ph.smallp);
+  const double pr = floor_pressure(f, ph, qr[E2D_IP], rr);
   const double ur = qr[E2D_IU];
-  const double hrr = half(rr);
-  double ecinr = hrr * ur * ur;
-  ecinr = ecinr + hrr * qr[E2D_IV] * qr[E2D_IV];
-  const double etotr = pr * ph.entho + ecinr;
-  const double cfastl = sqrt(max_pos(ph.gamma0 * pl / rl, ph.smallc2));
-  const double cfastr = sqrt(max_pos(ph.gamma0 * pr / rr, ph.smallc2));
-  const double cmax = max_nn(cfastl, cfastr);
-  const double SL = min_any(ul, ur) - cmax;
-  const double SR = max_any(ul, ur) + cmax;
-  const double rcl = rl * (ul - SL);
-  const double rcr = rr * (SR - ur);
-  const double ustar = (rcr * ur + rcl * ul + (pl - pr)) / (rcr + rcl);
-  const double ptotstar = (rcr * pl + rcl * pr + rcl * rcr * (ul - ur)) / (rcr + rcl);
-  const bool lft = gt0(ustar);
+  const double c2l = max_pos(quot(f.mul(ph.gamma0, pl), rl), ph.smallc2);
+  const double c2r = max_pos(quot(f.mul(ph.gamma0, pr), rr), ph.smallc2);
+  const double cmax = root(max_nn(c2l, c2r));
+  const double SL = f.sub(min_any(ul, ur), cmax);
+  const double SR = f.add(max_any(ul, ur), cmax);
+  const double rcl = f.mul(rl, f.sub(ul, SL));
+  const double rcr = f.mul(rr, f.sub(SR, ur));
+  const Divisor rc = divisor(f.add(rcr, rcl));
+  const double ustar = quot(f.add(f.add(f.mul(rcr, ur), f.mul(rcl, ul)), f.sub(pl, pr)), rc);
+  const double ptotstar =
+      quot(f.add(f.add(f.mul(rcr, pl), f.mul(rcl, pr)), f.mul(f.mul(rcl, rcr), f.sub(ul, ur))), rc);
+  const bool own_l = gt0(SL);
+  const bool lft = own_l || gt0(ustar);
+  const bool own = own_l || !(lft || gt0(SR));
   const double S = lft ? SL : SR;
-  const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr;
-  const double es = lft ? etotl : etotr;
-  const double sdu = S - us;
-  const double sds = S - ustar;
-  const double rstar = rs * sdu / sds;
-  const double etotstar = (sdu * es - ps * us + ptotstar * ustar) / sds;
-  double ro, uo, ptoto, etoto;
-  if (gt0(SL)) {
-    ro = rl, uo = ul, ptoto = pl, etoto = etotl;
-  } else if (lft || gt0(SR)) {
-    ro = rstar, uo = ustar, ptoto = ptotstar, etoto = etotstar;
-  } else {
-    ro = rr, uo = ur, ptoto = pr, etoto = etotr;
-  }
-  flux[E2D_ID] = ro * uo;
-  flux[E2D_IU] = flux[E2D_ID] * uo + ptoto;
-  flux[E2D_IP] = (etoto + ptoto) * uo;
-  flux[E2D_IV] = gt0(flux[E2D_ID]) ? flux[E2D_ID] * ql[E2D_IV] : flux[E2D_ID] * qr[E2D_IV];
+  const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr, vs = lft ? ql[E2D_IV] : qr[E2D_IV];
+  const double hrs = half(rs);
+  const double es = f.add(f.mul(ps, ph.entho), f.add(f.mul(f.mul(hrs, us), us), f.mul(f.mul(hrs, vs), vs)));
+  const double sdu = f.sub(S, us);
+  const Divisor sds = divisor(f.sub(S, ustar));
+  const double rstar = quot(f.mul(rs, sdu), sds);
+  const double etotstar = quot(f.add(f.sub(f.mul(sdu, es), f.mul(ps, us)), f.mul(ptotstar, ustar)), sds);
+  const double ro = own ? rs : rstar, uo = own ? us : ustar, ptoto = own ? ps : ptotstar;
+  const double etoto = own ? es : etotstar;
+  flux[E2D_ID] = f.mul(ro, uo);
+  flux[E2D_IU] = f.add(f.mul(flux[E2D_ID], uo), ptoto);
+  flux[E2D_IP] = f.mul(f.add(etoto, ptoto), uo);
+  flux[E2D_IV] = f.mul(flux[E2D_ID], gt0(flux[E2D_ID]) ? ql[E2D_IV] : qr[E2D_IV]);
 }
 
 // HLL flux (Harten, Lax, van Leer; Toro, "Riemann Solvers and Numerical
@@ -206,37 +237,35 @@ __device__ __forceinline__ void riemann_hllc(const KPhys<double> &ph, const doub
 // RIEMANN_HLL but has no solver; this uses riemann_hllc's cut-offs and Davis
 // wave speeds; the star flux multiplies by one reciprocal of SR - SL.
 // Operation order matches the oracle's riemann_hll.
-__device__ __forceinline__ void riemann_hll(const KPhys<double> &ph, const double *ql,
+__device__ __forceinline__ void riemann_hll(const Fp &f, const KPhys<double> &ph, const double *ql,
                                             const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
-  const double pl = max_pos(ql[E2D_IP], rl * ph.smallp);
+  const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
   const double ul = ql[E2D_IU], vl = ql[E2D_IV];
   const double rr = max_pos(qr[E2D_ID], ph.smallr);
-  const double pr = max_pos(qr[E2D_IP], rr * ph.smallp);
+  const double pr = floor_pressure(f, ph, qr[E2D_IP], rr);
   const double ur = qr[E2D_IU], vr = qr[E2D_IV];
-  const double hrl = half(rl), hrr = half(rr);
-  double ecinl = hrl * ul * ul;
-  ecinl = ecinl + hrl * vl * vl;
-  const double etotl = pl * ph.entho + ecinl;
-  double ecinr = hrr * ur * ur;
-  ecinr = ecinr + hrr * vr * vr;
-  const double etotr = pr * ph.entho + ecinr;
-  const double cfastl = sqrt(max_pos(ph.gamma0 * pl / rl, ph.smallc2));
-  const double cfastr = sqrt(max_pos(ph.gamma0 * pr / rr, ph.smallc2));
-  const double cmax = max_nn(cfastl, cfastr);
-  const double SL = min_any(ul, ur) - cmax;
-  const double SR = max_any(ul, ur) + cmax;
-  const double UL[4] = {rl, etotl, rl * ul, rl * vl};
-  const double UR[4] = {rr, etotr, rr * ur, rr * vr};
+  auto energy = [&](double r, double p, double u, double v) {
+    const double h = half(r);
+    return f.add(f.mul(p, ph.entho), f.add(f.mul(f.mul(h, u), u), f.mul(f.mul(h, v), v)));
+  };
+  const double etotl = energy(rl, pl, ul, vl), etotr = energy(rr, pr, ur, vr);
+  const double c2l = max_pos(quot(f.mul(ph.gamma0, pl), rl), ph.smallc2);
+  const double c2r = max_pos(quot(f.mul(ph.gamma0, pr), rr), ph.smallc2);
+  const double cmax = root(max_nn(c2l, c2r));
+  const double SL = f.sub(min_any(ul, ur), cmax);
+  const double SR = f.add(max_any(ul, ur), cmax);
+  const double UL[4] = {rl, etotl, f.mul(rl, ul), f.mul(rl, vl)};
+  const double UR[4] = {rr, etotr, f.mul(rr, ur), f.mul(rr, vr)};
   double FL[4], FR[4];
   FL[E2D_ID] = UL[E2D_IU];
-  FL[E2D_IP] = (etotl + pl) * ul;
-  FL[E2D_IU] = UL[E2D_IU] * ul + pl;
-  FL[E2D_IV] = UL[E2D_IU] * vl;
+  FL[E2D_IP] = f.mul(f.add(etotl, pl), ul);
+  FL[E2D_IU] = f.add(f.mul(UL[E2D_IU], ul), pl);
+  FL[E2D_IV] = f.mul(UL[E2D_IU], vl);
   FR[E2D_ID] = UR[E2D_IU];
-  FR[E2D_IP] = (etotr + pr) * ur;
-  FR[E2D_IU] = UR[E2D_IU] * ur + pr;
-  FR[E2D_IV] = UR[E2D_IU] * vr;
+  FR[E2D_IP] = f.mul(f.add(etotr, pr), ur);
+  FR[E2D_IU] = f.add(f.mul(UR[E2D_IU], ur), pr);
+  FR[E2D_IV] = f.mul(UR[E2D_IU], vr);
   if (gt0(SL)) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) flux[v] = FL[v];
@@ -245,164 +274,145 @@ __device__ __forceinline__ void riemann_hll(const KPhys<double> &ph, const doubl
     for (int v = 0; v < 4; ++v) flux[v] = FR[v];
   } else {
     // one division: the four star fluxes share the factor 1 / (SR - SL)
-    const double sls = SL * SR;
-    const double rden = 1.0 / (SR - SL);
+    const double sls = f.mul(SL, SR);
+    const double rden = quot(f.one, f.sub(SR, SL));
 #pragma unroll
-    for (int v = 0; v < 4; ++v) flux[v] = (SR * FL[v] - SL * FR[v] + sls * (UR[v] - UL[v])) * rden;
+    for (int v = 0; v < 4; ++v)
+      flux[v] = f.mul(f.add(f.sub(f.mul(SR, FL[v]), f.mul(SL, FR[v])), f.mul(sls, f.sub(UR[v], UL[v]))), rden);
   }
 }
 
 template <int RS>
-__device__ __forceinline__ void riemann(const KPhys<double> &ph, const double *ql, const double *qr,
+__device__ __forceinline__ void riemann(const Fp &f, const KPhys<double> &ph, const double *ql, const double *qr,
                                         double *flux) {
   if (RS == E2D_RIEMANN_HLLC)
-    riemann_hllc(ph, ql, qr, flux);
+    riemann_hllc(f, ph, ql, qr, flux);
   else if (RS == E2D_RIEMANN_HLL)
-    riemann_hll(ph, ql, qr, flux);
+    riemann_hll(f, ph, ql, qr, flux);
   else
-    riemann_approx(ph, ql, qr, flux);
+    riemann_approx(f, ph, ql, qr, flux);
 }
 
 // CFL wave-speed term of a cell from its primitives (src/HydroRunFunctors.h:56-72):
 // (c + |u|) / dx + (c + |v|) / dy, c = sqrt(gamma p / d); a division by a
 // power-of-two dx, dy is the exact product by its reciprocal.
-__device__ __forceinline__ double cfl_term(const KPhys<double> &ph, double dd, double p, double ux, double uy) {
-  const double c = sqrt(ph.gamma0 * p / dd);
-  const double vx = c + fabs(ux);
-  const double vy = c + fabs(uy);
-  const double tx = ph.inv_dx_pow2 != 0.0 ? vx * ph.inv_dx_pow2 : vx / ph.dx;
-  const double ty = ph.inv_dy_pow2 != 0.0 ? vy * ph.inv_dy_pow2 : vy / ph.dy;
-  return tx + ty;
+__device__ __forceinline__ double cfl_term(const Fp &f, const KPhys<double> &ph, const Divisor &dd, double p,
+                                           double ux, double uy) {
+  const double c = root(quot(f.mul(ph.gamma0, p), dd));
+  const double vx = f.add(c, fabs(ux));
+  const double vy = f.add(c, fabs(uy));
+  const double tx = ph.inv_dx_pow2 != 0.0 ? f.mul(vx, ph.inv_dx_pow2) : quot(vx, ph.dx);
+  const double ty = ph.inv_dy_pow2 != 0.0 ? f.mul(vy, ph.inv_dy_pow2) : quot(vy, ph.dy);
+  return f.add(tx, ty);
 }
 
 // E2D_FLAG_* bits of a cell's conserved values.
 __device__ __forceinline__ unsigned int state_flags(double rho, double e, double mx, double my) {
   unsigned int f = 0;
   if (nonfinite(rho) || nonfinite(e) || nonfinite(mx) || nonfinite(my)) f |= E2D_FLAG_NONFINITE;
-  if (!(rho > 0.0)) f |= E2D_FLAG_DENSITY;
+  if (!gt0(rho)) f |= E2D_FLAG_DENSITY;
   return f;
 }
 
 
 // ------------------------------------------------------------ fast forms
 // The opt-in E2D_PRECISION_FP64_FAST step: the same formulas with a*b + c
-// contracted into one FMA where it falls naturally and every division
-// replaced by a product with a reciprocal computed once per denominator.
-// Results differ from the reference's by rounding (not bit-identical); the
-// tests hold them to 1e-12 on dt and 1e-10 relative L1.
-
-// 1/b: the hardware estimate (rcp.approx.ftz.f64) refined by two
-// Newton-Raphson iterations for f(y) = 1/y - b, y <- y + y (1 - b y), each
-// of which roughly doubles the number of correct bits.  For normal b
-// (denominators here are densities >= smallr and sums of positive terms).
-__device__ __forceinline__ double rcp_nr(double b) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-  double e = fma(-b, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-b, y, 1.0);
-  return fma(y, e, y);
-}
-
-// primitives() with one reciprocal of the density (returned in rd).
-__device__ __forceinline__ void primitives_fast(const KPhys<double> &ph, double rho, double e, double mx,
-                                                double my, double &d, double &p, double &ux, double &uy,
-                                                double &rd) {
+// contracted into one FMA where it falls naturally (quotients and roots cost
+// no FP64 instruction, so they stay as they are).  Results differ from the
+// reference's by rounding (not bit-identical); the tests hold them to 1e-12
+// on dt and 1e-10 relative L1.
+__device__ __forceinline__ void primitives_fast(const Fp &f, const KPhys<double> &ph, double rho, double e,
+                                                double mx, double my, double &d, double &p, double &ux, double &uy,
+                                                Divisor &dv) {
   d = max_pos(rho, ph.smallr);
-  rd = rcp_nr(d);
-  ux = mx * rd;
-  uy = my * rd;
-  const double ei = fma(e, rd, -0.5 * fma(ux, ux, uy * uy));
-  p = max_pos(ph.gm1 * d * ei, d * ph.smallp);
+  dv = divisor(d);
+  ux = quot(mx, dv);
+  uy = quot(my, dv);
+  const double ei = f.sub(quot(e, dv), half(fma(ux, ux, f.mul(uy, uy))));
+  p = floor_pressure(f, ph, f.mul(f.mul(ph.gm1, d), ei), d);
 }
 
-__device__ __forceinline__ void trace_sources_fast(const KPhys<double> &ph, const double q[4], const double dqx[4],
-                                                   const double dqy[4], double s0[4]) {
+__device__ __forceinline__ void trace_sources_fast(const Fp &f, const KPhys<double> &ph, const double q[4],
+                                                   const double dqx[4], const double dqy[4], double s0[4]) {
   const double r = q[E2D_ID], p = q[E2D_IP], u = q[E2D_IU], v = q[E2D_IV];
-  const double div = dqx[E2D_IU] + dqy[E2D_IV];
-  const double ir = rcp_nr(r);
-  s0[E2D_ID] = fma(-u, dqx[E2D_ID], fma(-v, dqy[E2D_ID], -div * r));
-  s0[E2D_IP] = fma(-u, dqx[E2D_IP], fma(-v, dqy[E2D_IP], -div * ph.gamma0 * p));
-  s0[E2D_IU] = fma(-u, dqx[E2D_IU], fma(-v, dqy[E2D_IU], -dqx[E2D_IP] * ir));
-  s0[E2D_IV] = fma(-u, dqx[E2D_IV], fma(-v, dqy[E2D_IV], -dqy[E2D_IP] * ir));
+  const Divisor dr = divisor(r);
+  const double div = f.add(dqx[E2D_IU], dqy[E2D_IV]);
+  s0[E2D_ID] = fma(-u, dqx[E2D_ID], fma(-v, dqy[E2D_ID], f.mul(-div, r)));
+  s0[E2D_IP] = fma(-u, dqx[E2D_IP], fma(-v, dqy[E2D_IP], f.mul(f.mul(-div, ph.gamma0), p)));
+  s0[E2D_IU] = fma(-u, dqx[E2D_IU], fma(-v, dqy[E2D_IU], -quot(dqx[E2D_IP], dr)));
+  s0[E2D_IV] = fma(-u, dqx[E2D_IV], fma(-v, dqy[E2D_IV], -quot(dqy[E2D_IP], dr)));
 }
 
 // face_pair() with hdtd = dt/dx / 2 (or dt/dy / 2).
-__device__ __forceinline__ void face_pair_fast(const KPhys<double> &ph, int v, double q, double dq, double s0,
-                                               double hdtd, double &fm, double &fp) {
+__device__ __forceinline__ void face_pair_fast(const Fp &f, const KPhys<double> &ph, int v, double q, double dq,
+                                               double s0, double hdtd, double &fm, double &fp) {
   const double qs = fma(s0, hdtd, q);
-  fm = fma(dq, -0.5, qs);
-  fp = fma(dq, 0.5, qs);
+  const double h = half(dq);
+  fm = f.sub(qs, h);
+  fp = f.add(qs, h);
   if (v == E2D_ID) {
     fm = max_pos(fm, ph.smallr);
     fp = max_pos(fp, ph.smallr);
   }
 }
 
-// riemann_hllc() with shared reciprocals: 1 / rl, 1 / rr, 1 / (rcr + rcl)
-// for u* and p*, 1 / (S - u*) for the star density and energy.
-__device__ __forceinline__ void riemann_hllc_fast(const KPhys<double> &ph, const double *ql, const double *qr,
-                                                  double *flux) {
+// riemann_hllc() with FMAs.
+__device__ __forceinline__ void riemann_hllc_fast(const Fp &f, const KPhys<double> &ph, const double *ql,
+                                                  const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
-  const double pl = max_pos(ql[E2D_IP], rl * ph.smallp);
+  const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
   const double ul = ql[E2D_IU];
-  const double etotl = fma(pl, ph.entho, 0.5 * rl * fma(ul, ul, ql[E2D_IV] * ql[E2D_IV]));
   const double rr = max_pos(qr[E2D_ID], ph.smallr);
-  const double pr = max_pos(qr[E2D_IP], rr * ph.smallp);
+  const double pr = floor_pressure(f, ph, qr[E2D_IP], rr);
   const double ur = qr[E2D_IU];
-  const double etotr = fma(pr, ph.entho, 0.5 * rr * fma(ur, ur, qr[E2D_IV] * qr[E2D_IV]));
-  const double cfastl = sqrt(max_pos(ph.gamma0 * pl * rcp_nr(rl), ph.smallc2));
-  const double cfastr = sqrt(max_pos(ph.gamma0 * pr * rcp_nr(rr), ph.smallc2));
-  const double cmax = max_nn(cfastl, cfastr);
-  const double SL = min_any(ul, ur) - cmax;
-  const double SR = max_any(ul, ur) + cmax;
-  const double rcl = rl * (ul - SL);
-  const double rcr = rr * (SR - ur);
-  const double isum = rcp_nr(rcr + rcl);
-  const double ustar = fma(rcr, ur, fma(rcl, ul, pl - pr)) * isum;
-  const double ptotstar = fma(rcr, pl, fma(rcl, pr, rcl * rcr * (ul - ur))) * isum;
-  const bool lft = gt0(ustar);
+  const double c2l = max_pos(quot(f.mul(ph.gamma0, pl), rl), ph.smallc2);
+  const double c2r = max_pos(quot(f.mul(ph.gamma0, pr), rr), ph.smallc2);
+  const double cmax = root(max_nn(c2l, c2r));
+  const double SL = f.sub(min_any(ul, ur), cmax);
+  const double SR = f.add(max_any(ul, ur), cmax);
+  const double rcl = f.mul(rl, f.sub(ul, SL));
+  const double rcr = f.mul(rr, f.sub(SR, ur));
+  const Divisor rc = divisor(f.add(rcr, rcl));
+  const double ustar = quot(fma(rcr, ur, fma(rcl, ul, f.sub(pl, pr))), rc);
+  const double ptotstar = quot(fma(rcr, pl, fma(rcl, pr, f.mul(f.mul(rcl, rcr), f.sub(ul, ur)))), rc);
+  const bool own_l = gt0(SL);
+  const bool lft = own_l || gt0(ustar);
+  const bool own = own_l || !(lft || gt0(SR));
   const double S = lft ? SL : SR;
-  const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr;
-  const double es = lft ? etotl : etotr;
-  const double sdu = S - us;
-  const double isds = rcp_nr(S - ustar);
-  const double rstar = rs * sdu * isds;
-  const double etotstar = fma(sdu, es, fma(-ps, us, ptotstar * ustar)) * isds;
-  double ro, uo, ptoto, etoto;
-  if (gt0(SL)) {
-    ro = rl, uo = ul, ptoto = pl, etoto = etotl;
-  } else if (lft || gt0(SR)) {
-    ro = rstar, uo = ustar, ptoto = ptotstar, etoto = etotstar;
-  } else {
-    ro = rr, uo = ur, ptoto = pr, etoto = etotr;
-  }
-  flux[E2D_ID] = ro * uo;
+  const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr, vs = lft ? ql[E2D_IV] : qr[E2D_IV];
+  const double es = fma(ps, ph.entho, f.mul(half(rs), fma(us, us, f.mul(vs, vs))));
+  const double sdu = f.sub(S, us);
+  const Divisor sds = divisor(f.sub(S, ustar));
+  const double rstar = quot(f.mul(rs, sdu), sds);
+  const double etotstar = quot(fma(sdu, es, fma(-ps, us, f.mul(ptotstar, ustar))), sds);
+  const double ro = own ? rs : rstar, uo = own ? us : ustar, ptoto = own ? ps : ptotstar;
+  const double etoto = own ? es : etotstar;
+  flux[E2D_ID] = f.mul(ro, uo);
   flux[E2D_IU] = fma(flux[E2D_ID], uo, ptoto);
-  flux[E2D_IP] = (etoto + ptoto) * uo;
-  flux[E2D_IV] = gt0(flux[E2D_ID]) ? flux[E2D_ID] * ql[E2D_IV] : flux[E2D_ID] * qr[E2D_IV];
+  flux[E2D_IP] = f.mul(f.add(etoto, ptoto), uo);
+  flux[E2D_IV] = f.mul(flux[E2D_ID], gt0(flux[E2D_ID]) ? ql[E2D_IV] : qr[E2D_IV]);
 }
 
-// riemann_hll() with FMAs and reciprocals of rl, rr.
-__device__ __forceinline__ void riemann_hll_fast(const KPhys<double> &ph, const double *ql, const double *qr,
-                                                 double *flux) {
+// riemann_hll() with FMAs.
+__device__ __forceinline__ void riemann_hll_fast(const Fp &f, const KPhys<double> &ph, const double *ql,
+                                                 const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
-  const double pl = max_pos(ql[E2D_IP], rl * ph.smallp);
+  const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
   const double ul = ql[E2D_IU], vl = ql[E2D_IV];
   const double rr = max_pos(qr[E2D_ID], ph.smallr);
-  const double pr = max_pos(qr[E2D_IP], rr * ph.smallp);
+  const double pr = floor_pressure(f, ph, qr[E2D_IP], rr);
   const double ur = qr[E2D_IU], vr = qr[E2D_IV];
-  const double etotl = fma(pl, ph.entho, 0.5 * rl * fma(ul, ul, vl * vl));
-  const double etotr = fma(pr, ph.entho, 0.5 * rr * fma(ur, ur, vr * vr));
-  const double cfastl = sqrt(max_pos(ph.gamma0 * pl * rcp_nr(rl), ph.smallc2));
-  const double cfastr = sqrt(max_pos(ph.gamma0 * pr * rcp_nr(rr), ph.smallc2));
-  const double cmax = max_nn(cfastl, cfastr);
-  const double SL = min_any(ul, ur) - cmax;
-  const double SR = max_any(ul, ur) + cmax;
-  const double UL[4] = {rl, etotl, rl * ul, rl * vl};
-  const double UR[4] = {rr, etotr, rr * ur, rr * vr};
-  const double FL[4] = {UL[E2D_IU], (etotl + pl) * ul, fma(UL[E2D_IU], ul, pl), UL[E2D_IU] * vl};
-  const double FR[4] = {UR[E2D_IU], (etotr + pr) * ur, fma(UR[E2D_IU], ur, pr), UR[E2D_IU] * vr};
+  const double etotl = fma(pl, ph.entho, f.mul(half(rl), fma(ul, ul, f.mul(vl, vl))));
+  const double etotr = fma(pr, ph.entho, f.mul(half(rr), fma(ur, ur, f.mul(vr, vr))));
+  const double c2l = max_pos(quot(f.mul(ph.gamma0, pl), rl), ph.smallc2);
+  const double c2r = max_pos(quot(f.mul(ph.gamma0, pr), rr), ph.smallc2);
+  const double cmax = root(max_nn(c2l, c2r));
+  const double SL = f.sub(min_any(ul, ur), cmax);
+  const double SR = f.add(max_any(ul, ur), cmax);
+  const double UL[4] = {rl, etotl, f.mul(rl, ul), f.mul(rl, vl)};
+  const double UR[4] = {rr, etotr, f.mul(rr, ur), f.mul(rr, vr)};
+  const double FL[4] = {UL[E2D_IU], f.mul(f.add(etotl, pl), ul), fma(UL[E2D_IU], ul, pl), f.mul(UL[E2D_IU], vl)};
+  const double FR[4] = {UR[E2D_IU], f.mul(f.add(etotr, pr), ur), fma(UR[E2D_IU], ur, pr), f.mul(UR[E2D_IU], vr)};
   if (gt0(SL)) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) flux[v] = FL[v];
@@ -410,36 +420,36 @@ __device__ __forceinline__ void riemann_hll_fast(const KPhys<double> &ph, const 
 #pragma unroll
     for (int v = 0; v < 4; ++v) flux[v] = FR[v];
   } else {
-    const double sls = SL * SR;
-    const double rden = rcp_nr(SR - SL);
+    const double sls = f.mul(SL, SR);
+    const double rden = quot(f.one, f.sub(SR, SL));
 #pragma unroll
-    for (int v = 0; v < 4; ++v) flux[v] = fma(sls, UR[v] - UL[v], fma(SR, FL[v], -SL * FR[v])) * rden;
+    for (int v = 0; v < 4; ++v)
+      flux[v] = f.mul(fma(sls, f.sub(UR[v], UL[v]), fma(SR, FL[v], f.mul(-SL, FR[v]))), rden);
   }
 }
 
 template <int RS, bool FAST>
-__device__ __forceinline__ void riemann_sel(const KPhys<double> &ph, const double *ql, const double *qr,
-                                            double *flux) {
+__device__ __forceinline__ void riemann_sel(const Fp &f, const KPhys<double> &ph, const double *ql,
+                                            const double *qr, double *flux) {
   if (FAST && RS == E2D_RIEMANN_HLLC)
-    riemann_hllc_fast(ph, ql, qr, flux);
+    riemann_hllc_fast(f, ph, ql, qr, flux);
   else if (FAST && RS == E2D_RIEMANN_HLL)
-    riemann_hll_fast(ph, ql, qr, flux);
+    riemann_hll_fast(f, ph, ql, qr, flux);
   else
-    riemann<RS>(ph, ql, qr, flux);
+    riemann<RS>(f, ph, ql, qr, flux);
 }
 
-// cfl_term() from the reciprocal of the density.
-__device__ __forceinline__ double cfl_term_fast(const KPhys<double> &ph, double rd, double p, double ux,
-                                                double uy) {
-  const double c = sqrt(ph.gamma0 * p * rd);
-  return fma(c + fabs(ux), ph.inv_dx, (c + fabs(uy)) * ph.inv_dy);
+__device__ __forceinline__ double cfl_term_fast(const Fp &f, const KPhys<double> &ph, const Divisor &dd, double p,
+                                                double ux, double uy) {
+  const double c = root(quot(f.mul(ph.gamma0, p), dd));
+  return fma(f.add(c, fabs(ux)), ph.inv_dx, f.mul(f.add(c, fabs(uy)), ph.inv_dy));
 }
 
 // dt of a step from the CFL maximum (src/main.cpp:128-134).
 __device__ __forceinline__ double step_dt(const KPhys<double> &ph, unsigned long long invdt_bits, double t,
                                           double t_end) {
   const double inv_dt = __longlong_as_double((long long)invdt_bits);
-  double dt = ph.cfl / inv_dt;
+  double dt = quot(ph.cfl, inv_dt);
   if (t + dt > t_end) dt = t_end - t;
   return dt;
 }

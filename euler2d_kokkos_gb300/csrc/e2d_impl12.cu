@@ -36,8 +36,8 @@ __device__ __forceinline__ void step_ratios(const KPhys<double> &ph, const DevCl
     run = clk->t < clk->t_end;
     dt = step_dt(ph, clk->invdt_bits, clk->t, clk->t_end);
   }
-  dtdx = dt / ph.dx;
-  dtdy = dt / ph.dy;
+  dtdx = quot(dt, ph.dx);
+  dtdy = quot(dt, ph.dy);
 }
 
 __device__ __forceinline__ int st_kind_of(const KPhys<double> &ph) {
@@ -45,49 +45,49 @@ __device__ __forceinline__ int st_kind_of(const KPhys<double> &ph) {
 }
 
 // Primitives and both slopes of cell s (row stride isize).
-__device__ __forceinline__ void cell_slopes(const KGeom &g, const KPhys<double> &ph, const double *__restrict__ q,
+__device__ __forceinline__ void cell_slopes(const Fp &f, const KGeom &g, const KPhys<double> &ph, const double *__restrict__ q,
                                             size_t s, double qc[4], double dqx[4], double dqy[4]) {
   const int st = st_kind_of(ph);
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     const double *P = q + v * g.plane;
     qc[v] = P[s];
-    dqx[v] = slope(st, qc[v], P[s + 1], P[s - 1]);
-    dqy[v] = slope(st, qc[v], P[s + g.isize], P[s - g.isize]);
+    dqx[v] = slope(f, st, qc[v], P[s + 1], P[s - 1]);
+    dqy[v] = slope(f, st, qc[v], P[s + g.isize], P[s - g.isize]);
   }
 }
 
 // Face states of one cell along one direction: its minus (XMIN / YMIN) and
 // plus (XMAX / YMAX) faces.
-__device__ __forceinline__ void cell_faces(const KPhys<double> &ph, const double qc[4], const double dqx[4],
+__device__ __forceinline__ void cell_faces(const Fp &f, const KPhys<double> &ph, const double qc[4], const double dqx[4],
                                            const double dqy[4], bool xdir, double dtdx, double dtdy,
                                            double fm[4], double fp[4]) {
   double s0[4];
-  trace_sources(ph, qc, dqx, dqy, s0);
+  trace_sources(f, ph, qc, dqx, dqy, s0);
 #pragma unroll
   for (int v = 0; v < 4; ++v)
-    face_pair(ph, v, qc[v], xdir ? dqx[v] : dqy[v], s0[v], xdir ? dtdx : dtdy, fm[v], fp[v]);
+    face_pair(f, ph, v, qc[v], xdir ? dqx[v] : dqy[v], s0[v], xdir ? dtdx : dtdy, fm[v], fp[v]);
 }
 
 // Scaled flux through the face between the left/lower state ql and the
 // right/upper state qr (y: normal velocity first, src/HydroRunFunctors.h:628-632).
 template <int RS>
-__device__ __forceinline__ void face_flux(const KPhys<double> &ph, bool xdir, const double ql[4],
+__device__ __forceinline__ void face_flux(const Fp &o, const KPhys<double> &ph, bool xdir, const double ql[4],
                                           const double qr[4], double dtd, double f[4]) {
   if (xdir) {
-    riemann<RS>(ph, ql, qr, f);
+    riemann<RS>(o, ph, ql, qr, f);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) f[v] = f[v] * dtd;
+    for (int v = 0; v < 4; ++v) f[v] = o.mul(f[v], dtd);
     return;
   }
   const double l[4] = {ql[E2D_ID], ql[E2D_IP], ql[E2D_IV], ql[E2D_IU]};
   const double r[4] = {qr[E2D_ID], qr[E2D_IP], qr[E2D_IV], qr[E2D_IU]};
   double g[4];
-  riemann<RS>(ph, l, r, g);
-  f[E2D_ID] = g[E2D_ID] * dtd;
-  f[E2D_IP] = g[E2D_IP] * dtd;
-  f[E2D_IU] = g[E2D_IV] * dtd;
-  f[E2D_IV] = g[E2D_IU] * dtd;
+  riemann<RS>(o, ph, l, r, g);
+  f[E2D_ID] = o.mul(g[E2D_ID], dtd);
+  f[E2D_IP] = o.mul(g[E2D_IP], dtd);
+  f[E2D_IU] = o.mul(g[E2D_IV], dtd);
+  f[E2D_IV] = o.mul(g[E2D_IU], dtd);
 }
 
 // --------------------------------------------------------- implementation 1
@@ -99,8 +99,9 @@ __global__ void __launch_bounds__(BX *BY)
   const int i = blockIdx.x * BX + threadIdx.x, j = blockIdx.y * BY + threadIdx.y;
   if (i < 1 || i > g.isize - 2 || j < 1 || j > g.jsize - 2) return;
   const size_t s = (size_t)i + (size_t)g.isize * j;
+  const Fp o;
   double qc[4], dqx[4], dqy[4];
-  cell_slopes(g, kp.ph, q, s, qc, dqx, dqy);
+  cell_slopes(o, g, kp.ph, q, s, qc, dqx, dqy);
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     sx[s + v * g.plane] = dqx[v];
@@ -134,10 +135,11 @@ __global__ void __launch_bounds__(BX *BY)
     nqx[v] = sx[n + v * g.plane];
     nqy[v] = sy[n + v * g.plane];
   }
+  const Fp o;
   double cm[4], cp[4], nm[4], np[4], fl[4];
-  cell_faces(kp.ph, qc, dqx, dqy, xdir, dtdx, dtdy, cm, cp);   // right state: the cell's minus face
-  cell_faces(kp.ph, qn, nqx, nqy, xdir, dtdx, dtdy, nm, np);   // left state: the neighbour's plus face
-  face_flux<RS>(kp.ph, xdir, np, cm, xdir ? dtdx : dtdy, fl);
+  cell_faces(o, kp.ph, qc, dqx, dqy, xdir, dtdx, dtdy, cm, cp);   // right state: the cell's minus face
+  cell_faces(o, kp.ph, qn, nqx, nqy, xdir, dtdx, dtdy, nm, np);   // left state: the neighbour's plus face
+  face_flux<RS>(o, kp.ph, xdir, np, cm, xdir ? dtdx : dtdy, fl);
 #pragma unroll
   for (int v = 0; v < 4; ++v) f[s + v * g.plane] = fl[v];
 }
@@ -177,16 +179,17 @@ __global__ void __launch_bounds__(BX *BY)
   step_ratios(kp.ph, clk, use_clock, host_dt, dtdx, dtdy, run);
   if (!run) return;
   const size_t s = (size_t)i + (size_t)g.isize * j;
+  const Fp o;
   double qc[4], dqx[4], dqy[4];
-  cell_slopes(g, kp.ph, q, s, qc, dqx, dqy);
+  cell_slopes(o, g, kp.ph, q, s, qc, dqx, dqy);
   for (int d = 0; d < 2; ++d) {
     const bool xdir = d == 0;
     const size_t n = xdir ? s - 1 : s - g.isize;
     double qn[4], nqx[4], nqy[4], cm[4], cp[4], nm[4], np[4], fl[4];
-    cell_slopes(g, kp.ph, q, n, qn, nqx, nqy);
-    cell_faces(kp.ph, qc, dqx, dqy, xdir, dtdx, dtdy, cm, cp);
-    cell_faces(kp.ph, qn, nqx, nqy, xdir, dtdx, dtdy, nm, np);
-    face_flux<RS>(kp.ph, xdir, np, cm, xdir ? dtdx : dtdy, fl);
+    cell_slopes(o, g, kp.ph, q, n, qn, nqx, nqy);
+    cell_faces(o, kp.ph, qc, dqx, dqy, xdir, dtdx, dtdy, cm, cp);
+    cell_faces(o, kp.ph, qn, nqx, nqy, xdir, dtdx, dtdy, nm, np);
+    face_flux<RS>(o, kp.ph, xdir, np, cm, xdir ? dtdx : dtdy, fl);
     // src/HydroRunFunctors.h:881-895 (x) and :957-971 (y)
     const bool own = j < g.jsize - 2 && i < g.isize - 2;
     const bool nbr = xdir ? (j < g.jsize - 2 && i > 2) : (j > 2 && i < g.isize - 2);
