@@ -303,6 +303,7 @@ int admit64(e2d_batch *b, const e2d_params &p, double t_end, const double *u0, i
   if (cudaMemcpyAsync(u1d, u0d, state_bytes, cudaMemcpyDeviceToDevice, b->stream) != cudaSuccess)
     return undo(E2D_ECUDA, "admit: copy");
   BatchInst64 I{};
+  batch_f64_shape(kp, &I.nbx, &I.nfill, &I.ntx, &I.ntiles);
   I.kp = kp;
   I.u[0] = u0d;
   I.u[1] = u1d;
@@ -311,7 +312,6 @@ int admit64(e2d_batch *b, const e2d_params &p, double t_end, const double *u0, i
   I.t = 0.0;
   I.t_end = t_end;
   I.active = I.t < I.t_end;
-  batch_f64_shape(kp, &I.nbx, &I.nfill, &I.ntx, &I.ntiles);
   HostInst &h = b->slots[slot];
   if (cudaMemcpyAsync(&b->d_insts64[slot], &I, sizeof(I), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
       launch_batch_prime_f64(&b->d_insts64[slot], I.nfill, b->stream) != cudaSuccess ||

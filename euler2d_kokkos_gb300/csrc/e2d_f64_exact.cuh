@@ -17,28 +17,14 @@
 namespace e2d {
 namespace f64x {
 
-// Additions and products as fused multiply-adds of three registers.  The FP64
-// pipe takes 16 clocks per SM for a warp's DFMA whose operands are all
-// registers and 19 for a DADD, a DMUL or any form with a constant or uniform
-// operand (measured: 625 against 527 G operations/s), so x + y is issued as
-// x * 1 + y and x * y as x * y + (-0): the same roundings and the same signs
-// of zero.  1 and -0 have to sit in registers the compiler knows nothing of;
-// each lane loads them from its own address.
-static __device__ double2 g_unit[32] = {
-#define E2D_U4 {1.0, -0.0}, {1.0, -0.0}, {1.0, -0.0}, {1.0, -0.0}
-    E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4
-#undef E2D_U4
-};
-struct Fp {
-  double one, mzero;
-  __device__ __forceinline__ Fp() {
-    const double2 *p = g_unit + (threadIdx.x & 31);
-    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(one), "=d"(mzero) : "l"(p));
-  }
-  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
-  __device__ __forceinline__ double sub(double a, double b) const { return fma(a, one, -b); }
-  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, mzero); }
-};
+constexpr unsigned long long kMag = 0x7fffffffffffffffull;
+constexpr unsigned long long kSign = 0x8000000000000000ull;
+
+__device__ __forceinline__ unsigned long long ubits(double x) { return f64i::bits(x); }
+__device__ __forceinline__ long long sbits(double x) { return (long long)f64i::bits(x); }
+__device__ __forceinline__ double from_bits(unsigned long long b) {
+  return f64i::make((uint32_t)(b >> 32), (uint32_t)b);
+}
 
 // a / b and sqrt(x) as the IEEE operations give them, on the integer pipes
 // (e2d_f64_intdiv.h); operands outside their range run the operation itself.
@@ -49,7 +35,7 @@ using f64i::divisor;
 __device__ __forceinline__ double quot(double a, const Divisor &d) {
   bool ok;
   double q = f64i::quotient(a, d, ok);
-  if (!ok) q = div_slow(a, __hiloint2double((int)d.hi, (int)d.lo));
+  if (!ok) q = div_slow(a, f64i::make(d.hi, d.lo));
   return q;
 }
 __device__ __forceinline__ double quot(double a, double b) { return quot(a, divisor(b)); }
@@ -58,17 +44,6 @@ __device__ __forceinline__ double root(double x) {
   double s = f64i::root(x, ok);
   if (!ok) s = sqrt_slow(x);
   return s;
-}
-
-constexpr unsigned long long kMag = 0x7fffffffffffffffull;
-constexpr unsigned long long kSign = 0x8000000000000000ull;
-
-__device__ __forceinline__ long long sbits(double x) { return __double_as_longlong(x); }
-__device__ __forceinline__ unsigned long long ubits(double x) {
-  return (unsigned long long)__double_as_longlong(x);
-}
-__device__ __forceinline__ double from_bits(unsigned long long b) {
-  return __longlong_as_double((long long)b);
 }
 
 // FP64 multiply kept out of line so that it runs only on the lanes that need
@@ -106,10 +81,10 @@ __device__ __forceinline__ bool gt_pos(double x, double c) { return sbits(x) > s
 // [2, 2046]; zeros are unchanged; subnormal results need rounding and use the
 // FP64 multiply; Inf/NaN are unchanged.
 __device__ __forceinline__ double half(double x) {
-  const int hi = __double2hiint(x);
-  const int lo = __double2loint(x);
+  const int hi = (int)f64i::high(x);
+  const int lo = (int)f64i::low(x);
   const int e = (hi >> 20) & 0x7ff;
-  if (e >= 2 && e < 0x7ff) return __hiloint2double(hi - 0x00100000, lo);
+  if (e >= 2 && e < 0x7ff) return f64i::make((uint32_t)hi - 0x00100000u, (uint32_t)lo);
   if (((hi & 0x7fffffff) | lo) == 0 || e == 0x7ff) return x;
   return mul_slow(0.5, x);
 }
@@ -117,44 +92,119 @@ __device__ __forceinline__ double half(double x) {
 // 2.0 * x: increment the exponent of normal numbers below 2^1023 ...; zeros
 // unchanged; subnormals and overflow use the FP64 multiply.
 __device__ __forceinline__ double twice(double x) {
-  const int hi = __double2hiint(x);
-  const int lo = __double2loint(x);
+  const int hi = (int)f64i::high(x);
+  const int lo = (int)f64i::low(x);
   const int e = (hi >> 20) & 0x7ff;
-  if (e >= 1 && e < 0x7fe) return __hiloint2double(hi + 0x00100000, lo);
+  if (e >= 1 && e < 0x7fe) return f64i::make((uint32_t)hi + 0x00100000u, (uint32_t)lo);
   if (((hi & 0x7fffffff) | lo) == 0 || e == 0x7ff) return x;
   return mul_slow(2.0, x);
 }
 
-static __device__ __noinline__ bool product_le0_slow(double a, double b) { return (a * b) <= 0.0; }
+// Additions and products as fused multiply-adds of three registers.  The FP64
+// pipe takes 16 clocks per SM for a warp's DFMA whose operands are all
+// registers and 19 for a DADD, a DMUL or any form with a constant or uniform
+// operand (measured: 625 against 527 G operations/s), so x + y is issued as
+// x * 1 + y, x - y as y * (-1) + x and x * y as x * y + (-0): the same
+// roundings and the same signs of zero.  1 and -0 have to sit in registers the compiler knows nothing of;
+// each lane loads them from its own address.
+static __device__ double2 g_unit[32] = {
+#define E2D_U4 {1.0, -0.0}, {1.0, -0.0}, {1.0, -0.0}, {1.0, -0.0}
+    E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4, E2D_U4
+#undef E2D_U4
+};
+//
+// XMUL: xmul() forms the product on the integer pipes (35 instructions, about
+// 60 clocks, overlapping the FP64 pipe's 64).  With about a fifth of a step's
+// products there -- face increments, transport terms, contact sums, energies,
+// flux scaling -- the two pipes run side by side: 1.556 instead of 1.69 ms a
+// 2048^2 HLLC step; with more of them the step slows down again (1.57 to 1.63
+// ms).  Where each SM holds one small tile the step waits on latency, not on
+// the FP64 pipe, and the plain product is the faster one (64x48: 16.0
+// against 17.1 us a step).
+template <bool XMUL>
+struct FpT {
+  double one, mzero, mone;
+  __device__ __forceinline__ FpT() {
+    const double2 *p = g_unit + (threadIdx.x & 31);
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(one), "=d"(mzero) : "l"(p));
+    mone = neg(one);
+  }
+  // sign changes on the integer pipe: a negated FP64 operand that several
+  // instructions read is otherwise formed by an FP64 instruction of its own
+  static __device__ __forceinline__ double neg(double x) {
+    return f64i::make(f64i::high(x) ^ 0x80000000u, f64i::low(x));
+  }
+  static __device__ __forceinline__ double abs(double x) {
+    return f64i::make(f64i::high(x) & 0x7fffffffu, f64i::low(x));
+  }
+  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return fma(b, mone, a); }
+  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, mzero); }
+  __device__ __forceinline__ double xmul(double a, double b) const {
+    if (!XMUL) return mul(a, b);
+    bool ok;
+    double p = f64i::product(a, b, ok);
+    if (!ok) p = mul_slow(a, b);
+    return p;
+  }
+  // 0.5 * (a * b) given hb = 0.5 * b: one product, unless halving would round
+  // (a result below the smallest normal double)
+  __device__ __forceinline__ double half_product(double a, double b, double hb) const {
+    if (XMUL) return half(xmul(a, b));
+    double p = mul(a, hb);
+    if ((f64i::high(p) & 0x7ff00000u) == 0u && ((f64i::high(a) & 0x7fffffffu) | f64i::low(a)) != 0u)
+      p = mul_slow(0.5, mul_slow(a, b));
+    return p;
+  }
+};
+using Fp = FpT<true>;
 
 // src/HydroBaseFunctor.h:421-455, one direction, for slope_type st in {1, 2}:
 //   dlft = st*(q-qm); drgt = st*(qp-q); dcen = 0.5*(qp-qm)
 //   dsgn = dcen >= 0 ? 1 : -1; slop = fmin(|dlft|, |drgt|)
 //   dlim = (dlft*drgt <= 0) ? 0 : slop;  dq = dsgn * fmin(dlim, |dcen|)
-// The three differences are FP64; scaling by st and 0.5 is exact, min of
-// non-negative values and all sign logic are integer operations.  The product
-// test dlft*drgt <= 0 equals "a zero or opposite signs" unless the product
-// underflows to zero, which needs both magnitudes below 2^-511: that case is
-// decided by the FP64 product itself.
-__device__ __forceinline__ double slope_limited(const Fp &f, bool st2, double q, double qp, double qm) {
+// from the three differences, as written.
+static __device__ __noinline__ double limit_slow(bool st2, double d1, double d2, double dc) {
+  const double st = st2 ? 2.0 : 1.0;
+  const double dl = mul_slow(st, d1), dr = mul_slow(st, d2), dcen = mul_slow(0.5, dc);
+  const double slop = fmin(fabs(dl), fabs(dr));
+  const double dlim = (dl * dr <= 0.0) ? 0.0 : slop;
+  const double r = fmin(dlim, fabs(dcen));
+  return dcen >= 0.0 ? r : -r;
+}
+
+// The same on the integer pipe but for the three differences.  The product
+// test is "a zero or opposite signs" (the product underflows only below
+// 2^-511); of one sign, the differences' sum dc has it too and is at least as
+// large as either, so scaling by 2 and by 0.5 moves only the exponents.
+// Differences outside [2^-511, 2^1023) that are not zero take the form above.
+// h: dq / 2, which the face states need (exact: 0 or at least 2^-512).
+template <class F>
+__device__ __forceinline__ void slope_limited(const F &f, bool st2, double q, double qp, double qm, double &dq,
+                                              double &h) {
   const double d1 = f.sub(q, qm);
   const double d2 = f.sub(qp, q);
   const double dc = f.sub(qp, qm);
-  const long long b1 = sbits(d1), b2 = sbits(d2);
-  const unsigned long long a1 = (unsigned long long)b1 & kMag;
-  const unsigned long long a2 = (unsigned long long)b2 & kMag;
-  bool kill = (a1 == 0ull) | (a2 == 0ull) | ((b1 ^ b2) < 0);
-  constexpr unsigned long long kTiny = 512ull << 52;  // 2^-511
-  if (!kill && (a1 < kTiny || a2 < kTiny)) {
-    const double st = st2 ? 2.0 : 1.0;
-    kill = product_le0_slow(mul_slow(st, d1), mul_slow(st, d2));
-  }
+  const unsigned int h1 = f64i::high(d1), h2 = f64i::high(d2), hc = f64i::high(dc), lc = f64i::low(dc);
+  const unsigned long long a1 = ((unsigned long long)(h1 & 0x7fffffffu) << 32) | f64i::low(d1);
+  const unsigned long long a2 = ((unsigned long long)(h2 & 0x7fffffffu) << 32) | f64i::low(d2);
   const unsigned long long m = a1 < a2 ? a1 : a2;
-  const double dlim = kill ? 0.0 : (st2 ? twice(from_bits(m)) : from_bits(m));
-  const double hc = half(from_bits(ubits(dc) & kMag));  // |dcen|
-  const unsigned long long r = ubits(dlim) < ubits(hc) ? ubits(dlim) : ubits(hc);
-  const bool neg = (sbits(dc) < 0) && (ubits(hc) != 0ull);  // dcen < 0
-  return from_bits(r | (neg ? kSign : 0ull));
+  const unsigned int mh = (unsigned int)(m >> 32), ac = hc & 0x7fffffffu;
+  const bool mz = m == 0ull, cz = (ac | lc) == 0u;
+  if ((mh < 0x20000000u && !mz) || (ac - 0x00200000u >= 0x7fc00000u && !cz)) {
+    dq = limit_slow(st2, d1, d2, dc);
+    h = 0.5 * dq;
+    return;
+  }
+  // min(st m, |dc| / 2), halved once more below
+  const unsigned long long lim = m + (st2 ? 1ull << 52 : 0ull);
+  const unsigned long long cen = (((unsigned long long)ac << 32) | lc) - (1ull << 52);
+  unsigned long long r = lim < cen ? lim : cen;
+  const bool kill = mz || (int)(h1 ^ h2) < 0;
+  const unsigned int sg = cz ? 0u : hc & 0x80000000u;  // dcen < 0
+  const unsigned int rh = (unsigned int)(r >> 32), rl = kill ? 0u : (unsigned int)r;
+  dq = f64i::make(sg | (kill ? 0u : rh), rl);
+  h = f64i::make(sg | (kill ? 0u : rh - 0x00100000u), rl);
 }
 
 }  // namespace f64x

@@ -25,6 +25,7 @@
 
 #include <cudaTypedefs.h>
 
+#include <cmath>
 #include <cstdint>
 
 namespace e2d {
@@ -32,19 +33,19 @@ namespace {
 
 constexpr int FILL_BX = 64, FILL_BY = 4;
 
-// Shared memory of a TX x TY tile of the flux kernel: primitives with a
-// 2-cell halo, then XMIN/XMAX states of cells x in [-1, TX] and YMIN/YMAX
-// states of cells y in [-1, TY].
-template <int TX, int TY>
+// Shared memory of a tile of up to TX x TYM cells: primitives with a 2-cell
+// halo, then XMIN/XMAX states of cells x in [-1, TX] and YMIN/YMAX states of
+// cells y in [-1, TYM].
+template <int TX, int TYM>
 constexpr size_t flux_smem_bytes() {
-  return sizeof(double) * (4 * (TY + 4) * (TX + 4) + 2 * (4 * TY * (TX + 2)) + 2 * (4 * (TY + 2) * TX));
+  return sizeof(double) * (4 * (TYM + 4) * (TX + 4) + 2 * (4 * TYM * (TX + 2)) + 2 * (4 * (TYM + 2) * TX));
 }
 
 // The fused step's shared memory: the same tile + alignment slack of the
 // TMA destination.
-template <int TX, int TY>
+template <int TX, int TYM>
 constexpr size_t step_smem_bytes() {
-  return flux_smem_bytes<TX, TY>() + 128;
+  return flux_smem_bytes<TX, TYM>() + 128;
 }
 
 // Ghost fill + primitives + CFL term of array cell (i, j) (see the file
@@ -147,27 +148,25 @@ __global__ void __launch_bounds__(FILL_BX *FILL_BY)
 }
 
 // ------------------------------------------------------------ kernel 2
-// Tile shapes (kp.tile): 0 -> 32 x 32 cells, 512 threads, 1 block per SM
-// (180.7 KB shared; 1.125 slope/trace evaluations and 2.06 Riemann solves
-// per cell); 1 -> 32 x 16, 256 threads, 2 blocks per SM (94.7 KB; 1.19 and
-// 2.09).  Measured on the 4096^2 blast: 15.12 and 15.38 ms per step; smaller
-// tiles (16 x 16, 32 x 8: 16.1, 16.7 ms) lose more to halo work than they
-// gain in residency.  Results do not depend on the shape.
+// Tiles are TX x ty cells, ty <= TYM chosen at run time per grid (see
+// choose_f64_tile); results do not depend on the shape.
 
 // Shared memory of a tile: primitives with a 2-cell halo, then the face
-// states (the scaled fluxes replace the XMIN / YMIN states in stage 3).
-template <int TX, int TY>
+// states (the scaled fluxes replace the XMIN / YMIN states in stage 3).  The
+// primitives' planes are ty + 4 rows each (as a TMA copy writes them), the
+// face states' planes TYM or TYM + 2.
+template <int TX, int TYM>
 struct TileSmem {
   static constexpr int QW = TX + 4;  // primitives tile width (2-cell halo)
-  static constexpr int QH = TY + 4;
+  static constexpr int QH = TYM + 4;
   static constexpr int XW = TX + 2;  // x-face states: cells x in [-1, TX]
-  static constexpr int YH = TY + 2;  // y-face states: cells y in [-1, TY]
+  static constexpr int YH = TYM + 2; // y-face states: cells y in [-1, TYM]
   double *sQ, *sXm, *sXp, *sYm, *sYp;
   __device__ explicit TileSmem(double *smem) {
-    sQ = smem;                   // [4][QH][QW]  primitives with halo
-    sXm = sQ + 4 * QH * QW;      // [4][TY][XW]  XMIN states, then x-fluxes
-    sXp = sXm + 4 * TY * XW;     // [4][TY][XW]  XMAX states
-    sYm = sXp + 4 * TY * XW;     // [4][YH][TX]  YMIN states, then y-fluxes
+    sQ = smem;                   // [4][ty + 4][QW]  primitives with halo
+    sXm = sQ + 4 * QH * QW;      // [4][TYM][XW]  XMIN states, then x-fluxes
+    sXp = sXm + 4 * TYM * XW;    // [4][TYM][XW]  XMAX states
+    sYm = sXp + 4 * TYM * XW;    // [4][YH][TX]  YMIN states, then y-fluxes
     sYp = sYm + 4 * YH * TX;     // [4][YH][TX]  YMAX states
   }
 };
@@ -175,20 +174,21 @@ struct TileSmem {
 // Stage 1 of the two-launch step: primitives of the tile and its 2-cell
 // halo from the primitives array (ghost cells included, written by the fill
 // kernel); cells beyond the array get a harmless 1.0.
-template <int TX, int TY, int NT>
-__device__ __forceinline__ void load_qtile(const KGeom &g, const double *__restrict__ q, int i0, int j0,
+template <int TX, int NT>
+__device__ __forceinline__ void load_qtile(const KGeom &g, const double *__restrict__ q, int i0, int j0, int ty,
                                            double *sQ) {
-  constexpr int QW = TX + 4, QH = TY + 4;
-  for (int k = threadIdx.x; k < QH * QW; k += NT) {
+  constexpr int QW = TX + 4;
+  const int n = (ty + 4) * QW;
+  for (int k = threadIdx.x; k < n; k += NT) {
     const int y = k / QW, x = k - y * QW;
     const int gi = i0 + x, gj = j0 + y;
     if (gi < g.isize && gj < g.jsize) {
       const size_t s = (size_t)gi + (size_t)g.isize * gj;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sQ[v * QH * QW + k] = q[s + v * g.plane];
+      for (int v = 0; v < 4; ++v) sQ[v * n + k] = q[s + v * g.plane];
     } else {
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sQ[v * QH * QW + k] = 1.0;
+      for (int v = 0; v < 4; ++v) sQ[v * n + k] = 1.0;
     }
   }
 }
@@ -199,11 +199,12 @@ __device__ __forceinline__ void load_qtile(const KGeom &g, const double *__restr
 // primitives of the reference's ghost-filled state (u = mx / d changes only
 // its sign with mx; e, p and c depend on u^2).  Only interior cells of q are
 // read.
-template <int TX, int TY, int NT>
-__device__ __forceinline__ void gather_qtile(const KGeom &g, const double *__restrict__ q, int i0, int j0,
+template <int TX, int NT>
+__device__ __forceinline__ void gather_qtile(const KGeom &g, const double *__restrict__ q, int i0, int j0, int ty,
                                              double *sQ) {
-  constexpr int QW = TX + 4, QH = TY + 4;
-  for (int k = threadIdx.x; k < QH * QW; k += NT) {
+  constexpr int QW = TX + 4;
+  const int n = (ty + 4) * QW;
+  for (int k = threadIdx.x; k < n; k += NT) {
     const int y = k / QW, x = k - y * QW;
     const int gi = i0 + x, gj = j0 + y;
     if (gi < g.isize && gj < g.jsize) {
@@ -213,63 +214,58 @@ __device__ __forceinline__ void gather_qtile(const KGeom &g, const double *__res
       const size_t s = (size_t)si + (size_t)g.isize * sj;
       const double ux = q[s + 2 * g.plane], uy = q[s + 3 * g.plane];
       sQ[k] = q[s];
-      sQ[QH * QW + k] = q[s + g.plane];
-      sQ[2 * QH * QW + k] = fu ? -ux : ux;
-      sQ[3 * QH * QW + k] = fv ? -uy : uy;
+      sQ[n + k] = q[s + g.plane];
+      sQ[2 * n + k] = fu ? Fp::neg(ux) : ux;
+      sQ[3 * n + k] = fv ? Fp::neg(uy) : uy;
     } else {
 #pragma unroll
-      for (int v = 0; v < 4; ++v) sQ[v * QH * QW + k] = 1.0;
+      for (int v = 0; v < 4; ++v) sQ[v * n + k] = 1.0;
     }
   }
 }
 
-// Stages 2 and 3 of a tile whose primitives are in shared memory (the
-// caller has synchronised after writing them): slopes, trace sources and
-// face states of the tile cells and of the 1-cell ring (corners excluded)
-// -- src/HydroBaseFunctor.h:214-291 --, then one Riemann solve per face.
-// On return (after a block barrier) sXm holds the x-fluxes scaled by dt/dx
-// and sYm the y-fluxes scaled by dt/dy.
-template <int RS, int TX, int TY, int NT, bool FAST = false>
-__device__ __forceinline__ void tile_fluxes(const Fp &fp64, const KPhys<double> &ph, const double dtdx, const double dtdy,
-                                            double *smem) {
-  using T = TileSmem<TX, TY>;
-  constexpr int QW = T::QW, QH = T::QH, XW = T::XW, YH = T::YH;
+// Stage 2 of a tile whose primitives are in shared memory (the caller has
+// synchronised after writing them): slopes, trace sources and face states of
+// the tile cells and of the 1-cell ring (corners excluded) --
+// src/HydroBaseFunctor.h:214-291.
+template <int TX, int TYM, int NT, bool FAST, class F>
+__device__ __forceinline__ void tile_faces(const F &fp64, const KPhys<double> &ph, const double dtdx,
+                                           const double dtdy, const int ty, double *smem) {
+  using T = TileSmem<TX, TYM>;
+  constexpr int QW = T::QW, XW = T::XW, YH = T::YH;
   const T sm(smem);
   const double *sQ = sm.sQ;
-  double *sXm = sm.sXm, *sXp = sm.sXp, *sYm = sm.sYm, *sYp = sm.sYp;
-  const int tid = threadIdx.x;
-
-  // stage 2: slopes, trace sources and face states.  Items enumerate the
-  // tile and its 1-cell ring without the ring's four corners (which carry no
-  // face), so the last partial round of 32 x 32 tiles is 4 whole warps -- one
-  // per scheduler -- instead of 4 warps and 4 threads.  The FP64 pipe takes
-  // as long for a warp instruction with a few active lanes as for a full
-  // one, so a partial round costs what its busiest scheduler's warps cost.
+  const int qs = QW * (ty + 4);
+  // Items enumerate the tile and its 1-cell ring without the ring's four
+  // corners, which carry no face.  The FP64 pipe takes as long for a warp
+  // instruction with a few active lanes as for a full one, so a partial
+  // round costs what its busiest scheduler's warps cost.
   const int st_kind = (ph.slope_type == 2.0) ? 2 : (ph.slope_type == 1.0) ? 1 : 0;
-  constexpr int NS2 = YH * XW - 4;
-  for (int k = tid; k < NS2; k += NT) {
+  const int ns2 = (ty + 2) * XW - 4;
+  const double hdtdx = half(dtdx), hdtdy = half(dtdy);
+  for (int k = threadIdx.x; k < ns2; k += NT) {
     int yy, xx;  // cell (xx-1, yy-1) of the tile
     if (k < TX) {
       yy = 0;
       xx = k + 1;
-    } else if (k < TX + TY * XW) {
+    } else if (k < TX + ty * XW) {
       const int r = k - TX;
       yy = 1 + r / XW;
       xx = r - (yy - 1) * XW;
     } else {
-      yy = YH - 1;
-      xx = k - (TX + TY * XW) + 1;
+      yy = ty + 1;
+      xx = k - (TX + ty * XW) + 1;
     }
     const bool xin = (xx >= 1) && (xx <= TX);
-    const bool yin = (yy >= 1) && (yy <= TY);
+    const bool yin = (yy >= 1) && (yy <= ty);
     const int c = (yy + 1) * QW + (xx + 1);
-    double qc[4], dqx[4], dqy[4];
+    double qc[4], dqx[4], dqy[4], hx[4], hy[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-      const double *P = sQ + v * QH * QW;
+      const double *P = sQ + v * qs;
       qc[v] = P[c];
-      dqx[v] = slope(fp64, st_kind, qc[v], P[c + 1], P[c - 1]);
-      dqy[v] = slope(fp64, st_kind, qc[v], P[c + QW], P[c - QW]);
+      slope(fp64, st_kind, qc[v], P[c + 1], P[c - 1], dqx[v], hx[v]);
+      slope(fp64, st_kind, qc[v], P[c + QW], P[c - QW], dqy[v], hy[v]);
     }
     double s0[4];
     if (FAST)
@@ -282,11 +278,11 @@ __device__ __forceinline__ void tile_fluxes(const Fp &fp64, const KPhys<double> 
       for (int v = 0; v < 4; ++v) {
         double fm, fp;
         if (FAST)
-          face_pair_fast(fp64, ph, v, qc[v], dqx[v], s0[v], 0.5 * dtdx, fm, fp);
+          face_pair_fast(fp64, ph, v, qc[v], hx[v], s0[v], hdtdx, fm, fp);
         else
-          face_pair(fp64, ph, v, qc[v], dqx[v], s0[v], dtdx, fm, fp);
-        if (xx >= 1) sXm[v * TY * XW + o] = fm;
-        if (xx <= TX) sXp[v * TY * XW + o] = fp;
+          face_pair(fp64, ph, v, qc[v], hx[v], s0[v], dtdx, hdtdx, fm, fp);
+        if (xx >= 1) sm.sXm[v * TYM * XW + o] = fm;
+        if (xx <= TX) sm.sXp[v * TYM * XW + o] = fp;
       }
     }
     if (xin) {
@@ -295,96 +291,131 @@ __device__ __forceinline__ void tile_fluxes(const Fp &fp64, const KPhys<double> 
       for (int v = 0; v < 4; ++v) {
         double fm, fp;
         if (FAST)
-          face_pair_fast(fp64, ph, v, qc[v], dqy[v], s0[v], 0.5 * dtdy, fm, fp);
+          face_pair_fast(fp64, ph, v, qc[v], hy[v], s0[v], hdtdy, fm, fp);
         else
-          face_pair(fp64, ph, v, qc[v], dqy[v], s0[v], dtdy, fm, fp);
-        if (yy >= 1) sYm[v * YH * TX + o] = fm;
-        if (yy <= TY) sYp[v * YH * TX + o] = fp;
+          face_pair(fp64, ph, v, qc[v], hy[v], s0[v], dtdy, hdtdy, fm, fp);
+        if (yy >= 1) sm.sYm[v * YH * TX + o] = fm;
+        if (yy <= ty) sm.sYp[v * YH * TX + o] = fp;
       }
     }
   }
-  __syncthreads();
-
-  // stage 3: one Riemann solve per face; the scaled flux replaces the
-  // right-hand state, which no other face reads
-  constexpr int NXF = (TX + 1) * TY;
-  constexpr int NYF = TX * (TY + 1);
-  for (int k = tid; k < NXF + NYF; k += NT) {
-    double ql[4], qr[4], f[4];
-    if (k < NXF) {
-      const int y = k / (TX + 1), fx = k - y * (TX + 1);
-      const int ol = y * XW + fx, orr = ol + 1;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        ql[v] = sXp[v * TY * XW + ol];
-        qr[v] = sXm[v * TY * XW + orr];
-      }
-      riemann_sel<RS, FAST>(fp64, ph, ql, qr, f);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) sXm[v * TY * XW + orr] = fp64.mul(f[v], dtdx);
-    } else {
-      const int kk = k - NXF;
-      const int fy = kk / TX, x = kk - fy * TX;
-      const int ol = fy * TX + x, orr = ol + TX;
-      // normal velocity first: swap IU/IV (src/HydroRunFunctors.h:628-632)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int vs = (v == E2D_IU) ? E2D_IV : (v == E2D_IV) ? E2D_IU : v;
-        ql[vs] = sYp[v * YH * TX + ol];
-        qr[vs] = sYm[v * YH * TX + orr];
-      }
-      riemann_sel<RS, FAST>(fp64, ph, ql, qr, f);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int vs = (v == E2D_IU) ? E2D_IV : (v == E2D_IV) ? E2D_IU : v;
-        sYm[v * YH * TX + orr] = fp64.mul(f[vs], dtdy);
-      }
-    }
-  }
-  __syncthreads();
 }
 
+// Stage 3 (after a block barrier): one Riemann solve per face; the flux,
+// scaled by dt/dx or dt/dy (the fast forms scale in the update), replaces
+// the right-hand state, which no other face reads.
+template <int RS, int TX, int TYM, int NT, bool FAST, class F>
+__device__ __forceinline__ void tile_riemann(const F &fp64, const KPhys<double> &ph, const double dtdx,
+                                             const double dtdy, const int ty, double *smem) {
+  using T = TileSmem<TX, TYM>;
+  constexpr int XW = T::XW, YH = T::YH;
+  const T sm(smem);
+  const int nxf = (TX + 1) * ty;
+  const int nf = nxf + TX * (ty + 1);
+  // one copy of the solver for both directions: the faces' states by
+  // pointer, with the plane stride and the planes of the normal and the
+  // tangential velocity (y: swapped, src/HydroRunFunctors.h:628-632)
+  for (int k = threadIdx.x; k < nf; k += NT) {
+    const bool xd = k < nxf;
+    const int kk = xd ? k : k - nxf;
+    const int w = xd ? TX + 1 : TX;
+    const int y = xd ? kk / (TX + 1) : kk / TX, x = kk - y * w;
+    const int ol = xd ? y * XW + x : kk;
+    const int ps = xd ? TYM * XW : YH * TX;
+    const double *pl = (xd ? sm.sXp : sm.sYp) + ol;
+    double *pr = (xd ? sm.sXm + 1 : sm.sYm + TX) + ol;
+    const int on = xd ? 2 * ps : 3 * ps, ot = xd ? 3 * ps : 2 * ps;
+    const double ql[4] = {pl[0], pl[ps], pl[on], pl[ot]}, qr[4] = {pr[0], pr[ps], pr[on], pr[ot]};
+    double f[4];
+    riemann_sel<RS, FAST>(fp64, ph, ql, qr, f);
+    if (!FAST) {
+      const double dtd = xd ? dtdx : dtdy;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) f[v] = fp64.xmul(f[v], dtd);
+    }
+    pr[0] = f[E2D_ID];
+    pr[ps] = f[E2D_IP];
+    pr[on] = f[E2D_IU];
+    pr[ot] = f[E2D_IV];
+  }
+}
+
+// The input values of a thread's cells of the tile, loaded before the
+// Riemann solves so that the update does not wait for them.
+template <int TX, int TYM, int NT>
+struct TileCells {
+  static constexpr int N = (TX * TYM + NT - 1) / NT;
+  double u[N][4];
+  // cell n of the thread: its offset in a plane, or -1
+  static __device__ __forceinline__ long long offset(const KGeom &g, int i0, int j0, int ty, int n, int &x, int &y) {
+    const int k = threadIdx.x + n * NT;
+    y = k / TX;
+    x = k - y * TX;
+    const int gi = i0 + 2 + x, gj = j0 + 2 + y;
+    return (y < ty && gi < g.nx + 2 && gj < g.ny + 2) ? gi + (long long)g.isize * gj : -1;
+  }
+  __device__ __forceinline__ void load(const KGeom &g, const double *__restrict__ u_in, int i0, int j0, int ty) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      int x, y;
+      const long long s = offset(g, i0, j0, ty, n, x, y);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) u[n][v] = s >= 0 ? u_in[s + v * g.plane] : 0.0;
+    }
+  }
+};
+
 // The conservative update of cell (x, y) of a tile in the reference's order
-// (src/HydroRunFunctors.h:691-713): +Fx(i) -Fx(i+1) +Fy(j) -Fy(j+1).
-template <int TX, int TY>
-__device__ __forceinline__ double update_var(const Fp &f, const TileSmem<TX, TY> &sm, int v, int x, int y,
-                                             double uu) {
-  using T = TileSmem<TX, TY>;
-  uu = f.add(uu, sm.sXm[v * TY * T::XW + y * T::XW + x + 1]);
-  uu = f.sub(uu, sm.sXm[v * TY * T::XW + y * T::XW + x + 2]);
-  uu = f.add(uu, sm.sYm[v * T::YH * TX + (y + 1) * TX + x]);
-  uu = f.sub(uu, sm.sYm[v * T::YH * TX + (y + 2) * TX + x]);
+// (src/HydroRunFunctors.h:691-713): +Fx(i) -Fx(i+1) +Fy(j) -Fy(j+1).  The
+// fast forms take unscaled fluxes: one difference and one FMA a direction.
+template <int TX, int TYM, bool FAST, class F>
+__device__ __forceinline__ double update_var(const F &f, const TileSmem<TX, TYM> &sm, int v, int x, int y,
+                                             double uu, double dtdx, double dtdy) {
+  using T = TileSmem<TX, TYM>;
+  const double *fx = sm.sXm + v * TYM * T::XW + y * T::XW + x + 1;
+  const double *fy = sm.sYm + v * T::YH * TX + (y + 1) * TX + x;
+  if (FAST) return fma(f.sub(fx[0], fx[1]), dtdx, fma(f.sub(fy[0], fy[TX]), dtdy, uu));
+  uu = f.add(uu, fx[0]);
+  uu = f.sub(uu, fx[1]);
+  uu = f.add(uu, fy[0]);
+  uu = f.sub(uu, fy[TX]);
   return uu;
 }
 
 // Stages 1-4 of the two-launch step for tile (bx, by) of a grid,
-// block-wide; the caller provides dt/dx, dt/dy and TX x TY shared memory.
-template <int RS, int TX, int TY, int NT>
+// block-wide; the caller provides dt/dx, dt/dy and the tile's shared memory.
+template <int RS, int TX, int TYM, int NT, class F>
 __device__ __forceinline__ void flux_tile(const KParams64 &kp, const double *__restrict__ q,
                                           const double *__restrict__ u_in, double *__restrict__ u_out,
-                                          const int bx, const int by, const double dtdx, const double dtdy,
-                                          double *smem) {
+                                          const int bx, const int by, const int ty, const double dtdx,
+                                          const double dtdy, double *smem) {
   const KGeom &g = kp.g;
   const int i0 = bx * TX;  // array column of the tile's first halo cell
-  const int j0 = by * TY;
-  const Fp f;
-  load_qtile<TX, TY, NT>(g, q, i0, j0, smem);
+  const int j0 = by * ty;
+  const F f;
+  load_qtile<TX, NT>(g, q, i0, j0, ty, smem);
   __syncthreads();
-  tile_fluxes<RS, TX, TY, NT>(f, kp.ph, dtdx, dtdy, smem);
-  const TileSmem<TX, TY> sm(smem);
+  tile_faces<TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+  TileCells<TX, TYM, NT> cells;
+  cells.load(g, u_in, i0, j0, ty);
+  __syncthreads();
+  tile_riemann<RS, TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+  __syncthreads();
+  const TileSmem<TX, TYM> sm(smem);
   // stage 4: conservative update
-  for (int k = threadIdx.x; k < TX * TY; k += NT) {
-    const int y = k / TX, x = k - y * TX;
-    const int gi = i0 + 2 + x, gj = j0 + 2 + y;
-    if (gi < g.nx + 2 && gj < g.ny + 2) {
-      const size_t s = (size_t)gi + (size_t)g.isize * gj;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) u_out[s + v * g.plane] = update_var<TX, TY>(f, sm, v, x, y, u_in[s + v * g.plane]);
+  for (int n = 0; n < cells.N; ++n) {
+    int x, y;
+    const long long s = cells.offset(g, i0, j0, ty, n, x, y);
+    if (s >= 0) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        u_out[s + v * g.plane] = update_var<TX, TYM, false>(f, sm, v, x, y, cells.u[n][v], dtdx, dtdy);
     }
   }
 }
 
-template <int RS, int TX, int TY, int NT, int MINB>
+template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL>
 __global__ void __launch_bounds__(NT, MINB)
     k_flux_update_f64(const KParams64 kp, const double *__restrict__ q,
                       const double *__restrict__ u_in, double *__restrict__ u_out, DevClock *clk,
@@ -412,7 +443,7 @@ __global__ void __launch_bounds__(NT, MINB)
   __syncthreads();
   if (!s_run) return;
   const double dt = s_dt[0];
-  flux_tile<RS, TX, TY, NT>(kp, q, u_in, u_out, blockIdx.x, blockIdx.y, s_dt[1], s_dt[2], smem);
+  flux_tile<RS, TX, TYM, NT, f64x::FpT<XMUL>>(kp, q, u_in, u_out, blockIdx.x, blockIdx.y, kp.ty, s_dt[1], s_dt[2], smem);
 
   if (!use_clock) return;
   // the last block to finish advances the loop state (src/main.cpp:139-143)
@@ -471,22 +502,23 @@ __device__ __forceinline__ void block_fold(double term, unsigned int flags, unsi
 // The fused step's epilogue for the cells of a tile whose fluxes are in
 // shared memory: the conservative update into u_out, the primitives of the
 // new cells into q_out and the running maximum of their CFL terms and flags.
-template <int TX, int TY, int NT, bool FAST>
-__device__ __forceinline__ void step_epilogue(const Fp &f, const KParams64 &kp, const double *__restrict__ u_in,
+template <int TX, int TYM, int NT, bool FAST, class F>
+__device__ __forceinline__ void step_epilogue(const F &f, const KParams64 &kp, const TileCells<TX, TYM, NT> &cells,
                                               double *__restrict__ u_out, double *__restrict__ q_out, int i0,
-                                              int j0, double *smem, double &term, unsigned int &flags) {
+                                              int j0, int ty, double dtdx, double dtdy, double *smem, double &term,
+                                              unsigned int &flags) {
   const KGeom &g = kp.g;
   const KPhys<double> &ph = kp.ph;
-  const TileSmem<TX, TY> sm(smem);
-  for (int k = threadIdx.x; k < TX * TY; k += NT) {
-    const int y = k / TX, x = k - y * TX;
-    const int gi = i0 + 2 + x, gj = j0 + 2 + y;
-    if (gi < g.nx + 2 && gj < g.ny + 2) {
-      const size_t s = (size_t)gi + (size_t)g.isize * gj;
+  const TileSmem<TX, TYM> sm(smem);
+#pragma unroll
+  for (int n = 0; n < cells.N; ++n) {
+    int x, y;
+    const long long s = cells.offset(g, i0, j0, ty, n, x, y);
+    if (s >= 0) {
       double un[4];
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        un[v] = update_var<TX, TY>(f, sm, v, x, y, u_in[s + v * g.plane]);
+        un[v] = update_var<TX, TYM, FAST>(f, sm, v, x, y, cells.u[n][v], dtdx, dtdy);
         u_out[s + v * g.plane] = un[v];
       }
       double dd, p, ux, uy;
@@ -508,12 +540,12 @@ __device__ __forceinline__ void step_epilogue(const Fp &f, const KParams64 &kp, 
 // The ghost cells next to a tile -- those whose nearest interior cell is in
 // it -- receive the ghost fill of u_in in both states, read from interior
 // cells of u_in only (no block writes those during a step).
-template <int TX, int TY, int NT>
+template <int TX, int NT>
 __device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *__restrict__ u_in, double *__restrict__ u_out,
-                                                int i0, int j0, bool lo_x, bool hi_x, bool lo_y, bool hi_y) {
+                                                int i0, int j0, int ty, bool lo_x, bool hi_x, bool lo_y, bool hi_y) {
   if (!(lo_x || hi_x || lo_y || hi_y)) return;
   const int xa = lo_x ? 0 : i0 + 2, xb = hi_x ? g.isize : i0 + 2 + TX;
-  const int ya = lo_y ? 0 : j0 + 2, yb = hi_y ? g.jsize : j0 + 2 + TY;
+  const int ya = lo_y ? 0 : j0 + 2, yb = hi_y ? g.jsize : j0 + 2 + ty;
   const int w = xb - xa, n = w * (yb - ya);
   for (int k = threadIdx.x; k < n; k += NT) {
     const int j = ya + k / w, i = xa + k % w;
@@ -533,13 +565,8 @@ __device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *__restri
   }
 }
 
-template <int TX, int TY>
-__host__ __device__ constexpr unsigned int qtile_bytes() {
-  return (unsigned int)(sizeof(double) * 4 * (TX + 4) * (TY + 4));
-}
-
 // One whole time step of the device loop (src/main.cpp:128-143 around
-// godunov_unsplit_impl, src/HydroRun.h:279-364), one TX x TY tile per block:
+// godunov_unsplit_impl, src/HydroRun.h:279-364), one TX x ty tile per block:
 //  - dt from the CFL maximum of the input state, clock->acc[nstep & 1],
 //    which the previous step (or the prologue fill) folded;
 //  - stage 1: primitives of the tile and its 2-cell halo, from q_in (the
@@ -554,7 +581,7 @@ __host__ __device__ constexpr unsigned int qtile_bytes() {
 //    only interior cells of u_in, which no block writes;
 //  - the last block to finish advances the loop state.
 // Bit-identical to the two-launch step; FP64 work per cell is the same.
-template <int RS, int TX, int TY, int NT, int MINB, bool FAST>
+template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL, bool FAST>
 __global__ void __launch_bounds__(NT, MINB)
     k_step_f64(const KParams64 kp, const __grid_constant__ CUtensorMap tm_q, const int use_tma,
                const double *__restrict__ q_in, double *__restrict__ q_out, double *__restrict__ u_in,
@@ -569,9 +596,10 @@ __global__ void __launch_bounds__(NT, MINB)
   const KPhys<double> &ph = kp.ph;
   const int tid = threadIdx.x;
   const int bx = blockIdx.x, by = blockIdx.y;
-  const int i0 = bx * TX, j0 = by * TY;  // array cell of the halo box's corner
-  constexpr int QW = TX + 4, QH = TY + 4;
-  const bool tma_tile = use_tma && i0 >= 2 && j0 >= 2 && i0 + QW <= g.nx + 2 && j0 + QH <= g.ny + 2;
+  const int ty = kp.ty;
+  const int i0 = bx * TX, j0 = by * ty;  // array cell of the halo box's corner
+  constexpr int QW = TX + 4;
+  const bool tma_tile = use_tma && i0 >= 2 && j0 >= 2 && i0 + QW <= g.nx + 2 && j0 + ty + 4 <= g.ny + 2;
   if (tid == 0) {
     const int run = clk->t < clk->t_end;
     const int par = clk->nstep & 1;
@@ -586,7 +614,7 @@ __global__ void __launch_bounds__(NT, MINB)
       mbar_init_fence();
       // wait_test: tile (1, 1) never copies, so its bounded wait runs out
       if (!(kp.wait_test && bx == 1 && by == 1)) {
-        mbar_arrive_expect(&s_bar, qtile_bytes<TX, TY>());
+        mbar_arrive_expect(&s_bar, (unsigned int)(sizeof(double) * 4 * QW) * (unsigned int)(ty + 4));
         tma_load_3d(smem, &tm_q, i0, j0, 0, &s_bar);
       }
     }
@@ -605,19 +633,25 @@ __global__ void __launch_bounds__(NT, MINB)
       __syncthreads();
     }
   } else {
-    gather_qtile<TX, TY, NT>(g, q_in, i0, j0, smem);
+    gather_qtile<TX, NT>(g, q_in, i0, j0, ty, smem);
     __syncthreads();
   }
 
-  const Fp f;
+  const f64x::FpT<XMUL> f;
   double term = 0.0;
   unsigned int flags = 0;
   if (ok) {
-    tile_fluxes<RS, TX, TY, NT, FAST>(f, ph, s_dt[1], s_dt[2], smem);
-    step_epilogue<TX, TY, NT, FAST>(f, kp, u_in, u_out, q_out, i0, j0, smem, term, flags);
+    const double dtdx = s_dt[1], dtdy = s_dt[2];
+    tile_faces<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+    TileCells<TX, TYM, NT> cells;
+    cells.load(g, u_in, i0, j0, ty);
+    __syncthreads();
+    tile_riemann<RS, TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+    __syncthreads();
+    step_epilogue<TX, TYM, NT, FAST>(f, kp, cells, u_out, q_out, i0, j0, ty, dtdx, dtdy, smem, term, flags);
   }
-  ghost_fill_tile<TX, TY, NT>(g, u_in, u_out, i0, j0, bx == 0, bx == (int)gridDim.x - 1, by == 0,
-                              by == (int)gridDim.y - 1);
+  ghost_fill_tile<TX, NT>(g, u_in, u_out, i0, j0, ty, bx == 0, bx == (int)gridDim.x - 1, by == 0,
+                          by == (int)gridDim.y - 1);
 
   block_fold<NT>(term, flags, &clk->acc[par ^ 1], &clk->status);
 
@@ -669,12 +703,13 @@ __global__ void __launch_bounds__(FILL_BX *FILL_BY) k_batch_prime_f64(BatchInst6
 }
 
 // One iteration of every listed FP64 instance in one persistent launch: each
-// block takes 32 x 32 tiles from the work list (instance k's tiles are
+// block takes tiles from the work list (instance k's tiles are
 // tile_begin[k] .. tile_begin[k+1]-1) and runs the fused step on each with
 // its instance's dt, primitives and ghost cells (tiles gathered, no TMA);
 // the instance's last tile advances its loop state.
+constexpr int BTX = 32, BTY = 32, BNT = 512, BMINB = 1;
 template <int RS>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(BNT, BMINB)
     k_batch_step_f64(BatchInst64 *__restrict__ insts, const int *__restrict__ list_slots,
                      const int *__restrict__ tile_begin, const int n_inst, const int total_tiles) {
   extern __shared__ unsigned char smem_raw[];
@@ -697,16 +732,24 @@ __global__ void __launch_bounds__(512, 1)
     const int b = w - tile_begin[k];
     const int by = b / I.ntx, bx = b - by * I.ntx;
     const int nty = I.ntiles / I.ntx;
-    const int i0 = bx * 32, j0 = by * 32;
-    gather_qtile<32, 32, 512>(kp.g, I.q[par], i0, j0, smem);
+    const int ty = kp.ty;
+    const int i0 = bx * BTX, j0 = by * ty;
+    gather_qtile<BTX, BNT>(kp.g, I.q[par], i0, j0, ty, smem);
     __syncthreads();
     double term = 0.0;
     unsigned int flags = 0;
-    tile_fluxes<RS, 32, 32, 512>(f, kp.ph, s_dt[1], s_dt[2], smem);
-    step_epilogue<32, 32, 512, false>(f, kp, I.u[par], I.u[par ^ 1], I.q[par ^ 1], i0, j0, smem, term, flags);
-    ghost_fill_tile<32, 32, 512>(kp.g, I.u[par], I.u[par ^ 1], i0, j0, bx == 0, bx == I.ntx - 1, by == 0,
-                                 by == nty - 1);
-    block_fold<512>(term, flags, &I.acc[par ^ 1], &I.status);
+    const double dtdx = s_dt[1], dtdy = s_dt[2];
+    tile_faces<BTX, BTY, BNT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+    TileCells<BTX, BTY, BNT> cells;
+    cells.load(kp.g, I.u[par], i0, j0, ty);
+    __syncthreads();
+    tile_riemann<RS, BTX, BTY, BNT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+    __syncthreads();
+    step_epilogue<BTX, BTY, BNT, false>(f, kp, cells, I.u[par ^ 1], I.q[par ^ 1], i0, j0, ty, dtdx, dtdy, smem, term,
+                                        flags);
+    ghost_fill_tile<BTX, BNT>(kp.g, I.u[par], I.u[par ^ 1], i0, j0, ty, bx == 0, bx == I.ntx - 1, by == 0,
+                              by == nty - 1);
+    block_fold<BNT>(term, flags, &I.acc[par ^ 1], &I.status);
     __syncthreads();
     if (tid == 0) {
       __threadfence();
@@ -768,7 +811,8 @@ __global__ void k_eval_f64(const KParams64 kp, const int what, const int n,
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       double fm, fp;
-      face_pair(f, ph, v, s[v], xdir ? s[4 + v] : s[8 + v], s0[v], xdir ? dtdx : dtdy, fm, fp);
+      const double dtd = xdir ? dtdx : dtdy;
+      face_pair(f, ph, v, s[v], half(xdir ? s[4 + v] : s[8 + v]), s0[v], dtd, half(dtd), fm, fp);
       out[4 * k + v] = (face == 0 || face == 2) ? fm : fp;
     }
   } else {
@@ -872,54 +916,124 @@ cudaError_t launch_fill_f64(const KParams64 &kp, double *u_in, double *u_out, do
   return cudaGetLastError();
 }
 
-template <int RS, int TX, int TY, int NT, int MINB>
-static cudaError_t launch_flux_shape(const KParams64 &kp, const double *q, const double *u_in,
-                                     double *u_out, DevClock *clk, int use_clock, double host_dt,
-                                     double *dt_trace, cudaStream_t s) {
-  dim3 grid((kp.g.nx + TX - 1) / TX, (kp.g.ny + TY - 1) / TY);
-  k_flux_update_f64<RS, TX, TY, NT, MINB><<<grid, NT, flux_smem_bytes<TX, TY>(), s>>>(
-      kp, q, u_in, u_out, clk, use_clock, host_dt, dt_trace);
-  return cudaGetLastError();
+// Tile shapes of the fused step and of the two-launch step's flux kernel: TX
+// columns, up to TYM rows, NT threads, MINB blocks on an SM; XMUL: see FpT.
+template <int SHAPE>
+struct Shape;
+template <>
+struct Shape<0> {
+  static constexpr int TX = 32, TYM = 16, NT = 256, MINB = 2;
+  static constexpr bool XMUL = true;
+};
+template <>
+struct Shape<1> {
+  static constexpr int TX = 16, TYM = 16, NT = 128, MINB = 4;
+  static constexpr bool XMUL = true;
+};
+template <>
+struct Shape<2> {
+  static constexpr int TX = 8, TYM = 8, NT = 160, MINB = 3;
+  static constexpr bool XMUL = false;
+};
+constexpr int kShapes = 3;
+template <class F>
+static void with_shape(int shape, F &&f) {
+  switch (shape) {
+    case 1: f(Shape<1>{}); break;
+    case 2: f(Shape<2>{}); break;
+    default: f(Shape<0>{}); break;
+  }
+}
+
+// The tile of a grid: the shape and rows whose step a simple model of the
+// launch puts lowest.  A tile's stages take whole warps of face-state cells,
+// Riemann solves and updates (W2, W3, W4); one tile alone takes L, a latency
+// per round of its block's warps; k tiles on an SM share the FP64 pipe,
+// k (80 W2 + 50 W3 + 34 W4) instructions at 5 ns; the two add with exponent
+// 1.26; tiles beyond what is resident make further waves, which average out
+// once there are four.  The constants are fitted to 380 timings (14 grids
+// from 64x48 to 2048^2, every shape, 4 to 16 rows; 4 % rms), on which the
+// model's choice is within 0.6 % of the fastest tile of every grid.
+// What it buys (us a step, HLLC; before: 32 x 32 tiles for every grid):
+// 64x48 71 -> 15.9 (8 x 4), 128^2 71 -> 17.2 (8 x 7), 256^2 72 -> 36.2
+// (32 x 7), 500x300 128 -> 63.6 (32 x 16), 2048^2 1832 -> 1553 (32 x 13: the
+// Riemann solves of 13 rows fill their last round of warps, those of 16 do
+// not: 1580).
+void choose_f64_tile(int nx, int ny, int tile, int *shape, int *ty) {
+  struct Info {
+    int tx, most, warps, resident;
+  };
+  auto info = [](int sh) {
+    Info i{};
+    with_shape(sh, [&](auto s) {
+      using S = decltype(s);
+      i = Info{S::TX, S::TYM, S::NT / 32, S::MINB};
+    });
+    return i;
+  };
+  if (tile >= 0) {
+    *shape = tile % 100 < kShapes ? tile % 100 : 0;
+    const int m = info(*shape).most;
+    *ty = tile >= 100 && tile / 100 < m ? tile / 100 : m;
+    return;
+  }
+  static const double lat[kShapes][3] = {{4.47, 2.49, 2.29}, {3.65, 3.30, 2.25}, {4.34, 1.87, 5.41}};  // us
+  constexpr double kSms = 152.0, kFixed = 4.3, kInst = 0.005, kExp = 1.26;
+  auto up = [](int a, int b) { return (a + b - 1) / b; };
+  double best = 0.0;
+  for (int sh = 0; sh < kShapes; ++sh) {
+    const Info i = info(sh);
+    for (int y = 3; y <= i.most; ++y) {
+      const int w[3] = {up((i.tx + 2) * (y + 2) - 4, 32), up((i.tx + 1) * y + i.tx * (y + 1), 32), up(i.tx * y, 32)};
+      const double inst = kInst * (80 * w[0] + 50 * w[1] + 34 * w[2]);
+      double alone = 0.0;
+      for (int k = 0; k < 3; ++k) alone += up(w[k], i.warps) * lat[sh][k];
+      auto wave = [&](double k) { return std::pow(std::pow(alone, kExp) + std::pow(k * inst, kExp), 1.0 / kExp); };
+      const double tiles = (double)up(nx, i.tx) * up(ny, y), per_wave = kSms * i.resident;
+      const double full = std::floor(tiles / per_wave), rest = tiles - full * per_wave;
+      const double t = full >= 4 ? wave(i.resident) * tiles / per_wave + 0.5 * wave(1)
+                                 : full * wave(i.resident) + (rest > 0 ? wave(std::ceil(rest / kSms)) : 0.0);
+      if (best == 0.0 || kFixed + t < best) {
+        best = kFixed + t;
+        *shape = sh;
+        *ty = y;
+      }
+    }
+  }
 }
 
 template <int RS>
 static cudaError_t launch_flux_t(const KParams64 &kp, const double *q, const double *u_in,
                                  double *u_out, DevClock *clk, int use_clock, double host_dt,
                                  double *dt_trace, cudaStream_t s) {
-  if (kp.tile == 1)
-    return launch_flux_shape<RS, 32, 16, 256, 2>(kp, q, u_in, u_out, clk, use_clock, host_dt, dt_trace, s);
-  return launch_flux_shape<RS, 32, 32, 512, 1>(kp, q, u_in, u_out, clk, use_clock, host_dt, dt_trace, s);
-}
-
-template <int RS, int TX, int TY, int NT, int MINB>
-static cudaError_t set_flux_smem() {
-  return cudaFuncSetAttribute(k_flux_update_f64<RS, TX, TY, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)flux_smem_bytes<TX, TY>());
-}
-
-template <int RS, int TX, int TY, int NT, int MINB, bool FAST = false>
-static cudaError_t set_step_smem() {
-  return cudaFuncSetAttribute(k_step_f64<RS, TX, TY, NT, MINB, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)step_smem_bytes<TX, TY>());
+  with_shape(kp.shape, [&](auto sh) {
+    using S = decltype(sh);
+    dim3 grid((kp.g.nx + S::TX - 1) / S::TX, (kp.g.ny + kp.ty - 1) / kp.ty);
+    k_flux_update_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL><<<grid, S::NT, flux_smem_bytes<S::TX, S::TYM>(), s>>>(
+        kp, q, u_in, u_out, clk, use_clock, host_dt, dt_trace);
+  });
+  return cudaGetLastError();
 }
 
 template <int RS>
 static cudaError_t configure_rs() {
-  cudaError_t e = set_flux_smem<RS, 32, 32, 512, 1>();
-  if (e == cudaSuccess) e = set_flux_smem<RS, 32, 16, 256, 2>();
-  if (e == cudaSuccess) e = set_step_smem<RS, 32, 32, 512, 1>();
-  if (e == cudaSuccess) e = set_step_smem<RS, 32, 16, 256, 2>();
-  if (e == cudaSuccess) e = set_step_smem<RS, 32, 31, 512, 1>();
-  if (e == cudaSuccess) e = set_step_smem<RS, 32, 15, 256, 2>();
-  if (e == cudaSuccess) e = set_step_smem<RS, 32, 32, 512, 1, true>();
-  if (e == cudaSuccess) e = set_step_smem<RS, 32, 16, 256, 2, true>();
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < kShapes; ++k)
+    with_shape(k, [&](auto sh) {
+      using S = decltype(sh);
+      constexpr int step = (int)step_smem_bytes<S::TX, S::TYM>(), flux = (int)flux_smem_bytes<S::TX, S::TYM>();
+      constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux_update_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL>, attr, flux);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>, attr, step);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>, attr, step);
+    });
   return e;
 }
 
 template <int RS>
 static cudaError_t set_batch_flux_smem() {
   return cudaFuncSetAttribute(k_batch_step_f64<RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)step_smem_bytes<32, 32>());
+                              (int)step_smem_bytes<BTX, BTY>());
 }
 
 cudaError_t configure_f64_kernels() {
@@ -932,11 +1046,12 @@ cudaError_t configure_f64_kernels() {
   return e;
 }
 
-void batch_f64_shape(const KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles) {
+void batch_f64_shape(KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles) {
   *nbx = (kp.g.isize + FILL_BX - 1) / FILL_BX;
   *nfill = *nbx * ((kp.g.jsize + FILL_BY - 1) / FILL_BY);
-  *ntx = (kp.g.nx + 31) / 32;
-  *ntiles = *ntx * ((kp.g.ny + 31) / 32);
+  kp.ty = BTY;
+  *ntx = (kp.g.nx + BTX - 1) / BTX;
+  *ntiles = *ntx * ((kp.g.ny + kp.ty - 1) / kp.ty);
 }
 
 cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s) {
@@ -947,17 +1062,17 @@ cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s)
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
                              int n_inst, int total_tiles, int grid_blocks, cudaStream_t s) {
   if (n_inst <= 0 || total_tiles <= 0) return cudaSuccess;
-  const size_t sm = step_smem_bytes<32, 32>();
+  const size_t sm = step_smem_bytes<BTX, BTY>();
   const int grid = grid_blocks < total_tiles ? grid_blocks : total_tiles;
   switch (riemann) {
     case E2D_RIEMANN_HLLC:
-      k_batch_step_f64<E2D_RIEMANN_HLLC><<<grid, 512, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
+      k_batch_step_f64<E2D_RIEMANN_HLLC><<<grid, BNT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
       break;
     case E2D_RIEMANN_HLL:
-      k_batch_step_f64<E2D_RIEMANN_HLL><<<grid, 512, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
+      k_batch_step_f64<E2D_RIEMANN_HLL><<<grid, BNT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
       break;
     default:
-      k_batch_step_f64<E2D_RIEMANN_APPROX><<<grid, 512, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
+      k_batch_step_f64<E2D_RIEMANN_APPROX><<<grid, BNT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
       break;
   }
   return cudaGetLastError();
@@ -977,39 +1092,22 @@ cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const doubl
   }
 }
 
-// Fused-step tile shapes (kp.tile): 32 x 32 cells, 512 threads, one block
-// per SM (the default); 1 -> 32 x 16, 256 threads, two blocks per SM (0.6 %
-// slower per 4096^2 HLLC step: 5 % more instructions per cell for the halo,
-// the FP64 pipe 86 % instead of 82 % busy); 2 -> 32 x 31 (2047 Riemann
-// solves: four full rounds of 512 threads); 3 -> 32 x 15 (two blocks per SM,
-// 1007 solves: four rounds of 256).  The fast forms exist for 32 x 32 and
-// 32 x 16.  Results do not depend on the shape.
-template <int RS, int TX, int TY, int NT, int MINB, bool FAST = false>
-static cudaError_t launch_step_shape(const KParams64 &kp, const CUtensorMap &tm_q, int use_tma, const double *q_in,
-                                     double *q_out, double *u_in, double *u_out, DevClock *clk, double *dt_trace,
-                                     cudaStream_t s) {
-  dim3 grid((kp.g.nx + TX - 1) / TX, (kp.g.ny + TY - 1) / TY);
-  k_step_f64<RS, TX, TY, NT, MINB, FAST><<<grid, NT, step_smem_bytes<TX, TY>(), s>>>(kp, tm_q, use_tma, q_in, q_out,
-                                                                                      u_in, u_out, clk, dt_trace);
-  return cudaGetLastError();
-}
-
 template <int RS>
 static cudaError_t launch_step_t(const KParams64 &kp, const CUtensorMap &tm_q, int use_tma, const double *q_in,
                                  double *q_out, double *u_in, double *u_out, DevClock *clk, double *dt_trace,
                                  cudaStream_t s) {
-  if (kp.fast) {  // the fast forms: 32 x 32 (default) and 32 x 16 tiles
-    if (kp.tile == 1)
-      return launch_step_shape<RS, 32, 16, 256, 2, true>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace,
-                                                         s);
-    return launch_step_shape<RS, 32, 32, 512, 1, true>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace, s);
-  }
-  switch (kp.tile) {
-    case 1: return launch_step_shape<RS, 32, 16, 256, 2>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace, s);
-    case 2: return launch_step_shape<RS, 32, 31, 512, 1>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace, s);
-    case 3: return launch_step_shape<RS, 32, 15, 256, 2>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace, s);
-    default: return launch_step_shape<RS, 32, 32, 512, 1>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace, s);
-  }
+  with_shape(kp.shape, [&](auto sh) {
+    using S = decltype(sh);
+    dim3 grid((kp.g.nx + S::TX - 1) / S::TX, (kp.g.ny + kp.ty - 1) / kp.ty);
+    constexpr size_t sm = step_smem_bytes<S::TX, S::TYM>();
+    if (kp.fast)
+      k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>
+          <<<grid, S::NT, sm, s>>>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace);
+    else
+      k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>
+          <<<grid, S::NT, sm, s>>>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace);
+  });
+  return cudaGetLastError();
 }
 
 cudaError_t launch_step_f64(const KParams64 &kp, int riemann, const CUtensorMap &tm_q, int use_tma,
@@ -1026,7 +1124,7 @@ cudaError_t launch_step_f64(const KParams64 &kp, int riemann, const CUtensorMap 
 }
 
 // The box of the fused step's primitives tile for the tile shape of kp:
-// dimensions (isize, jsize, 4 planes), box (TX + 4) x (TY + 4) x 4.  Row and
+// dimensions (isize, jsize, 4 planes), box (TX + 4) x (ty + 4) x 4.  Row and
 // plane strides must be multiples of 16 bytes, so isize must be even; false
 // (tiles are then gathered) otherwise or if the driver cannot encode it.
 bool encode_q_map(CUtensorMap *map, const double *q, const KParams64 &kp) {
@@ -1039,10 +1137,11 @@ bool encode_q_map(CUtensorMap *map, const double *q, const KParams64 &kp) {
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   }();
   if (!encode || (kp.g.isize & 1) || (reinterpret_cast<uintptr_t>(q) & 15u)) return false;
-  const int ty = kp.tile == 1 ? 16 : kp.tile == 2 && !kp.fast ? 31 : kp.tile == 3 && !kp.fast ? 15 : 32;
   const cuuint64_t dims[3] = {(cuuint64_t)kp.g.isize, (cuuint64_t)kp.g.jsize, 4};
   const cuuint64_t strides[2] = {(cuuint64_t)kp.g.isize * sizeof(double), (cuuint64_t)kp.g.plane * sizeof(double)};
-  const cuuint32_t box[3] = {32 + 4, (cuuint32_t)ty + 4, 4};
+  int tx = 0;
+  with_shape(kp.shape, [&](auto sh) { tx = decltype(sh)::TX; });
+  const cuuint32_t box[3] = {(cuuint32_t)tx + 4, (cuuint32_t)kp.ty + 4, 4};
   const cuuint32_t estr[3] = {1, 1, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(q), dims, strides, box, estr,
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

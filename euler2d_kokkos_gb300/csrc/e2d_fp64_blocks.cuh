@@ -23,7 +23,7 @@ using f64x::min_any;
 __device__ __forceinline__ int src_lo_hi(int i, int n, int bc_lo, int bc_hi, bool &flip) {
   return ghost_source(i, n, bc_lo, bc_hi, flip);
 }
-__device__ __forceinline__ bool nonfinite(double x) { return nonfinite64(x); }
+__device__ __forceinline__ bool nonfinite(double x) { return (f64i::high(x) & 0x7ff00000u) == 0x7ff00000u; }
 
 // ------------------------------------------------------------ numerics
 using f64x::divisor;
@@ -37,15 +37,18 @@ using f64x::root;
 // certain when they differ by more than smallp's exponent plus two; only then
 // is the product not formed (one FP64 instruction of the two each face state
 // would take; every cell of an ordinary flow).
-__device__ __forceinline__ double floor_pressure(const Fp &f, const KPhys<double> &ph, double p, double d) {
-  const int lim = (__double2hiint(ph.smallp) & 0x7ff00000) - (1020 << 20);  // (exponent + 3) 2^20
-  if (__double2hiint(p) >= 0x00100000 && __double2hiint(p) - __double2hiint(d) > lim) return p;
+template <class F>
+__device__ __forceinline__ double floor_pressure(const F &f, const KPhys<double> &ph, double p, double d) {
+  const int lim = (int)(f64i::high(ph.smallp) & 0x7ff00000u) - (1020 << 20);  // (exponent + 3) 2^20
+  const int hp = (int)f64i::high(p), hd = (int)f64i::high(d);
+  if (hp >= 0x00100000 && hp - hd > lim) return p;
   return max_pos(p, f.mul(d, ph.smallp));
 }
 
 // src/HydroBaseFunctor.h:76-102 (computePrimitives) without the sound speed.
 // `dv`: the density, ready as a divisor.
-__device__ __forceinline__ void primitives(const Fp &f, const KPhys<double> &ph, double rho, double e, double mx,
+template <class F>
+__device__ __forceinline__ void primitives(const F &f, const KPhys<double> &ph, double rho, double e, double mx,
                                            double my, double &d, double &p, double &ux, double &uy, Divisor &dv) {
   d = max_pos(rho, ph.smallr);
   dv = divisor(d);
@@ -57,19 +60,28 @@ __device__ __forceinline__ void primitives(const Fp &f, const KPhys<double> &ph,
 }
 
 // src/HydroBaseFunctor.h:475-516 for one variable and direction: slope_type
-// 0 gives a zero slope, 1 and 2 the limited slope.
-__device__ __forceinline__ double slope(const Fp &f, int st_kind, double q, double qp, double qm) {
-  if (st_kind == 0) return 0.0;
-  return f64x::slope_limited(f, st_kind == 2, q, qp, qm);
+// 0 gives a zero slope, 1 and 2 the limited slope.  h: half of it.
+template <class F>
+__device__ __forceinline__ void slope(const F &f, int st_kind, double q, double qp, double qm, double &dq, double &h) {
+  dq = h = 0.0;
+  if (st_kind != 0) f64x::slope_limited(f, st_kind == 2, q, qp, qm, dq, h);
+}
+template <class F>
+__device__ __forceinline__ double slope(const F &f, int st_kind, double q, double qp, double qm) {
+  double dq, h;
+  slope(f, st_kind, q, qp, qm, dq, h);
+  return dq;
 }
 
 // Sources of trace_unsplit_2d_along_dir (src/HydroBaseFunctor.h:246-249).
-__device__ __forceinline__ void trace_sources(const Fp &f, const KPhys<double> &ph, const double q[4],
+template <class F>
+__device__ __forceinline__ void trace_sources(const F &f, const KPhys<double> &ph, const double q[4],
                                               const double dqx[4], const double dqy[4], double s0[4]) {
   const double r = q[E2D_ID], p = q[E2D_IP], u = q[E2D_IU], v = q[E2D_IV];
   const Divisor dr = divisor(r);
   const double div = f.add(dqx[E2D_IU], dqy[E2D_IV]);
-  auto advect = [&](int k) { return f.sub(f.mul(-u, dqx[k]), f.mul(v, dqy[k])); };  // -u*dqx - v*dqy
+  const double nu = f.neg(u);
+  auto advect = [&](int k) { return f.sub(f.xmul(nu, dqx[k]), f.xmul(v, dqy[k])); };  // -u*dqx - v*dqy
   s0[E2D_ID] = f.sub(advect(E2D_ID), f.mul(div, r));
   s0[E2D_IP] = f.sub(advect(E2D_IP), f.mul(f.mul(div, ph.gamma0), p));
   s0[E2D_IU] = f.sub(advect(E2D_IU), quot(dqx[E2D_IP], dr));
@@ -78,11 +90,11 @@ __device__ __forceinline__ void trace_sources(const Fp &f, const KPhys<double> &
 
 // The two face states of one direction (src/HydroBaseFunctor.h:251-289):
 // minus face q - dq/2 + s0*dtd/2, plus face q + dq/2 + s0*dtd/2, density
-// clamped at smallr.
-__device__ __forceinline__ void face_pair(const Fp &f, const KPhys<double> &ph, int v, double q, double dq,
-                                          double s0, double dtd, double &fm, double &fp) {
-  const double h = half(dq);
-  const double sx = half(f.mul(s0, dtd));
+// clamped at smallr.  h = dq/2, hdtd = dtd/2.
+template <class F>
+__device__ __forceinline__ void face_pair(const F &f, const KPhys<double> &ph, int v, double q, double h,
+                                          double s0, double dtd, double hdtd, double &fm, double &fp) {
+  const double sx = f.half_product(s0, dtd, hdtd);
   fm = f.add(f.sub(q, h), sx);
   fp = f.add(f.add(q, h), sx);
   if (v == E2D_ID) {
@@ -92,7 +104,8 @@ __device__ __forceinline__ void face_pair(const Fp &f, const KPhys<double> &ph, 
 }
 
 // src/HydroBaseFunctor.h:523-547.
-__device__ __forceinline__ void cmpflx(const Fp &o, const KPhys<double> &ph, const double g[4], double f[4]) {
+template <class F>
+__device__ __forceinline__ void cmpflx(const F &o, const KPhys<double> &ph, const double g[4], double f[4]) {
   f[E2D_ID] = o.mul(g[E2D_ID], g[E2D_IU]);
   f[E2D_IU] = o.add(o.mul(f[E2D_ID], g[E2D_IU]), g[E2D_IP]);
   f[E2D_IV] = o.mul(f[E2D_ID], g[E2D_IV]);
@@ -107,7 +120,8 @@ __device__ __forceinline__ double fmax_any(double a, double b) {
 }
 
 // src/HydroBaseFunctor.h:558-693 (riemann_approx).
-__device__ __noinline__ void riemann_approx(const Fp &f, const KPhys<double> &ph, const double *ql,
+template <class F>
+__device__ __noinline__ void riemann_approx(const F &f, const KPhys<double> &ph, const double *ql,
                                             const double *qr, double *flux) {
   const double gamma0 = ph.gamma0, gamma6 = ph.gamma6;
   const double rl = fmax_any(ql[E2D_ID], ph.smallr), ul = ql[E2D_IU];
@@ -137,9 +151,9 @@ __device__ __noinline__ void riemann_approx(const Fp &f, const KPhys<double> &ph
     const double qxr = quot(f.mul(f.mul(f64x::twice(wwr), wwr), wwr), f.add(w2r, cr));
     const double usl = f.sub(ul, quot(f.sub(pold, pl), wwl));
     const double usr = f.add(ur, quot(f.sub(pold, pr), wwr));
-    const double delp = fmax_any(f.mul(quot(f.mul(qxr, qxl), f.add(qxr, qxl)), f.sub(usl, usr)), -pold);
+    const double delp = fmax_any(f.mul(quot(f.mul(qxr, qxl), f.add(qxr, qxl)), f.sub(usl, usr)), f.neg(pold));
     pold = f.add(pold, delp);
-    conv = fabs(quot(delp, f.add(pold, ph.smallpp)));
+    conv = f.abs(quot(delp, f.add(pold, ph.smallpp)));
   }
   pstar = pold;
   wl = wave(cl, pstar, pl, dpl);
@@ -147,13 +161,13 @@ __device__ __noinline__ void riemann_approx(const Fp &f, const KPhys<double> &ph
   const double ustar =
       half(f.sub(f.add(f.add(ul, quot(f.sub(pl, pstar), wl)), ur), quot(f.sub(pr, pstar), wr)));
   const bool lft = f64x::sbits(ustar) >= 0;  // copysign(1, ustar) > 0
-  auto signed_by = [&](double x) { return lft ? x : -x; };  // sgnm * x
+  auto signed_by = [&](double x) { return lft ? x : f.neg(x); };  // sgnm * x
   const double ro = lft ? rl : rr, uo = lft ? ul : ur, po = lft ? pl : pr, wo = lft ? wl : wr;
   const Divisor dro = divisor(ro);
-  const double co = fmax_any(ph.smallc, root(fabs(quot(f.mul(gamma0, po), dro))));
+  const double co = fmax_any(ph.smallc, root(f.abs(quot(f.mul(gamma0, po), dro))));
   const double rstar = fmax_any(
       quot(ro, f.add(f.one, quot(f.mul(ro, f.sub(po, pstar)), f.mul(wo, wo)))), ph.smallr);
-  const double cstar = fmax_any(ph.smallc, root(fabs(quot(f.mul(gamma0, pstar), rstar))));
+  const double cstar = fmax_any(ph.smallc, root(f.abs(quot(f.mul(gamma0, pstar), rstar))));
   double spout = f.sub(co, signed_by(uo));
   double spin = f.sub(cstar, signed_by(ustar));
   const double ushock = f.sub(quot(wo, dro), signed_by(uo));
@@ -162,7 +176,7 @@ __device__ __noinline__ void riemann_approx(const Fp &f, const KPhys<double> &ph
     spout = ushock;
   }
   const double spsum = f.add(spout, spin);
-  const double scr = fmax_any(f.sub(spout, spin), f.add(ph.smallc, fabs(spsum)));
+  const double scr = fmax_any(f.sub(spout, spin), f.add(ph.smallc, f.abs(spsum)));
   double frac = half(f.add(f.one, quot(spsum, scr)));
   if (f64x::is_nan(frac))
     frac = 0.0;
@@ -194,7 +208,8 @@ __device__ __noinline__ void riemann_approx(const Fp &f, const KPhys<double> &ph
 // larger square (a correctly rounded root is monotonic): the same values.
 // Cut-offs, maxima, the 0.5 factors and the sign tests use the exact integer
 // forms of e2d_f64_exact.cuh.
-__device__ __forceinline__ void riemann_hllc(const Fp &f, const KPhys<double> &ph, const double *ql,
+template <class F>
+__device__ __forceinline__ void riemann_hllc(const F &f, const KPhys<double> &ph, const double *ql,
                                              const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
   const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
@@ -210,16 +225,16 @@ __device__ __forceinline__ void riemann_hllc(const Fp &f, const KPhys<double> &p
   const double rcl = f.mul(rl, f.sub(ul, SL));
   const double rcr = f.mul(rr, f.sub(SR, ur));
   const Divisor rc = divisor(f.add(rcr, rcl));
-  const double ustar = quot(f.add(f.add(f.mul(rcr, ur), f.mul(rcl, ul)), f.sub(pl, pr)), rc);
+  const double ustar = quot(f.add(f.add(f.xmul(rcr, ur), f.xmul(rcl, ul)), f.sub(pl, pr)), rc);
   const double ptotstar =
-      quot(f.add(f.add(f.mul(rcr, pl), f.mul(rcl, pr)), f.mul(f.mul(rcl, rcr), f.sub(ul, ur))), rc);
+      quot(f.add(f.add(f.xmul(rcr, pl), f.xmul(rcl, pr)), f.mul(f.mul(rcl, rcr), f.sub(ul, ur))), rc);
   const bool own_l = gt0(SL);
   const bool lft = own_l || gt0(ustar);
   const bool own = own_l || !(lft || gt0(SR));
   const double S = lft ? SL : SR;
   const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr, vs = lft ? ql[E2D_IV] : qr[E2D_IV];
   const double hrs = half(rs);
-  const double es = f.add(f.mul(ps, ph.entho), f.add(f.mul(f.mul(hrs, us), us), f.mul(f.mul(hrs, vs), vs)));
+  const double es = f.add(f.xmul(ps, ph.entho), f.add(f.xmul(f.xmul(hrs, us), us), f.xmul(f.xmul(hrs, vs), vs)));
   const double sdu = f.sub(S, us);
   const Divisor sds = divisor(f.sub(S, ustar));
   const double rstar = quot(f.mul(rs, sdu), sds);
@@ -237,7 +252,8 @@ __device__ __forceinline__ void riemann_hllc(const Fp &f, const KPhys<double> &p
 // RIEMANN_HLL but has no solver; this uses riemann_hllc's cut-offs and Davis
 // wave speeds; the star flux multiplies by one reciprocal of SR - SL.
 // Operation order matches the oracle's riemann_hll.
-__device__ __forceinline__ void riemann_hll(const Fp &f, const KPhys<double> &ph, const double *ql,
+template <class F>
+__device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph, const double *ql,
                                             const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
   const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
@@ -282,8 +298,8 @@ __device__ __forceinline__ void riemann_hll(const Fp &f, const KPhys<double> &ph
   }
 }
 
-template <int RS>
-__device__ __forceinline__ void riemann(const Fp &f, const KPhys<double> &ph, const double *ql, const double *qr,
+template <int RS, class F>
+__device__ __forceinline__ void riemann(const F &f, const KPhys<double> &ph, const double *ql, const double *qr,
                                         double *flux) {
   if (RS == E2D_RIEMANN_HLLC)
     riemann_hllc(f, ph, ql, qr, flux);
@@ -296,11 +312,12 @@ __device__ __forceinline__ void riemann(const Fp &f, const KPhys<double> &ph, co
 // CFL wave-speed term of a cell from its primitives (src/HydroRunFunctors.h:56-72):
 // (c + |u|) / dx + (c + |v|) / dy, c = sqrt(gamma p / d); a division by a
 // power-of-two dx, dy is the exact product by its reciprocal.
-__device__ __forceinline__ double cfl_term(const Fp &f, const KPhys<double> &ph, const Divisor &dd, double p,
+template <class F>
+__device__ __forceinline__ double cfl_term(const F &f, const KPhys<double> &ph, const Divisor &dd, double p,
                                            double ux, double uy) {
   const double c = root(quot(f.mul(ph.gamma0, p), dd));
-  const double vx = f.add(c, fabs(ux));
-  const double vy = f.add(c, fabs(uy));
+  const double vx = f.add(c, f.abs(ux));
+  const double vy = f.add(c, f.abs(uy));
   const double tx = ph.inv_dx_pow2 != 0.0 ? f.mul(vx, ph.inv_dx_pow2) : quot(vx, ph.dx);
   const double ty = ph.inv_dy_pow2 != 0.0 ? f.mul(vy, ph.inv_dy_pow2) : quot(vy, ph.dy);
   return f.add(tx, ty);
@@ -321,7 +338,8 @@ __device__ __forceinline__ unsigned int state_flags(double rho, double e, double
 // no FP64 instruction, so they stay as they are).  Results differ from the
 // reference's by rounding (not bit-identical); the tests hold them to 1e-12
 // on dt and 1e-10 relative L1.
-__device__ __forceinline__ void primitives_fast(const Fp &f, const KPhys<double> &ph, double rho, double e,
+template <class F>
+__device__ __forceinline__ void primitives_fast(const F &f, const KPhys<double> &ph, double rho, double e,
                                                 double mx, double my, double &d, double &p, double &ux, double &uy,
                                                 Divisor &dv) {
   d = max_pos(rho, ph.smallr);
@@ -332,22 +350,22 @@ __device__ __forceinline__ void primitives_fast(const Fp &f, const KPhys<double>
   p = floor_pressure(f, ph, f.mul(f.mul(ph.gm1, d), ei), d);
 }
 
-__device__ __forceinline__ void trace_sources_fast(const Fp &f, const KPhys<double> &ph, const double q[4],
+template <class F>
+__device__ __forceinline__ void trace_sources_fast(const F &f, const KPhys<double> &ph, const double q[4],
                                                    const double dqx[4], const double dqy[4], double s0[4]) {
   const double r = q[E2D_ID], p = q[E2D_IP], u = q[E2D_IU], v = q[E2D_IV];
   const Divisor dr = divisor(r);
-  const double div = f.add(dqx[E2D_IU], dqy[E2D_IV]);
-  s0[E2D_ID] = fma(-u, dqx[E2D_ID], fma(-v, dqy[E2D_ID], f.mul(-div, r)));
-  s0[E2D_IP] = fma(-u, dqx[E2D_IP], fma(-v, dqy[E2D_IP], f.mul(f.mul(-div, ph.gamma0), p)));
-  s0[E2D_IU] = fma(-u, dqx[E2D_IU], fma(-v, dqy[E2D_IU], -quot(dqx[E2D_IP], dr)));
-  s0[E2D_IV] = fma(-u, dqx[E2D_IV], fma(-v, dqy[E2D_IV], -quot(dqy[E2D_IP], dr)));
+  const double nu = f.neg(u), nv = f.neg(v), ndiv = f.neg(f.add(dqx[E2D_IU], dqy[E2D_IV]));
+  s0[E2D_ID] = fma(nu, dqx[E2D_ID], fma(nv, dqy[E2D_ID], f.mul(ndiv, r)));
+  s0[E2D_IP] = fma(nu, dqx[E2D_IP], fma(nv, dqy[E2D_IP], f.mul(f.mul(ndiv, ph.gamma0), p)));
+  s0[E2D_IU] = fma(nu, dqx[E2D_IU], fma(nv, dqy[E2D_IU], f.neg(quot(dqx[E2D_IP], dr))));
+  s0[E2D_IV] = fma(nu, dqx[E2D_IV], fma(nv, dqy[E2D_IV], f.neg(quot(dqy[E2D_IP], dr))));
 }
 
-// face_pair() with hdtd = dt/dx / 2 (or dt/dy / 2).
-__device__ __forceinline__ void face_pair_fast(const Fp &f, const KPhys<double> &ph, int v, double q, double dq,
+template <class F>
+__device__ __forceinline__ void face_pair_fast(const F &f, const KPhys<double> &ph, int v, double q, double h,
                                                double s0, double hdtd, double &fm, double &fp) {
   const double qs = fma(s0, hdtd, q);
-  const double h = half(dq);
   fm = f.sub(qs, h);
   fp = f.add(qs, h);
   if (v == E2D_ID) {
@@ -357,7 +375,8 @@ __device__ __forceinline__ void face_pair_fast(const Fp &f, const KPhys<double> 
 }
 
 // riemann_hllc() with FMAs.
-__device__ __forceinline__ void riemann_hllc_fast(const Fp &f, const KPhys<double> &ph, const double *ql,
+template <class F>
+__device__ __forceinline__ void riemann_hllc_fast(const F &f, const KPhys<double> &ph, const double *ql,
                                                   const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
   const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
@@ -384,7 +403,7 @@ __device__ __forceinline__ void riemann_hllc_fast(const Fp &f, const KPhys<doubl
   const double sdu = f.sub(S, us);
   const Divisor sds = divisor(f.sub(S, ustar));
   const double rstar = quot(f.mul(rs, sdu), sds);
-  const double etotstar = quot(fma(sdu, es, fma(-ps, us, f.mul(ptotstar, ustar))), sds);
+  const double etotstar = quot(fma(sdu, es, fma(f.neg(ps), us, f.mul(ptotstar, ustar))), sds);
   const double ro = own ? rs : rstar, uo = own ? us : ustar, ptoto = own ? ps : ptotstar;
   const double etoto = own ? es : etotstar;
   flux[E2D_ID] = f.mul(ro, uo);
@@ -394,7 +413,8 @@ __device__ __forceinline__ void riemann_hllc_fast(const Fp &f, const KPhys<doubl
 }
 
 // riemann_hll() with FMAs.
-__device__ __forceinline__ void riemann_hll_fast(const Fp &f, const KPhys<double> &ph, const double *ql,
+template <class F>
+__device__ __forceinline__ void riemann_hll_fast(const F &f, const KPhys<double> &ph, const double *ql,
                                                  const double *qr, double *flux) {
   const double rl = max_pos(ql[E2D_ID], ph.smallr);
   const double pl = floor_pressure(f, ph, ql[E2D_IP], rl);
@@ -424,12 +444,12 @@ __device__ __forceinline__ void riemann_hll_fast(const Fp &f, const KPhys<double
     const double rden = quot(f.one, f.sub(SR, SL));
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      flux[v] = f.mul(fma(sls, f.sub(UR[v], UL[v]), fma(SR, FL[v], f.mul(-SL, FR[v]))), rden);
+      flux[v] = f.mul(fma(sls, f.sub(UR[v], UL[v]), fma(SR, FL[v], f.mul(f.neg(SL), FR[v]))), rden);
   }
 }
 
-template <int RS, bool FAST>
-__device__ __forceinline__ void riemann_sel(const Fp &f, const KPhys<double> &ph, const double *ql,
+template <int RS, bool FAST, class F>
+__device__ __forceinline__ void riemann_sel(const F &f, const KPhys<double> &ph, const double *ql,
                                             const double *qr, double *flux) {
   if (FAST && RS == E2D_RIEMANN_HLLC)
     riemann_hllc_fast(f, ph, ql, qr, flux);
@@ -439,10 +459,11 @@ __device__ __forceinline__ void riemann_sel(const Fp &f, const KPhys<double> &ph
     riemann<RS>(f, ph, ql, qr, flux);
 }
 
-__device__ __forceinline__ double cfl_term_fast(const Fp &f, const KPhys<double> &ph, const Divisor &dd, double p,
+template <class F>
+__device__ __forceinline__ double cfl_term_fast(const F &f, const KPhys<double> &ph, const Divisor &dd, double p,
                                                 double ux, double uy) {
   const double c = root(quot(f.mul(ph.gamma0, p), dd));
-  return fma(f.add(c, fabs(ux)), ph.inv_dx, f.mul(f.add(c, fabs(uy)), ph.inv_dy));
+  return fma(f.add(c, f.abs(ux)), ph.inv_dx, f.mul(f.add(c, f.abs(uy)), ph.inv_dy));
 }
 
 // dt of a step from the CFL maximum (src/main.cpp:128-134).

@@ -66,7 +66,8 @@ __device__ __forceinline__ void cell_faces(const Fp &f, const KPhys<double> &ph,
   trace_sources(f, ph, qc, dqx, dqy, s0);
 #pragma unroll
   for (int v = 0; v < 4; ++v)
-    face_pair(f, ph, v, qc[v], xdir ? dqx[v] : dqy[v], s0[v], xdir ? dtdx : dtdy, fm[v], fp[v]);
+    face_pair(f, ph, v, qc[v], half(xdir ? dqx[v] : dqy[v]), s0[v], xdir ? dtdx : dtdy, half(xdir ? dtdx : dtdy), fm[v],
+              fp[v]);
 }
 
 // Scaled flux through the face between the left/lower state ql and the

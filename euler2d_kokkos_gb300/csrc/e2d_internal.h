@@ -58,8 +58,7 @@ struct KPhys {
 struct KParams64 {
   KGeom g;
   KPhys<double> ph;
-  int tile;       // tile shape: -1 the default (32 x 32), else see launch_step_f64 and
-                  // launch_flux_update_f64
+  int shape, ty;  // tile shape of the step and its rows (choose_f64_tile)
   int fast;       // E2D_PRECISION_FP64_FAST: the fused step's fast forms (not bit-identical)
   int wait_test;  // nonzero: tile (1, 1) of the fused step never stages its primitives,
                   // so its bounded wait runs out (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
@@ -145,6 +144,9 @@ cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const doubl
                                    const double *u_in, double *u_out, DevClock *clk,
                                    int use_clock, double host_dt, double *dt_trace,
                                    cudaStream_t s);
+// Tile shape and rows of a grid (e2d_fp64.cu); tile >= 0 forces shape
+// tile % 100 with tile / 100 rows (0: the shape's most).
+void choose_f64_tile(int nx, int ny, int tile, int *shape, int *ty);
 // Sets the kernels' shared-memory limits; call once per device before any
 // launch or graph capture.
 cudaError_t configure_f64_kernels();
@@ -222,8 +224,8 @@ cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s)
 // total_tiles).
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
                              int n_inst, int total_tiles, int grid_blocks, cudaStream_t s);
-// Fill blocks and flux tiles of an FP64 instance.
-void batch_f64_shape(const KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles);
+// Fill blocks and tiles of an FP64 instance; sets its tile rows.
+void batch_f64_shape(KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles);
 
 // One iteration over every strip of every listed instance: list entry k is
 // table slot list_slots[k]; strip_begin[k] is its first global strip

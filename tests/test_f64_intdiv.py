@@ -1,5 +1,5 @@
-"""Integer-pipe FP64 division and square root (csrc/e2d_f64_intdiv.h): bit for
-bit the IEEE operations, on the host build of the header (CPU) and through the
+"""Integer-pipe FP64 division, square root and product (csrc/e2d_f64_intdiv.h):
+bit for bit the IEEE operations, on the host build of the header (CPU) and through the
 device's primitives block (GPU)."""
 import os
 import shutil
@@ -42,6 +42,9 @@ int main() {
     refused += !ok;
     bad += ok && bits(q) != bits(t);
     const double x = std::fabs(a), y = b * b;
+    const double pr = product(a, b, ok);
+    refused += !ok;
+    bad += ok && bits(pr) != bits(a * b);
     for (double z : {x, y, std::nextafter(y, 0.0), std::nextafter(y, 1e300)}) {
       const double s = root(z, ok);
       bad += ok && bits(s) != bits(std::sqrt(z));
@@ -54,6 +57,11 @@ int main() {
   for (double a : {1e-310, (double)INFINITY, (double)NAN}) quotient(a, divisor(1.5), ok), any |= ok;
   quotient(1e300, divisor(1e-140), ok), any |= ok;
   quotient(1e-300, divisor(1e140), ok), any |= ok;
+  product(1e-200, 1e-200, ok), any |= ok;
+  product(1e200, -1e200, ok), any |= ok;
+  product(1e-310, 1.5, ok), any |= ok;
+  product(0.0, (double)INFINITY, ok), any |= ok;
+  product(1.0, (double)NAN, ok), any |= ok;
   for (double x : {0.0, -1.0, -0.0, 1e-310, 1e300, (double)INFINITY, (double)NAN}) root(x, ok), any |= ok;
   std::printf("%ld %ld %d\n", bad, refused, any ? 1 : 0);
   return 0;
