@@ -4,6 +4,7 @@
 #include "e2d_internal.h"
 
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -27,6 +28,7 @@ struct e2d_sim {
   CUtensorMap QTM[2];                 // FP64: TMA maps of Q[0], Q[1] (fused step's tile staging)
   int q_tma = 0;                      // FP64: both maps encoded (isize even)
   int f64_split = 0;                  // FP64 device loop as two launches per step (E2D_F64_SPLIT=1)
+  int loop_blocks = 0;                // blocks of a multi-step launch (0: one launch per step)
   int impl = 0;                       // FP64: implementationVersion (1, 2: the debug orchestrations)
   // FP64 fused step: the parity whose primitives (Q[par], interior) and CFL
   // maximum (q_acc) on the device are those of U[par] as the last device-loop
@@ -297,10 +299,17 @@ int e2d_create(const e2d_params *pin, e2d_sim **out) {
   s->fp32 = (p.precision == E2D_PRECISION_FP32C) ? 1 : 0;
   make_kparams(p, &s->kp);
   make_kparams32(p, &s->kp32);
-  if (const char *v = std::getenv("E2D_F32C_VARIANT")) s->kp32.variant = std::atoi(v);
-  // strip heights are whole 16-row CFL fold units
+  if (const char *v = std::getenv("E2D_F32C_VARIANT")) {
+    s->kp32.variant = std::atoi(v);
+    s->kp32.short_rows = 0;
+  }
+  // strip heights are whole 16-row CFL fold units, or 2, 4 or 8 rows of one
   if (const char *v = std::getenv("E2D_F32C_STRIP_H"))
-    if (std::atoi(v) > 0 && std::atoi(v) <= 512) s->kp32.strip_h = (std::atoi(v) + 15) / 16 * 16;
+    if (std::atoi(v) > 0 && std::atoi(v) <= 512) {
+      const int h = std::atoi(v);
+      s->kp32.short_rows = h == 2 || h == 4 || h == 8 ? h : 0;
+      s->kp32.strip_h = (h + 15) / 16 * 16;
+    }
   auto fail = [&](int status) {
     e2d_destroy(s);
     return status;
@@ -337,6 +346,13 @@ int e2d_create(const e2d_params *pin, e2d_sim **out) {
     }
     if (const size_t k = impl12_scratch_doubles(s->kp, s->impl))
       if (cudaMalloc(&s->impl_scratch, sizeof(double) * k) != cudaSuccess) return fail(E2D_ENOMEM);
+  }
+  const char *lp = std::getenv("E2D_LOOP");
+  if (!(lp && std::atoi(lp) == 0)) {
+    if (s->fp32)
+      s->loop_blocks = f32c_loop_blocks(s->kp32, p.riemannSolverType);
+    else if (!s->f64_split && s->impl == 0 && !s->kp.wait_test)
+      s->loop_blocks = f64_loop_blocks(s->kp, p.riemannSolverType);
   }
   if (cudaMalloc(&s->partial, sizeof(double) * reduce_partial_count(s->kp.g)) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMalloc(&s->red_out, sizeof(double) * 8) != cudaSuccess) return fail(E2D_ENOMEM);
@@ -625,6 +641,20 @@ int e2d_step_n(e2d_sim *s, int n, double t_end, double *t, int *nStep, double *d
   } else {
     if (prologue) E2D_CK(s, enqueue_prologue(s, par0, *nStep), "prologue");
     int done = 0;
+    // small grids: many steps per launch, a grid barrier between them
+    while (s->loop_blocks > 0 && done < n) {
+      const int k = n - done < kLoopSteps ? n - done : kLoopSteps;
+      if (done > 0)
+        E2D_CK(s, cudaMemsetAsync(&s->clk->arrived, 0, sizeof(DevClock) - offsetof(DevClock, arrived), s->stream),
+               "loop reset");
+      if (s->fp32)
+        E2D_CK(s, launch_loop_f32c(s->kp32, s->p.riemannSolverType, s->loop_blocks, s->W, s->clk, k, s->stream),
+               "loop launch");
+      else
+        E2D_CK(s, launch_loop_f64(s->kp, s->p.riemannSolverType, s->loop_blocks, s->U, s->Q, s->clk, s->dt_trace, k,
+                                  s->stream), "loop launch");
+      done += k;
+    }
     while (n - done >= kGraphSteps) {
       cudaGraphExec_t g;
       rc = get_graph(s, kGraphSteps, (par0 + done) & 1, &g);
@@ -642,7 +672,7 @@ int e2d_step_n(e2d_sim *s, int n, double t_end, double *t, int *nStep, double *d
   *t = s->clk_host->t;
   *nStep = s->clk_host->nstep;
   if (s->clk_host->status & E2D_FLAG_TIMEOUT)
-    return set_err(s, E2D_ETIMEOUT, "a staging wait gave up: the state of this call is incomplete");
+    return set_err(s, E2D_ETIMEOUT, "a bounded device wait gave up: the state of this call is incomplete");
   if (s->clk_host->status & (E2D_FLAG_NONFINITE | E2D_FLAG_BAD_DT))
     return set_err(s, E2D_ENUMERIC, (s->clk_host->status & E2D_FLAG_NONFINITE) ? "non-finite state value"
                                                                               : "non-positive or non-finite dt");

@@ -27,6 +27,7 @@
 // ghost cells of the arrays are never read.  Algorithmic traffic: 32 B read
 // + 32 B written per cell.
 #include "e2d_common.cuh"
+#include "e2d_f64_intdiv.h"
 #include "e2d_internal.h"
 #include "e2d_tma.cuh"
 
@@ -282,16 +283,36 @@ __device__ __forceinline__ void riemann2(const KPhys<float> &ph, const C2 &k, co
   }
 }
 
+// FP64 division and square root on the integer pipes (e2d_f64_intdiv.h): one
+// lane's quotient arrives after about 300 clocks instead of 600, and a step's
+// dt and its CFL winners are chains of them.
+static __device__ __noinline__ double div64_slow(double a, double b) { return a / b; }
+static __device__ __noinline__ double sqrt64_slow(double x) { return sqrt(x); }
+__device__ __forceinline__ double quot64(double a, const f64i::Divisor &d) {
+  bool ok;
+  double q = f64i::quotient(a, d, ok);
+  if (!ok) q = div64_slow(a, f64i::make(d.hi, d.lo));
+  return q;
+}
+__device__ __forceinline__ double quot64(double a, double b) { return quot64(a, f64i::divisor(b)); }
+__device__ __forceinline__ double root64(double x) {
+  bool ok;
+  double s = f64i::root(x, ok);
+  if (!ok) s = sqrt64_slow(x);
+  return s;
+}
+
 // CFL term of src/HydroRunFunctors.h:56-72, FP64, from a compensated cell.
 __device__ __forceinline__ double cfl_term64(const KPhys<double> &ph, double rho, double e, double mx,
                                              double my) {
   const double d = fmax(rho, ph.smallr);
-  const double ux = mx / d, uy = my / d;
+  const f64i::Divisor dv = f64i::divisor(d);
+  const double ux = quot64(mx, dv), uy = quot64(my, dv);
   const double eken = 0.5 * (ux * ux + uy * uy);
-  const double ei = e / d - eken;
+  const double ei = quot64(e, dv) - eken;
   const double p = fmax(ph.gm1 * d * ei, d * ph.smallp);
-  const double c = sqrt(ph.gamma0 * p / d);
-  return (c + fabs(ux)) / ph.dx + (c + fabs(uy)) / ph.dy;
+  const double c = root64(quot64(ph.gamma0 * p, dv));
+  return quot64(c + fabs(ux), ph.dx) + quot64(c + fabs(uy), ph.dy);
 }
 
 // The CFL term of two cells from their conserved values; idx = (1/dx, 1/dy).
@@ -315,11 +336,14 @@ __device__ __forceinline__ void fold_candidate(const KParams32 &kp, float term, 
                                                const float *w, unsigned long long *target,
                                                unsigned int *status) {
   const double cur = __longlong_as_double((long long)(*(volatile unsigned long long *)target));
-  if ((double)term < cur * (1.0 - 1e-4)) return;
   const long long P = kp.wplane;
+  float h[8];  // on their way beside the maximum
+#pragma unroll
+  for (int v = 0; v < 8; ++v) h[v] = w[cell + v * P];
+  if ((double)term < cur * (1.0 - 1e-4)) return;
   double u[4];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) u[v] = (double)w[cell + v * P] + (double)w[cell + (4 + v) * P];
+  for (int v = 0; v < 4; ++v) u[v] = (double)h[v] + (double)h[4 + v];
   const double t64 = cfl_term64(kp.ph64, u[E2D_ID], u[E2D_IP], u[E2D_IU], u[E2D_IV]);
   if (t64 > 0.0 && !nonfinite64(t64))
     atomicMax(target, (unsigned long long)__double_as_longlong(t64));
@@ -461,7 +485,9 @@ constexpr int SLOT = 8 * 64;  // floats per slot
 constexpr int kMaxSlots = 8;  // ring slots (PFD + 3) a warp may have
 // (+128 bytes: the ring starts at the first 128-byte boundary of the
 // dynamic shared memory, the alignment a tiled TMA destination needs)
-constexpr size_t ring_bytes(int pfd) { return pfd > 0 ? sizeof(float) * WPB * (pfd + 3) * SLOT + 128 : 0; }
+constexpr size_t ring_bytes(int pfd, int warps = WPB) {
+  return pfd > 0 ? sizeof(float) * warps * (pfd + 3) * SLOT + 128 : 0;
+}
 
 __device__ __forceinline__ void cp_async16(float *dst, const float *src) {
   const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
@@ -499,28 +525,42 @@ __device__ __forceinline__ int source_row(const KGeom &g, int r, bool yghost, bo
   return ghost_source(min(max(r, 0), g.jsize - 1), g.ny, g.bc_ymin, g.bc_ymax, fv);
 }
 
-// Copies array row r into a ring slot.  `direct` strips (64 interior
-// columns starting at array column cs, a multiple of 4) copy 16-byte chunks,
-// lane l taking chunk l % 16 of planes l / 16, +2, +4, +6, so a lane reads
-// columns another lane copied; other strips copy each lane's two columns
-// s0, s1 (the boundary map of c0, c0 + 1) element by element.
+// Copies array row r into a ring slot: the 64 columns from array column cs (a
+// multiple of 4) of the 8 planes, in 16-byte chunks, lane l taking chunk l %
+// 16 of planes l / 16, +2, +4, +6, so a lane reads columns another lane
+// copied.  In strips that are not `direct` (64 interior columns) the chunks
+// with a ghost column in them -- the array's first one, and those of columns
+// nx + 2 and nx + 3 -- are copied column by column through the boundary map
+// (lane l: column l % 4 of plane l / 4), and columns beyond the grid, which
+// no written cell depends on, not at all.  (Copying every column of such a
+// strip by itself took 16 requests a row, most of them of one and the same
+// word: 7500 to 19000 clocks for a 256-column grid's last strip to get under
+// way, against 2600.)
 __device__ __forceinline__ void stage_row(const KParams32 &kp, const float *__restrict__ w, int r, int cs,
-                                          int lane, bool direct, bool yghost, int s0, int s1, float *slot) {
+                                          int lane, bool direct, bool yghost, float *slot) {
+  const KGeom &g = kp.g;
   bool fv;
-  const float *row = w + (long long)source_row(kp.g, r, yghost, fv) * kp.wpitch;
-  if (direct) {
-    const int chunk = lane & 15;
+  const float *row = w + (long long)source_row(g, r, yghost, fv) * kp.wpitch;
+  const int chunk = lane & 15, c4 = cs + 4 * chunk;
+  if (direct || (c4 >= 2 && c4 + 3 < g.nx + 2)) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int v = (lane >> 4) + 2 * k;
       cp_async16(slot + v * 64 + 4 * chunk, row + v * kp.wplane + cs + 4 * chunk);
     }
-  } else {
-#pragma unroll
-    for (int v = 0; v < 8; ++v) {
-      cp_async4(slot + v * 64 + 2 * lane, row + v * kp.wplane + s0);
-      cp_async4(slot + v * 64 + 2 * lane + 1, row + v * kp.wplane + s1);
-    }
+  }
+  if (!direct) {
+    auto ghost_chunk = [&](int q) {  // columns 4 q .. 4 q + 3 of the array
+      const int c = 4 * q + (lane & 3), v = lane >> 2;
+      if (4 * q < cs || 4 * q >= cs + 64 || c > g.nx + 3) return;
+      bool f;
+      const int src = ghost_source(c, g.nx, g.bc_xmin, g.bc_xmax, f);
+      cp_async4(slot + v * 64 + (c - cs), row + v * kp.wplane + src);
+    };
+    if (cs == 0) ghost_chunk(0);
+    const int q0 = (g.nx + 2) >> 2, q1 = (g.nx + 3) >> 2;  // never the first chunk unless nx < 2
+    if (q0 > 0) ghost_chunk(q0);
+    if (q1 > q0) ghost_chunk(q1);
   }
 }
 
@@ -547,13 +587,20 @@ __device__ __forceinline__ void stage_row_tma(const KGeom &g, const CUtensorMap 
 // kernel or the batch (strip_h must be a multiple of CFL_UNIT_ROWS and at
 // most 32 units).  Each unit's FP32 arg-max is parked in lane `unit`; the
 // parked winners are recomputed in FP64 together when the strip ends.
-template <int RS, int PFD, int TMA, bool INTERIOR, bool TGT>
+// SUB > 0: a short strip of SUB rows, part of a fold unit whose other strips
+// are marched by the block's other warps.  The caller has staged its first
+// PFD + 2 rows (stage_first_rows), and it folds the unit: `lane_best` and
+// `lane_local` receive the lane's best cell, numbered from the unit's first
+// row, which is `urow` rows above the strip's.
+template <int RS, int PFD, int TMA, bool INTERIOR, bool TGT, int SUB = 0>
 __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *__restrict__ w_in,
                                             float *__restrict__ w_out, const float2 dtdx,
                                             const float2 dtdy, const int sx, const int sy,
                                             const int lane, unsigned long long *target,
                                             unsigned int *status, float *ring, const CUtensorMap *map,
-                                            unsigned long long *bars, unsigned int &phase) {
+                                            unsigned long long *bars, unsigned int &phase, const int urow = 0,
+                                            float *lane_best = nullptr, int *lane_local = nullptr) {
+  static_assert(SUB == 0 || (TMA == 0 && PFD > 0 && TGT), "short strips: rows staged by cp.async, CFL folded");
   // sum of the lane's new conserved values over the strip: NaN or infinite
   // when one of them is (a sum that overflows FP32 reads as non-finite too)
   float2 nfacc = f2(0.0f);
@@ -564,7 +611,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
   int unit = 0;
   const KGeom &g = kp.g;
   const KPhys<float> &ph = kp.ph;
-  const int SH = kp.strip_h;
+  const int SH = SUB > 0 ? SUB : kp.strip_h;
   const int cb = 2 + sx * OUTW;       // array column of the strip's first output column
   const int rb = 2 + sy * SH;         // array row of the strip's first output row
   const int re = min(rb + SH, g.ny + 2);
@@ -588,10 +635,9 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
   float2 pf[4];  // (register path) conserved hi of row m+1, loaded one iteration ahead
   // (staged path) the boundary map of the lane's columns and its ring slots
   bool f0 = false, f1 = false;
-  int s0 = c0, s1 = c0 + 1;
-  if ((PFD > 0) && !direct) {
-    s0 = ghost_source(min(max(c0, 0), g.isize - 1), g.nx, g.bc_xmin, g.bc_xmax, f0);
-    s1 = ghost_source(min(max(c0 + 1, 0), g.isize - 1), g.nx, g.bc_xmin, g.bc_xmax, f1);
+  if ((PFD > 0) && !direct) {  // the flips of the lane's two columns
+    ghost_source(min(max(c0, 0), g.isize - 1), g.nx, g.bc_xmin, g.bc_xmax, f0);
+    ghost_source(min(max(c0 + 1, 0), g.isize - 1), g.nx, g.bc_xmin, g.bc_xmax, f1);
   }
   constexpr int R = PFD + 3;  // ring slots; row r sits in slot (r - rb + 2) mod R
   static_assert(TMA != 2 || R == 6, "row pairs need a ring of three pairs");
@@ -629,7 +675,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
       stage_row_tma(g, map, r, cb - 2, lane, yghost, slot_of(sl), bars + sl);
       pending |= 1u << sl;
     } else {
-      stage_row(kp, w_in, r, cb - 2, lane, direct, yghost, s0, s1, slot_of(sl));
+      stage_row(kp, w_in, r, cb - 2, lane, direct, yghost, slot_of(sl));
     }
   };
   auto wait_slot = [&](int sl) {
@@ -664,8 +710,10 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
     // rows rb-2 .. rb+PFD-1 into slots 0 .. PFD+1 (one commit group each on
     // the cp.async path), after every lane is done with the ring's previous
     // strip
-    __syncwarp();
-    if (pairs) {
+    if (SUB == 0) __syncwarp();
+    if (SUB > 0) {
+      cp_async_wait<(PFD > 0 ? PFD : 0)>();
+    } else if (pairs) {
       stage_pair(0);
       stage_pair(1);
       if (!wait_slot(0)) return give_up();
@@ -807,8 +855,13 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
       float2 yl[4] = {ymax_prev[E2D_ID], ymax_prev[E2D_IP], ymax_prev[E2D_IV], ymax_prev[E2D_IU]};
       float2 yr[4] = {ymin[E2D_ID], ymin[E2D_IP], ymin[E2D_IV], ymin[E2D_IU]};
       float2 f[4];
-      riemann2<RS>(ph, k, xl, xr, fx);
-      riemann2<RS>(ph, k, yl, yr, f);
+      if (SUB > 0 && m < rb) {  // a short strip: two of its few solves saved
+#pragma unroll
+        for (int v = 0; v < 4; ++v) fx[v] = f[v] = f2(0.0f);
+      } else {
+        riemann2<RS>(ph, k, xl, xr, fx);
+        riemann2<RS>(ph, k, yl, yr, f);
+      }
       // unscaled: dt/dx and dt/dy are applied in the update
       fy[E2D_ID] = f[E2D_ID];
       fy[E2D_IP] = f[E2D_IP];
@@ -846,7 +899,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
         }
         if (TGT || target) {
           const float2 t = cfl_term2(k, idx, nh);
-          const int loc = (m - 1 - rb) * 64 + 2 * lane + 1;
+          const int loc = (m - 1 - rb + urow) * 64 + 2 * lane + 1;
           // non-finite states: a NaN term never wins the arg-max, and the
           // fmaxf cut-offs drop a NaN density or energy, so the new density
           // and energy are summed with the term, which a non-finite momentum
@@ -860,7 +913,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
       }
       const int r = m - 1;  // >= rb >= 2, so the low bits of r - 2 are its remainder
       static_assert((CFL_UNIT_ROWS & (CFL_UNIT_ROWS - 1)) == 0, "fold units are a power of two rows");
-      if ((TGT || target) && (((r - 2) & (CFL_UNIT_ROWS - 1)) == CFL_UNIT_ROWS - 1 || r == re - 1)) {
+      if (SUB == 0 && (TGT || target) && (((r - 2) & (CFL_UNIT_ROWS - 1)) == CFL_UNIT_ROWS - 1 || r == re - 1)) {
         float ut;
         const int win = unit_argmax(best, blocal, &ut);
         if (lane == unit) pend_term = ut, pend_local = win;
@@ -886,6 +939,11 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
     const float kInf = __int_as_float(0x7f800000);
     const bool nonfin = !(fabsf(nfacc.x) < kInf) || !(fabsf(nfacc.y) < kInf);
     if (__any_sync(0xffffffffu, nonfin) && lane == 0) atomicOr(status, (unsigned)E2D_FLAG_NONFINITE);
+    if (SUB > 0) {
+      *lane_best = best;
+      *lane_local = blocal;
+      return true;
+    }
     __syncwarp();  // the winners were written by lanes of this warp
     if (pend_local > 0) {
       const int L = pend_local - 1;
@@ -921,6 +979,25 @@ __device__ __forceinline__ bool march_strip(const KParams32 &kp, const float *__
                                                    ring, map, bars, phase);
 }
 
+// The last block to finish a step advances the loop state
+// (src/main.cpp:139-143); one thread per block, after a block barrier.
+__device__ __forceinline__ void finish_step(DevClock *clk, const double dt, const int slot) {
+  __threadfence();
+  const unsigned int ticket = atomicAdd(&clk->done_blocks, 1u);
+  if (ticket != gridDim.x - 1) return;
+  __threadfence();
+  const int ns = clk->nstep;
+  const int tslot = ns - clk->trace_base;
+  if (clk->trace && tslot >= 0 && tslot < clk->trace_cap) clk->trace[tslot] = dt;
+  if (!(dt > 0.0) || nonfinite64(dt)) clk->status |= E2D_FLAG_BAD_DT;
+  clk->dt = dt;
+  clk->t = clk->t + dt;  // only this block writes t during the step
+  clk->nstep = ns + 1;
+  clk->acc[slot] = 0ull;
+  clk->done_blocks = 0u;
+  __threadfence();
+}
+
 extern __shared__ __align__(16) float g_ring[];
 
 // The warp's row ring: g_ring rounded up to 128 bytes (ring_bytes reserves
@@ -954,12 +1031,12 @@ __global__ void __launch_bounds__(NT, MINB)
       run = t < t_end;
       slot = clk->nstep & 1;
       const double inv_dt = __longlong_as_double((long long)clk->acc[slot]);
-      dt = kp.ph64.cfl / inv_dt;
+      dt = quot64(kp.ph64.cfl, inv_dt);
       if (t + dt > t_end) dt = t_end - t;
     }
     s_dt[0] = dt;
-    s_dt[1] = dt / kp.ph64.dx;
-    s_dt[2] = dt / kp.ph64.dy;
+    s_dt[1] = quot64(dt, kp.ph64.dx);
+    s_dt[2] = quot64(dt, kp.ph64.dy);
     s_run = run;
     s_slot = slot;
   }
@@ -983,27 +1060,151 @@ __global__ void __launch_bounds__(NT, MINB)
   }
   if (!use_clock) return;
 
-  // the last block to finish advances the loop state (src/main.cpp:139-143)
   __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    const unsigned int nblocks = gridDim.x;
-    const unsigned int ticket = atomicAdd(&clk->done_blocks, 1u);
-    if (ticket == nblocks - 1) {
-      __threadfence();
-      const double dt = s_dt[0];
-      const int ns = clk->nstep;
-      const int tslot = ns - clk->trace_base;
-      if (clk->trace && tslot >= 0 && tslot < clk->trace_cap) clk->trace[tslot] = dt;
-      if (!(dt > 0.0) || nonfinite64(dt)) clk->status |= E2D_FLAG_BAD_DT;
-      clk->dt = dt;
-      clk->t = clk->t + dt;  // only this block writes t during the step
-      clk->nstep = ns + 1;
-      clk->acc[slot] = 0ull;
-      clk->done_blocks = 0u;
-      __threadfence();
+  if (tid == 0) finish_step(clk, s_dt[0], slot);
+}
+
+// Stages the first PFD + 2 rows of a strip (from array row rb - 2) into the
+// warp's ring, one commit group each.
+template <int PFD>
+__device__ __forceinline__ void stage_first_rows(const KParams32 &kp, const float *__restrict__ w, int sx, int rb,
+                                                 int re, int lane, float *ring) {
+  const KGeom &g = kp.g;
+  const int cb = 2 + sx * OUTW;
+  const bool direct = (cb - 2 >= 2) && (cb + OUTW + 1 <= g.nx + 1);
+  const bool yghost = (rb - 2 < 2) || (re + 1 > g.ny + 1);
+  for (int k = 0; k < PFD + 2; ++k) {
+    stage_row(kp, w, rb - 2 + k, cb - 2, lane, direct, yghost, ring + k * SLOT);
+    cp_async_commit();
+  }
+}
+
+// One step of a grid too small to fill the GPU with strips of a whole fold
+// unit: each block takes one unit (60 columns by 16 rows), each of its 16/SUB
+// warps SUB rows of it.  A step of such a grid costs what one warp's march
+// costs, about 1 us a row plus a fixed part, so a shorter strip is a faster
+// step as long as the warps stay few (see short_rows); the extra halo rows
+// run on SMs that would stand idle.  The unit's winner -- the lanes' earliest
+// rows first, then the largest cell -- is the one a 16-row strip finds, so
+// states and dts are the same bits.
+constexpr int SHORT_PFD = 4;  // rows staged ahead: all of a 2-row strip's before its march
+
+// Unit `unit` of a step from w_in to w_out; dt() (called by every thread
+// once the unit's first rows are on their way) gives dt/dx and dt/dy.  The
+// unit's CFL winner is folded into *target by thread 0.
+template <int RS, int SUB, class DT>
+__device__ __forceinline__ void short_unit(const KParams32 &kp, const float *w_in, float *w_out, const int unit,
+                                           unsigned long long *target, unsigned int *status, const DT &dt) {
+  constexpr int W = CFL_UNIT_ROWS / SUB;
+  const KGeom &g = kp.g;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ float s_best[W][LANES];
+  __shared__ int s_local[W][LANES];
+  const int nsx = (g.nx + OUTW - 1) / OUTW;
+  const int sx = unit % nsx;
+  const int ub = 2 + (unit / nsx) * CFL_UNIT_ROWS;  // the unit's first row
+  const int rb = ub + warp * SUB, re = min(rb + SUB, g.ny + 2);
+  const bool has = rb < g.ny + 2;
+  float *ring = warp_ring<SHORT_PFD>(warp);
+  if (has) stage_first_rows<SHORT_PFD>(kp, w_in, sx, rb, re, lane, ring);
+  const float2 d = dt();
+  float best = -1.0f;
+  int local = 0;
+  if (has) {
+    const float2 dtdx = f2(d.x), dtdy = f2(d.y);
+    const int sy = (rb - 2) / SUB;
+    unsigned int phase = 0u;
+    const int cb = 2 + sx * OUTW;
+    const bool interior = (cb - 2 >= 2) && (cb + OUTW + 1 <= g.nx + 1) && !(rb - 2 < 2) && !(re + 1 > g.ny + 1);
+    if (interior)
+      march_strip_t<RS, SHORT_PFD, 0, true, true, SUB>(kp, w_in, w_out, dtdx, dtdy, sx, sy, lane, target, status, ring,
+                                                       nullptr, nullptr, phase, rb - ub, &best, &local);
+    else
+      march_strip_t<RS, SHORT_PFD, 0, false, true, SUB>(kp, w_in, w_out, dtdx, dtdy, sx, sy, lane, target, status,
+                                                        ring, nullptr, nullptr, phase, rb - ub, &best, &local);
+    cp_async_wait<0>();  // rows past a strip cut short by the grid's end
+  }
+  s_best[warp][lane] = best;
+  s_local[warp][lane] = local;
+  __syncthreads();
+  if (warp != 0) return;
+  // a lane's best cell over the unit's rows: the first of equal terms, as one
+  // warp marching all 16 rows keeps it
+#pragma unroll
+  for (int k = 1; k < W; ++k)
+    if (s_best[k][lane] > best) best = s_best[k][lane], local = s_local[k][lane];
+  float term;
+  const int win = unit_argmax(best, local, &term);
+  if (lane == 0 && win > 0) {
+    const int L = win - 1;
+    fold_candidate(kp, term, (long long)kp.wpitch * (ub + L / 64) + (2 + sx * OUTW - 2) + (L % 64), w_out, target,
+                   status);
+  }
+}
+
+template <int RS, int SUB, int MINB>
+__global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
+    k_step_f32c_short(const KParams32 kp, const float *__restrict__ w_in, float *__restrict__ w_out, DevClock *clk) {
+  __shared__ double s_dt[3];
+  const int slot = clk->nstep & 1;
+  if (!(clk->t < clk->t_end)) return;
+  short_unit<RS, SUB>(kp, w_in, w_out, blockIdx.x, &clk->acc[slot ^ 1], &clk->status, [&]() {
+    if (threadIdx.x == 0) {
+      const double t = clk->t, t_end = clk->t_end;
+      double dt = quot64(kp.ph64.cfl, __longlong_as_double((long long)clk->acc[slot]));
+      if (t + dt > t_end) dt = t_end - t;
+      s_dt[0] = dt;
+      s_dt[1] = quot64(dt, kp.ph64.dx);
+      s_dt[2] = quot64(dt, kp.ph64.dy);
+    }
+    __syncthreads();
+    return make_float2((float)s_dt[1], (float)s_dt[2]);
+  });
+  if (threadIdx.x == 0) finish_step(clk, s_dt[0], slot);
+}
+
+// Up to `steps` steps in one cooperative launch, a grid barrier between them
+// (see k_loop_f64); states are read by cp.async and written through, so what
+// other blocks wrote before the barrier is what is read.
+template <int RS, int SUB, int MINB>
+__global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
+    k_loop_f32c(const KParams32 kp, float *w0, float *w1, DevClock *clk, const int units, const int steps) {
+  __shared__ double s_dt[3];
+  LoopClock c = loop_begin(clk);
+  int s = 0;
+  for (; s < steps && c.t < c.t_end; ++s) {
+    const bool odd = c.ns & 1;
+    bool first = true;
+    // asked for before the rows, whose requests it would queue behind
+    const unsigned long long cfl = threadIdx.x == 0 ? loop_cfl(clk, c, s) : 0ull;
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      short_unit<RS, SUB>(kp, odd ? w1 : w0, odd ? w0 : w1, u, &clk->acc3[(s + 1) % 3], &clk->status, [&]() {
+        if (first) {
+          if (threadIdx.x == 0) {
+            double dt = quot64(kp.ph64.cfl, __longlong_as_double((long long)cfl));
+            if (c.t + dt > c.t_end) dt = c.t_end - c.t;
+            s_dt[0] = dt;
+            s_dt[1] = quot64(dt, kp.ph64.dx);
+            s_dt[2] = quot64(dt, kp.ph64.dy);
+          }
+          __syncthreads();
+        }
+        return make_float2((float)s_dt[1], (float)s_dt[2]);
+      });
+      first = false;
+      if (u + gridDim.x < units) __syncthreads();  // the winners' table is rewritten by the next unit
+    }
+    const double dt = s_dt[0];
+    if (blockIdx.x == 0 && threadIdx.x == 0) loop_record(clk, c, s, dt, clk->trace);
+    c.t = c.t + dt;
+    c.ns += 1;
+    // wait_test: a block more than there are, so the bounded wait runs out
+    if (!grid_barrier(&clk->arrived, (unsigned)(s + 1) * gridDim.x + (kp.wait_test ? 1u : 0u))) {
+      if (threadIdx.x == 0) atomicOr(&clk->status, (unsigned)E2D_FLAG_TIMEOUT);
+      return;
     }
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) loop_end(clk, c, s);
 }
 
 // ------------------------------------------------------------ batches
@@ -1199,6 +1400,20 @@ int default_strip_h(int nx, int ny) {
   return 16;
 }
 
+// Rows of a grid's short strips (0: strips of default_strip_h rows), by the
+// number of 60 x 16 fold units, a block each: 2 rows while every block has an
+// SM of its own, 4 while all are resident two to an SM, 8 while the extra
+// halo rows (10 marched for 8 written) cost less than a 16-row march's
+// latency.  Measured, us a step, HLLC, multi-step launches, 2 / 4 / 8 rows
+// against 16: 256^2 (80 units) 10.5 / 10.8 / 15.1 against 27.3; 512^2 (288)
+// 17.1 / 12.0 / 16.2 against 30.2; 700^2 (528) 35.9 / 21.4 / 19.6 against
+// 36.3; 1201x700 (924) 57 / 39 / 31.1 against 35.0; 1024^2 (1152) 70 / 44 /
+// 37.6 against 35.7.
+int default_short_rows(int nx, int ny) {
+  const long long units = (long long)((nx + OUTW - 1) / OUTW) * ((ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS);
+  return units <= 152 ? 2 : units <= 304 ? 4 : units <= 1000 ? 8 : 0;
+}
+
 void make_kparams32(const e2d_params &p, KParams32 *kp) {
   KParams64 k64;
   make_kparams(p, &k64);
@@ -1212,8 +1427,21 @@ void make_kparams32(const e2d_params &p, KParams32 *kp) {
   kp->wplane = (long long)kp->wpitch * p.jsize;
   kp->variant = 4;  // 3 blocks per SM, rows staged by cp.async (fastest at 8192^2)
   kp->strip_h = default_strip_h(p.nx, p.ny);
+  kp->short_rows = default_short_rows(p.nx, p.ny);
   const char *wt = std::getenv("E2D_TEST_WAIT_TIMEOUT");
   kp->wait_test = (wt && std::atoi(wt) != 0) ? 1 : 0;
+}
+
+// Rows of a short strip (see k_step_f32c_short), as template arguments with
+// the resident blocks per SM their launch bounds ask for.
+template <class F>
+static void with_short(int rows, F &&f) {
+  using std::integral_constant;
+  switch (rows) {
+    case 2: f(integral_constant<int, 2>{}, integral_constant<int, 1>{}); break;
+    case 4: f(integral_constant<int, 4>{}, integral_constant<int, 2>{}); break;
+    default: f(integral_constant<int, 8>{}, integral_constant<int, 4>{}); break;
+  }
 }
 
 // Dynamic plus static shared memory above 48 KB must be enabled per kernel
@@ -1230,6 +1458,13 @@ static cudaError_t configure_rs() {
           e = cudaFuncSetAttribute(k_batch_f32c<RS, M, P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)ring_bytes(P));
       }
+    });
+  for (int rows = 2; rows <= 8 && e == cudaSuccess; rows *= 2)
+    with_short(rows, [&](auto sub, auto minb) {
+      constexpr int S = decltype(sub)::value, M = decltype(minb)::value;
+      constexpr int bytes = (int)ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / S);
+      e = cudaFuncSetAttribute(k_step_f32c_short<RS, S, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loop_f32c<RS, S, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     });
   if (e == cudaSuccess)  // variant 7 (single-grid step only)
     e = cudaFuncSetAttribute(k_step_f32c<RS, 3, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes(3));
@@ -1288,9 +1523,81 @@ static void launch_step_v(const KParams32 &kp, int riemann, int blocks, const fl
   }
 }
 
+template <int SUB, int MINB>
+static void launch_short_v(const KParams32 &kp, int riemann, int blocks, const float *w_in, float *w_out,
+                           DevClock *clk, cudaStream_t s) {
+  constexpr int threads = 32 * (CFL_UNIT_ROWS / SUB);
+  const size_t sm = ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / SUB);
+  switch (riemann) {
+    case E2D_RIEMANN_HLLC:
+      k_step_f32c_short<E2D_RIEMANN_HLLC, SUB, MINB><<<blocks, threads, sm, s>>>(kp, w_in, w_out, clk);
+      break;
+    case E2D_RIEMANN_HLL:
+      k_step_f32c_short<E2D_RIEMANN_HLL, SUB, MINB><<<blocks, threads, sm, s>>>(kp, w_in, w_out, clk);
+      break;
+    default:
+      k_step_f32c_short<E2D_RIEMANN_APPROX, SUB, MINB><<<blocks, threads, sm, s>>>(kp, w_in, w_out, clk);
+      break;
+  }
+}
+
+static int units_of(const KParams32 &kp) {
+  return ((kp.g.nx + OUTW - 1) / OUTW) * ((kp.g.ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS);
+}
+
+template <class F>
+static void with_loop(const KParams32 &kp, int riemann, F &&f) {
+  with_short(kp.short_rows, [&](auto sub, auto minb) {
+    constexpr int S = decltype(sub)::value, M = decltype(minb)::value;
+    constexpr int threads = 32 * (CFL_UNIT_ROWS / S);
+    const size_t sm = ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / S);
+    switch (riemann) {
+      case E2D_RIEMANN_HLLC: f(k_loop_f32c<E2D_RIEMANN_HLLC, S, M>, threads, sm); break;
+      case E2D_RIEMANN_HLL: f(k_loop_f32c<E2D_RIEMANN_HLL, S, M>, threads, sm); break;
+      default: f(k_loop_f32c<E2D_RIEMANN_APPROX, S, M>, threads, sm); break;
+    }
+  });
+}
+
+int f32c_loop_blocks(const KParams32 &kp, int riemann) {
+  if (kp.short_rows <= 0) return 0;
+  int blocks = 0;
+  with_loop(kp, riemann, [&](auto kernel, int threads, size_t sm) {
+    int dev = 0, sms = 0, per_sm = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sm) != cudaSuccess)
+      return;
+    const int units = units_of(kp);
+    if (units <= 2 * sms * per_sm) blocks = units < sms * per_sm ? units : sms * per_sm;
+  });
+  return blocks;
+}
+
+cudaError_t launch_loop_f32c(const KParams32 &kp, int riemann, int blocks, float *const w[2], DevClock *clk, int steps,
+                             cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  with_loop(kp, riemann, [&](auto kernel, int threads, size_t sm) {
+    KParams32 p = kp;
+    float *w0 = w[0], *w1 = w[1];
+    int units = units_of(kp);
+    void *args[] = {&p, &w0, &w1, &clk, &units, &steps};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(blocks), dim3(threads), args, sm, s);
+  });
+  return e;
+}
+
 cudaError_t launch_f32c_step(const KParams32 &kp, int riemann, const float *w_in, float *w_out,
                              const CUtensorMap &tm_in, DevClock *clk, int use_clock, double host_dt,
                              cudaStream_t s) {
+  if (use_clock && kp.short_rows > 0) {
+    const int units = units_of(kp);
+    with_short(kp.short_rows, [&](auto sub, auto minb) {
+      launch_short_v<decltype(sub)::value, decltype(minb)::value>(kp, riemann, units, w_in, w_out, clk, s);
+    });
+    return cudaGetLastError();
+  }
   const int nsx = (kp.g.nx + OUTW - 1) / OUTW;
   const int nsy = (kp.g.ny + kp.strip_h - 1) / kp.strip_h;
   const int blocks = (nsx * nsy + WPB - 1) / WPB;

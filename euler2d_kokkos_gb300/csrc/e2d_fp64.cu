@@ -200,7 +200,7 @@ __device__ __forceinline__ void load_qtile(const KGeom &g, const double *__restr
 // its sign with mx; e, p and c depend on u^2).  Only interior cells of q are
 // read.
 template <int TX, int NT>
-__device__ __forceinline__ void gather_qtile(const KGeom &g, const double *__restrict__ q, int i0, int j0, int ty,
+__device__ __forceinline__ void gather_qtile(const KGeom &g, const double *q, int i0, int j0, int ty,
                                              double *sQ) {
   constexpr int QW = TX + 4;
   const int n = (ty + 4) * QW;
@@ -212,9 +212,9 @@ __device__ __forceinline__ void gather_qtile(const KGeom &g, const double *__res
       const int si = src_lo_hi(gi, g.nx, g.bc_xmin, g.bc_xmax, fu);
       const int sj = src_lo_hi(gj, g.ny, g.bc_ymin, g.bc_ymax, fv);
       const size_t s = (size_t)si + (size_t)g.isize * sj;
-      const double ux = q[s + 2 * g.plane], uy = q[s + 3 * g.plane];
-      sQ[k] = q[s];
-      sQ[n + k] = q[s + g.plane];
+      const double ux = __ldcg(q + s + 2 * g.plane), uy = __ldcg(q + s + 3 * g.plane);
+      sQ[k] = __ldcg(q + s);
+      sQ[n + k] = __ldcg(q + s + g.plane);
       sQ[2 * n + k] = fu ? Fp::neg(ux) : ux;
       sQ[3 * n + k] = fv ? Fp::neg(uy) : uy;
     } else {
@@ -354,13 +354,13 @@ struct TileCells {
     const int gi = i0 + 2 + x, gj = j0 + 2 + y;
     return (y < ty && gi < g.nx + 2 && gj < g.ny + 2) ? gi + (long long)g.isize * gj : -1;
   }
-  __device__ __forceinline__ void load(const KGeom &g, const double *__restrict__ u_in, int i0, int j0, int ty) {
+  __device__ __forceinline__ void load(const KGeom &g, const double *u_in, int i0, int j0, int ty) {
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       int x, y;
       const long long s = offset(g, i0, j0, ty, n, x, y);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) u[n][v] = s >= 0 ? u_in[s + v * g.plane] : 0.0;
+      for (int v = 0; v < 4; ++v) u[n][v] = s >= 0 ? __ldcg(u_in + s + v * g.plane) : 0.0;
     }
   }
 };
@@ -504,8 +504,7 @@ __device__ __forceinline__ void block_fold(double term, unsigned int flags, unsi
 // new cells into q_out and the running maximum of their CFL terms and flags.
 template <int TX, int TYM, int NT, bool FAST, class F>
 __device__ __forceinline__ void step_epilogue(const F &f, const KParams64 &kp, const TileCells<TX, TYM, NT> &cells,
-                                              double *__restrict__ u_out, double *__restrict__ q_out, int i0,
-                                              int j0, int ty, double dtdx, double dtdy, double *smem, double &term,
+                                              double *u_out, double *q_out, int i0, int j0, int ty, double dtdx, double dtdy, double *smem, double &term,
                                               unsigned int &flags) {
   const KGeom &g = kp.g;
   const KPhys<double> &ph = kp.ph;
@@ -541,7 +540,7 @@ __device__ __forceinline__ void step_epilogue(const F &f, const KParams64 &kp, c
 // it -- receive the ghost fill of u_in in both states, read from interior
 // cells of u_in only (no block writes those during a step).
 template <int TX, int NT>
-__device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *__restrict__ u_in, double *__restrict__ u_out,
+__device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *u_in, double *u_out,
                                                 int i0, int j0, int ty, bool lo_x, bool hi_x, bool lo_y, bool hi_y) {
   if (!(lo_x || hi_x || lo_y || hi_y)) return;
   const int xa = lo_x ? 0 : i0 + 2, xb = hi_x ? g.isize : i0 + 2 + TX;
@@ -554,7 +553,9 @@ __device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *__restri
     const int si = src_lo_hi(i, g.nx, g.bc_xmin, g.bc_xmax, fu);
     const int sj = src_lo_hi(j, g.ny, g.bc_ymin, g.bc_ymax, fv);
     const size_t s = (size_t)si + (size_t)g.isize * sj, d = (size_t)i + (size_t)g.isize * j;
-    double v4[4] = {u_in[s], u_in[s + g.plane], u_in[s + 2 * g.plane], u_in[s + 3 * g.plane]};
+    double v4[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) v4[v] = __ldcg(u_in + s + v * g.plane);
     if (fu) v4[E2D_IU] = -v4[E2D_IU];
     if (fv) v4[E2D_IV] = -v4[E2D_IV];
 #pragma unroll
@@ -675,6 +676,69 @@ __global__ void __launch_bounds__(NT, MINB)
       __threadfence();
     }
   }
+}
+
+// Up to `steps` steps of the device loop in one cooperative launch, a grid
+// barrier between them: each block takes the same tiles in every step.  A
+// launch per step costs a small grid about 4 us of it -- the drain, the next
+// launch and instructions fetched anew -- and a barrier 1.5.  Tiles are
+// gathered with L2 loads (what other blocks wrote in this launch must not
+// come from an L1 line or the read-only path); arithmetic and bits are
+// k_step_f64's.
+template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL, bool FAST>
+__global__ void __launch_bounds__(NT, MINB)
+    k_loop_f64(const KParams64 kp, double *q0, double *q1, double *u0, double *u1, DevClock *clk, double *dt_trace,
+               const int steps) {
+  extern __shared__ unsigned char smem_raw[];
+  double *smem = reinterpret_cast<double *>(smem_raw);
+  __shared__ double s_dt[3];
+  const KGeom &g = kp.g;
+  const KPhys<double> &ph = kp.ph;
+  const int tid = threadIdx.x, ty = kp.ty;
+  const int ntx = (g.nx + TX - 1) / TX, nty = (g.ny + ty - 1) / ty;
+  const f64x::FpT<XMUL> f;
+  LoopClock c = loop_begin(clk);
+  int s = 0;
+  for (; s < steps && c.t < c.t_end; ++s) {
+    if (tid == 0) {
+      const double dt = step_dt(ph, loop_cfl(clk, c, s), c.t, c.t_end);
+      s_dt[0] = dt;
+      s_dt[1] = quot(dt, ph.dx);
+      s_dt[2] = quot(dt, ph.dy);
+    }
+    const bool odd = c.ns & 1;
+    double *u_in = odd ? u1 : u0, *u_out = odd ? u0 : u1;
+    const double *q_in = odd ? q1 : q0;
+    double *q_out = odd ? q0 : q1;
+    double term = 0.0;
+    unsigned int flags = 0;
+    for (int w = blockIdx.x; w < ntx * nty; w += gridDim.x) {
+      const int by = w / ntx, bx = w - by * ntx;
+      const int i0 = bx * TX, j0 = by * ty;
+      gather_qtile<TX, NT>(g, q_in, i0, j0, ty, smem);
+      __syncthreads();
+      const double dtdx = s_dt[1], dtdy = s_dt[2];
+      tile_faces<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+      TileCells<TX, TYM, NT> cells;
+      cells.load(g, u_in, i0, j0, ty);
+      __syncthreads();
+      tile_riemann<RS, TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+      __syncthreads();
+      step_epilogue<TX, TYM, NT, FAST>(f, kp, cells, u_out, q_out, i0, j0, ty, dtdx, dtdy, smem, term, flags);
+      ghost_fill_tile<TX, NT>(g, u_in, u_out, i0, j0, ty, bx == 0, bx == ntx - 1, by == 0, by == nty - 1);
+      __syncthreads();
+    }
+    block_fold<NT>(term, flags, &clk->acc3[(s + 1) % 3], &clk->status);
+    const double dt = s_dt[0];
+    if (blockIdx.x == 0 && tid == 0) loop_record(clk, c, s, dt, dt_trace);
+    c.t = c.t + dt;
+    c.ns += 1;
+    if (!grid_barrier(&clk->arrived, (unsigned)(s + 1) * gridDim.x)) {
+      if (tid == 0) atomicOr(&clk->status, E2D_FLAG_TIMEOUT);
+      return;
+    }
+  }
+  if (blockIdx.x == 0 && tid == 0) loop_end(clk, c, s);
 }
 
 // ------------------------------------------------------------ batches
@@ -936,6 +1000,8 @@ struct Shape<2> {
   static constexpr bool XMUL = false;
 };
 constexpr int kShapes = 3;
+// Waves of tiles up to which a grid's steps run in one launch.
+constexpr int LOOP_WAVES = 4;
 template <class F>
 static void with_shape(int shape, F &&f) {
   switch (shape) {
@@ -1026,6 +1092,8 @@ static cudaError_t configure_rs() {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_flux_update_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL>, attr, flux);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>, attr, step);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>, attr, step);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>, attr, flux);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>, attr, flux);
     });
   return e;
 }
@@ -1108,6 +1176,53 @@ static cudaError_t launch_step_t(const KParams64 &kp, const CUtensorMap &tm_q, i
           <<<grid, S::NT, sm, s>>>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace);
   });
   return cudaGetLastError();
+}
+
+template <int RS, class F>
+static void with_loop(const KParams64 &kp, F &&f) {
+  with_shape(kp.shape, [&](auto sh) {
+    using S = decltype(sh);
+    constexpr size_t sm = flux_smem_bytes<S::TX, S::TYM>();
+    const int tiles = ((kp.g.nx + S::TX - 1) / S::TX) * ((kp.g.ny + kp.ty - 1) / kp.ty);
+    if (kp.fast)
+      f(k_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>, S::NT, sm, tiles);
+    else
+      f(k_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>, S::NT, sm, tiles);
+  });
+}
+template <class F>
+static void with_loop(int riemann, const KParams64 &kp, F &&f) {
+  switch (riemann) {
+    case E2D_RIEMANN_HLLC: with_loop<E2D_RIEMANN_HLLC>(kp, f); break;
+    case E2D_RIEMANN_HLL: with_loop<E2D_RIEMANN_HLL>(kp, f); break;
+    default: with_loop<E2D_RIEMANN_APPROX>(kp, f); break;
+  }
+}
+
+int f64_loop_blocks(const KParams64 &kp, int riemann) {
+  int blocks = 0;
+  with_loop(riemann, kp, [&](auto kernel, int threads, size_t sm, int tiles) {
+    int dev = 0, sms = 0, per_sm = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sm) != cudaSuccess)
+      return;
+    if (tiles <= sms * per_sm * LOOP_WAVES) blocks = tiles < sms * per_sm ? tiles : sms * per_sm;
+  });
+  return blocks;
+}
+
+cudaError_t launch_loop_f64(const KParams64 &kp, int riemann, int blocks, double *const u[2], double *const q[2],
+                            DevClock *clk, double *dt_trace, int steps, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  with_loop(riemann, kp, [&](auto kernel, int threads, size_t sm, int) {
+    KParams64 p = kp;
+    double *q0 = q[0], *q1 = q[1], *u0 = u[0], *u1 = u[1];
+    void *args[] = {&p, &q0, &q1, &u0, &u1, &clk, &dt_trace, &steps};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(blocks), dim3(threads), args, sm, s);
+  });
+  return e;
 }
 
 cudaError_t launch_step_f64(const KParams64 &kp, int riemann, const CUtensorMap &tm_q, int use_tma,

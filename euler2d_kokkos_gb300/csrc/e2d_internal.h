@@ -75,10 +75,13 @@ struct KParams32 {
   long long wplane;  // wpitch * jsize
   int variant;       // step kernel register-budget variant (see launch_f32c_step)
   int strip_h;       // rows per warp strip of the step kernel
-  int wait_test;     // nonzero: strip (1, 0) never stages its first row, so its bounded
-                     // wait runs out (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
+  int short_rows;    // 2, 4 or 8: the single grid's step runs short strips of so many rows; 0: strip_h
+  int wait_test;     // nonzero: strip (1, 0) never stages its first row, or a multi-step launch's
+                     // barrier waits for a block too many, so that the bounded wait runs out
+                     // (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
 };
 int default_strip_h(int nx, int ny);
+int default_short_rows(int nx, int ny);
 
 // Device-resident loop state of the time loop of src/main.cpp:100-145.
 struct DevClock {
@@ -97,7 +100,15 @@ struct DevClock {
   // acc[(n + 1) & 1]
   unsigned long long acc[2];
   double *trace;  // FP32 path: device dt trace (trace_cap entries) or null
+  // multi-step launches (k_loop_*): blocks that reached the step's barrier,
+  // and the CFL maxima of three consecutive states (step s reads [s % 3],
+  // folds into [(s + 1) % 3] and clears [(s + 2) % 3])
+  unsigned int arrived;
+  unsigned int loop_pad;
+  unsigned long long acc3[3];
 };
+// Most steps one multi-step launch takes.
+constexpr int kLoopSteps = 1024;
 
 enum : unsigned int {
   E2D_FLAG_NONFINITE = 1u,  // a state value is NaN or Inf
@@ -127,6 +138,13 @@ cudaError_t launch_fill_f64(const KParams64 &kp, double *u_in, double *u_out, do
 cudaError_t launch_step_f64(const KParams64 &kp, int riemann, const CUtensorMap &tm_q, int use_tma,
                             const double *q_in, double *q_out, double *u_in, double *u_out, DevClock *clk,
                             double *dt_trace, cudaStream_t s);
+// Blocks of a multi-step launch of the fused step, all resident at once
+// (0: the grid is too large for it), and that launch: up to `steps` steps
+// with a grid barrier between them, from states u[0], u[1] and their
+// primitives, beginning at clk's t and nstep.
+int f64_loop_blocks(const KParams64 &kp, int riemann);
+cudaError_t launch_loop_f64(const KParams64 &kp, int riemann, int blocks, double *const u[2], double *const q[2],
+                            DevClock *clk, double *dt_trace, int steps, cudaStream_t s);
 // The reference's implementations 1 and 2 of the step (e2d_impl12.cu), after
 // a fill with FILL_WRITE_Q | FILL_GHOSTS_IN | FILL_COPY_OUT (and FILL_DT |
 // FILL_DEVICE_CLOCK in the device loop, use_clock = 1); implementation 1 needs
@@ -177,6 +195,11 @@ bool encode_f32c_map(CUtensorMap *map, const float *w, const KParams32 &kp);
 // One FP32C step; tm_in: the map of w_in.
 cudaError_t launch_f32c_step(const KParams32 &kp, int riemann, const float *w_in, float *w_out,
                              const CUtensorMap &tm_in, DevClock *clk, int use_clock, double host_dt,
+                             cudaStream_t s);
+
+// The same as f64_loop_blocks and launch_loop_f64, for grids that run short strips.
+int f32c_loop_blocks(const KParams32 &kp, int riemann);
+cudaError_t launch_loop_f32c(const KParams32 &kp, int riemann, int blocks, float *const w[2], DevClock *clk, int steps,
                              cudaStream_t s);
 
 // ---------------------------------------------------------------- batches
