@@ -1,8 +1,9 @@
 // e2d_batch.cu -- batched solves: many independent simulations of uneven
 // size resident in one device memory pool, advanced together by one kernel
-// launch per iteration for the FP32C instances (k_batch_f32c) and one for
-// the FP64 ones (k_batch_step_f64) with per-instance dt, replayed from CUDA
-// graphs; admission by free pool bytes; strip height per size class and
+// launch per iteration for the FP32C instances (k_batch_f32c, replayed from
+// CUDA graphs), or one per run call when they are few (k_batch_loop_f32c),
+// and one per run call for the FP64 ones (k_batch_loop_f64), with
+// per-instance dt; admission by free pool bytes; strip height per size class and
 // the kernel's register budget set by a measured autotuner.
 #include "e2d_internal.h"
 
@@ -86,6 +87,20 @@ struct HostInst {
   unsigned int status() const { return fp64 ? mirror64.status : mirror.status; }
 };
 
+// A table entry from a kernel argument: the record is taken at the launch,
+// so the caller need not keep it (or wait) as for a copy from host memory.
+template <class T>
+__global__ void k_put_record(T *dst, const __grid_constant__ T rec) {
+  static_assert(sizeof(T) % 4 == 0, "copied by words");
+  const int *src = reinterpret_cast<const int *>(&rec);
+  for (int k = threadIdx.x; k < (int)(sizeof(T) / 4); k += blockDim.x) reinterpret_cast<int *>(dst)[k] = src[k];
+}
+template <class T>
+cudaError_t put_record(T *dst, const T &rec, cudaStream_t s) {
+  k_put_record<T><<<1, 128, 0, s>>>(dst, rec);
+  return cudaGetLastError();
+}
+
 int size_class_of(int nx, int ny) {
   const int s = std::max(nx, ny);
   return s <= 192 ? 0 : s <= 512 ? 1 : 2;
@@ -111,12 +126,19 @@ struct e2d_batch {
   int *d_list64 = nullptr;           // slots (max_inst), then tile_begin (max_inst + 1)
   std::vector<int> list64;           // slots of the current FP64 work list
   int total_tiles = 0;
-  int sm_count = 152;  // multiprocessors of the batch's device (the FP64 kernel's persistent grid)
+  int shape64 = 0, ty64 = 16;  // tile of the current FP64 work list
+  int short_rows = 0;          // rows of the FP32C list's short strips (the list counts fold units); 0: strips
+  bool tuned_by_caller = false;  // set_tuning named a kernel variant: lists keep to it
+  unsigned int *d_arrived = nullptr;  // barrier words of the multi-iteration launches (FP32C, FP64)
   bool list_dirty = true;
   int grid = 0;
   std::map<int, cudaGraphExec_t> graphs;  // iterations -> graph of the current list
   std::string err;
   long long cell_updates = 0;  // interior cell-updates done by run calls
+  // pinned copies of the device tables' used part, where the mirrors are read from
+  BatchInst *h_insts = nullptr;
+  BatchInst64 *h_insts64 = nullptr;
+  bool mirrors_stale = false;  // an instance admitted since the tables were last read back
 };
 
 namespace {
@@ -144,37 +166,47 @@ size_t inst_bytes(const KParams32 &kp) { return (size_t)2 * 8 * kp.wplane * size
 size_t inst_bytes64(const KGeom &g) { return (size_t)4 * 4 * g.plane * sizeof(double); }
 
 int sync_mirrors(e2d_batch *b) {
-  std::vector<BatchInst> tmp(b->max_inst);
-  std::vector<BatchInst64> tmp64(b->max_inst);
-  B_CK(b, cudaMemcpyAsync(tmp.data(), b->d_insts, sizeof(BatchInst) * b->max_inst, cudaMemcpyDeviceToHost,
-                          b->stream), "table download");
-  B_CK(b, cudaMemcpyAsync(tmp64.data(), b->d_insts64, sizeof(BatchInst64) * b->max_inst, cudaMemcpyDeviceToHost,
-                          b->stream), "table download");
+  int n32 = 0, n64 = 0;  // table entries up to the last used one of each kind
+  for (int k = 0; k < b->max_inst; ++k)
+    if (b->slots[k].used) (b->slots[k].fp64 ? n64 : n32) = k + 1;
+  if (n32)
+    B_CK(b, cudaMemcpyAsync(b->h_insts, b->d_insts, sizeof(BatchInst) * n32, cudaMemcpyDeviceToHost, b->stream),
+         "table download");
+  if (n64)
+    B_CK(b, cudaMemcpyAsync(b->h_insts64, b->d_insts64, sizeof(BatchInst64) * n64, cudaMemcpyDeviceToHost, b->stream),
+         "table download");
   B_CK(b, cudaStreamSynchronize(b->stream), "table sync");
   for (int k = 0; k < b->max_inst; ++k) {
     HostInst &h = b->slots[k];
     if (!h.used) continue;
     if (h.fp64)
-      h.mirror64 = tmp64[k];
+      h.mirror64 = b->h_insts64[k];
     else
-      h.mirror = tmp[k];
+      h.mirror = b->h_insts[k];
   }
+  b->mirrors_stale = false;
   return E2D_OK;
 }
 
-// The FP64 work list: used, active FP64 instances with their tiles.
+// The FP64 work list: used, active FP64 instances with their tiles, of the
+// shape that suits them together.
 int rebuild_list64(e2d_batch *b) {
-  std::vector<int> list, tb;
-  int nt = 0;
+  std::vector<int> list, tb, dims;
   for (int k = 0; k < b->max_inst; ++k) {
     HostInst &h = b->slots[k];
     if (!h.used || !h.fp64 || !h.mirror64.active) continue;
     list.push_back(k);
-    tb.push_back(nt);
-    nt += h.mirror64.ntiles;
+    dims.push_back(h.p.nx);
+    dims.push_back(h.p.ny);
   }
-  tb.push_back(nt);
+  int nt = 0;
   if (!list.empty()) {
+    choose_f64_tile(reinterpret_cast<const int(*)[2]>(dims.data()), (int)list.size(), false, -1, &b->shape64, &b->ty64);
+    for (int k : list) {
+      tb.push_back(nt);
+      nt += f64_tiles(b->slots[k].p.nx, b->slots[k].p.ny, b->shape64, b->ty64);
+    }
+    tb.push_back(nt);
     const size_t m = (size_t)b->max_inst;
     B_CK(b, cudaMemcpyAsync(b->d_list64, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, b->stream),
          "list upload");
@@ -190,12 +222,18 @@ int rebuild_list64(e2d_batch *b) {
 // size class, lowered (to 16 rows at least) while the list has fewer strips
 // than the grid has warps -- the tail of a batch, when a few large instances
 // are left, would otherwise leave SMs idle.  Results do not depend on it.
+// A list of few fold units runs in short strips instead (short_rows_for):
+// its iterations wait on the march of one strip, not on throughput.
 int rebuild_list(e2d_batch *b) {
   std::vector<int> list, begin;
-  const int per_sm = batch_blocks_per_sm(b->riemann, b->variant);
+  long long units = 0;
+  for (HostInst &h : b->slots)
+    if (h.used && !h.fp64 && h.mirror.active) units += units_of(h.mirror.kp);
+  b->short_rows = b->tuned_by_caller ? 0 : short_rows_for(units);
+  const int per_sm = b->short_rows > 0 ? 1 : batch_blocks_per_sm(b->riemann, b->variant);
   const long long warps = 152LL * per_sm * 4;
   int shift = 0;
-  for (;; ++shift) {
+  for (; b->short_rows == 0; ++shift) {
     long long n = 0;
     bool all_min = true;
     for (int k = 0; k < b->max_inst; ++k) {
@@ -212,6 +250,12 @@ int rebuild_list(e2d_batch *b) {
   for (int k = 0; k < b->max_inst; ++k) {
     HostInst &h = b->slots[k];
     if (!h.used || h.fp64 || !h.mirror.active) continue;
+    list.push_back(k);
+    begin.push_back(total);
+    if (b->short_rows > 0) {
+      total += units_of(h.mirror.kp);
+      continue;
+    }
     const int sh = std::max(16, ((b->strip_h[h.size_class] >> shift) / 16) * 16);
     if (h.mirror.kp.strip_h != sh) {
       h.mirror.kp.strip_h = sh;
@@ -221,8 +265,6 @@ int rebuild_list(e2d_batch *b) {
       B_CK(b, cudaMemcpyAsync(&b->d_insts[k].nstrips, &h.mirror.nstrips, sizeof(int), cudaMemcpyHostToDevice,
                               b->stream), "nstrips upload");
     }
-    list.push_back(k);
-    begin.push_back(total);
     total += h.mirror.nstrips;
   }
   begin.push_back(total);
@@ -246,21 +288,27 @@ int rebuild_list(e2d_batch *b) {
 }
 
 int launch_iterations(e2d_batch *b, int iterations) {
+  const int m = b->max_inst;
+  if (!b->list64.empty())
+    B_CK(b, launch_batch_f64(b->riemann, b->d_insts64, b->d_list64, b->d_list64 + m, (int)b->list64.size(),
+                             b->total_tiles, b->shape64, b->ty64, iterations, b->d_arrived + 1, b->stream),
+         "batch launch");
+  if (b->list.empty()) return E2D_OK;
+  if (b->short_rows > 0) {
+    B_CK(b, launch_batch_loop_f32c(b->riemann, b->short_rows, b->d_insts, b->d_list, b->d_list + m,
+                                   (int)b->list.size(), b->total_strips, iterations, b->d_arrived, b->stream),
+         "batch launch");
+    return E2D_OK;
+  }
   auto it = b->graphs.find(iterations);
   cudaGraphExec_t exec = nullptr;
   if (it == b->graphs.end()) {
     cudaGraph_t graph;
     B_CK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "capture");
     cudaError_t le = cudaSuccess;
-    const int m = b->max_inst;
-    for (int k = 0; k < iterations && le == cudaSuccess; ++k) {
-      if (!b->list.empty())
-        le = launch_batch_f32c(b->riemann, b->variant, b->d_insts, b->d_list, b->d_list + m, (int)b->list.size(),
-                               b->total_strips, b->grid, b->stream);
-      if (le == cudaSuccess && !b->list64.empty())
-        le = launch_batch_f64(b->riemann, b->d_insts64, b->d_list64, b->d_list64 + m, (int)b->list64.size(),
-                              b->total_tiles, b->sm_count, b->stream);
-    }
+    for (int k = 0; k < iterations && le == cudaSuccess; ++k)
+      le = launch_batch_f32c(b->riemann, b->variant, b->d_insts, b->d_list, b->d_list + m, (int)b->list.size(),
+                             b->total_strips, b->grid, b->stream);
     cudaError_t ee = cudaStreamEndCapture(b->stream, &graph);
     if (le != cudaSuccess || ee != cudaSuccess) return berr(b, E2D_ECUDA, "batch capture");
     cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
@@ -303,7 +351,7 @@ int admit64(e2d_batch *b, const e2d_params &p, double t_end, const double *u0, i
   if (cudaMemcpyAsync(u1d, u0d, state_bytes, cudaMemcpyDeviceToDevice, b->stream) != cudaSuccess)
     return undo(E2D_ECUDA, "admit: copy");
   BatchInst64 I{};
-  batch_f64_shape(kp, &I.nbx, &I.nfill, &I.ntx, &I.ntiles);
+  batch_f64_shape(kp, &I.nbx, &I.nfill);
   I.kp = kp;
   I.u[0] = u0d;
   I.u[1] = u1d;
@@ -313,11 +361,11 @@ int admit64(e2d_batch *b, const e2d_params &p, double t_end, const double *u0, i
   I.t_end = t_end;
   I.active = I.t < I.t_end;
   HostInst &h = b->slots[slot];
-  if (cudaMemcpyAsync(&b->d_insts64[slot], &I, sizeof(I), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
+  if (put_record(&b->d_insts64[slot], I, b->stream) != cudaSuccess ||
       launch_batch_prime_f64(&b->d_insts64[slot], I.nfill, b->stream) != cudaSuccess ||
-      cudaMemcpyAsync(&I, &b->d_insts64[slot], sizeof(I), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
-      cudaStreamSynchronize(b->stream) != cudaSuccess)
+      (u0 && cudaStreamSynchronize(b->stream) != cudaSuccess))  // u0 is the caller's again
     return undo(E2D_ECUDA, "admit: table upload");
+  b->mirrors_stale = true;
   h.used = true;
   h.fp64 = true;
   h.p = p;
@@ -347,19 +395,16 @@ int e2d_batch_create(int riemann, size_t pool_bytes, int max_instances, e2d_batc
     return st;
   };
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(E2D_ECUDA);
-  {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      return fail(E2D_ECUDA);
-    b->sm_count = sms;
-  }
   if (cudaMalloc(&b->pool, pool_bytes) != cudaSuccess) return fail(E2D_ENOMEM);
   b->pool_bytes = pool_bytes;
   b->alloc.reset(pool_bytes);
   if (cudaMalloc(&b->d_insts, sizeof(BatchInst) * (size_t)max_instances) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMalloc(&b->d_list, sizeof(int) * (2 * (size_t)max_instances + 1)) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMalloc(&b->d_insts64, sizeof(BatchInst64) * (size_t)max_instances) != cudaSuccess) return fail(E2D_ENOMEM);
+  if (cudaMallocHost(&b->h_insts, (sizeof(BatchInst) + sizeof(BatchInst64)) * (size_t)max_instances) != cudaSuccess)
+    return fail(E2D_ENOMEM);
+  b->h_insts64 = reinterpret_cast<BatchInst64 *>(b->h_insts + max_instances);
+  if (cudaMalloc(&b->d_arrived, 2 * sizeof(unsigned int)) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMalloc(&b->d_list64, sizeof(int) * (2 * (size_t)max_instances + 1)) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMemsetAsync(b->d_insts, 0, sizeof(BatchInst) * (size_t)max_instances, b->stream) != cudaSuccess ||
       cudaMemsetAsync(b->d_insts64, 0, sizeof(BatchInst64) * (size_t)max_instances, b->stream) != cudaSuccess)
@@ -381,6 +426,9 @@ int e2d_batch_destroy(e2d_batch *b) {
   if (b->d_list) cudaFree(b->d_list);
   if (b->d_insts64) cudaFree(b->d_insts64);
   if (b->d_list64) cudaFree(b->d_list64);
+  if (b->d_arrived) cudaFree(b->d_arrived);
+  if (b->h_insts) cudaFreeHost(b->h_insts);
+
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return E2D_OK;
@@ -466,15 +514,18 @@ int e2d_batch_admit(e2d_batch *b, const e2d_params *pin, double t_end, const dou
   I.nsx = (kp.g.nx + 59) / 60;
   I.nstrips = strips_of(kp);
   BatchInst *dI = &b->d_insts[slot];
-  if (cudaMemcpyAsync(dI, &I, sizeof(I), cudaMemcpyHostToDevice, b->stream) != cudaSuccess)
+  if (put_record(dI, I, b->stream) != cudaSuccess)
     return undo(E2D_ECUDA, "admit: table upload");
   if (launch_f32c_dt_to(kp, w0, &dI->acc[0], &dI->status, b->stream) != cudaSuccess)
     return undo(E2D_ECUDA, "admit: dt");
   if (launch_batch_arm(dI, b->stream) != cudaSuccess) return undo(E2D_ECUDA, "admit: arm");
+  // the caller's u0 is its own again after this call; everything else --
+  // the staging bytes included -- is used in stream order
+  if (u0 && cudaStreamSynchronize(b->stream) != cudaSuccess) return undo(E2D_ECUDA, "admit: sync");
   HostInst &h = b->slots[slot];
-  if (cudaMemcpyAsync(&h.mirror, dI, sizeof(BatchInst), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
-      cudaStreamSynchronize(b->stream) != cudaSuccess)
-    return undo(E2D_ECUDA, "admit: sync");
+  I.active = I.t < I.t_end;  // as k_batch_arm finds it unless the state is bad
+  h.mirror = I;
+  b->mirrors_stale = true;
   b->alloc.release(soff, stage_bytes);
   h.used = true;
   h.fp64 = false;
@@ -489,21 +540,22 @@ int e2d_batch_admit(e2d_batch *b, const e2d_params *pin, double t_end, const dou
 
 int e2d_batch_release(e2d_batch *b, int id) {
   if (!b || id < 0 || id >= b->max_inst || !b->slots[id].used) return E2D_EINVAL;
-  B_CK(b, cudaStreamSynchronize(b->stream), "release sync");
   HostInst &h = b->slots[id];
+  // in stream order: the bytes' and the entry's next user comes after
+  B_CK(b, h.fp64 ? cudaMemsetAsync(&b->d_insts64[id], 0, sizeof(BatchInst64), b->stream)
+                 : cudaMemsetAsync(&b->d_insts[id], 0, sizeof(BatchInst), b->stream), "release");
   b->alloc.release(h.off, h.bytes);
   h.used = false;
-  BatchInst zero{};
-  BatchInst64 zero64{};
-  B_CK(b, cudaMemcpyAsync(&b->d_insts[id], &zero, sizeof(zero), cudaMemcpyHostToDevice, b->stream), "release");
-  B_CK(b, cudaMemcpyAsync(&b->d_insts64[id], &zero64, sizeof(zero64), cudaMemcpyHostToDevice, b->stream), "release");
-  B_CK(b, cudaStreamSynchronize(b->stream), "release sync");
   b->list_dirty = true;
   return E2D_OK;
 }
 
 int e2d_batch_query(e2d_batch *b, int id, double *t, int *nstep, int *active) {
   if (!b || id < 0 || id >= b->max_inst || !b->slots[id].used) return E2D_EINVAL;
+  if (b->mirrors_stale) {
+    const int rc = sync_mirrors(b);
+    if (rc != E2D_OK) return rc;
+  }
   const HostInst &m = b->slots[id];
   if (t) *t = m.t();
   if (nstep) *nstep = m.nstep();
@@ -585,7 +637,10 @@ int e2d_batch_stats(e2d_batch *b, long long *cell_updates, int *n_used) {
 
 int e2d_batch_set_tuning(e2d_batch *b, int variant, const int strip_h[3]) {
   if (!b) return E2D_EINVAL;
-  if (variant >= 0 && variant < kF32cVariants) b->variant = variant;
+  if (variant >= 0 && variant < kF32cVariants) {
+    b->variant = variant;
+    b->tuned_by_caller = true;
+  }
   // strip heights are whole CFL fold units (16 rows)
   if (strip_h)
     for (int c = 0; c < 3; ++c)
@@ -608,6 +663,13 @@ int e2d_batch_get_tuning(const e2d_batch *b, int *variant, int strip_h[3]) {
 // timing candidates are ordinary progress of the batch.
 int e2d_batch_autotune(e2d_batch *b, int iters_per_trial) {
   if (!b || iters_per_trial <= 0) return E2D_EINVAL;
+  b->tuned_by_caller = false;
+  {
+    // a list in short strips leaves nothing to choose
+    int rc = rebuild_list(b);
+    if (rc != E2D_OK) return rc;
+    if (b->list.empty() || b->short_rows > 0) return E2D_OK;
+  }
   cudaEvent_t e0, e1;
   B_CK(b, cudaEventCreate(&e0), "event");
   B_CK(b, cudaEventCreate(&e1), "event");

@@ -114,7 +114,8 @@ void e2d::make_kparams(const e2d_params &p, KParams64 *kp) {
   kp->ph.inv_dy = 1.0 / p.dy;
   kp->fast = p.precision == E2D_PRECISION_FP64_FAST ? 1 : 0;
   const char *tile = std::getenv("E2D_F64_TILE");
-  choose_f64_tile(p.nx, p.ny, tile ? std::atoi(tile) : -1, &kp->shape, &kp->ty);
+  const int dims[1][2] = {{p.nx, p.ny}};
+  choose_f64_tile(dims, 1, kp->fast != 0, tile ? std::atoi(tile) : -1, &kp->shape, &kp->ty);
   const char *wt = std::getenv("E2D_TEST_WAIT_TIMEOUT");
   kp->wait_test = (wt && std::atoi(wt) != 0) ? 1 : 0;
 }

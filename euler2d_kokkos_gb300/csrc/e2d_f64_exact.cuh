@@ -115,12 +115,14 @@ static __device__ double2 g_unit[32] = {
 //
 // XMUL: xmul() forms the product on the integer pipes (35 instructions, about
 // 60 clocks, overlapping the FP64 pipe's 64).  With about a fifth of a step's
-// products there -- face increments, transport terms, contact sums, energies,
-// flux scaling -- the two pipes run side by side: 1.556 instead of 1.69 ms a
-// 2048^2 HLLC step; with more of them the step slows down again (1.57 to 1.63
-// ms).  Where each SM holds one small tile the step waits on latency, not on
-// the FP64 pipe, and the plain product is the faster one (64x48: 16.0
-// against 17.1 us a step).
+// products there the two pipes run side by side.  HLLC: face increments,
+// transport terms, contact sums, energies, flux scaling, 1.556 instead of 1.69
+// ms a 2048^2 step; with more of them the step slows down again (1.57 to 1.63
+// ms).  HLL: energies, momentum and energy fluxes, jump terms too, 1.866 ->
+// 1.761 ms.  The fast forms, which have the fewest FP64 instructions: all
+// products that are not part of an FMA, 1.308 -> 1.236 ms.  Where each SM holds
+// one small tile the step waits on latency, not on the FP64 pipe, and the
+// plain product is the faster one (64x48: 16.0 against 17.1 us a step).
 template <bool XMUL>
 struct FpT {
   double one, mzero, mone;

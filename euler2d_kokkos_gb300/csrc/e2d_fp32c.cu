@@ -35,6 +35,8 @@
 
 #include <cstdint>
 #include <cstdlib>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 namespace e2d {
@@ -1211,21 +1213,25 @@ __global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
 // The loop-state advance of src/main.cpp:139-143 plus the next dt (:128-134)
 // for one instance; run by the instance's last strip of an iteration.
 __device__ __forceinline__ void batch_finalize(BatchInst &I) {
-  const int n = I.nstep;
-  const double dt = I.dt;
-  if (!(dt > 0.0) || nonfinite64(dt)) I.status |= E2D_FLAG_BAD_DT;
-  const double t = I.t + dt;
+  const int n = __ldcg(&I.nstep);
+  const double dt = __ldcg(&I.dt), t_end = __ldcg(&I.t_end);
+  const double inv_dt = __longlong_as_double((long long)__ldcg(&I.acc[(n + 1) & 1]));
+  unsigned int status = __ldcg(&I.status);
+  if (!(dt > 0.0) || nonfinite64(dt)) {
+    status |= E2D_FLAG_BAD_DT;
+    I.status = status;
+  }
+  const double t = __ldcg(&I.t) + dt;
   I.t = t;
   I.nstep = n + 1;
-  I.par ^= 1;
+  I.par = __ldcg(&I.par) ^ 1;
   I.acc[n & 1] = 0ull;
-  const double inv_dt = __longlong_as_double((long long)I.acc[(n + 1) & 1]);
-  double dtn = I.kp.ph64.cfl / inv_dt;
-  if (t + dtn > I.t_end) dtn = I.t_end - t;
+  double dtn = quot64(I.kp.ph64.cfl, inv_dt);
+  if (t + dtn > t_end) dtn = t_end - t;
   I.dt = dtn;
-  I.dtdx = (float)(dtn / I.kp.ph64.dx);
-  I.dtdy = (float)(dtn / I.kp.ph64.dy);
-  I.active = (t < I.t_end) && !(I.status & (E2D_FLAG_NONFINITE | E2D_FLAG_BAD_DT | E2D_FLAG_TIMEOUT));
+  I.dtdx = (float)quot64(dtn, I.kp.ph64.dx);
+  I.dtdy = (float)quot64(dtn, I.kp.ph64.dy);
+  I.active = (t < t_end) && !(status & (E2D_FLAG_NONFINITE | E2D_FLAG_BAD_DT | E2D_FLAG_TIMEOUT));
   I.done = 0u;
 }
 
@@ -1283,6 +1289,66 @@ __global__ void __launch_bounds__(NT, MINB)
       }
     }
     __syncwarp();
+  }
+}
+
+// `iterations` steps of a batch too small to fill the GPU with whole fold
+// units, in one cooperative launch: each block takes the same units of the
+// list in every iteration, marches them in short strips (short_unit) with the
+// instance's own dt, and the last unit of an instance advances its loop
+// state; a grid barrier separates iterations.
+template <int RS, int SUB, int MINB>
+__global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
+    k_batch_loop_f32c(BatchInst *insts, const int *__restrict__ list_slots, const int *__restrict__ unit_begin,
+                      const int n_inst, const int units, const int iterations, unsigned int *arrived) {
+  constexpr int NTS = 32 * (CFL_UNIT_ROWS / SUB);
+  __shared__ KParams32 s_kp;  // of the instance at hand
+  int held = -1;
+  for (int it = 0; it < iterations; ++it) {
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+      int lo = 0, hi = n_inst;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (unit_begin[mid] <= u)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      BatchInst &I = insts[list_slots[lo]];
+      const int active = __ldcg(&I.active), par = __ldcg(&I.par), ns = __ldcg(&I.nstep);
+      const float dtdx = __ldcg(&I.dtdx), dtdy = __ldcg(&I.dtdy);
+      __syncthreads();  // the previous unit is done with s_kp and the winners' table
+      if (lo != held) {
+        static_assert(sizeof(KParams32) % 4 == 0, "copied by words");
+        for (int j = threadIdx.x; j < (int)(sizeof(KParams32) / 4); j += NTS)
+          reinterpret_cast<int *>(&s_kp)[j] = reinterpret_cast<const int *>(&I.kp)[j];
+        held = lo;
+        __syncthreads();
+      }
+      if (!active) continue;  // block-uniform
+      short_unit<RS, SUB>(s_kp, I.w[par], I.w[par ^ 1], u - unit_begin[lo], &I.acc[(ns + 1) & 1], &I.status,
+                          [&]() { return make_float2(dtdx, dtdy); });
+      if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned int ticket = atomicAdd(&I.done, 1u);
+        const int nsx = (s_kp.g.nx + OUTW - 1) / OUTW;
+        if (ticket == (unsigned)(nsx * ((s_kp.g.ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS)) - 1u) {
+          __threadfence();
+          batch_finalize(I);
+          __threadfence();
+        }
+      }
+    }
+    if (!grid_barrier(arrived, (unsigned)(it + 1) * gridDim.x)) {
+      // the states of this block's units are incomplete: their instances stop
+      for (int u = blockIdx.x; threadIdx.x == 0 && u < units; u += gridDim.x) {
+        int k = 0;
+        while (k + 1 < n_inst && unit_begin[k + 1] <= u) ++k;
+        atomicOr(&insts[list_slots[k]].status, (unsigned)E2D_FLAG_TIMEOUT);
+        insts[list_slots[k]].active = 0;
+      }
+      return;
+    }
   }
 }
 
@@ -1387,17 +1453,19 @@ int batch_blocks_per_sm(int riemann, int variant) {
   }
 }
 
-// Rows per warp strip: the largest of 64, 32, 16 that still gives at least
-// four waves of strips for the resident warps (152 SMs x 12 warps of the
-// default variant): taller strips cost less halo ((h + 4) / h rows loaded per
-// output row), more waves leave less of the last one idle.  Measured, FP32C
-// HLLC: 8192^2 64 rows (55.4 Gcell/s; 32: 54.0), 4096^2 32 rows (48.5; 64:
-// 46.8, 16: 45.2), 2048^2 all within 1 %.
+// Rows per warp strip, by the strips it gives against the warps that run at
+// once (152 SMs x 12): the shortest while its strips are one wave; one wave
+// of taller strips rather than a second wave begun (1500^2: 32 rows 59.5 us a
+// step, 16 64.9); 16 while 32 would begin a second wave (2048^2: 97.6, 32
+// rows 103.4); then the tallest with two waves of 32 rows (3000^2: 169 against
+// 176 with 16) or four of 64 (8192^2: 992; 32 rows 1016): taller strips load
+// and march less halo, more waves leave less of the last one idle.
 int default_strip_h(int nx, int ny) {
-  const long long nsx = (nx + OUTW - 1) / OUTW;
-  for (int h = 64; h > 16; h /= 2)
-    if (nsx * ((ny + h - 1) / h) >= 152LL * 12 * 4) return h;
-  return 16;
+  const long long wave = 152 * 12;
+  auto strips = [&](int h) { return (long long)((nx + OUTW - 1) / OUTW) * ((ny + h - 1) / h); };
+  if (strips(64) >= 4 * wave) return 64;
+  if (strips(32) >= 2 * wave) return 32;
+  return strips(16) > wave && strips(32) <= wave ? 32 : 16;
 }
 
 // Rows of a grid's short strips (0: strips of default_strip_h rows), by the
@@ -1409,9 +1477,9 @@ int default_strip_h(int nx, int ny) {
 // 17.1 / 12.0 / 16.2 against 30.2; 700^2 (528) 35.9 / 21.4 / 19.6 against
 // 36.3; 1201x700 (924) 57 / 39 / 31.1 against 35.0; 1024^2 (1152) 70 / 44 /
 // 37.6 against 35.7.
+int short_rows_for(long long units) { return units <= 152 ? 2 : units <= 304 ? 4 : units <= 1000 ? 8 : 0; }
 int default_short_rows(int nx, int ny) {
-  const long long units = (long long)((nx + OUTW - 1) / OUTW) * ((ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS);
-  return units <= 152 ? 2 : units <= 304 ? 4 : units <= 1000 ? 8 : 0;
+  return short_rows_for((long long)((nx + OUTW - 1) / OUTW) * ((ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS));
 }
 
 void make_kparams32(const e2d_params &p, KParams32 *kp) {
@@ -1465,6 +1533,8 @@ static cudaError_t configure_rs() {
       constexpr int bytes = (int)ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / S);
       e = cudaFuncSetAttribute(k_step_f32c_short<RS, S, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loop_f32c<RS, S, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_batch_loop_f32c<RS, S, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     });
   if (e == cudaSuccess)  // variant 7 (single-grid step only)
     e = cudaFuncSetAttribute(k_step_f32c<RS, 3, 3, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring_bytes(3));
@@ -1472,9 +1542,17 @@ static cudaError_t configure_rs() {
 }
 
 cudaError_t configure_f32c_kernels() {
-  cudaError_t e = configure_rs<E2D_RIEMANN_HLLC>();
+  static std::mutex mutex;
+  static std::map<int, bool> done;  // per device, for the life of the process
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mutex);
+  if (done[dev]) return cudaSuccess;
+  e = configure_rs<E2D_RIEMANN_HLLC>();
   if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_HLL>();
   if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_APPROX>();
+  done[dev] = e == cudaSuccess;
   return e;
 }
 
@@ -1541,7 +1619,7 @@ static void launch_short_v(const KParams32 &kp, int riemann, int blocks, const f
   }
 }
 
-static int units_of(const KParams32 &kp) {
+int units_of(const KParams32 &kp) {
   return ((kp.g.nx + OUTW - 1) / OUTW) * ((kp.g.ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS);
 }
 
@@ -1563,16 +1641,42 @@ int f32c_loop_blocks(const KParams32 &kp, int riemann) {
   if (kp.short_rows <= 0) return 0;
   int blocks = 0;
   with_loop(kp, riemann, [&](auto kernel, int threads, size_t sm) {
-    int dev = 0, sms = 0, per_sm = 0, coop = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sm) != cudaSuccess)
-      return;
+    const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), threads, sm);
     const int units = units_of(kp);
-    if (units <= 2 * sms * per_sm) blocks = units < sms * per_sm ? units : sms * per_sm;
+    if (units <= 2 * resident) blocks = units < resident ? units : resident;
   });
   return blocks;
+}
+
+template <int RS>
+static cudaError_t launch_batch_loop_t(int rows, BatchInst *insts, const int *list_slots, const int *unit_begin,
+                                       int n_inst, int units, int iterations, unsigned int *arrived, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
+  with_short(rows, [&](auto sub, auto minb) {
+    constexpr int S = decltype(sub)::value, M = decltype(minb)::value, threads = 32 * (CFL_UNIT_ROWS / S);
+    const void *kernel = reinterpret_cast<const void *>(k_batch_loop_f32c<RS, S, M>);
+    const size_t sm = ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / S);
+    const int resident = resident_blocks(kernel, threads, sm);
+    const int grid = units < resident ? units : resident;
+    void *args[] = {&insts, &list_slots, &unit_begin, &n_inst, &units, &iterations, &arrived};
+    if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, sm, s);
+  });
+  return e;
+}
+
+cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, const int *list_slots,
+                                   const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
+                                   cudaStream_t s) {
+  if (n_inst <= 0 || units <= 0 || iterations <= 0) return cudaSuccess;
+  switch (riemann) {
+    case E2D_RIEMANN_HLLC:
+      return launch_batch_loop_t<E2D_RIEMANN_HLLC>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived, s);
+    case E2D_RIEMANN_HLL:
+      return launch_batch_loop_t<E2D_RIEMANN_HLL>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived, s);
+    default:
+      return launch_batch_loop_t<E2D_RIEMANN_APPROX>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived, s);
+  }
 }
 
 cudaError_t launch_loop_f32c(const KParams32 &kp, int riemann, int blocks, float *const w[2], DevClock *clk, int steps,

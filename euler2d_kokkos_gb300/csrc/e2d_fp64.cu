@@ -5,7 +5,7 @@
 // The device time loop runs one fused launch per step (k_step_f64, after a
 // prologue k_fill_f64 that folds the first step's CFL maximum and writes the
 // primitives of the initial state); FP64 batch instances run the same fused
-// step in one persistent launch per iteration (k_batch_step_f64).  The
+// step in one launch per run call (k_batch_loop_f64).  The
 // host-driven godunov_unsplit runs it as two launches:
 //   k_fill_f64         ghost fill (make_boundaries, src/HydroRun.h:388-399)
 //                      into both states, primitives of every cell
@@ -27,6 +27,9 @@
 
 #include <cmath>
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <utility>
 
 namespace e2d {
 namespace {
@@ -766,73 +769,97 @@ __global__ void __launch_bounds__(FILL_BX *FILL_BY) k_batch_prime_f64(BatchInst6
   fill_reduce(term, flags, &I->acc[0], &I->status);
 }
 
-// One iteration of every listed FP64 instance in one persistent launch: each
-// block takes tiles from the work list (instance k's tiles are
-// tile_begin[k] .. tile_begin[k+1]-1) and runs the fused step on each with
-// its instance's dt, primitives and ghost cells (tiles gathered, no TMA);
-// the instance's last tile advances its loop state.
-constexpr int BTX = 32, BTY = 32, BNT = 512, BMINB = 1;
-template <int RS>
-__global__ void __launch_bounds__(BNT, BMINB)
-    k_batch_step_f64(BatchInst64 *__restrict__ insts, const int *__restrict__ list_slots,
-                     const int *__restrict__ tile_begin, const int n_inst, const int total_tiles) {
+// `iterations` steps of every listed FP64 instance in one cooperative launch,
+// a grid barrier between them: each block takes the same TX x ty tiles of the
+// work list (instance k's tiles are tile_begin[k] .. tile_begin[k+1]-1) in
+// every iteration and runs the fused step on each with its instance's dt,
+// primitives and ghost cells (tiles gathered); the instance's last tile of an
+// iteration advances its loop state.  The tile is chosen for the whole list
+// (choose_f64_tile), so the last few solves of a batch still use every SM:
+// 32 x 32 tiles left a lone 256^2 solve on 64 of 152.
+template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL>
+__global__ void __launch_bounds__(NT, MINB)
+    k_batch_loop_f64(BatchInst64 *insts, const int *__restrict__ list_slots, const int *__restrict__ tile_begin,
+                     const int n_inst, const int total_tiles, const int ty, const int iterations,
+                     unsigned int *arrived) {
   extern __shared__ unsigned char smem_raw[];
-  double *smem = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  double *smem = reinterpret_cast<double *>(smem_raw);
   __shared__ double s_dt[3];
+  __shared__ KParams64 s_kp;  // of the instance at hand
   const int tid = threadIdx.x;
-  const Fp f;
-  for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
-    const int k = list_entry(tile_begin, n_inst, w);
-    BatchInst64 &I = insts[list_slots[k]];
-    if (!I.active) continue;  // block-uniform
-    const KParams64 &kp = I.kp;
-    const int par = I.par;
-    if (tid == 0) {
-      const double dt = step_dt(kp.ph, I.acc[par], I.t, I.t_end);
-      s_dt[0] = dt;
-      s_dt[1] = quot(dt, kp.ph.dx);
-      s_dt[2] = quot(dt, kp.ph.dy);
-    }
-    const int b = w - tile_begin[k];
-    const int by = b / I.ntx, bx = b - by * I.ntx;
-    const int nty = I.ntiles / I.ntx;
-    const int ty = kp.ty;
-    const int i0 = bx * BTX, j0 = by * ty;
-    gather_qtile<BTX, BNT>(kp.g, I.q[par], i0, j0, ty, smem);
-    __syncthreads();
-    double term = 0.0;
-    unsigned int flags = 0;
-    const double dtdx = s_dt[1], dtdy = s_dt[2];
-    tile_faces<BTX, BTY, BNT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
-    TileCells<BTX, BTY, BNT> cells;
-    cells.load(kp.g, I.u[par], i0, j0, ty);
-    __syncthreads();
-    tile_riemann<RS, BTX, BTY, BNT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
-    __syncthreads();
-    step_epilogue<BTX, BTY, BNT, false>(f, kp, cells, I.u[par ^ 1], I.q[par ^ 1], i0, j0, ty, dtdx, dtdy, smem, term,
-                                        flags);
-    ghost_fill_tile<BTX, BNT>(kp.g, I.u[par], I.u[par ^ 1], i0, j0, ty, bx == 0, bx == I.ntx - 1, by == 0,
-                              by == nty - 1);
-    block_fold<BNT>(term, flags, &I.acc[par ^ 1], &I.status);
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      const unsigned int ticket = atomicAdd(&I.done, 1u);
-      if (ticket == (unsigned)I.ntiles - 1u) {
-        __threadfence();
-        const double dt = s_dt[0];
-        if (!(dt > 0.0) || nonfinite(dt)) I.status |= E2D_FLAG_BAD_DT;
-        I.dt = dt;
-        I.t = I.t + dt;
-        I.nstep = I.nstep + 1;
-        I.par = par ^ 1;
-        I.acc[par] = 0ull;  // read by this step; folded into by the next
-        I.done = 0u;
-        I.active = (I.t < I.t_end) && !(I.status & (E2D_FLAG_NONFINITE | E2D_FLAG_BAD_DT));
-        __threadfence();
+  const f64x::FpT<XMUL> f;
+  const KParams64 &kp = s_kp;
+  int held = -1;  // list entry whose parameters are in s_kp
+  for (int it = 0; it < iterations; ++it) {
+    for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
+      const int k = list_entry(tile_begin, n_inst, w);
+      BatchInst64 &I = insts[list_slots[k]];
+      if (k != held) {
+        __syncthreads();
+        static_assert(sizeof(KParams64) % 4 == 0, "copied by words");
+        for (int j = tid; j < (int)(sizeof(KParams64) / 4); j += NT)
+          reinterpret_cast<int *>(&s_kp)[j] = reinterpret_cast<const int *>(&I.kp)[j];
+        held = k;
       }
+      if (!__ldcg(&I.active)) continue;  // block-uniform
+      const int par = __ldcg(&I.par);
+      __syncthreads();
+      if (tid == 0) {
+        const double dt = step_dt(kp.ph, __ldcg(&I.acc[par]), __ldcg(&I.t), __ldcg(&I.t_end));
+        s_dt[0] = dt;
+        s_dt[1] = quot(dt, kp.ph.dx);
+        s_dt[2] = quot(dt, kp.ph.dy);
+      }
+      const int ntx = (kp.g.nx + TX - 1) / TX, nty = (kp.g.ny + ty - 1) / ty;
+      const int b = w - tile_begin[k];
+      const int by = b / ntx, bx = b - by * ntx;
+      const int i0 = bx * TX, j0 = by * ty;
+      gather_qtile<TX, NT>(kp.g, I.q[par], i0, j0, ty, smem);
+      __syncthreads();
+      double term = 0.0;
+      unsigned int flags = 0;
+      const double dtdx = s_dt[1], dtdy = s_dt[2];
+      tile_faces<TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+      TileCells<TX, TYM, NT> cells;
+      cells.load(kp.g, I.u[par], i0, j0, ty);
+      __syncthreads();
+      tile_riemann<RS, TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+      __syncthreads();
+      step_epilogue<TX, TYM, NT, false>(f, kp, cells, I.u[par ^ 1], I.q[par ^ 1], i0, j0, ty, dtdx, dtdy, smem, term,
+                                        flags);
+      ghost_fill_tile<TX, NT>(kp.g, I.u[par], I.u[par ^ 1], i0, j0, ty, bx == 0, bx == ntx - 1, by == 0,
+                              by == nty - 1);
+      block_fold<NT>(term, flags, &I.acc[par ^ 1], &I.status);
+      __syncthreads();
+      if (tid == 0) {
+        __threadfence();
+        const unsigned int ticket = atomicAdd(&I.done, 1u);
+        if (ticket == (unsigned)(ntx * nty) - 1u) {
+          __threadfence();
+          const double dt = s_dt[0];
+          if (!(dt > 0.0) || nonfinite(dt)) atomicOr(&I.status, (unsigned)E2D_FLAG_BAD_DT);
+          const double t = __ldcg(&I.t) + dt;
+          I.dt = dt;
+          I.t = t;
+          I.nstep = __ldcg(&I.nstep) + 1;
+          I.par = par ^ 1;
+          I.acc[par] = 0ull;  // read by this step; folded into by the next
+          I.done = 0u;
+          I.active = (t < __ldcg(&I.t_end)) && !(__ldcg(&I.status) & (E2D_FLAG_NONFINITE | E2D_FLAG_BAD_DT));
+          __threadfence();
+        }
+      }
+      __syncthreads();  // s_dt and the shared tile are rewritten by the next tile
     }
-    __syncthreads();  // s_dt and the shared tile are rewritten by the next tile
+    if (!grid_barrier(arrived, (unsigned)(it + 1) * gridDim.x)) {
+      // the states of this block's tiles are incomplete: their instances stop
+      for (int w = blockIdx.x; tid == 0 && w < total_tiles; w += gridDim.x) {
+        BatchInst64 &I = insts[list_slots[list_entry(tile_begin, n_inst, w)]];
+        atomicOr(&I.status, (unsigned)E2D_FLAG_TIMEOUT);
+        I.active = 0;
+      }
+      return;
+    }
   }
 }
 
@@ -1011,8 +1038,8 @@ static void with_shape(int shape, F &&f) {
   }
 }
 
-// The tile of a grid: the shape and rows whose step a simple model of the
-// launch puts lowest.  A tile's stages take whole warps of face-state cells,
+// The tile of a grid, or of a batch's grids together: the shape and rows
+// whose step a simple model of the launch puts lowest.  A tile's stages take whole warps of face-state cells,
 // Riemann solves and updates (W2, W3, W4); one tile alone takes L, a latency
 // per round of its block's warps; k tiles on an SM share the FP64 pipe,
 // k (80 W2 + 50 W3 + 34 W4) instructions at 5 ns; the two add with exponent
@@ -1024,8 +1051,10 @@ static void with_shape(int shape, F &&f) {
 // 64x48 71 -> 15.9 (8 x 4), 128^2 71 -> 17.2 (8 x 7), 256^2 72 -> 36.2
 // (32 x 7), 500x300 128 -> 63.6 (32 x 16), 2048^2 1832 -> 1553 (32 x 13: the
 // Riemann solves of 13 rows fill their last round of warps, those of 16 do
-// not: 1580).
-void choose_f64_tile(int nx, int ny, int tile, int *shape, int *ty) {
+// not: 1580).  The fast forms' rounds are shorter and a tile's fixed part
+// weighs more: with many waves they take the most rows (2048^2: 1236 us with
+// 16, 1260 with 13).
+void choose_f64_tile(const int (*dims)[2], int n, bool fast, int tile, int *shape, int *ty) {
   struct Info {
     int tx, most, warps, resident;
   };
@@ -1055,8 +1084,11 @@ void choose_f64_tile(int nx, int ny, int tile, int *shape, int *ty) {
       double alone = 0.0;
       for (int k = 0; k < 3; ++k) alone += up(w[k], i.warps) * lat[sh][k];
       auto wave = [&](double k) { return std::pow(std::pow(alone, kExp) + std::pow(k * inst, kExp), 1.0 / kExp); };
-      const double tiles = (double)up(nx, i.tx) * up(ny, y), per_wave = kSms * i.resident;
+      double tiles = 0.0;
+      for (int k = 0; k < n; ++k) tiles += (double)up(dims[k][0], i.tx) * up(dims[k][1], y);
+      const double per_wave = kSms * i.resident;
       const double full = std::floor(tiles / per_wave), rest = tiles - full * per_wave;
+      if (fast && full >= 4 && y < i.most) continue;
       const double t = full >= 4 ? wave(i.resident) * tiles / per_wave + 0.5 * wave(1)
                                  : full * wave(i.resident) + (rest > 0 ? wave(std::ceil(rest / kSms)) : 0.0);
       if (best == 0.0 || kFixed + t < best) {
@@ -1066,6 +1098,25 @@ void choose_f64_tile(int nx, int ny, int tile, int *shape, int *ty) {
       }
     }
   }
+}
+
+// Blocks of a kernel that are resident on the current device at once, 0 if
+// it cannot launch cooperatively (kept per kernel and device: the occupancy
+// query costs more than a launch).
+int resident_blocks(const void *kernel, int threads, size_t smem) {
+  static std::mutex mutex;
+  static std::map<std::pair<const void *, int>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mutex);
+  auto it = known.find({kernel, dev});
+  if (it != known.end()) return it->second;
+  int sms = 0, per_sm = 0, coop = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess)
+    return 0;
+  return known[{kernel, dev}] = sms * per_sm;
 }
 
 template <int RS>
@@ -1094,32 +1145,35 @@ static cudaError_t configure_rs() {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>, attr, step);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>, attr, flux);
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, true>, attr, flux);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_batch_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL>, attr, flux);
     });
   return e;
 }
 
-template <int RS>
-static cudaError_t set_batch_flux_smem() {
-  return cudaFuncSetAttribute(k_batch_step_f64<RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)step_smem_bytes<BTX, BTY>());
-}
-
 cudaError_t configure_f64_kernels() {
-  cudaError_t e = configure_rs<E2D_RIEMANN_HLLC>();
+  static std::mutex mutex;
+  static std::map<int, bool> done;  // per device, for the life of the process
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mutex);
+  if (done[dev]) return cudaSuccess;
+  e = configure_rs<E2D_RIEMANN_HLLC>();
   if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_HLL>();
   if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_APPROX>();
-  if (e == cudaSuccess) e = set_batch_flux_smem<E2D_RIEMANN_HLLC>();
-  if (e == cudaSuccess) e = set_batch_flux_smem<E2D_RIEMANN_HLL>();
-  if (e == cudaSuccess) e = set_batch_flux_smem<E2D_RIEMANN_APPROX>();
+  done[dev] = e == cudaSuccess;
   return e;
 }
 
-void batch_f64_shape(KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles) {
+void batch_f64_shape(const KParams64 &kp, int *nbx, int *nfill) {
   *nbx = (kp.g.isize + FILL_BX - 1) / FILL_BX;
   *nfill = *nbx * ((kp.g.jsize + FILL_BY - 1) / FILL_BY);
-  kp.ty = BTY;
-  *ntx = (kp.g.nx + BTX - 1) / BTX;
-  *ntiles = *ntx * ((kp.g.ny + kp.ty - 1) / kp.ty);
+}
+
+int f64_tiles(int nx, int ny, int shape, int ty) {
+  int tx = 0;
+  with_shape(shape, [&](auto sh) { tx = decltype(sh)::TX; });
+  return ((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
 }
 
 cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s) {
@@ -1127,23 +1181,40 @@ cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s)
   return cudaGetLastError();
 }
 
+template <int RS>
+static cudaError_t launch_batch_t(BatchInst64 *insts, const int *list_slots, const int *tile_begin, int n_inst,
+                                  int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
+                                  cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
+  with_shape(shape, [&](auto sh) {
+    using S = decltype(sh);
+    auto kernel = k_batch_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL>;
+    constexpr size_t sm = flux_smem_bytes<S::TX, S::TYM>();
+    const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), S::NT, sm);
+    const int grid = total_tiles < resident ? total_tiles : resident;
+    void *args[] = {&insts, &list_slots, &tile_begin, &n_inst, &total_tiles, &ty, &iterations, &arrived};
+    if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(S::NT), args, sm, s);
+  });
+  return e;
+}
+
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
-                             int n_inst, int total_tiles, int grid_blocks, cudaStream_t s) {
-  if (n_inst <= 0 || total_tiles <= 0) return cudaSuccess;
-  const size_t sm = step_smem_bytes<BTX, BTY>();
-  const int grid = grid_blocks < total_tiles ? grid_blocks : total_tiles;
+                             int n_inst, int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
+                             cudaStream_t s) {
+  if (n_inst <= 0 || total_tiles <= 0 || iterations <= 0) return cudaSuccess;
   switch (riemann) {
     case E2D_RIEMANN_HLLC:
-      k_batch_step_f64<E2D_RIEMANN_HLLC><<<grid, BNT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
-      break;
+      return launch_batch_t<E2D_RIEMANN_HLLC>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty, iterations,
+                                              arrived, s);
     case E2D_RIEMANN_HLL:
-      k_batch_step_f64<E2D_RIEMANN_HLL><<<grid, BNT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
-      break;
+      return launch_batch_t<E2D_RIEMANN_HLL>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty, iterations,
+                                             arrived, s);
     default:
-      k_batch_step_f64<E2D_RIEMANN_APPROX><<<grid, BNT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles);
-      break;
+      return launch_batch_t<E2D_RIEMANN_APPROX>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty,
+                                                iterations, arrived, s);
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const double *q,
@@ -1202,13 +1273,8 @@ static void with_loop(int riemann, const KParams64 &kp, F &&f) {
 int f64_loop_blocks(const KParams64 &kp, int riemann) {
   int blocks = 0;
   with_loop(riemann, kp, [&](auto kernel, int threads, size_t sm, int tiles) {
-    int dev = 0, sms = 0, per_sm = 0, coop = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sm) != cudaSuccess)
-      return;
-    if (tiles <= sms * per_sm * LOOP_WAVES) blocks = tiles < sms * per_sm ? tiles : sms * per_sm;
+    const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), threads, sm);
+    if (tiles <= resident * LOOP_WAVES) blocks = tiles < resident ? tiles : resident;
   });
   return blocks;
 }

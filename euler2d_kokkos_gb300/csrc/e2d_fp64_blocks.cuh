@@ -263,7 +263,7 @@ __device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph,
   const double ur = qr[E2D_IU], vr = qr[E2D_IV];
   auto energy = [&](double r, double p, double u, double v) {
     const double h = half(r);
-    return f.add(f.mul(p, ph.entho), f.add(f.mul(f.mul(h, u), u), f.mul(f.mul(h, v), v)));
+    return f.add(f.xmul(p, ph.entho), f.add(f.xmul(f.xmul(h, u), u), f.xmul(f.xmul(h, v), v)));
   };
   const double etotl = energy(rl, pl, ul, vl), etotr = energy(rr, pr, ur, vr);
   const double c2l = max_pos(quot(f.mul(ph.gamma0, pl), rl), ph.smallc2);
@@ -275,13 +275,13 @@ __device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph,
   const double UR[4] = {rr, etotr, f.mul(rr, ur), f.mul(rr, vr)};
   double FL[4], FR[4];
   FL[E2D_ID] = UL[E2D_IU];
-  FL[E2D_IP] = f.mul(f.add(etotl, pl), ul);
+  FL[E2D_IP] = f.xmul(f.add(etotl, pl), ul);
   FL[E2D_IU] = f.add(f.mul(UL[E2D_IU], ul), pl);
-  FL[E2D_IV] = f.mul(UL[E2D_IU], vl);
+  FL[E2D_IV] = f.xmul(UL[E2D_IU], vl);
   FR[E2D_ID] = UR[E2D_IU];
-  FR[E2D_IP] = f.mul(f.add(etotr, pr), ur);
+  FR[E2D_IP] = f.xmul(f.add(etotr, pr), ur);
   FR[E2D_IU] = f.add(f.mul(UR[E2D_IU], ur), pr);
-  FR[E2D_IV] = f.mul(UR[E2D_IU], vr);
+  FR[E2D_IV] = f.xmul(UR[E2D_IU], vr);
   if (gt0(SL)) {
 #pragma unroll
     for (int v = 0; v < 4; ++v) flux[v] = FL[v];
@@ -294,7 +294,7 @@ __device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph,
     const double rden = quot(f.one, f.sub(SR, SL));
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      flux[v] = f.mul(f.add(f.sub(f.mul(SR, FL[v]), f.mul(SL, FR[v])), f.mul(sls, f.sub(UR[v], UL[v]))), rden);
+      flux[v] = f.mul(f.add(f.sub(f.mul(SR, FL[v]), f.mul(SL, FR[v])), f.xmul(sls, f.sub(UR[v], UL[v]))), rden);
   }
 }
 
@@ -356,8 +356,8 @@ __device__ __forceinline__ void trace_sources_fast(const F &f, const KPhys<doubl
   const double r = q[E2D_ID], p = q[E2D_IP], u = q[E2D_IU], v = q[E2D_IV];
   const Divisor dr = divisor(r);
   const double nu = f.neg(u), nv = f.neg(v), ndiv = f.neg(f.add(dqx[E2D_IU], dqy[E2D_IV]));
-  s0[E2D_ID] = fma(nu, dqx[E2D_ID], fma(nv, dqy[E2D_ID], f.mul(ndiv, r)));
-  s0[E2D_IP] = fma(nu, dqx[E2D_IP], fma(nv, dqy[E2D_IP], f.mul(f.mul(ndiv, ph.gamma0), p)));
+  s0[E2D_ID] = fma(nu, dqx[E2D_ID], fma(nv, dqy[E2D_ID], f.xmul(ndiv, r)));
+  s0[E2D_IP] = fma(nu, dqx[E2D_IP], fma(nv, dqy[E2D_IP], f.xmul(f.xmul(ndiv, ph.gamma0), p)));
   s0[E2D_IU] = fma(nu, dqx[E2D_IU], fma(nv, dqy[E2D_IU], f.neg(quot(dqx[E2D_IP], dr))));
   s0[E2D_IV] = fma(nu, dqx[E2D_IV], fma(nv, dqy[E2D_IV], f.neg(quot(dqy[E2D_IP], dr))));
 }
@@ -393,23 +393,23 @@ __device__ __forceinline__ void riemann_hllc_fast(const F &f, const KPhys<double
   const double rcr = f.mul(rr, f.sub(SR, ur));
   const Divisor rc = divisor(f.add(rcr, rcl));
   const double ustar = quot(fma(rcr, ur, fma(rcl, ul, f.sub(pl, pr))), rc);
-  const double ptotstar = quot(fma(rcr, pl, fma(rcl, pr, f.mul(f.mul(rcl, rcr), f.sub(ul, ur)))), rc);
+  const double ptotstar = quot(fma(rcr, pl, fma(rcl, pr, f.xmul(f.xmul(rcl, rcr), f.sub(ul, ur)))), rc);
   const bool own_l = gt0(SL);
   const bool lft = own_l || gt0(ustar);
   const bool own = own_l || !(lft || gt0(SR));
   const double S = lft ? SL : SR;
   const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr, vs = lft ? ql[E2D_IV] : qr[E2D_IV];
-  const double es = fma(ps, ph.entho, f.mul(half(rs), fma(us, us, f.mul(vs, vs))));
+  const double es = fma(ps, ph.entho, f.xmul(half(rs), fma(us, us, f.xmul(vs, vs))));
   const double sdu = f.sub(S, us);
   const Divisor sds = divisor(f.sub(S, ustar));
-  const double rstar = quot(f.mul(rs, sdu), sds);
-  const double etotstar = quot(fma(sdu, es, fma(f.neg(ps), us, f.mul(ptotstar, ustar))), sds);
+  const double rstar = quot(f.xmul(rs, sdu), sds);
+  const double etotstar = quot(fma(sdu, es, fma(f.neg(ps), us, f.xmul(ptotstar, ustar))), sds);
   const double ro = own ? rs : rstar, uo = own ? us : ustar, ptoto = own ? ps : ptotstar;
   const double etoto = own ? es : etotstar;
-  flux[E2D_ID] = f.mul(ro, uo);
+  flux[E2D_ID] = f.xmul(ro, uo);
   flux[E2D_IU] = fma(flux[E2D_ID], uo, ptoto);
-  flux[E2D_IP] = f.mul(f.add(etoto, ptoto), uo);
-  flux[E2D_IV] = f.mul(flux[E2D_ID], gt0(flux[E2D_ID]) ? ql[E2D_IV] : qr[E2D_IV]);
+  flux[E2D_IP] = f.xmul(f.add(etoto, ptoto), uo);
+  flux[E2D_IV] = f.xmul(flux[E2D_ID], gt0(flux[E2D_ID]) ? ql[E2D_IV] : qr[E2D_IV]);
 }
 
 // riemann_hll() with FMAs.

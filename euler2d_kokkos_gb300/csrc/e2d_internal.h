@@ -162,9 +162,14 @@ cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const doubl
                                    const double *u_in, double *u_out, DevClock *clk,
                                    int use_clock, double host_dt, double *dt_trace,
                                    cudaStream_t s);
-// Tile shape and rows of a grid (e2d_fp64.cu); tile >= 0 forces shape
-// tile % 100 with tile / 100 rows (0: the shape's most).
-void choose_f64_tile(int nx, int ny, int tile, int *shape, int *ty);
+// Tile shape and rows of a grid, or of n grids stepped together
+// (e2d_fp64.cu); tile >= 0 forces shape tile % 100 with tile / 100 rows (0:
+// the shape's most).
+void choose_f64_tile(const int (*dims)[2], int n, bool fast, int tile, int *shape, int *ty);
+int f64_tiles(int nx, int ny, int shape, int ty);
+// Blocks of a kernel resident on the current device at once (0: it cannot
+// launch cooperatively).
+int resident_blocks(const void *kernel, int threads, size_t smem);
 // Sets the kernels' shared-memory limits; call once per device before any
 // launch or graph capture.
 cudaError_t configure_f64_kernels();
@@ -223,7 +228,7 @@ struct BatchInst {
 
 // An FP64 instance of a batch: the reference's two states and the
 // primitives of each in the pool, stepped by the fused step
-// (k_batch_step_f64) after one prologue at admission (k_batch_prime_f64).
+// (k_batch_loop_f64) after one prologue at admission (k_batch_prime_f64).
 struct BatchInst64 {
   KParams64 kp;
   double *u[2];
@@ -234,21 +239,21 @@ struct BatchInst64 {
   int active;                    // 1 while t < t_end
   int nstep;
   int nbx, nfill;                // prologue blocks per row, total
-  int ntx, ntiles;               // 32 x 32 tiles per row, total
   unsigned int done;             // tiles finished in the current iteration
   unsigned int status;           // E2D_FLAG_* bits
 };
 
 // The prologue of a newly admitted FP64 instance (q[0], acc[0] from u[0]).
 cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s);
-// One FP64 iteration of every listed FP64 instance in one persistent launch
-// of at most grid_blocks blocks: list entry k is table slot list_slots[k];
-// tile_begin[k] is its first global tile (n_inst + 1 entries, the last =
-// total_tiles).
+// `iterations` steps of every listed FP64 instance in one cooperative launch:
+// list entry k is table slot list_slots[k]; tile_begin[k] is its first global
+// tile of that shape (n_inst + 1 entries, the last = total_tiles); arrived: a
+// device word for the launch's barriers.
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
-                             int n_inst, int total_tiles, int grid_blocks, cudaStream_t s);
-// Fill blocks and tiles of an FP64 instance; sets its tile rows.
-void batch_f64_shape(KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles);
+                             int n_inst, int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
+                             cudaStream_t s);
+// Prologue blocks of an FP64 instance.
+void batch_f64_shape(const KParams64 &kp, int *nbx, int *nfill);
 
 // One iteration over every strip of every listed instance: list entry k is
 // table slot list_slots[k]; strip_begin[k] is its first global strip
@@ -256,6 +261,13 @@ void batch_f64_shape(KParams64 &kp, int *nbx, int *nfill, int *ntx, int *ntiles)
 cudaError_t launch_batch_f32c(int riemann, int variant, BatchInst *insts, const int *list_slots,
                               const int *strip_begin, int n_inst, int total_strips, int grid_blocks,
                               cudaStream_t s);
+// `iterations` steps over the fold units of every listed instance in short
+// strips of `rows` rows, in one cooperative launch (unit_begin as strip_begin).
+cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, const int *list_slots,
+                                   const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
+                                   cudaStream_t s);
+int units_of(const KParams32 &kp);
+int short_rows_for(long long units);
 // dt, dt/dx, dt/dy and `active` of an instance from acc[nstep & 1].
 cudaError_t launch_batch_arm(BatchInst *inst, cudaStream_t s);
 // Resident blocks per SM of the batch kernel variant (occupancy).
