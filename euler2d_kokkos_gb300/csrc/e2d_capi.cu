@@ -36,6 +36,13 @@ struct e2d_sim {
   // have changed a state
   int q_ready = -1;
   unsigned long long q_acc = 0ull;
+  // the state whose primitives compute_dt left in Q[h_ready], for the
+  // godunov_unsplit that follows it; -1 once anything may have changed the
+  // state, and always once its device address has been given out
+  int h_ready = -1;
+  bool address_out = false;
+  DtAcc *dt_acc = nullptr;            // compute_dt: accumulators (zero between calls)
+  DtResult *dt_result = nullptr;      // and result (pinned)
   double *impl_scratch = nullptr;     // FP64, implementation 1: stored slopes and fluxes
   float *W[2] = {nullptr, nullptr};   // FP32C: compensated U and U2 (8 float planes)
   CUtensorMap TM[2];                  // FP32C: TMA maps of W[0], W[1] (row staging)
@@ -122,6 +129,12 @@ void e2d::make_kparams(const e2d_params &p, KParams64 *kp) {
 
 namespace {
 
+// A state may have changed: what was kept of it is void.
+void touch(e2d_sim *s) {
+  s->q_ready = -1;
+  s->h_ready = -1;
+}
+
 size_t cells(const e2d_sim *s) { return (size_t)s->p.isize * s->p.jsize; }
 
 // LayoutRight (OpenMP backend) <-> LayoutLeft (CUDA backend) on the host.
@@ -158,7 +171,7 @@ cudaError_t enqueue_step(e2d_sim *s, int par) {
   if (!s->f64_split)
     return launch_step_f64(s->kp, s->p.riemannSolverType, s->QTM[par], s->q_tma, s->Q[par], s->Q[par ^ 1], in,
                            out, s->clk, s->dt_trace, s->stream);
-  const int mode = FILL_WRITE_Q | FILL_GHOSTS_IN | FILL_GHOSTS_OUT | FILL_DT | FILL_DEVICE_CLOCK;
+  const int mode = FILL_WRITE_Q | FILL_DT | FILL_DEVICE_CLOCK;
   cudaError_t e = launch_fill_f64(s->kp, in, out, s->Q[0], s->clk, mode, s->stream);
   if (e != cudaSuccess) return e;
   return launch_flux_update_f64(s->kp, s->p.riemannSolverType, s->Q[0], in, out, s->clk, 1, 0.0,
@@ -316,7 +329,8 @@ int e2d_create(const e2d_params *pin, e2d_sim **out) {
     return status;
   };
   if (cudaGetDevice(&s->device) != cudaSuccess) return fail(E2D_ECUDA);
-  if (configure_f64_kernels() != cudaSuccess || configure_f32c_kernels() != cudaSuccess) return fail(E2D_ECUDA);
+  if ((s->fp32 ? configure_f32c_kernels(p.riemannSolverType) : configure_f64_kernels(p.riemannSolverType)) != cudaSuccess)
+    return fail(E2D_ECUDA);
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(E2D_ECUDA);
   const size_t n = cells(s);
   if (s->fp32) {
@@ -358,8 +372,12 @@ int e2d_create(const e2d_params *pin, e2d_sim **out) {
   if (cudaMalloc(&s->partial, sizeof(double) * reduce_partial_count(s->kp.g)) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMalloc(&s->red_out, sizeof(double) * 8) != cudaSuccess) return fail(E2D_ENOMEM);
   if (cudaMalloc(&s->clk, sizeof(DevClock)) != cudaSuccess) return fail(E2D_ENOMEM);
-  if (cudaMallocHost(&s->clk_host, sizeof(DevClock)) != cudaSuccess) return fail(E2D_ENOMEM);
-  std::memset(s->clk_host, 0, sizeof(DevClock));
+  if (cudaMallocHost(&s->clk_host, sizeof(DevClock) + sizeof(DtResult)) != cudaSuccess) return fail(E2D_ENOMEM);
+  if (cudaMalloc(&s->dt_acc, sizeof(DtAcc)) != cudaSuccess) return fail(E2D_ENOMEM);
+  // one pinned block: the clock's mirror, then compute_dt's result
+  s->dt_result = reinterpret_cast<DtResult *>(s->clk_host + 1);
+  if (cudaMemsetAsync(s->dt_acc, 0, sizeof(DtAcc), s->stream) != cudaSuccess) return fail(E2D_ECUDA);
+  std::memset(s->clk_host, 0, sizeof(DevClock) + sizeof(DtResult));
   if (cudaMemsetAsync(s->clk, 0, sizeof(DevClock), s->stream) != cudaSuccess) return fail(E2D_ECUDA);
   if (ensure_trace(s, 1024) != E2D_OK) return fail(E2D_ENOMEM);
   if (cudaStreamSynchronize(s->stream) != cudaSuccess) return fail(E2D_ECUDA);
@@ -383,6 +401,7 @@ int e2d_destroy(e2d_sim *s) {
   if (s->partial) cudaFree(s->partial);
   if (s->red_out) cudaFree(s->red_out);
   if (s->clk) cudaFree(s->clk);
+  if (s->dt_acc) cudaFree(s->dt_acc);
   if (s->clk_host) cudaFreeHost(s->clk_host);
   if (s->dt_trace) cudaFree(s->dt_trace);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -406,7 +425,8 @@ int e2d_get_stream(e2d_sim *s, void **stream) {
 
 int e2d_device_state(e2d_sim *s, int which, double **dptr) {
   if (!s || !dptr || (which != 0 && which != 1)) return E2D_EINVAL;
-  s->q_ready = -1;  // the caller may write through the pointer
+  touch(s);  // the caller may write through the pointer, now or later
+  s->address_out = true;
   int rc = fp64_view(s, which, dptr);
   if (rc != E2D_OK) return rc;
   if (s->fp32) E2D_CK(s, cudaStreamSynchronize(s->stream), "device_state sync");
@@ -415,7 +435,7 @@ int e2d_device_state(e2d_sim *s, int which, double **dptr) {
 
 int e2d_init_problem(e2d_sim *s) {
   if (!s) return E2D_EINVAL;
-  s->q_ready = -1;
+  touch(s);
   if (s->fp32) {
     E2D_CK(s, launch_init_f64(s->kp, s->p, s->stage, s->stream), "init problem");
     E2D_CK(s, launch_f32c_from_f64(s->kp32, s->stage, s->W[0], s->stream), "init convert");
@@ -431,7 +451,7 @@ int e2d_init_problem(e2d_sim *s) {
 int e2d_set_state(e2d_sim *s, int which, const double *host, int layout) {
   if (!s || !host || (which != 0 && which != 1)) return set_err(s, E2D_EINVAL, "bad set_state args");
   if (layout != E2D_LAYOUT_LEFT && layout != E2D_LAYOUT_RIGHT) return set_err(s, E2D_EINVAL, "bad layout");
-  s->q_ready = -1;
+  touch(s);
   const size_t n = 4 * cells(s);
   std::vector<double> tmp;
   const double *src = host;
@@ -514,7 +534,7 @@ int e2d_save_vtk(e2d_sim *s, int which, const char *filename) {
 
 int e2d_make_boundaries(e2d_sim *s, int which) {
   if (!s || (which != 0 && which != 1)) return set_err(s, E2D_EINVAL, "bad make_boundaries args");
-  s->q_ready = -1;
+  touch(s);
   // FP32C states keep no ghost cells: every reader maps them on the fly
   if (s->fp32) return E2D_OK;
   E2D_CK(s, launch_fill_f64(s->kp, s->U[which], nullptr, nullptr, s->clk, FILL_GHOSTS_IN, s->stream), "make_boundaries");
@@ -524,26 +544,34 @@ int e2d_make_boundaries(e2d_sim *s, int which) {
 int e2d_compute_dt(e2d_sim *s, int useU, double *dt) {
   if (!s || !dt) return set_err(s, E2D_EINVAL, "bad compute_dt args");
   const int which = (useU == 0) ? 0 : 1;
-  E2D_CK(s, cudaMemsetAsync(&s->clk->invdt_bits, 0, sizeof(unsigned long long), s->stream), "dt reset");
-  E2D_CK(s, cudaMemsetAsync(&s->clk->status, 0, sizeof(unsigned int), s->stream), "dt reset");
-  if (s->fp32)
-    E2D_CK(s, launch_f32c_dt(s->kp32, s->W[which], s->clk, -1, s->stream), "compute_dt");
-  else
-    E2D_CK(s, launch_fill_f64(s->kp, s->U[which], nullptr, nullptr, s->clk, FILL_DT, s->stream), "compute_dt");
-  E2D_CK(s, cudaMemcpyAsync(s->clk_host, s->clk, sizeof(DevClock), cudaMemcpyDeviceToHost, s->stream), "dt copy");
-  E2D_CK(s, cudaStreamSynchronize(s->stream), "dt sync");
+  if (!s->fp32) {
+    // exact primitives: not into the fast forms' arrays
+    double *q = s->kp.fast ? nullptr : s->Q[which];
+    E2D_CK(s, launch_dt_f64(s->kp, s->U[which], q, s->dt_acc, s->dt_result, s->stream), "compute_dt");
+    E2D_CK(s, cudaStreamSynchronize(s->stream), "dt sync");
+    if (q && !s->address_out) s->h_ready = which;
+  } else {
+    E2D_CK(s, cudaMemsetAsync(s->dt_acc, 0, sizeof(DtAcc), s->stream), "dt reset");
+    E2D_CK(s, launch_f32c_dt_to(s->kp32, s->W[which], &s->dt_acc->bits, &s->dt_acc->status, s->stream), "compute_dt");
+    E2D_CK(s, cudaMemcpyAsync(s->dt_result, s->dt_acc, sizeof(DtResult), cudaMemcpyDeviceToHost, s->stream), "dt copy");
+    E2D_CK(s, cudaStreamSynchronize(s->stream), "dt sync");
+  }
+  static_assert(offsetof(DtAcc, bits) == offsetof(DtResult, bits) && offsetof(DtAcc, status) == offsetof(DtResult, status) &&
+                    sizeof(DtResult) <= sizeof(DtAcc), "the result is the accumulators' head");
+  const DtResult r = *s->dt_result;
   double inv;
-  std::memcpy(&inv, &s->clk_host->invdt_bits, sizeof(double));
+  std::memcpy(&inv, &r.bits, sizeof(double));
   *dt = s->p.cfl / inv;  // src/HydroRun.h:248
-  if (s->clk_host->status & E2D_FLAG_NONFINITE) return set_err(s, E2D_ENUMERIC, "non-finite state value");
+  if (r.status & E2D_FLAG_NONFINITE) return set_err(s, E2D_ENUMERIC, "non-finite state value");
   return E2D_OK;
 }
 
 int e2d_godunov_unsplit(e2d_sim *s, int nStep, double dt) {
   if (!s) return E2D_EINVAL;
   if (s->kp.fast) return set_err(s, E2D_EINVAL, "fp64_fast runs through the device time loop (e2d_step_n) only");
-  s->q_ready = -1;
   const int par = (nStep % 2 == 0) ? 0 : 1;  // src/HydroRun.h:263-270
+  const bool have_q = s->h_ready == par;
+  touch(s);
   if (s->fp32) {
     E2D_CK(s, launch_f32c_step(s->kp32, s->p.riemannSolverType, s->W[par], s->W[par ^ 1], s->TM[par], s->clk, 0, dt,
                                s->stream), "godunov step");
@@ -557,9 +585,9 @@ int e2d_godunov_unsplit(e2d_sim *s, int nStep, double dt) {
                                 dt, nullptr, s->stream), "godunov implementation 1/2");
     return E2D_OK;
   }
-  const int mode = FILL_WRITE_Q | FILL_GHOSTS_IN | FILL_GHOSTS_OUT;
-  E2D_CK(s, launch_fill_f64(s->kp, in, out, s->Q[0], s->clk, mode, s->stream), "godunov primitives");
-  E2D_CK(s, launch_flux_update_f64(s->kp, s->p.riemannSolverType, s->Q[0], in, out, s->clk, 0, dt,
+  if (!have_q)
+    E2D_CK(s, launch_fill_f64(s->kp, in, nullptr, s->Q[par], s->clk, FILL_WRITE_Q, s->stream), "godunov primitives");
+  E2D_CK(s, launch_flux_update_f64(s->kp, s->p.riemannSolverType, s->Q[par], in, out, s->clk, 0, dt,
                                    nullptr, s->stream), "godunov fluxes");
   return E2D_OK;
 }
@@ -583,7 +611,7 @@ int e2d_step_n(e2d_sim *s, int n, double t_end, double *t, int *nStep, double *d
   const bool fused = !s->fp32 && !s->f64_split && s->impl == 0;
   const bool prologue = fused && s->q_ready != par0;
   if (fused && !prologue) c.acc[par0] = s->q_acc;
-  s->q_ready = -1;
+  touch(s);
   *s->clk_host = c;
   E2D_CK(s, cudaMemcpyAsync(s->clk, s->clk_host, sizeof(DevClock), cudaMemcpyHostToDevice, s->stream), "clock upload");
   // FP32C and the fused FP64 step: the first step's CFL maximum (and the
@@ -624,7 +652,7 @@ int e2d_step_n(e2d_sim *s, int n, double t_end, double *t, int *nStep, double *d
       double *in = s->U[par], *out = s->U[par ^ 1];
       E2D_CK(s, cudaEventRecord(a, s->stream), "event");
       E2D_CK(s, launch_fill_f64(s->kp, in, out, s->Q[0], s->clk,
-                                FILL_WRITE_Q | FILL_GHOSTS_IN | FILL_GHOSTS_OUT | FILL_DT | FILL_DEVICE_CLOCK,
+                                FILL_WRITE_Q | FILL_DT | FILL_DEVICE_CLOCK,
                                 s->stream), "fill");
       E2D_CK(s, cudaEventRecord(b, s->stream), "event");
       E2D_CK(s, launch_flux_update_f64(s->kp, s->p.riemannSolverType, s->Q[0], in, out, s->clk, 1, 0.0,

@@ -38,6 +38,7 @@
 #include <map>
 #include <mutex>
 #include <type_traits>
+#include <utility>
 
 namespace e2d {
 namespace {
@@ -1541,18 +1542,19 @@ static cudaError_t configure_rs() {
   return e;
 }
 
-cudaError_t configure_f32c_kernels() {
+cudaError_t configure_f32c_kernels(int riemann) {
   static std::mutex mutex;
-  static std::map<int, bool> done;  // per device, for the life of the process
+  static std::map<std::pair<int, int>, bool> done;  // per device and solver, for the life of the process
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mutex);
-  if (done[dev]) return cudaSuccess;
-  e = configure_rs<E2D_RIEMANN_HLLC>();
-  if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_HLL>();
-  if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_APPROX>();
-  done[dev] = e == cudaSuccess;
+  bool &ready = done[{dev, riemann}];
+  if (ready) return cudaSuccess;
+  e = riemann == E2D_RIEMANN_HLLC  ? configure_rs<E2D_RIEMANN_HLLC>()
+      : riemann == E2D_RIEMANN_HLL ? configure_rs<E2D_RIEMANN_HLL>()
+                                   : configure_rs<E2D_RIEMANN_APPROX>();
+  ready = e == cudaSuccess;
   return e;
 }
 

@@ -4,20 +4,23 @@
 //
 // The device time loop runs one fused launch per step (k_step_f64, after a
 // prologue k_fill_f64 that folds the first step's CFL maximum and writes the
-// primitives of the initial state); FP64 batch instances run the same fused
-// step in one launch per run call (k_batch_loop_f64).  The
-// host-driven godunov_unsplit runs it as two launches:
-//   k_fill_f64         ghost fill (make_boundaries, src/HydroRun.h:388-399)
-//                      into both states, primitives of every cell
+// primitives of the initial state), or many steps in one cooperative launch
+// where the grid is small (k_loop_f64); FP64 batch instances run the same
+// fused step in one launch per run call (k_batch_loop_f64).  The host-driven
+// loop runs a step as two launches:
+//   k_dt_f64           (compute_dt) primitives of every cell
 //                      (ConvertToPrimitivesFunctor, src/HydroRunFunctors.h:84-143)
 //                      and the CFL maximum of the interior
 //                      (ComputeDtFunctor, src/HydroRunFunctors.h:17-79);
-//   k_flux_update_f64  per 32x32 tile: limited slopes once per cell, the
-//                      half-step trace once per cell and face, one Riemann
-//                      solve per face, the conservative update
+//                      k_fill_f64 writes the primitives where no compute_dt
+//                      of the state came before;
+//   k_flux_update_f64  (godunov_unsplit) per tile: limited slopes once per
+//                      cell, the half-step trace once per cell and face, one
+//                      Riemann solve per face, the conservative update
 //                      (ComputeAndStoreFluxesFunctor + UpdateFunctor,
-//                      src/HydroRunFunctors.h:412-723) and the time-loop
-//                      bookkeeping of src/main.cpp:128-143.
+//                      src/HydroRunFunctors.h:412-723) and the ghost fill
+//                      into both states (make_boundaries, deep_copy,
+//                      src/HydroRun.h:388-399,302).
 // The reference evaluates the slopes of a cell three times and the trace
 // sources four times per cell; evaluating each once gives the same bits.
 #include "e2d_fp64_blocks.cuh"
@@ -85,12 +88,6 @@ __device__ __forceinline__ void fill_cell(const KParams64 &kp, double *__restric
       u_in[d + 2 * g.plane] = mx;
       u_in[d + 3 * g.plane] = my;
     }
-    if (mode & FILL_GHOSTS_OUT) {
-      u_out[d] = rho;
-      u_out[d + g.plane] = e;
-      u_out[d + 2 * g.plane] = mx;
-      u_out[d + 3 * g.plane] = my;
-    }
   }
   if (mode & (FILL_WRITE_Q | FILL_DT)) {
     const Fp f;
@@ -150,6 +147,30 @@ __global__ void __launch_bounds__(FILL_BX *FILL_BY)
     fill_reduce(term, flags, acc_slot < 0 ? &clk->invdt_bits : &clk->acc[acc_slot & 1], &clk->status);
 }
 
+// compute_dt in one launch: the interior's primitives into q, its CFL maximum
+// and flags by the last block to finish into *result (pinned host memory),
+// and the accumulators cleared for the next call.
+__global__ void __launch_bounds__(FILL_BX *FILL_BY)
+    k_dt_f64(const KParams64 kp, double *__restrict__ u_in, double *__restrict__ q, DtAcc *acc, DtResult *result) {
+  double term = 0.0;
+  unsigned int flags = 0;
+  fill_cell(kp, u_in, nullptr, q, q ? FILL_WRITE_Q | FILL_DT : FILL_DT, blockIdx.x * FILL_BX + threadIdx.x,
+            blockIdx.y * FILL_BY + threadIdx.y, term, flags);
+  fill_reduce(term, flags, &acc->bits, &acc->status);
+  if (threadIdx.x == 0 && threadIdx.y == 0) {  // the thread that folded
+    __threadfence();
+    if (atomicAdd(&acc->done, 1u) == gridDim.x * gridDim.y - 1) {
+      __threadfence();
+      result->bits = __ldcg(&acc->bits);
+      result->status = __ldcg(&acc->status);
+      acc->bits = 0ull;
+      acc->status = 0u;
+      acc->done = 0u;
+      __threadfence_system();
+    }
+  }
+}
+
 // ------------------------------------------------------------ kernel 2
 // Tiles are TX x ty cells, ty <= TYM chosen at run time per grid (see
 // choose_f64_tile); results do not depend on the shape.
@@ -174,29 +195,8 @@ struct TileSmem {
   }
 };
 
-// Stage 1 of the two-launch step: primitives of the tile and its 2-cell
-// halo from the primitives array (ghost cells included, written by the fill
-// kernel); cells beyond the array get a harmless 1.0.
-template <int TX, int NT>
-__device__ __forceinline__ void load_qtile(const KGeom &g, const double *__restrict__ q, int i0, int j0, int ty,
-                                           double *sQ) {
-  constexpr int QW = TX + 4;
-  const int n = (ty + 4) * QW;
-  for (int k = threadIdx.x; k < n; k += NT) {
-    const int y = k / QW, x = k - y * QW;
-    const int gi = i0 + x, gj = j0 + y;
-    if (gi < g.isize && gj < g.jsize) {
-      const size_t s = (size_t)gi + (size_t)g.isize * gj;
-#pragma unroll
-      for (int v = 0; v < 4; ++v) sQ[v * n + k] = q[s + v * g.plane];
-    } else {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) sQ[v * n + k] = 1.0;
-    }
-  }
-}
-
-// Stage 1 of the fused step for tiles whose halo reaches ghost cells: the
+// Stage 1 from the primitives of the interior cells (the fused step where its
+// halo reaches ghost cells, the other steps throughout): the
 // primitives of a ghost cell are those of its source cell with the normal
 // velocity negated where the boundary reflects -- bit for bit the
 // primitives of the reference's ghost-filled state (u = mx / d changes only
@@ -304,6 +304,84 @@ __device__ __forceinline__ void tile_faces(const F &fp64, const KPhys<double> &p
   }
 }
 
+// Stage 2 with a lane per cell and variable, for tiles so small that their
+// cells do not fill the block's warps: a quarter of the instructions in each
+// warp's chain (23 FP64 instead of 80; 21 % more of them in all).  The lanes
+// of a cell exchange what the trace sources need of the other variables.
+// Same operations, same bits.
+template <int TX, int TYM, int NT, bool FAST, class F>
+__device__ __forceinline__ void tile_faces_split(const F &f, const KPhys<double> &ph, const double dtdx,
+                                                 const double dtdy, const int ty, double *smem) {
+  using T = TileSmem<TX, TYM>;
+  constexpr int QW = T::QW, XW = T::XW, YH = T::YH;
+  const T sm(smem);
+  const int qs = QW * (ty + 4);
+  const int st_kind = (ph.slope_type == 2.0) ? 2 : (ph.slope_type == 1.0) ? 1 : 0;
+  const int ns2 = (ty + 2) * XW - 4;
+  const double hdtdx = half(dtdx), hdtdy = half(dtdy);
+  const int v = threadIdx.x & 3;
+  auto other = [](double x, int w) { return __shfl_sync(0xffffffffu, x, w, 4); };
+  for (int k0 = threadIdx.x >> 2; (k0 & ~7) < ns2; k0 += NT / 4) {  // whole warps
+    const int k = k0 < ns2 ? k0 : ns2 - 1;
+    int yy, xx;  // cell (xx-1, yy-1) of the tile
+    if (k < TX) {
+      yy = 0;
+      xx = k + 1;
+    } else if (k < TX + ty * XW) {
+      const int r = k - TX;
+      yy = 1 + r / XW;
+      xx = r - (yy - 1) * XW;
+    } else {
+      yy = ty + 1;
+      xx = k - (TX + ty * XW) + 1;
+    }
+    const double *P = sm.sQ + v * qs + (yy + 1) * QW + (xx + 1);
+    const double q = P[0];
+    double dqx, dqy, hx, hy;
+    slope(f, st_kind, q, P[1], P[-1], dqx, hx);
+    slope(f, st_kind, q, P[QW], P[-QW], dqy, hy);
+    const double r = other(q, E2D_ID), u = other(q, E2D_IU), w = other(q, E2D_IV);
+    const double div = f.add(other(dqx, E2D_IU), other(dqy, E2D_IV));
+    const double dpx = other(dqx, E2D_IP), dpy = other(dqy, E2D_IP);
+    // the term of the variable's source beside its transport
+    const double dg = f.mul(div, ph.gamma0);
+    const double m = f.mul(v == E2D_IP ? dg : div, q), g = quot(v == E2D_IU ? dpx : dpy, r);
+    const double ex = v < E2D_IU ? m : g;
+    const double nu = f.neg(u);
+    const double s0 = FAST ? fma(nu, dqx, fma(f.neg(w), dqy, f.neg(ex)))
+                           : f.sub(f.sub(f.mul(nu, dqx), f.mul(w, dqy)), ex);
+    double xm, xp, ym, yp;
+    if (FAST) {
+      face_pair_fast(f, ph, v, q, hx, s0, hdtdx, xm, xp);
+      face_pair_fast(f, ph, v, q, hy, s0, hdtdy, ym, yp);
+    } else {
+      face_pair(f, ph, v, q, hx, s0, dtdx, hdtdx, xm, xp);
+      face_pair(f, ph, v, q, hy, s0, dtdy, hdtdy, ym, yp);
+    }
+    if (k0 < ns2 && yy >= 1 && yy <= ty) {
+      const int o = v * TYM * XW + (yy - 1) * XW + xx;
+      if (xx >= 1) sm.sXm[o] = xm;
+      if (xx <= TX) sm.sXp[o] = xp;
+    }
+    if (k0 < ns2 && xx >= 1 && xx <= TX) {
+      const int o = v * YH * TX + yy * TX + (xx - 1);
+      if (yy >= 1) sm.sYm[o] = ym;
+      if (yy <= ty) sm.sYp[o] = yp;
+    }
+  }
+}
+
+// Stage 2 of a tile: by variable for the small tiles (which are the ones
+// without integer products), else by cell.
+template <int TX, int TYM, int NT, bool FAST, class F>
+__device__ __forceinline__ void tile_stage2(const F &f, const KPhys<double> &ph, const double dtdx, const double dtdy,
+                                            const int ty, double *smem) {
+  if constexpr (TX <= 8)
+    tile_faces_split<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+  else
+    tile_faces<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+}
+
 // Stage 3 (after a block barrier): one Riemann solve per face; the flux,
 // scaled by dt/dx or dt/dy (the fast forms scale in the update), replaces
 // the right-hand state, which no other face reads.
@@ -385,20 +463,49 @@ __device__ __forceinline__ double update_var(const F &f, const TileSmem<TX, TYM>
   return uu;
 }
 
+// The ghost cells next to a tile -- those whose nearest interior cell is in
+// it -- receive the ghost fill of u_in in both states, read from interior
+// cells of u_in only (no block writes those during a step).
+template <int TX, int NT>
+__device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *u_in, double *u_out,
+                                                int i0, int j0, int ty, bool lo_x, bool hi_x, bool lo_y, bool hi_y) {
+  if (!(lo_x || hi_x || lo_y || hi_y)) return;
+  const int xa = lo_x ? 0 : i0 + 2, xb = hi_x ? g.isize : i0 + 2 + TX;
+  const int ya = lo_y ? 0 : j0 + 2, yb = hi_y ? g.jsize : j0 + 2 + ty;
+  const int w = xb - xa, n = w * (yb - ya);
+  for (int k = threadIdx.x; k < n; k += NT) {
+    const int j = ya + k / w, i = xa + k % w;
+    if (i >= 2 && i < g.nx + 2 && j >= 2 && j < g.ny + 2) continue;
+    bool fu, fv;
+    const int si = src_lo_hi(i, g.nx, g.bc_xmin, g.bc_xmax, fu);
+    const int sj = src_lo_hi(j, g.ny, g.bc_ymin, g.bc_ymax, fv);
+    const size_t s = (size_t)si + (size_t)g.isize * sj, d = (size_t)i + (size_t)g.isize * j;
+    double v4[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) v4[v] = __ldcg(u_in + s + v * g.plane);
+    if (fu) v4[E2D_IU] = -v4[E2D_IU];
+    if (fv) v4[E2D_IV] = -v4[E2D_IV];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      u_in[d + v * g.plane] = v4[v];
+      u_out[d + v * g.plane] = v4[v];
+    }
+  }
+}
+
 // Stages 1-4 of the two-launch step for tile (bx, by) of a grid,
 // block-wide; the caller provides dt/dx, dt/dy and the tile's shared memory.
 template <int RS, int TX, int TYM, int NT, class F>
-__device__ __forceinline__ void flux_tile(const KParams64 &kp, const double *__restrict__ q,
-                                          const double *__restrict__ u_in, double *__restrict__ u_out,
+__device__ __forceinline__ void flux_tile(const KParams64 &kp, const double *q, double *u_in, double *u_out,
                                           const int bx, const int by, const int ty, const double dtdx,
                                           const double dtdy, double *smem) {
   const KGeom &g = kp.g;
   const int i0 = bx * TX;  // array column of the tile's first halo cell
   const int j0 = by * ty;
   const F f;
-  load_qtile<TX, NT>(g, q, i0, j0, ty, smem);
+  gather_qtile<TX, NT>(g, q, i0, j0, ty, smem);
   __syncthreads();
-  tile_faces<TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+  tile_stage2<TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
   TileCells<TX, TYM, NT> cells;
   cells.load(g, u_in, i0, j0, ty);
   __syncthreads();
@@ -416,13 +523,14 @@ __device__ __forceinline__ void flux_tile(const KParams64 &kp, const double *__r
         u_out[s + v * g.plane] = update_var<TX, TYM, false>(f, sm, v, x, y, cells.u[n][v], dtdx, dtdy);
     }
   }
+  ghost_fill_tile<TX, NT>(g, u_in, u_out, i0, j0, ty, bx == 0, bx == (int)gridDim.x - 1, by == 0,
+                          by == (int)gridDim.y - 1);
 }
 
 template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL>
 __global__ void __launch_bounds__(NT, MINB)
-    k_flux_update_f64(const KParams64 kp, const double *__restrict__ q,
-                      const double *__restrict__ u_in, double *__restrict__ u_out, DevClock *clk,
-                      const int use_clock, const double host_dt, double *__restrict__ dt_trace) {
+    k_flux_update_f64(const KParams64 kp, const double *q, double *u_in, double *u_out, DevClock *clk,
+                      const int use_clock, const double host_dt, double *dt_trace) {
   extern __shared__ double smem[];
   const KPhys<double> &ph = kp.ph;
   const int tid = threadIdx.x;
@@ -539,36 +647,6 @@ __device__ __forceinline__ void step_epilogue(const F &f, const KParams64 &kp, c
   }
 }
 
-// The ghost cells next to a tile -- those whose nearest interior cell is in
-// it -- receive the ghost fill of u_in in both states, read from interior
-// cells of u_in only (no block writes those during a step).
-template <int TX, int NT>
-__device__ __forceinline__ void ghost_fill_tile(const KGeom &g, double *u_in, double *u_out,
-                                                int i0, int j0, int ty, bool lo_x, bool hi_x, bool lo_y, bool hi_y) {
-  if (!(lo_x || hi_x || lo_y || hi_y)) return;
-  const int xa = lo_x ? 0 : i0 + 2, xb = hi_x ? g.isize : i0 + 2 + TX;
-  const int ya = lo_y ? 0 : j0 + 2, yb = hi_y ? g.jsize : j0 + 2 + ty;
-  const int w = xb - xa, n = w * (yb - ya);
-  for (int k = threadIdx.x; k < n; k += NT) {
-    const int j = ya + k / w, i = xa + k % w;
-    if (i >= 2 && i < g.nx + 2 && j >= 2 && j < g.ny + 2) continue;
-    bool fu, fv;
-    const int si = src_lo_hi(i, g.nx, g.bc_xmin, g.bc_xmax, fu);
-    const int sj = src_lo_hi(j, g.ny, g.bc_ymin, g.bc_ymax, fv);
-    const size_t s = (size_t)si + (size_t)g.isize * sj, d = (size_t)i + (size_t)g.isize * j;
-    double v4[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) v4[v] = __ldcg(u_in + s + v * g.plane);
-    if (fu) v4[E2D_IU] = -v4[E2D_IU];
-    if (fv) v4[E2D_IV] = -v4[E2D_IV];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      u_in[d + v * g.plane] = v4[v];
-      u_out[d + v * g.plane] = v4[v];
-    }
-  }
-}
-
 // One whole time step of the device loop (src/main.cpp:128-143 around
 // godunov_unsplit_impl, src/HydroRun.h:279-364), one TX x ty tile per block:
 //  - dt from the CFL maximum of the input state, clock->acc[nstep & 1],
@@ -646,7 +724,7 @@ __global__ void __launch_bounds__(NT, MINB)
   unsigned int flags = 0;
   if (ok) {
     const double dtdx = s_dt[1], dtdy = s_dt[2];
-    tile_faces<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+    tile_stage2<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
     TileCells<TX, TYM, NT> cells;
     cells.load(g, u_in, i0, j0, ty);
     __syncthreads();
@@ -721,7 +799,7 @@ __global__ void __launch_bounds__(NT, MINB)
       gather_qtile<TX, NT>(g, q_in, i0, j0, ty, smem);
       __syncthreads();
       const double dtdx = s_dt[1], dtdy = s_dt[2];
-      tile_faces<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
+      tile_stage2<TX, TYM, NT, FAST>(f, ph, dtdx, dtdy, ty, smem);
       TileCells<TX, TYM, NT> cells;
       cells.load(g, u_in, i0, j0, ty);
       __syncthreads();
@@ -819,7 +897,7 @@ __global__ void __launch_bounds__(NT, MINB)
       double term = 0.0;
       unsigned int flags = 0;
       const double dtdx = s_dt[1], dtdy = s_dt[2];
-      tile_faces<TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
+      tile_stage2<TX, TYM, NT, false>(f, kp.ph, dtdx, dtdy, ty, smem);
       TileCells<TX, TYM, NT> cells;
       cells.load(kp.g, I.u[par], i0, j0, ty);
       __syncthreads();
@@ -1023,7 +1101,7 @@ struct Shape<1> {
 };
 template <>
 struct Shape<2> {
-  static constexpr int TX = 8, TYM = 8, NT = 160, MINB = 3;
+  static constexpr int TX = 8, TYM = 8, NT = 256, MINB = 2;
   static constexpr bool XMUL = false;
 };
 constexpr int kShapes = 3;
@@ -1039,17 +1117,18 @@ static void with_shape(int shape, F &&f) {
 }
 
 // The tile of a grid, or of a batch's grids together: the shape and rows
-// whose step a simple model of the launch puts lowest.  A tile's stages take whole warps of face-state cells,
-// Riemann solves and updates (W2, W3, W4); one tile alone takes L, a latency
-// per round of its block's warps; k tiles on an SM share the FP64 pipe,
-// k (80 W2 + 50 W3 + 34 W4) instructions at 5 ns; the two add with exponent
-// 1.26; tiles beyond what is resident make further waves, which average out
-// once there are four.  The constants are fitted to 380 timings (14 grids
-// from 64x48 to 2048^2, every shape, 4 to 16 rows; 4 % rms), on which the
-// model's choice is within 0.6 % of the fastest tile of every grid.
+// whose step a simple model of the launch puts lowest.  A tile's stages take
+// whole warps of face-state cells (lanes of cell and variable for the 8-column
+// shape), Riemann solves and updates (W2, W3, W4); one tile alone takes L, a
+// latency per round of its block's warps; k tiles on an SM share the FP64
+// pipe, k (80 W2 + 50 W3 + 34 W4) instructions (23 W2 by variable) at 5.07 ns;
+// the two add with exponent 1.3; tiles beyond what is resident make further
+// waves, which average out once there are four.  The constants are fitted to
+// 300 timings (16 grids from 32x20 to 2048^2, every shape, 3 to 16 rows; 4 %
+// rms), on which the model's choice is the fastest tile of every grid.
 // What it buys (us a step, HLLC; before: 32 x 32 tiles for every grid):
-// 64x48 71 -> 15.9 (8 x 4), 128^2 71 -> 17.2 (8 x 7), 256^2 72 -> 36.2
-// (32 x 7), 500x300 128 -> 63.6 (32 x 16), 2048^2 1832 -> 1553 (32 x 13: the
+// 64x48 71 -> 10.9 (8 x 3), 128^2 71 -> 15.1 (8 x 7), 256^2 72 -> 33.4
+// (32 x 7), 500x300 128 -> 61 (32 x 16), 2048^2 1832 -> 1553 (32 x 13: the
 // Riemann solves of 13 rows fill their last round of warps, those of 16 do
 // not: 1580).  The fast forms' rounds are shorter and a tile's fixed part
 // weighs more: with many waves they take the most rows (2048^2: 1236 us with
@@ -1072,15 +1151,17 @@ void choose_f64_tile(const int (*dims)[2], int n, bool fast, int tile, int *shap
     *ty = tile >= 100 && tile / 100 < m ? tile / 100 : m;
     return;
   }
-  static const double lat[kShapes][3] = {{4.47, 2.49, 2.29}, {3.65, 3.30, 2.25}, {4.34, 1.87, 5.41}};  // us
-  constexpr double kSms = 152.0, kFixed = 4.3, kInst = 0.005, kExp = 1.26;
+  static const double lat[kShapes][3] = {{4.77, 2.49, 1.83}, {3.93, 2.24, 3.95}, {1.62, 0.42, 5.36}};  // us
+  constexpr double kSms = 152.0, kFixed = 2.7, kInst = 0.00507, kExp = 1.3;
   auto up = [](int a, int b) { return (a + b - 1) / b; };
   double best = 0.0;
   for (int sh = 0; sh < kShapes; ++sh) {
     const Info i = info(sh);
     for (int y = 3; y <= i.most; ++y) {
-      const int w[3] = {up((i.tx + 2) * (y + 2) - 4, 32), up((i.tx + 1) * y + i.tx * (y + 1), 32), up(i.tx * y, 32)};
-      const double inst = kInst * (80 * w[0] + 50 * w[1] + 34 * w[2]);
+      const bool split = i.tx <= 8;  // tile_stage2
+      const int w[3] = {up(((i.tx + 2) * (y + 2) - 4) * (split ? 4 : 1), 32),
+                        up((i.tx + 1) * y + i.tx * (y + 1), 32), up(i.tx * y, 32)};
+      const double inst = kInst * ((split ? 23 : 80) * w[0] + 50 * w[1] + 34 * w[2]);
       double alone = 0.0;
       for (int k = 0; k < 3; ++k) alone += up(w[k], i.warps) * lat[sh][k];
       auto wave = [&](double k) { return std::pow(std::pow(alone, kExp) + std::pow(k * inst, kExp), 1.0 / kExp); };
@@ -1120,7 +1201,7 @@ int resident_blocks(const void *kernel, int threads, size_t smem) {
 }
 
 template <int RS>
-static cudaError_t launch_flux_t(const KParams64 &kp, const double *q, const double *u_in,
+static cudaError_t launch_flux_t(const KParams64 &kp, const double *q, double *u_in,
                                  double *u_out, DevClock *clk, int use_clock, double host_dt,
                                  double *dt_trace, cudaStream_t s) {
   with_shape(kp.shape, [&](auto sh) {
@@ -1150,18 +1231,19 @@ static cudaError_t configure_rs() {
   return e;
 }
 
-cudaError_t configure_f64_kernels() {
+cudaError_t configure_f64_kernels(int riemann) {
   static std::mutex mutex;
-  static std::map<int, bool> done;  // per device, for the life of the process
+  static std::map<std::pair<int, int>, bool> done;  // per device and solver, for the life of the process
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mutex);
-  if (done[dev]) return cudaSuccess;
-  e = configure_rs<E2D_RIEMANN_HLLC>();
-  if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_HLL>();
-  if (e == cudaSuccess) e = configure_rs<E2D_RIEMANN_APPROX>();
-  done[dev] = e == cudaSuccess;
+  bool &ready = done[{dev, riemann}];
+  if (ready) return cudaSuccess;
+  e = riemann == E2D_RIEMANN_HLLC  ? configure_rs<E2D_RIEMANN_HLLC>()
+      : riemann == E2D_RIEMANN_HLL ? configure_rs<E2D_RIEMANN_HLL>()
+                                   : configure_rs<E2D_RIEMANN_APPROX>();
+  ready = e == cudaSuccess;
   return e;
 }
 
@@ -1218,7 +1300,7 @@ cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_sl
 }
 
 cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const double *q,
-                                   const double *u_in, double *u_out, DevClock *clk,
+                                   double *u_in, double *u_out, DevClock *clk,
                                    int use_clock, double host_dt, double *dt_trace,
                                    cudaStream_t s) {
   switch (riemann) {
@@ -1246,6 +1328,13 @@ static cudaError_t launch_step_t(const KParams64 &kp, const CUtensorMap &tm_q, i
       k_step_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL, false>
           <<<grid, S::NT, sm, s>>>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk, dt_trace);
   });
+  return cudaGetLastError();
+}
+
+cudaError_t launch_dt_f64(const KParams64 &kp, double *u, double *q, DtAcc *acc, DtResult *result, cudaStream_t s) {
+  dim3 block(FILL_BX, FILL_BY);
+  dim3 grid((kp.g.isize + FILL_BX - 1) / FILL_BX, (kp.g.jsize + FILL_BY - 1) / FILL_BY);
+  k_dt_f64<<<grid, block, 0, s>>>(kp, u, q, acc, result);
   return cudaGetLastError();
 }
 

@@ -110,6 +110,16 @@ struct DevClock {
 // Most steps one multi-step launch takes.
 constexpr int kLoopSteps = 1024;
 
+// compute_dt's accumulators on the device and its result in pinned host memory.
+struct DtAcc {
+  unsigned long long bits;
+  unsigned int status, done;
+};
+struct DtResult {
+  unsigned long long bits;
+  unsigned int status;
+};
+
 enum : unsigned int {
   E2D_FLAG_NONFINITE = 1u,  // a state value is NaN or Inf
   E2D_FLAG_DENSITY = 2u,    // a density <= 0 was clamped to smallr
@@ -122,7 +132,6 @@ enum : unsigned int {
 enum : int {
   FILL_WRITE_Q = 1,          // store primitives of every cell
   FILL_GHOSTS_IN = 2,        // store the ghost fill into the input state (make_boundaries)
-  FILL_GHOSTS_OUT = 4,       // store the ghost fill into the output state (deep_copy)
   FILL_DT = 8,               // fold the CFL term of interior cells into clock->invdt_bits (or acc[slot])
   FILL_DEVICE_CLOCK = 16,    // do nothing once clock->t >= clock->t_end
   FILL_COPY_OUT = 32,        // copy the whole ghost-filled input state into the output (deep_copy)
@@ -158,8 +167,9 @@ cudaError_t launch_impl12_f64(const KParams64 &kp, int impl, int riemann, const 
 bool encode_q_map(CUtensorMap *map, const double *q, const KParams64 &kp);
 // use_clock = 1: dt from clk (src/main.cpp:128-134 on the device) and the
 // loop bookkeeping; 0: the caller's host_dt, clock untouched.
+// q: primitives of u_in's interior; the ghost fill of u_in goes into both states.
 cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const double *q,
-                                   const double *u_in, double *u_out, DevClock *clk,
+                                   double *u_in, double *u_out, DevClock *clk,
                                    int use_clock, double host_dt, double *dt_trace,
                                    cudaStream_t s);
 // Tile shape and rows of a grid, or of n grids stepped together
@@ -170,9 +180,12 @@ int f64_tiles(int nx, int ny, int shape, int ty);
 // Blocks of a kernel resident on the current device at once (0: it cannot
 // launch cooperatively).
 int resident_blocks(const void *kernel, int threads, size_t smem);
-// Sets the kernels' shared-memory limits; call once per device before any
-// launch or graph capture.
-cudaError_t configure_f64_kernels();
+// Primitives of u into q (may be null) and its CFL maximum and flags into *result (pinned
+// host memory), in one launch; acc zeroed once, left zeroed by each launch.
+cudaError_t launch_dt_f64(const KParams64 &kp, double *u, double *q, DtAcc *acc, DtResult *result, cudaStream_t s);
+// Sets the shared-memory limits of a solver's kernels; call before any
+// launch or graph capture (done once per device).
+cudaError_t configure_f64_kernels(int riemann);
 cudaError_t launch_init_f64(const KParams64 &kp, const e2d_params &p, double *u, cudaStream_t s);
 cudaError_t launch_eval_f64(const KParams64 &kp, int what, int n, const double *in, double *out,
                             double dtdx, double dtdy, cudaStream_t s);
@@ -183,7 +196,7 @@ void make_kparams32(const e2d_params &p, KParams32 *kp);
 // float planes of isize*jsize: hi(rho, E, mx, my) then lo(rho, E, mx, my).
 // Ghost cells of these arrays are not maintained: the step reads ghosts
 // through the boundary map.
-cudaError_t configure_f32c_kernels();
+cudaError_t configure_f32c_kernels(int riemann);
 // FP32C step / batch kernel variants (register budget x row staging), see
 // with_variant in e2d_fp32c.cu.
 constexpr int kF32cVariants = 7;

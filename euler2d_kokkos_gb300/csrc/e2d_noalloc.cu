@@ -39,7 +39,8 @@ int setup_device(int dev, double **out) {
   if (!g_scratch_ptr[dev]) {
     double *ptr = nullptr;
     if (cudaGetSymbolAddress((void **)&ptr, g_noalloc_scratch) != cudaSuccess || !ptr) return E2D_ECUDA;
-    if (configure_f64_kernels() != cudaSuccess) return E2D_ECUDA;
+    for (int r = E2D_RIEMANN_APPROX; r <= E2D_RIEMANN_HLLC; ++r)
+      if (configure_f64_kernels(r) != cudaSuccess) return E2D_ECUDA;
     g_scratch_ptr[dev] = ptr;
   }
   *out = g_scratch_ptr[dev];
@@ -74,7 +75,7 @@ extern "C" int e2d_godunov_unsplit_noalloc(const e2d_params *pin, double *u_in, 
   // the primitives kernel writes every cell of q before the flux kernel reads
   // it, and neither kernel reads the clock in this mode: nothing left over
   // from an earlier call is used
-  if (launch_fill_f64(kp, u_in, u_out, q, clk, FILL_WRITE_Q | FILL_GHOSTS_IN | FILL_GHOSTS_OUT, s) != cudaSuccess)
+  if (launch_fill_f64(kp, u_in, nullptr, q, clk, FILL_WRITE_Q, s) != cudaSuccess)
     return E2D_ECUDA;
   if (launch_flux_update_f64(kp, p.riemannSolverType, q, u_in, u_out, clk, 0, dt, nullptr, s) != cudaSuccess)
     return E2D_ECUDA;
