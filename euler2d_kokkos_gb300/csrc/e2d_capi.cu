@@ -123,6 +123,8 @@ void e2d::make_kparams(const e2d_params &p, KParams64 *kp) {
   const char *tile = std::getenv("E2D_F64_TILE");
   const int dims[1][2] = {{p.nx, p.ny}};
   choose_f64_tile(dims, 1, kp->fast != 0, tile ? std::atoi(tile) : -1, &kp->shape, &kp->ty);
+  const char *mr = std::getenv("E2D_F64_MARCH");  // segment rows; 0: tiles, as with a forced tile
+  kp->march_rows = mr ? std::atoi(mr) : tile ? 0 : choose_f64_march(p.nx, p.ny, 0);
   const char *wt = std::getenv("E2D_TEST_WAIT_TIMEOUT");
   kp->wait_test = (wt && std::atoi(wt) != 0) ? 1 : 0;
 }

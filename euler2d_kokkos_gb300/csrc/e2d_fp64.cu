@@ -610,6 +610,48 @@ __device__ __forceinline__ void block_fold(double term, unsigned int flags, unsi
   }
 }
 
+// A new cell of the fused step: its state and primitives, its CFL term into
+// the running maximum and its flags.
+template <bool FAST, class F>
+__device__ __forceinline__ void finish_cell(const F &f, const KParams64 &kp, long long s, const double un[4],
+                                            double *u_out, double *q_out, double &term, unsigned int &flags) {
+  const KGeom &g = kp.g;
+  const KPhys<double> &ph = kp.ph;
+#pragma unroll
+  for (int v = 0; v < 4; ++v) u_out[s + v * g.plane] = un[v];
+  double dd, p, ux, uy;
+  Divisor dv;
+  if (FAST)
+    primitives_fast(f, ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, dv);
+  else
+    primitives(f, ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, dv);
+  q_out[s] = dd;
+  q_out[s + g.plane] = p;
+  q_out[s + 2 * g.plane] = ux;
+  q_out[s + 3 * g.plane] = uy;
+  term = fmax_any(term, FAST ? cfl_term_fast(f, ph, dv, p, ux, uy) : cfl_term(f, ph, dv, p, ux, uy));
+  flags |= state_flags(un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV]);
+}
+
+// The last block to finish a step advances the loop state
+// (src/main.cpp:139-143); one thread per block, after a block barrier.
+__device__ __forceinline__ void finish_step64(DevClock *clk, const double dt, const int par, double *dt_trace) {
+  __threadfence();
+  const unsigned int ticket = atomicAdd(&clk->done_blocks, 1u);
+  if (ticket != gridDim.x * gridDim.y - 1) return;
+  __threadfence();
+  const int ns = clk->nstep;
+  const int slot = ns - clk->trace_base;
+  if (dt_trace && slot >= 0 && slot < clk->trace_cap) dt_trace[slot] = dt;
+  if (!(dt > 0.0) || nonfinite(dt)) clk->status |= E2D_FLAG_BAD_DT;
+  clk->dt = dt;
+  clk->t = clk->t + dt;  // only this block writes t during the step
+  clk->nstep = ns + 1;
+  clk->acc[par] = 0ull;  // read by this step; folded into by the next
+  clk->done_blocks = 0u;
+  __threadfence();
+}
+
 // The fused step's epilogue for the cells of a tile whose fluxes are in
 // shared memory: the conservative update into u_out, the primitives of the
 // new cells into q_out and the running maximum of their CFL terms and flags.
@@ -629,20 +671,8 @@ __device__ __forceinline__ void step_epilogue(const F &f, const KParams64 &kp, c
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         un[v] = update_var<TX, TYM, FAST>(f, sm, v, x, y, cells.u[n][v], dtdx, dtdy);
-        u_out[s + v * g.plane] = un[v];
       }
-      double dd, p, ux, uy;
-      Divisor dv;
-      if (FAST)
-        primitives_fast(f, ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, dv);
-      else
-        primitives(f, ph, un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV], dd, p, ux, uy, dv);
-      q_out[s] = dd;
-      q_out[s + g.plane] = p;
-      q_out[s + 2 * g.plane] = ux;
-      q_out[s + 3 * g.plane] = uy;
-      term = fmax_any(term, FAST ? cfl_term_fast(f, ph, dv, p, ux, uy) : cfl_term(f, ph, dv, p, ux, uy));
-      flags |= state_flags(un[E2D_ID], un[E2D_IP], un[E2D_IU], un[E2D_IV]);
+      finish_cell<FAST>(f, kp, s, un, u_out, q_out, term, flags);
     }
   }
 }
@@ -737,26 +767,215 @@ __global__ void __launch_bounds__(NT, MINB)
 
   block_fold<NT>(term, flags, &clk->acc[par ^ 1], &clk->status);
 
-  // the last block to finish advances the loop state (src/main.cpp:139-143)
   __syncthreads();
+  if (tid == 0) finish_step64(clk, s_dt[0], par, dt_trace);
+}
+
+// ------------------------------------------------------------ the march
+// The fused step of a large grid: a block walks a segment of a 32-column
+// strip upwards in chunks of CHUNK rows.  Each chunk traces its own rows
+// once -- the face states, x- and y-fluxes of the last row stay in shared
+// memory for the next chunk (16 rows of each, used as rings) -- so only the
+// strip's two side columns are traced twice, where a tile traces a ring of
+// cells around it.  15 rows make 16 warps of traced cells and 31 of Riemann
+// solves, two and four full rounds of the block's 8 warps, which is what 13
+// rows of a tile take.  The next chunk's primitives arrive by TMA (where the
+// strip is away from the boundary) while this one is computed, and dt, the
+// CFL fold and the block's launch are paid once a segment.
+//
+// Rows of a chunk are numbered 1 .. CHUNK (array rows r0 .. r0 + CHUNK - 1),
+// row 0 is the last one of the chunk before; the chunk updates rows 0 ..
+// CHUNK - 1, whose upper y-flux it has.  A segment of rows jb .. je starts at
+// r0 = jb - 1 and ends once row je + 1 is traced.
+constexpr int MTX = 32, CHUNK = 15, MNT = 256, MRING = 16;
+constexpr int MQW = MTX + 4, MQH = CHUNK + 2, MXW = MTX + 2;
+static_assert((MRING & (MRING - 1)) == 0 && MRING == CHUNK + 1, "row k of a chunk sits in slot (base + k) mod 16");
+constexpr size_t kMarchQ = sizeof(double) * 4 * MQH * MQW;  // one chunk's primitives
+static_assert(kMarchQ % 128 == 0, "a TMA destination is 128-byte aligned");
+constexpr size_t march_smem_bytes() {
+  return 2 * kMarchQ + sizeof(double) * (2 * 4 * MRING * MXW + 2 * 4 * MRING * MTX) + 128;
+}
+
+template <int RS, bool FAST>
+__global__ void __launch_bounds__(MNT, 2)
+    k_march_f64(const KParams64 kp, const __grid_constant__ CUtensorMap tm_q, const int use_tma, const double *q_in,
+                double *q_out, double *u_in, double *u_out, DevClock *clk, double *dt_trace) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char *base_ptr = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+  double *sQ[2] = {reinterpret_cast<double *>(base_ptr), reinterpret_cast<double *>(base_ptr + kMarchQ)};
+  double *sXm = reinterpret_cast<double *>(base_ptr + 2 * kMarchQ);  // [4][16][34] XMIN states, then x-fluxes
+  double *sXp = sXm + 4 * MRING * MXW;                               // [4][16][34] XMAX states
+  double *sYm = sXp + 4 * MRING * MXW;                               // [4][16][32] YMIN states, then y-fluxes
+  double *sYp = sYm + 4 * MRING * MTX;                               // [4][16][32] YMAX states
+  __shared__ double s_dt[3];
+  __shared__ int s_run, s_par;
+  __shared__ __align__(8) unsigned long long s_bar[2];
+  const KGeom &g = kp.g;
+  const KPhys<double> &ph = kp.ph;
+  const int tid = threadIdx.x;
+  const int bx = blockIdx.x, i0 = bx * MTX;
+  const int jb = 2 + blockIdx.y * kp.march_rows, je = min(jb + kp.march_rows, g.ny + 2) - 1;
+  const bool tma_x = use_tma && i0 >= 2 && i0 + MQW <= g.nx + 2;
+  // primitives of rows r0 - 1 .. r0 + CHUNK of a chunk by one TMA copy
+  auto by_tma = [&](int r0) { return tma_x && r0 - 1 >= 2 && r0 + CHUNK <= g.ny + 1; };
+  auto issue = [&](int r0, int b) {
+    // wait_test: block (1, 0)'s second chunk is never copied, so its wait runs out
+    if (kp.wait_test && bx == 1 && blockIdx.y == 0 && b == 1) return;
+    fence_proxy_async_smem();
+    mbar_arrive_expect(&s_bar[b], (unsigned int)kMarchQ);
+    tma_load_3d(sQ[b], &tm_q, i0, r0 - 1, 0, &s_bar[b]);
+  };
   if (tid == 0) {
-    __threadfence();
-    const unsigned int ticket = atomicAdd(&clk->done_blocks, 1u);
-    if (ticket == gridDim.x * gridDim.y - 1) {
-      __threadfence();
-      const double dt = s_dt[0];
-      const int ns = clk->nstep;
-      const int slot = ns - clk->trace_base;
-      if (dt_trace && slot >= 0 && slot < clk->trace_cap) dt_trace[slot] = dt;
-      if (!(dt > 0.0) || nonfinite(dt)) clk->status |= E2D_FLAG_BAD_DT;
-      clk->dt = dt;
-      clk->t = clk->t + dt;  // only this block writes t during the step
-      clk->nstep = ns + 1;
-      clk->acc[par] = 0ull;  // read by this step; folded into by the next
-      clk->done_blocks = 0u;
-      __threadfence();
-    }
+    mbar_init(&s_bar[0], 1u);
+    mbar_init(&s_bar[1], 1u);
+    mbar_init_fence();
+    const int run = clk->t < clk->t_end;
+    s_run = run;
+    s_par = clk->nstep & 1;
+    if (run && by_tma(jb - 1)) issue(jb - 1, 0);
+    const double dt = step_dt(ph, clk->acc[clk->nstep & 1], clk->t, clk->t_end);
+    s_dt[0] = dt;
+    s_dt[1] = quot(dt, ph.dx);
+    s_dt[2] = quot(dt, ph.dy);
   }
+  __syncthreads();
+  if (!s_run) return;  // past t_end: no copy was issued
+  const int par = s_par;
+  const double dtdx = s_dt[1], dtdy = s_dt[2];
+  const double hdtdx = half(dtdx), hdtdy = half(dtdy);
+  const int st_kind = (ph.slope_type == 2.0) ? 2 : (ph.slope_type == 1.0) ? 1 : 0;
+  const Fp f;
+  double term = 0.0;
+  unsigned int flags = 0, phase = 0;
+  bool ok = true;
+  int base = 0, buf = 0;
+  for (int r0 = jb - 1; r0 <= je + 1; r0 += CHUNK, buf ^= 1, base = (base + CHUNK) & (MRING - 1)) {
+    auto slot = [&](int k) { return (base + k) & (MRING - 1); };
+    // stage 1: this chunk's primitives; the next one's on their way (its
+    // buffer was last read before the barriers of the previous chunk)
+    if (by_tma(r0)) {
+      ok = __syncthreads_and(mbar_wait(&s_bar[buf], (phase >> buf) & 1u));
+      if (!ok) {
+        // flag the step, then wait (bounded) for the copy that may still land
+        // in this block's shared memory before leaving the segment
+        if (tid == 0) atomicOr(&clk->status, E2D_FLAG_TIMEOUT);
+        mbar_wait(&s_bar[buf], (phase >> buf) & 1u);
+        __syncthreads();
+        break;
+      }
+      phase ^= 1u << buf;
+    } else {
+      gather_qtile<MTX, MNT>(g, q_in, i0, r0 - 1, CHUNK - 2, sQ[buf]);
+      __syncthreads();
+    }
+    if (tid == 0 && r0 + CHUNK <= je + 1 && by_tma(r0 + CHUNK)) issue(r0 + CHUNK, buf ^ 1);
+
+    // stage 2: face states of rows 1 .. CHUNK, columns -1 .. 32
+    for (int k = tid; k < CHUNK * MXW; k += MNT) {
+      const int y = k / MXW, xx = k - y * MXW, sl = slot(y + 1);
+      const double *P = sQ[buf] + (y + 1) * MQW + (xx + 1);
+      double qc[4], dqx[4], dqy[4], hx[4], hy[4], s0[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v, P += MQH * MQW) {
+        qc[v] = P[0];
+        slope(f, st_kind, qc[v], P[1], P[-1], dqx[v], hx[v]);
+        slope(f, st_kind, qc[v], P[MQW], P[-MQW], dqy[v], hy[v]);
+      }
+      if (FAST)
+        trace_sources_fast(f, ph, qc, dqx, dqy, s0);
+      else
+        trace_sources(f, ph, qc, dqx, dqy, s0);
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        double fm, fp;
+        if (FAST)
+          face_pair_fast(f, ph, v, qc[v], hx[v], s0[v], hdtdx, fm, fp);
+        else
+          face_pair(f, ph, v, qc[v], hx[v], s0[v], dtdx, hdtdx, fm, fp);
+        const int o = (v * MRING + sl) * MXW + xx;
+        if (xx >= 1) sXm[o] = fm;
+        if (xx <= MTX) sXp[o] = fp;
+      }
+      if (xx >= 1 && xx <= MTX) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          double fm, fp;
+          if (FAST)
+            face_pair_fast(f, ph, v, qc[v], hy[v], s0[v], hdtdy, fm, fp);
+          else
+            face_pair(f, ph, v, qc[v], hy[v], s0[v], dtdy, hdtdy, fm, fp);
+          const int o = (v * MRING + sl) * MTX + xx - 1;
+          sYm[o] = fm;
+          sYp[o] = fp;
+        }
+      }
+    }
+    // the cells this chunk updates, loaded ahead of the Riemann solves
+    constexpr int N = (MTX * CHUNK + MNT - 1) / MNT;
+    double u[N][4];
+    long long at[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int k = tid + n * MNT, y = k / MTX, gi = i0 + 2 + (k - y * MTX), gj = r0 - 1 + y;
+      at[n] = (y < CHUNK && gi < g.nx + 2 && gj >= jb && gj <= je) ? gi + (long long)g.isize * gj : -1;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) u[n][v] = at[n] >= 0 ? __ldcg(u_in + at[n] + v * g.plane) : 0.0;
+    }
+    __syncthreads();
+
+    // stage 3: x-faces of rows 1 .. CHUNK, y-faces below them
+    constexpr int nxf = (MTX + 1) * CHUNK, nf = nxf + MTX * CHUNK;
+    for (int k = tid; k < nf; k += MNT) {
+      const bool xd = k < nxf;
+      const int kk = xd ? k : k - nxf;
+      const int y = xd ? kk / (MTX + 1) : kk / MTX, x = kk - y * (xd ? MTX + 1 : MTX);
+      const int sl = slot(y + 1), sb = slot(y);
+      const int ps = MRING * (xd ? MXW : MTX);
+      const double *pl = xd ? sXp + sl * MXW + x : sYp + sb * MTX + x;
+      double *pr = xd ? sXm + sl * MXW + x + 1 : sYm + sl * MTX + x;
+      const int on = xd ? 2 * ps : 3 * ps, ot = xd ? 3 * ps : 2 * ps;
+      const double ql[4] = {pl[0], pl[ps], pl[on], pl[ot]}, qr[4] = {pr[0], pr[ps], pr[on], pr[ot]};
+      double fl[4];
+      riemann_sel<RS, FAST>(f, ph, ql, qr, fl);
+      if (!FAST) {
+        const double dtd = xd ? dtdx : dtdy;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) fl[v] = f.xmul(fl[v], dtd);
+      }
+      pr[0] = fl[E2D_ID];
+      pr[ps] = fl[E2D_IP];
+      pr[on] = fl[E2D_IU];
+      pr[ot] = fl[E2D_IV];
+    }
+    __syncthreads();
+
+    // stage 4: rows 0 .. CHUNK - 1
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (at[n] < 0) continue;
+      const int k = tid + n * MNT, y = k / MTX, x = k - y * MTX;
+      const double *fx = sXm + slot(y) * MXW + x + 1;
+      const double *fy = sYm + slot(y) * MTX + x, *fz = sYm + slot(y + 1) * MTX + x;
+      double un[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int ox = v * MRING * MXW, oy = v * MRING * MTX;
+        if (FAST)
+          un[v] = fma(f.sub(fx[ox], fx[ox + 1]), dtdx, fma(f.sub(fy[oy], fz[oy]), dtdy, u[n][v]));
+        else
+          un[v] = f.sub(f.add(f.sub(f.add(u[n][v], fx[ox]), fx[ox + 1]), fy[oy]), fz[oy]);
+      }
+      finish_cell<FAST>(f, kp, at[n], un, u_out, q_out, term, flags);
+    }
+    // the rows this chunk read are rewritten two barriers from here at the
+    // earliest, but for the slots stage 2 of the next chunk writes
+    __syncthreads();
+  }
+  ghost_fill_tile<MTX, MNT>(g, u_in, u_out, i0, jb - 2, je - jb + 1, bx == 0, bx == (int)gridDim.x - 1,
+                            blockIdx.y == 0, blockIdx.y == gridDim.y - 1);
+  block_fold<MNT>(term, flags, &clk->acc[par ^ 1], &clk->status);
+  __syncthreads();
+  if (tid == 0) finish_step64(clk, s_dt[0], par, dt_trace);
 }
 
 // Up to `steps` steps of the device loop in one cooperative launch, a grid
@@ -1215,7 +1434,9 @@ static cudaError_t launch_flux_t(const KParams64 &kp, const double *q, double *u
 
 template <int RS>
 static cudaError_t configure_rs() {
-  cudaError_t e = cudaSuccess;
+  constexpr auto kDyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(k_march_f64<RS, false>, kDyn, (int)march_smem_bytes());
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_march_f64<RS, true>, kDyn, (int)march_smem_bytes());
   for (int k = 0; k < kShapes; ++k)
     with_shape(k, [&](auto sh) {
       using S = decltype(sh);
@@ -1313,10 +1534,45 @@ cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const doubl
   }
 }
 
+// Rows of a march's segments (0: tiles).  Grids march from 100 rows a
+// resident block on (two blocks an SM): 1024^2, 108 rows, takes 399 us a step
+// against 408 with tiles, 1531x797 HLL 526 against 547, 2048^2 1445 against
+// 1561, 4096^2 5535 against 6143 -- but 700^2, 51 rows, 205 against 197.  The
+// segment is the number of chunks whose waves of blocks take the fewest
+// chunks, a last wave with at most one block an SM counting 0.62 of a full
+// one (measured within 4 % over 10 segment lengths on 3000x1700; at 2048^2 and
+// 4096^2 the choice is within 2 % of the best of 13).
+int choose_f64_march(int nx, int ny, int rows) {
+  if (rows > 0) return rows;
+  constexpr double kSlots = 152.0 * 2, kMinRows = 100.0;
+  const double cols = (nx + MTX - 1) / MTX;
+  if (cols * ny < kMinRows * kSlots) return 0;
+  int best = 0;
+  double cost = 0.0;
+  for (int n = 4; n <= 20; ++n) {
+    const int h = CHUNK * n - 2;
+    const double waves = cols * std::ceil((double)ny / h) / kSlots, full = std::floor(waves), rest = waves - full;
+    // 0.3: a segment's start (dt, the first copy) and end (the fold)
+    const double c = (n + 0.3) * (full + (rest == 0.0 ? 0.0 : rest <= 0.5 ? 0.62 : 1.0));
+    if (best == 0 || c < cost) best = h, cost = c;
+  }
+  return best;
+}
+
 template <int RS>
 static cudaError_t launch_step_t(const KParams64 &kp, const CUtensorMap &tm_q, int use_tma, const double *q_in,
                                  double *q_out, double *u_in, double *u_out, DevClock *clk, double *dt_trace,
                                  cudaStream_t s) {
+  if (kp.march_rows > 0) {
+    dim3 grid((kp.g.nx + MTX - 1) / MTX, (kp.g.ny + kp.march_rows - 1) / kp.march_rows);
+    if (kp.fast)
+      k_march_f64<RS, true><<<grid, MNT, march_smem_bytes(), s>>>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk,
+                                                                  dt_trace);
+    else
+      k_march_f64<RS, false><<<grid, MNT, march_smem_bytes(), s>>>(kp, tm_q, use_tma, q_in, q_out, u_in, u_out, clk,
+                                                                   dt_trace);
+    return cudaGetLastError();
+  }
   with_shape(kp.shape, [&](auto sh) {
     using S = decltype(sh);
     dim3 grid((kp.g.nx + S::TX - 1) / S::TX, (kp.g.ny + kp.ty - 1) / kp.ty);
@@ -1360,6 +1616,7 @@ static void with_loop(int riemann, const KParams64 &kp, F &&f) {
 }
 
 int f64_loop_blocks(const KParams64 &kp, int riemann) {
+  if (kp.march_rows > 0) return 0;
   int blocks = 0;
   with_loop(riemann, kp, [&](auto kernel, int threads, size_t sm, int tiles) {
     const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), threads, sm);
@@ -1411,7 +1668,8 @@ bool encode_q_map(CUtensorMap *map, const double *q, const KParams64 &kp) {
   const cuuint64_t strides[2] = {(cuuint64_t)kp.g.isize * sizeof(double), (cuuint64_t)kp.g.plane * sizeof(double)};
   int tx = 0;
   with_shape(kp.shape, [&](auto sh) { tx = decltype(sh)::TX; });
-  const cuuint32_t box[3] = {(cuuint32_t)tx + 4, (cuuint32_t)kp.ty + 4, 4};
+  const cuuint32_t box[3] = {(cuuint32_t)(kp.march_rows > 0 ? MQW : tx + 4),
+                             (cuuint32_t)(kp.march_rows > 0 ? MQH : kp.ty + 4), 4};
   const cuuint32_t estr[3] = {1, 1, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(q), dims, strides, box, estr,
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

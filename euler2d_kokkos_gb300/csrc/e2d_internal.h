@@ -59,6 +59,7 @@ struct KParams64 {
   KGeom g;
   KPhys<double> ph;
   int shape, ty;  // tile shape of the step and its rows (choose_f64_tile)
+  int march_rows; // rows of the segments a large grid's step marches (choose_f64_march); 0: tiles
   int fast;       // E2D_PRECISION_FP64_FAST: the fused step's fast forms (not bit-identical)
   int wait_test;  // nonzero: tile (1, 1) of the fused step never stages its primitives,
                   // so its bounded wait runs out (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
@@ -177,6 +178,8 @@ cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const doubl
 // the shape's most).
 void choose_f64_tile(const int (*dims)[2], int n, bool fast, int tile, int *shape, int *ty);
 int f64_tiles(int nx, int ny, int shape, int ty);
+// Segment rows of a grid's march, 0 if it runs tiles; rows > 0 forces them.
+int choose_f64_march(int nx, int ny, int rows);
 // Blocks of a kernel resident on the current device at once (0: it cannot
 // launch cooperatively).
 int resident_blocks(const void *kernel, int threads, size_t smem);
