@@ -118,8 +118,9 @@ static __device__ double2 g_unit[32] = {
 // products there the two pipes run side by side.  HLLC: face increments,
 // transport terms, contact sums, energies, flux scaling, 1.556 instead of 1.69
 // ms a 2048^2 step; with more of them the step slows down again (1.57 to 1.63
-// ms).  HLL: energies, momentum and energy fluxes, jump terms too, 1.866 ->
-// 1.761 ms.  The fast forms, which have the fewest FP64 instructions: all
+// ms).  HLL: energies, transverse momentum and energy fluxes, jump
+// terms and the final scaling, 1.866 -> 1.761 ms with tiles, 1.574 -> 1.548
+// for the scaling (march).  The fast forms, which have the fewest FP64 instructions: all
 // products that are not part of an FMA, 1.308 -> 1.236 ms.  Where each SM holds
 // one small tile the step waits on latency, not on the FP64 pipe, and the
 // plain product is the faster one (64x48: 16.0 against 17.1 us a step).
@@ -138,6 +139,11 @@ struct FpT {
   }
   static __device__ __forceinline__ double abs(double x) {
     return f64i::make(f64i::high(x) & 0x7fffffffu, f64i::low(x));
+  }
+  // -x where x is a difference a - b: b - a (+0, not -0, where they are equal)
+  static __device__ __forceinline__ double reversed(double x) {
+    const unsigned int hi = f64i::high(x), lo = f64i::low(x);
+    return f64i::make(((hi << 1) | lo) != 0u ? hi ^ 0x80000000u : 0u, lo);
   }
   __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
   __device__ __forceinline__ double sub(double a, double b) const { return fma(b, mone, a); }

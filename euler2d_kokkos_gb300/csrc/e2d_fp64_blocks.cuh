@@ -147,13 +147,16 @@ __device__ __noinline__ void riemann_approx(const F &f, const KPhys<double> &ph,
     const double wwr = wave(cr, pold, pr, dpr);
     const double w2l = f.mul(wwl, wwl), w2r = f.mul(wwr, wwr);
     // 2 w w w: the doubling is exact wherever it is applied (no overflow here)
-    const double qxl = quot(f.mul(f.mul(f64x::twice(wwl), wwl), wwl), f.add(w2l, cl));
-    const double qxr = quot(f.mul(f.mul(f64x::twice(wwr), wwr), wwr), f.add(w2r, cr));
+    const double qxl = quot(f.mul(f64x::twice(w2l), wwl), f.add(w2l, cl));
+    const double qxr = quot(f.mul(f64x::twice(w2r), wwr), f.add(w2r, cr));
     const double usl = f.sub(ul, quot(f.sub(pold, pl), wwl));
     const double usr = f.add(ur, quot(f.sub(pold, pr), wwr));
     const double delp = fmax_any(f.mul(quot(f.mul(qxr, qxl), f.add(qxr, qxl)), f.sub(usl, usr)), f.neg(pold));
     pold = f.add(pold, delp);
-    conv = f.abs(quot(delp, f.add(pold, ph.smallpp)));
+    // pold + smallpp is pold where that is 2^55 times the larger
+    const int hs = (int)f64i::high(ph.smallpp);
+    const bool far = hs >= 0 && (int)f64i::high(pold) - hs > 55 << 20;
+    conv = f.abs(quot(delp, far ? pold : f.add(pold, ph.smallpp)));
   }
   pstar = pold;
   wl = wave(cl, pstar, pl, dpl);
@@ -206,6 +209,8 @@ __device__ __noinline__ void riemann_approx(const F &f, const KPhys<double> &ph,
 // star state of the side that is read are built (SL > 0 reads the left state,
 // else the contact selects), and the larger sound speed is the root of the
 // larger square (a correctly rounded root is monotonic): the same values.
+// S - us and rs (S - us) are, but for the sign, the differences and products
+// that rcl and rcr are made of.
 // Cut-offs, maxima, the 0.5 factors and the sign tests use the exact integer
 // forms of e2d_f64_exact.cuh.
 template <class F>
@@ -222,8 +227,9 @@ __device__ __forceinline__ void riemann_hllc(const F &f, const KPhys<double> &ph
   const double cmax = root(max_nn(c2l, c2r));
   const double SL = f.sub(min_any(ul, ur), cmax);
   const double SR = f.add(max_any(ul, ur), cmax);
-  const double rcl = f.mul(rl, f.sub(ul, SL));
-  const double rcr = f.mul(rr, f.sub(SR, ur));
+  const double dl = f.sub(ul, SL), dr = f.sub(SR, ur);
+  const double rcl = f.mul(rl, dl);
+  const double rcr = f.mul(rr, dr);
   const Divisor rc = divisor(f.add(rcr, rcl));
   const double ustar = quot(f.add(f.add(f.xmul(rcr, ur), f.xmul(rcl, ul)), f.sub(pl, pr)), rc);
   const double ptotstar =
@@ -235,9 +241,9 @@ __device__ __forceinline__ void riemann_hllc(const F &f, const KPhys<double> &ph
   const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr, vs = lft ? ql[E2D_IV] : qr[E2D_IV];
   const double hrs = half(rs);
   const double es = f.add(f.xmul(ps, ph.entho), f.add(f.xmul(f.xmul(hrs, us), us), f.xmul(f.xmul(hrs, vs), vs)));
-  const double sdu = f.sub(S, us);
+  const double sdu = lft ? f.reversed(dl) : dr, rsdu = lft ? f.reversed(rcl) : rcr;  // S - us, rs (S - us)
   const Divisor sds = divisor(f.sub(S, ustar));
-  const double rstar = quot(f.mul(rs, sdu), sds);
+  const double rstar = quot(rsdu, sds);
   const double etotstar = quot(f.add(f.sub(f.mul(sdu, es), f.mul(ps, us)), f.mul(ptotstar, ustar)), sds);
   const double ro = own ? rs : rstar, uo = own ? us : ustar, ptoto = own ? ps : ptotstar;
   const double etoto = own ? es : etotstar;
@@ -261,26 +267,30 @@ __device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph,
   const double rr = max_pos(qr[E2D_ID], ph.smallr);
   const double pr = floor_pressure(f, ph, qr[E2D_IP], rr);
   const double ur = qr[E2D_IU], vr = qr[E2D_IV];
-  auto energy = [&](double r, double p, double u, double v) {
-    const double h = half(r);
-    return f.add(f.xmul(p, ph.entho), f.add(f.xmul(f.xmul(h, u), u), f.xmul(f.xmul(h, v), v)));
-  };
-  const double etotl = energy(rl, pl, ul, vl), etotr = energy(rr, pr, ur, vr);
+  // r u, r v and r u u serve the state, the flux and the energy, whose factor
+  // 0.5 is exact wherever it is applied (barring underflow, and the energy's
+  // pressure term absorbs that): 12 products a cell fewer, 523 -> 495 us a
+  // 1531x797 step, 488 with the last product on the integer pipes in the
+  // room this leaves there (another 4 or 8 of a flux's: 492, 500).
+  const double mxl = f.mul(rl, ul), myl = f.mul(rl, vl), mxul = f.mul(mxl, ul);
+  const double mxr = f.mul(rr, ur), myr = f.mul(rr, vr), mxur = f.mul(mxr, ur);
+  const double etotl = f.add(f.xmul(pl, ph.entho), f.add(half(mxul), half(f.xmul(myl, vl))));
+  const double etotr = f.add(f.xmul(pr, ph.entho), f.add(half(mxur), half(f.xmul(myr, vr))));
   const double c2l = max_pos(quot(f.mul(ph.gamma0, pl), rl), ph.smallc2);
   const double c2r = max_pos(quot(f.mul(ph.gamma0, pr), rr), ph.smallc2);
   const double cmax = root(max_nn(c2l, c2r));
   const double SL = f.sub(min_any(ul, ur), cmax);
   const double SR = f.add(max_any(ul, ur), cmax);
-  const double UL[4] = {rl, etotl, f.mul(rl, ul), f.mul(rl, vl)};
-  const double UR[4] = {rr, etotr, f.mul(rr, ur), f.mul(rr, vr)};
+  const double UL[4] = {rl, etotl, mxl, myl};
+  const double UR[4] = {rr, etotr, mxr, myr};
   double FL[4], FR[4];
   FL[E2D_ID] = UL[E2D_IU];
   FL[E2D_IP] = f.xmul(f.add(etotl, pl), ul);
-  FL[E2D_IU] = f.add(f.mul(UL[E2D_IU], ul), pl);
+  FL[E2D_IU] = f.add(mxul, pl);
   FL[E2D_IV] = f.xmul(UL[E2D_IU], vl);
   FR[E2D_ID] = UR[E2D_IU];
   FR[E2D_IP] = f.xmul(f.add(etotr, pr), ur);
-  FR[E2D_IU] = f.add(f.mul(UR[E2D_IU], ur), pr);
+  FR[E2D_IU] = f.add(mxur, pr);
   FR[E2D_IV] = f.xmul(UR[E2D_IU], vr);
   if (gt0(SL)) {
 #pragma unroll
@@ -294,7 +304,7 @@ __device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph,
     const double rden = quot(f.one, f.sub(SR, SL));
 #pragma unroll
     for (int v = 0; v < 4; ++v)
-      flux[v] = f.mul(f.add(f.sub(f.mul(SR, FL[v]), f.mul(SL, FR[v])), f.xmul(sls, f.sub(UR[v], UL[v]))), rden);
+      flux[v] = f.xmul(f.add(f.sub(f.mul(SR, FL[v]), f.mul(SL, FR[v])), f.xmul(sls, f.sub(UR[v], UL[v]))), rden);
   }
 }
 
@@ -389,8 +399,9 @@ __device__ __forceinline__ void riemann_hllc_fast(const F &f, const KPhys<double
   const double cmax = root(max_nn(c2l, c2r));
   const double SL = f.sub(min_any(ul, ur), cmax);
   const double SR = f.add(max_any(ul, ur), cmax);
-  const double rcl = f.mul(rl, f.sub(ul, SL));
-  const double rcr = f.mul(rr, f.sub(SR, ur));
+  const double dl = f.sub(ul, SL), dr = f.sub(SR, ur);
+  const double rcl = f.mul(rl, dl);
+  const double rcr = f.mul(rr, dr);
   const Divisor rc = divisor(f.add(rcr, rcl));
   const double ustar = quot(fma(rcr, ur, fma(rcl, ul, f.sub(pl, pr))), rc);
   const double ptotstar = quot(fma(rcr, pl, fma(rcl, pr, f.xmul(f.xmul(rcl, rcr), f.sub(ul, ur)))), rc);
@@ -400,9 +411,9 @@ __device__ __forceinline__ void riemann_hllc_fast(const F &f, const KPhys<double
   const double S = lft ? SL : SR;
   const double rs = lft ? rl : rr, us = lft ? ul : ur, ps = lft ? pl : pr, vs = lft ? ql[E2D_IV] : qr[E2D_IV];
   const double es = fma(ps, ph.entho, f.xmul(half(rs), fma(us, us, f.xmul(vs, vs))));
-  const double sdu = f.sub(S, us);
+  const double sdu = lft ? f.reversed(dl) : dr, rsdu = lft ? f.reversed(rcl) : rcr;  // S - us, rs (S - us)
   const Divisor sds = divisor(f.sub(S, ustar));
-  const double rstar = quot(f.xmul(rs, sdu), sds);
+  const double rstar = quot(rsdu, sds);
   const double etotstar = quot(fma(sdu, es, fma(f.neg(ps), us, f.xmul(ptotstar, ustar))), sds);
   const double ro = own ? rs : rstar, uo = own ? us : ustar, ptoto = own ? ps : ptotstar;
   const double etoto = own ? es : etotstar;
