@@ -229,7 +229,7 @@ int rebuild_list(e2d_batch *b) {
   long long units = 0;
   for (HostInst &h : b->slots)
     if (h.used && !h.fp64 && h.mirror.active) units += units_of(h.mirror.kp);
-  b->short_rows = b->tuned_by_caller ? 0 : short_rows_for(units);
+  b->short_rows = b->tuned_by_caller ? 0 : short_rows_for(units, b->riemann);
   const int per_sm = b->short_rows > 0 ? 1 : batch_blocks_per_sm(b->riemann, b->variant);
   const long long warps = 152LL * per_sm * 4;
   int shift = 0;

@@ -1,6 +1,7 @@
 // e2d_capi.cu -- the C ABI of include/e2d.h: simulation handles, device
-// buffers, the HydroRun method mirrors and the graph-replayed time loop, for
-// both arithmetic modes (FP64 bit-identical, FP32 compensated).
+// buffers, the HydroRun method mirrors and the device time loop (many steps
+// per cooperative launch, or graph-replayed steps), for both arithmetic modes
+// (FP64 bit-identical, FP32 compensated).
 #include "e2d_internal.h"
 
 #include <cmath>
@@ -324,7 +325,8 @@ int e2d_create(const e2d_params *pin, e2d_sim **out) {
     if (std::atoi(v) > 0 && std::atoi(v) <= 512) {
       const int h = std::atoi(v);
       s->kp32.short_rows = h == 2 || h == 4 || h == 8 ? h : 0;
-      s->kp32.strip_h = (h + 15) / 16 * 16;
+      s->kp32.strip_h = s->kp32.tail_h = (h + 15) / 16 * 16;
+      s->kp32.tall = (p.ny + s->kp32.strip_h - 1) / s->kp32.strip_h;
     }
   auto fail = [&](int status) {
     e2d_destroy(s);

@@ -33,6 +33,8 @@
 
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdlib>
 #include <map>
@@ -540,27 +542,30 @@ __device__ __forceinline__ int source_row(const KGeom &g, int r, bool yghost, bo
 // word: 7500 to 19000 clocks for a 256-column grid's last strip to get under
 // way, against 2600.)  What a lane copies of them is the same for every row
 // of the strip and worked out once: with the boundary map in the row loop a
-// batch of 512 mixed solves, mostly boundary strips, took 2.08 s, so 1.975
+// batch of 512 mixed solves, mostly boundary strips, took 2.08 s, now 2.00
 // (every column by itself: 2.03).
 struct EdgeCopies {
-  bool whole;    // the lane's chunk has no ghost column
-  int edge[3];   // the lane's column of a chunk with one: source << 6 | column of the slot; -1: none
+  bool whole;   // the lane's chunk has no ghost column
+  bool third;   // a grid of one column of strips with three chunks that have
+  int edge[2];  // the lane's column of a chunk with one: source << 6 | column of the slot; -1: none
 };
+// The lane's column of the array's columns 4 q .. 4 q + 3.
+__device__ __forceinline__ int edge_column(const KGeom &g, int q, int cs, int lane) {
+  const int c = 4 * q + (lane & 3);
+  if (4 * q < cs || 4 * q >= cs + 64 || c > g.nx + 3) return -1;
+  bool f;
+  return ghost_source(c, g.nx, g.bc_xmin, g.bc_xmax, f) << 6 | (c - cs);
+}
 __device__ __forceinline__ EdgeCopies edge_copies(const KGeom &g, int cs, int lane, bool direct) {
-  EdgeCopies e{true, {-1, -1, -1}};
+  EdgeCopies e{true, false, {-1, -1}};
   if (direct) return e;
   const int c4 = cs + 4 * (lane & 15);
   e.whole = c4 >= 2 && c4 + 3 < g.nx + 2;
-  auto ghost_chunk = [&](int q) {  // columns 4 q .. 4 q + 3 of the array
-    const int c = 4 * q + (lane & 3);
-    if (4 * q < cs || 4 * q >= cs + 64 || c > g.nx + 3) return -1;
-    bool f;
-    return ghost_source(c, g.nx, g.bc_xmin, g.bc_xmax, f) << 6 | (c - cs);
-  };
   const int q0 = (g.nx + 2) >> 2, q1 = (g.nx + 3) >> 2;  // never the first chunk unless nx < 2
-  if (cs == 0) e.edge[0] = ghost_chunk(0);
-  if (q0 > 0) e.edge[1] = ghost_chunk(q0);
-  if (q1 > q0) e.edge[2] = ghost_chunk(q1);
+  if (cs == 0) e.edge[0] = edge_column(g, 0, cs, lane);
+  else if (q1 > q0) e.edge[0] = edge_column(g, q1, cs, lane);
+  if (q0 > 0) e.edge[1] = edge_column(g, q0, cs, lane);
+  e.third = cs == 0 && q1 < 16 && q1 > q0;
   return e;
 }
 
@@ -581,8 +586,12 @@ __device__ __forceinline__ void stage_row(const KParams32 &kp, const float *__re
     const float *from = row + (lane >> 2) * kp.wplane;
     float *to = slot + (lane >> 2) * 64;
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < 2; ++k)
       if (ec.edge[k] >= 0) cp_async4(to + (ec.edge[k] & 63), from + (ec.edge[k] >> 6));
+    if (ec.third) {
+      const int e = edge_column(g, (g.nx + 3) >> 2, cs, lane);
+      if (e >= 0) cp_async4(to + (e & 63), from + (e >> 6));
+    }
   }
 }
 
@@ -617,7 +626,7 @@ __device__ __forceinline__ void stage_row_tma(const KGeom &g, const CUtensorMap 
 template <int RS, int PFD, int TMA, bool INTERIOR, bool TGT, int SUB = 0>
 __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *__restrict__ w_in,
                                             float *__restrict__ w_out, const float2 dtdx,
-                                            const float2 dtdy, const int sx, const int sy,
+                                            const float2 dtdy, const int sx, const int rb, const int re,
                                             const int lane, unsigned long long *target,
                                             unsigned int *status, float *ring, const CUtensorMap *map,
                                             unsigned long long *bars, unsigned int &phase, const int urow = 0,
@@ -633,10 +642,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
   int unit = 0;
   const KGeom &g = kp.g;
   const KPhys<float> &ph = kp.ph;
-  const int SH = SUB > 0 ? SUB : kp.strip_h;
   const int cb = 2 + sx * OUTW;       // array column of the strip's first output column
-  const int rb = 2 + sy * SH;         // array row of the strip's first output row
-  const int re = min(rb + SH, g.ny + 2);
   const int c0 = cb - 2 + 2 * lane;   // the lane's columns: c0, c0 + 1
   const bool direct = INTERIOR || ((cb - 2 >= 2) && (cb + OUTW + 1 <= g.nx + 1));
   const bool writer = (lane >= 1) && (lane <= 30) && (c0 < g.nx + 2);
@@ -694,7 +700,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
   auto stage = [&](int r, int sl) {
     if (bulk && TMA == 1) {
       // wait_test: the first row of strip (1, 0) is never copied
-      if (kp.wait_test && sx == 1 && sy == 0 && r == rb - 2) return;
+      if (kp.wait_test && sx == 1 && rb == 2 && r == rb - 2) return;
       stage_row_tma(g, map, r, cb - 2, lane, yghost, slot_of(sl), bars + sl);
       pending |= 1u << sl;
     } else {
@@ -878,6 +884,19 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
       float2 yl[4] = {ymax_prev[E2D_ID], ymax_prev[E2D_IP], ymax_prev[E2D_IV], ymax_prev[E2D_IU]};
       float2 yr[4] = {ymin[E2D_ID], ymin[E2D_IP], ymin[E2D_IV], ymin[E2D_IU]};
       float2 f[4];
+      if (RS == E2D_RIEMANN_APPROX && !INTERIOR && c0 > g.nx) {
+        // beyond the grid's last faces the ring holds nothing: a state the
+        // iterative solver is done with at once (whatever else is there it
+        // iterates on, up to ten times for the whole warp: 1100^2 90 us a
+        // step against 82)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float still = v == E2D_ID || v == E2D_IP ? 1.0f : 0.0f;
+          if (c0 > g.nx + 2) xl[v].x = xr[v].x = still;
+          if (c0 > g.nx + 1) xl[v].y = xr[v].y = yl[v].x = yr[v].x = still;
+          yl[v].y = yr[v].y = still;
+        }
+      }
       if (SUB > 0 && m < rb) {  // a short strip: two of its few solves saved
 #pragma unroll
         for (int v = 0; v < 4; ++v) fx[v] = f[v] = f2(0.0f);
@@ -985,20 +1004,19 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
 template <int RS, int PFD, int TMA>
 __device__ __forceinline__ bool march_strip(const KParams32 &kp, const float *__restrict__ w_in,
                                             float *__restrict__ w_out, const float2 dtdx,
-                                            const float2 dtdy, const int sx, const int sy,
+                                            const float2 dtdy, const int sx, const int rb, const int re,
                                             const int lane, unsigned long long *target,
                                             unsigned int *status, float *ring, const CUtensorMap *map,
                                             unsigned long long *bars, unsigned int &phase) {
   const KGeom &g = kp.g;
-  const int cb = 2 + sx * OUTW, rb = 2 + sy * kp.strip_h;
-  const int re = min(rb + kp.strip_h, g.ny + 2);
+  const int cb = 2 + sx * OUTW;
   const bool interior = (cb - 2 >= 2) && (cb + OUTW + 1 <= g.nx + 1) && !(rb - 2 < 2) && !(re + 1 > g.ny + 1);
   if constexpr (PFD > 0) {
     if (interior && target)
-      return march_strip_t<RS, PFD, TMA, true, true>(kp, w_in, w_out, dtdx, dtdy, sx, sy, lane, target, status,
+      return march_strip_t<RS, PFD, TMA, true, true>(kp, w_in, w_out, dtdx, dtdy, sx, rb, re, lane, target, status,
                                                      ring, map, bars, phase);
   }
-  return march_strip_t<RS, PFD, TMA, false, false>(kp, w_in, w_out, dtdx, dtdy, sx, sy, lane, target, status,
+  return march_strip_t<RS, PFD, TMA, false, false>(kp, w_in, w_out, dtdx, dtdy, sx, rb, re, lane, target, status,
                                                    ring, map, bars, phase);
 }
 
@@ -1070,14 +1088,16 @@ __global__ void __launch_bounds__(NT, MINB)
   const float2 dtdy = f2((float)s_dt[2]);
 
   const int nsx = (g.nx + OUTW - 1) / OUTW;
-  const int SH = kp.strip_h;
-  const int nsy = (g.ny + SH - 1) / SH;
   const int strip = blockIdx.x * WPB + (tid >> 5);
+  // the tall strips first, then rows of shorter ones
+  const int tall = kp.tall * nsx;
+  const int sh = strip < tall ? kp.strip_h : kp.tail_h;
+  const int rb = 2 + (strip < tall ? strip / nsx * sh : kp.tall * kp.strip_h + (strip - tall) / nsx * sh);
   unsigned long long *bars = s_bars + (TMA ? (tid >> 5) * kMaxSlots : 0);
   unsigned int phase = 0u;
-  if (strip < nsx * nsy) {
+  if (rb < g.ny + 2) {
     if (TMA && PFD > 0) ring_bars_init(bars, PFD + 3, lane);
-    march_strip<RS, PFD, TMA>(kp, w_in, w_out, dtdx, dtdy, strip % nsx, strip / nsx, lane,
+    march_strip<RS, PFD, TMA>(kp, w_in, w_out, dtdx, dtdy, strip % nsx, rb, min(rb + sh, g.ny + 2), lane,
                          use_clock ? &clk->acc[slot ^ 1] : nullptr, &clk->status,
                          warp_ring<PFD>(tid >> 5), &tm_in, bars, phase);
   }
@@ -1136,15 +1156,14 @@ __device__ __forceinline__ void short_unit(const KParams32 &kp, const float *w_i
   int local = 0;
   if (has) {
     const float2 dtdx = f2(d.x), dtdy = f2(d.y);
-    const int sy = (rb - 2) / SUB;
     unsigned int phase = 0u;
     const int cb = 2 + sx * OUTW;
     const bool interior = (cb - 2 >= 2) && (cb + OUTW + 1 <= g.nx + 1) && !(rb - 2 < 2) && !(re + 1 > g.ny + 1);
     if (interior)
-      march_strip_t<RS, SHORT_PFD, 0, true, true, SUB>(kp, w_in, w_out, dtdx, dtdy, sx, sy, lane, target, status, ring,
+      march_strip_t<RS, SHORT_PFD, 0, true, true, SUB>(kp, w_in, w_out, dtdx, dtdy, sx, rb, re, lane, target, status, ring,
                                                        nullptr, nullptr, phase, rb - ub, &best, &local);
     else
-      march_strip_t<RS, SHORT_PFD, 0, false, true, SUB>(kp, w_in, w_out, dtdx, dtdy, sx, sy, lane, target, status,
+      march_strip_t<RS, SHORT_PFD, 0, false, true, SUB>(kp, w_in, w_out, dtdx, dtdy, sx, rb, re, lane, target, status,
                                                         ring, nullptr, nullptr, phase, rb - ub, &best, &local);
     cp_async_wait<0>();  // rows past a strip cut short by the grid's end
   }
@@ -1288,12 +1307,13 @@ __global__ void __launch_bounds__(NT, MINB)
     const KParams32 &kp = I.kp;
     const int par = I.par;
     const int strip = w - strip_begin[lo];
+    const int rb = 2 + strip / I.nsx * kp.strip_h;
     if (ring_ok) {
       // the general march only: a persistent warp takes strips of many
       // instances, mostly boundary strips of small grids, and a second
       // instantiation in this loop measured 14 % slower on the 512-solve mix
       ring_ok = march_strip_t<RS, PFD, TMA, false, false>(kp, I.w[par], I.w[par ^ 1], f2(I.dtdx), f2(I.dtdy),
-                                                          strip % I.nsx, strip / I.nsx, lane,
+                                                          strip % I.nsx, rb, min(rb + kp.strip_h, kp.g.ny + 2), lane,
                                                           &I.acc[(I.nstep + 1) & 1], &I.status,
                                                           warp_ring<PFD>(threadIdx.x >> 5), &I.tm[par], bars, phase);
     } else if (lane == 0) {
@@ -1475,22 +1495,61 @@ int batch_blocks_per_sm(int riemann, int variant) {
   }
 }
 
-// Rows per warp strip, by the strips it gives against the warps that run at
-// once (152 SMs x 12): the shortest while its strips are one wave; one wave
-// of taller strips rather than a second wave begun (1500^2: 32 rows 59.5 us a
-// step, 16 64.9); 16 while 32 would begin a second wave (2048^2: 97.6, 32
-// rows 103.4); then the tallest with two waves of 32 rows (3000^2: 169 against
-// 176 with 16) or four of 64 (8192^2: 992; 32 rows 1016): taller strips load
-// and march less halo, more waves leave less of the last one idle.
-int default_strip_h(int nx, int ny) {
-  const long long wave = 152 * 12;
-  auto strips = [&](int h) { return (long long)((nx + OUTW - 1) / OUTW) * ((ny + h - 1) / h); };
-  if (strips(64) >= 4 * wave) return 64;
-  if (strips(32) >= 2 * wave) return 32;
-  return strips(16) > wave && strips(32) <= wave ? 32 : 16;
+// The strips of a grid (152 SMs x 12 = 1824 warps are resident). Grids of less
+// than a wave of 32-row strips: the shortest while its strips are one wave,
+// and one wave of taller strips rather than a second wave begun (1500^2: 32
+// rows 59.5 us a step, 16 64.9). Larger grids: `tall` rows of strips of strip_h rows, as many as fill whole
+// waves, then strips of tail_h rows, which start as the tall ones end and
+// keep every SM busy to the last. Tall strips march fewer halo rows (4 a
+// strip), short ones leave less of a last wave idle; with one height a grid
+// had to choose. Cost, us: 4 + 1.55 a marched row in a full wave, less in
+// the last one if it has at most two thirds or one third of the warps; from
+// six waves on the strips' ends no longer coincide and a part of a wave costs
+// its part. (64 rows throughout do worse than that below 3.5 waves: 3500^2
+// 235 us against 223 with 32.) Measured, us a step, HLLC, against the best single height: 8192^2
+// 1034 -> 1004, 6000x3000 309 -> 288, 4096^2 296 -> 282, 2896^2 166 -> 153,
+// 2048^2 102 -> 92, 700x5000 106 -> 90, 6000x641 89 -> 78.
+// The iterative solver keeps one height, the tallest that gives four waves:
+// its warps iterate as long as their slowest face, so long strips drift apart
+// (4096^2: 595 us with strips of 32, 701 with 128 and 32; 1400^2: 123 with 16,
+// 156 with 32).
+static void choose_strips(const e2d_params &p, KParams32 *kp) {
+  const int nx = p.nx, ny = p.ny;
+  const int nsx = (nx + OUTW - 1) / OUTW;
+  const double wave = 152 * 12;
+  auto rows_of = [](int n, int h) { return n > 0 ? (n + h - 1) / h : 0; };
+  auto strips = [&](int h) { return (double)nsx * rows_of(ny, h); };
+  const bool approx = p.riemannSolverType == E2D_RIEMANN_APPROX;
+  int h = 16;
+  if (approx)
+    for (h = 64; h > 16 && strips(h) < 4 * wave;) h /= 2;
+  else if (strips(16) > wave)
+    h = 32;
+  kp->strip_h = kp->tail_h = h;
+  kp->tall = rows_of(ny, h);
+  if (approx || strips(32) < wave) return;
+  double best = 0.0;
+  auto consider = [&](int h1, int h2, int tall) {
+    const double w1 = nsx * (double)tall / wave, w2 = nsx * (double)rows_of(ny - tall * h1, h2) / wave;
+    const bool soft = w1 + w2 >= 6.0;
+    auto part = [&](double w, int h) {
+      const double full = std::floor(w), rest = w - full, row = h + 4;
+      if (soft) return w * (4.0 + 1.55 * row);
+      return full * (4.0 + 1.55 * row) +
+             (rest == 0.0 ? 0.0 : 4.0 + (rest <= 1.0 / 3 ? 1.0 : rest <= 2.0 / 3 ? 1.35 : 1.55) * row);
+    };
+    // the tall strips' last wave is all but full: it costs a whole one
+    const double t = part(soft ? w1 : std::ceil(w1), h1) + part(w2, h2) + (soft ? 0.3 * (4.0 + 1.55 * (h2 + 4)) : 0.0);
+    if (best == 0.0 || t < best) best = t, kp->strip_h = h1, kp->tail_h = h2, kp->tall = tall;
+  };
+  for (int u = strips(64) >= 3.5 * wave ? 64 : 32; u >= 16; u /= 2) consider(u, u, 0);
+  for (int h1 = 128; h1 >= 32; h1 /= 2)
+    for (int h2 = 32; h2 >= 16; h2 /= 2)
+      for (int k = (int)(nsx * (double)(ny / h1) / wave); h2 < h1 && k >= 1 && k >= (int)(nsx * (double)(ny / h1) / wave) - 1; --k)
+        consider(h1, h2, (int)(k * wave / nsx));
 }
 
-// Rows of a grid's short strips (0: strips of default_strip_h rows), by the
+// Rows of a grid's short strips (0: those of choose_strips), by the
 // number of 60 x 16 fold units, a block each: 2 rows while every block has an
 // SM of its own, 4 while all are resident two to an SM, 8 while the extra
 // halo rows (10 marched for 8 written) cost less than a 16-row march's
@@ -1498,10 +1557,15 @@ int default_strip_h(int nx, int ny) {
 // against 16: 256^2 (80 units) 10.5 / 10.8 / 15.1 against 27.3; 512^2 (288)
 // 17.1 / 12.0 / 16.2 against 30.2; 700^2 (528) 35.9 / 21.4 / 19.6 against
 // 36.3; 1201x700 (924) 57 / 39 / 31.1 against 35.0; 1024^2 (1152) 70 / 44 /
-// 37.6 against 35.7.
-int short_rows_for(long long units) { return units <= 152 ? 2 : units <= 304 ? 4 : units <= 1000 ? 8 : 0; }
-int default_short_rows(int nx, int ny) {
-  return short_rows_for((long long)((nx + OUTW - 1) / OUTW) * ((ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS));
+// 37.6 against 35.7. Just above 1000 units 8 rows and 16 are within 1 % for
+// HLLC, 8 ahead for HLL (450x2100, 1056: 38.6 against 39.9) and behind for
+// the iterative solver (75 against 69).
+int short_rows_for(long long units, int riemann) {
+  return units <= 152 ? 2 : units <= 304 ? 4 : units <= (riemann == E2D_RIEMANN_APPROX ? 1000 : 1100) ? 8 : 0;
+}
+static int default_short_rows(const e2d_params &p) {
+  return short_rows_for((long long)((p.nx + OUTW - 1) / OUTW) * ((p.ny + CFL_UNIT_ROWS - 1) / CFL_UNIT_ROWS),
+                        p.riemannSolverType);
 }
 
 void make_kparams32(const e2d_params &p, KParams32 *kp) {
@@ -1516,8 +1580,8 @@ void make_kparams32(const e2d_params &p, KParams32 *kp) {
   kp->wpitch = (p.isize + 3) & ~3;
   kp->wplane = (long long)kp->wpitch * p.jsize;
   kp->variant = 4;  // 3 blocks per SM, rows staged by cp.async (fastest at 8192^2)
-  kp->strip_h = default_strip_h(p.nx, p.ny);
-  kp->short_rows = default_short_rows(p.nx, p.ny);
+  choose_strips(p, kp);
+  kp->short_rows = default_short_rows(p);
   const char *wt = std::getenv("E2D_TEST_WAIT_TIMEOUT");
   kp->wait_test = (wt && std::atoi(wt) != 0) ? 1 : 0;
 }
@@ -1726,7 +1790,7 @@ cudaError_t launch_f32c_step(const KParams32 &kp, int riemann, const float *w_in
     return cudaGetLastError();
   }
   const int nsx = (kp.g.nx + OUTW - 1) / OUTW;
-  const int nsy = (kp.g.ny + kp.strip_h - 1) / kp.strip_h;
+  const int nsy = kp.tall + std::max(0, (kp.g.ny - kp.tall * kp.strip_h + kp.tail_h - 1) / kp.tail_h);
   const int blocks = (nsx * nsy + WPB - 1) / WPB;
   with_step_variant(kp.variant, [&](auto minb, auto pfd, auto tma) {
     launch_step_v<decltype(minb)::value, decltype(pfd)::value, decltype(tma)::value>(kp, riemann, blocks, w_in, w_out, tm_in, clk,

@@ -76,13 +76,12 @@ struct KParams32 {
   long long wplane;  // wpitch * jsize
   int variant;       // step kernel register-budget variant (see launch_f32c_step)
   int strip_h;       // rows per warp strip of the step kernel
+  int tall, tail_h;  // single grids: so many rows of strips of strip_h rows, then strips of tail_h
   int short_rows;    // 2, 4 or 8: the single grid's step runs short strips of so many rows; 0: strip_h
   int wait_test;     // nonzero: strip (1, 0) never stages its first row, or a multi-step launch's
                      // barrier waits for a block too many, so that the bounded wait runs out
                      // (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
 };
-int default_strip_h(int nx, int ny);
-int default_short_rows(int nx, int ny);
 
 // Device-resident loop state of the time loop of src/main.cpp:100-145.
 struct DevClock {
@@ -283,7 +282,7 @@ cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, cons
                                    const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
                                    cudaStream_t s);
 int units_of(const KParams32 &kp);
-int short_rows_for(long long units);
+int short_rows_for(long long units, int riemann);
 // dt, dt/dx, dt/dy and `active` of an instance from acc[nstep & 1].
 cudaError_t launch_batch_arm(BatchInst *inst, cudaStream_t s);
 // Resident blocks per SM of the batch kernel variant (occupancy).
