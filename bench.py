@@ -63,7 +63,7 @@ def parse():
                          "time; serve: Poisson arrivals into the batched loop; c3: the 8192^2 "
                          "four-quadrant problem to t = 0.3 in FP32C, in FP64 and in FP64 from a perturbed "
                          "initial state (about 40 min at 8192^2, 5 min at 4096^2); f64tiles: the FP64 "
-                         "step at every tile shape, fused and as two launches; fp64peak: the FP64 "
+                         "step as a march, at every tile shape and as two launches; fp64peak: the FP64 "
                          "operation rates of this GPU")
     ap.add_argument("--instances", type=int, default=512)
     ap.add_argument("--sample", type=int, default=0,
@@ -370,70 +370,6 @@ def roofline(kt, precision, cells, prefix):
     return r
 
 
-# FP64 operations of the fused FP64 step (k_step_f64 in
-# euler2d_kokkos_gb300/csrc/e2d_fp64.cu), counted from its source, by kind:
-# "addmul" (adds, subtracts, multiplies), "fma", "div", "sqrt" and "max"
-# (fmax and FP64 comparisons).  Each kind is weighted by its measured cost
-# in FMA-rate cycles (FMA rate / its rate: on GB300 adds and multiplies run
-# at ~0.84 of the FMA rate, a division or a square root costs ~9 FMAs).
-# Limiter min/max, sign tests, cut-offs against positive constants and the
-# exact scalings by 0.5 and 2 run on the integer pipe and are not counted.
-F64_OPS = {
-    # stage 2, per cell of the tile and of its 1-cell ring: 8 limited slopes
-    # (3 subtractions each, f64x::slope_limited) and the trace sources
-    # (trace_sources: 10 products and 10 sums; dpx / r and dpy / r)
-    "slopes_trace": {"addmul": 24 + 20, "div": 2},
-    # face_pair for the 4 variables of one direction: s0 * dtd, then
-    # q - h + sx and q + h + sx
-    "faces_dir": {"addmul": 4 * 5},
-    # stage 3, one solve plus the 4 products by dt/dx
-    "hllc": {"addmul": 51 + 4, "div": 6, "sqrt": 2},
-    "hll": {"addmul": 64 + 4, "div": 3, "sqrt": 2},
-    # epilogue per cell: the update (4 x 4 sums), primitives (7 + 3
-    # divisions), the CFL term (6 + a division and a square root), and
-    # fmax / comparisons (the running maximum, the dx / dy power-of-two
-    # tests, the density test, the block fold's shuffles, ~6)
-    "epilogue": {"addmul": 16 + 7 + 6, "div": 3 + 1, "sqrt": 1, "max": 6},
-}
-# The opt-in fast forms (precision fp64_fast, *_fast in e2d_fp64_blocks.cuh):
-# FMAs, and one reciprocal per denominator (rcp_nr: a hardware estimate on
-# the MUFU unit and two Newton steps, 4 FMAs) in place of the divisions.
-F64_OPS_FAST = {
-    "slopes_trace": {"addmul": 24 + 6, "fma": 12},
-    "faces_dir": {"fma": 4 * 3},
-    "hllc": {"addmul": 39, "fma": 27, "sqrt": 2},
-    "hll": {"addmul": 42, "fma": 26, "sqrt": 2},
-    "epilogue": {"addmul": 28, "fma": 7, "sqrt": 1, "max": 4},
-}
-F64_TILES = {-1: (32, 32), 0: (32, 32), 1: (32, 16), 2: (32, 31), 3: (32, 15)}  # E2D_F64_TILE -> shape
-
-
-def tile_shape(tile, fast=False):
-    """(TX, TY) of the fused FP64 step for an E2D_F64_TILE value (the fast
-    forms exist for 32 x 16 and 32 x 32)."""
-    if fast:
-        return (32, 16) if tile == 1 else (32, 32)
-    return F64_TILES.get(tile, (32, 32))
-
-
-def fp64_ops_per_cell(riemann, tile=-1, fast=False):
-    """FP64 operations per cell-update of the fused step by kind, for a tile
-    shape: per tile, (TX+2)(TY+2)-4 slope/trace evaluations, 2 TX TY + 2 TX
-    + 2 TY face-pair directions, (TX+1) TY + TX (TY+1) solves and TX TY
-    epilogues.  None for the iterative approx solver."""
-    ops = F64_OPS_FAST if fast else F64_OPS
-    if riemann not in ops:
-        return None
-    tx, ty = tile_shape(tile, fast)
-    n = {"slopes_trace": (tx + 2) * (ty + 2) - 4, "faces_dir": 2 * tx * ty + 2 * tx + 2 * ty,
-         riemann: (tx + 1) * ty + tx * (ty + 1), "epilogue": tx * ty}
-    tot = {"addmul": 0.0, "fma": 0.0, "div": 0.0, "sqrt": 0.0, "max": 0.0}
-    for part, cnt in n.items():
-        for kind, v in ops[part].items():
-            tot[kind] += cnt * v / (tx * ty)
-    return tot
-
-
 _FP64_RATES = None
 
 
@@ -446,34 +382,27 @@ def fp64_pipe_counts(kernel):
     return json.load(open(path)).get(kernel)
 
 
-def fp64_pipe_info(e2d, riemann, kernel_ms, cells, tile=-1, fast=False):
+def fp64_form(nx):
+    """The form of the fused FP64 step that a square nx^2 grid runs by default
+    and whose instructions are counted: "march" (large grids), else None."""
+    forced = os.environ.get("E2D_F64_TILE") or os.environ.get("E2D_F64_MARCH")
+    return "march" if not forced and nx >= 2048 else None
+
+
+def fp64_pipe_info(e2d, riemann, kernel_ms, cells, form, fast=False):
     """FP64-pipe roofline of the fused step, live: the probe's measured rates
-    (e2d_fp64_rates, this run), the source-counted operations per cell in FMA
-    equivalents, and the fraction of the FMA peak the kernel sustained."""
+    (e2d_fp64_rates, this run) and the share of the FMA rate at which the
+    kernel ran its FP64-pipe instructions.  Those are counted per cell by ncu
+    (one capture of the same kernel): adds, subtracts and products run as
+    three-register FMAs, divisions, square roots, comparisons and a part of
+    the products on the integer pipes, which overlap the FP64 pipe."""
     global _FP64_RATES
     if _FP64_RATES is None:
         _FP64_RATES = e2d.fp64_rates()
     r = _FP64_RATES
-    ops = fp64_ops_per_cell(riemann, tile, fast)
-    out = {"rates_gops": r, "peak_gops": r["fma"], "unit": "G FP64 FMA-equivalent ops/s",
+    out = {"rates_gops": r, "peak_gops": r["fma"], "unit": "G FP64-pipe instructions/s",
            "peak_source": "e2d_fp64_rates probe in this run (8 chains/thread, 8x256 threads/SM, CUDA events)"}
-    if not ops:
-        return out
-    cost = {"fma": 1.0, "addmul": r["fma"] / min(r["add"], r["mul"]), "div": r["fma"] / r["div"],
-            "sqrt": r["fma"] / r["sqrt"], "max": r["fma"] / r["max"]}
-    per_cell = sum(ops[k] * cost[k] for k in ops)
-    achieved = per_cell * cells / (kernel_ms * 1e-3) / 1e9
-    out.update({"ops_per_cell": ops, "fma_equivalent_per_cell": per_cell,
-                "cost_in_fma": {k: cost[k] for k in ("addmul", "div", "sqrt", "max")},
-                "achieved_gops": achieved, "frac_algorithmic": achieved / r["fma"],
-                "ops_source": "counted from k_step_f64's source (bench.py F64_OPS), divisions and square "
-                              "roots weighted by their measured cost"})
-    # the instructions the FP64 pipe actually executes per cell (one ncu
-    # capture of this kernel; the division and square-root sequences and the
-    # compiler add to the source count) at the live cell rate: the pipe's
-    # busy fraction, as ncu's sm__pipe_fp64_cycles_active measures it
-    tx, ty = tile_shape(tile, fast)
-    ic = fp64_pipe_counts(f"k_step_f64<{riemann}>" + (" fast" if fast else "") + f" {tx}x{ty}")
+    ic = fp64_pipe_counts(f"k_step_f64<{riemann}>" + (" fast" if fast else "") + f" {form}") if form else None
     if ic:
         inst = ic["fp64_pipe_inst_per_cell"] * cells / (kernel_ms * 1e-3) / 1e9
         out.update({"fp64_pipe_inst_per_cell": ic["fp64_pipe_inst_per_cell"], "achieved_inst_gops": inst,
@@ -706,8 +635,20 @@ def c3_mode(args):
     print(json.dumps(line), flush=True)
 
 
+# The forms of the FP64 step: a march of 32-column segments (the default of large
+# grids; here 208 rows each), tiles of every shape (E2D_F64_TILE = 100 * rows +
+# shape) and two launches per step.
+F64_FORMS = [("march", "fp64", {"E2D_F64_MARCH": "208"}),
+             ("tiles 32x13", "fp64", {"E2D_F64_TILE": "1300"}),
+             ("tiles 16x16", "fp64", {"E2D_F64_TILE": "1601"}),
+             ("tiles 8x8", "fp64", {"E2D_F64_TILE": "802"}),
+             ("two launches", "fp64", {"E2D_F64_SPLIT": "1"}),
+             ("fast, march", "fp64_fast", {"E2D_F64_MARCH": "208"}),
+             ("fast, tiles 32x16", "fp64_fast", {"E2D_F64_TILE": "1600"})]
+
+
 def f64tiles_mode(args):
-    """The FP64 blast (--nx, HLLC and HLL) at every fused-step tile shape and
+    """The FP64 blast (--nx, HLLC and HLL) in every form of the fused step and
     as two launches per step, CUDA events on the library's stream.  With
     --repeat R the HLLC forms are measured R times in turn instead and the
     line gives each form's median (timings of the forms interleave, so that
@@ -721,8 +662,7 @@ def f64tiles_mode(args):
     bar = torch.cuda.synchronize
     rows = []
     if args.repeat > 0:
-        forms = [("fused 32x16", {"E2D_F64_TILE": "1"}), ("fused 32x32", {"E2D_F64_TILE": "0"}),
-                 ("two launches 32x32", {"E2D_F64_SPLIT": "1", "E2D_F64_TILE": "0"})]
+        forms = [(f, env) for f, prec, env in F64_FORMS if prec == "fp64"]
         got = {f: [] for f, _ in forms}
         with ClockSampler(0) as clocks:
             for _ in range(args.repeat):
@@ -738,22 +678,15 @@ def f64tiles_mode(args):
         return
     with ClockSampler(0) as clocks:
         for rs in ("hllc", "hll"):
-            for label, prec, env in [
-                    ("fused 32x32 (default)", "fp64", {"E2D_F64_TILE": "0"}),
-                    ("fused 32x16", "fp64", {"E2D_F64_TILE": "1"}),
-                    ("fused 32x31", "fp64", {"E2D_F64_TILE": "2"}), ("fused 32x15", "fp64", {"E2D_F64_TILE": "3"}),
-                    ("two launches 32x32", "fp64", {"E2D_F64_SPLIT": "1", "E2D_F64_TILE": "0"}),
-                    ("fast, fused 32x32 (default)", "fp64_fast", {"E2D_F64_TILE": "0"}),
-                    ("fast, fused 32x16", "fp64_fast", {"E2D_F64_TILE": "1"})]:
+            for label, prec, env in F64_FORMS:
                 m = measure(e2d, torch, args, prec, "blast", nx, args.steps, args.warmup, 0, bar, None,
                             with_e2e=False, with_clocks=False, riemann=rs, env=env)
                 kt = {k: round(v[0] / v[1], 4) for k, v in m["kernels"].items()}
                 row = {"riemann": rs, "form": label, "ms_per_step": m["ms"] / args.steps,
                        "gcell_per_s": cells * args.steps / (m["ms"] / 1e3) / 1e9, "kernel_ms_avg": kt}
-                if "fused" in label:
+                if label.endswith("march"):
                     k = next(k for k in kt if k.startswith("k_step_f64"))
-                    row["fp64_pipe"] = fp64_pipe_info(e2d, rs, kt[k], cells, int(env["E2D_F64_TILE"]),
-                                                      fast=prec == "fp64_fast")
+                    row["fp64_pipe"] = fp64_pipe_info(e2d, rs, kt[k], cells, "march", fast=prec == "fp64_fast")
                 rows.append(row)
     line = {"metric": METRIC, "mode": "f64tiles", "config": config("blast", nx, "hllc/hll", "fp64"),
             "steps": args.steps, "rows": rows, "clocks": clocks.summary()}
@@ -821,8 +754,7 @@ def main():
     roof = roofline(kt, args.precision, cells, prefix)
     if roof and f64:
         roof["note"] = "the FP64 step is bound by GB300's FP64 pipe, not HBM: see fp64_pipe"
-        roof["fp64_pipe"] = fp64_pipe_info(e2d, args.riemann, roof["kernel_ms_avg"], cells,
-                                           int(os.environ.get("E2D_F64_TILE", "-1")),
+        roof["fp64_pipe"] = fp64_pipe_info(e2d, args.riemann, roof["kernel_ms_avg"], cells, fp64_form(nx),
                                            fast=args.precision == "fp64_fast")
     line = {"metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": m["ms"] / args.steps,
@@ -863,7 +795,7 @@ def main():
                      barrier, None, with_e2e=False, with_clocks=False, riemann="hll")
         rh = roofline(hl["kernels"], "fp64", cells, "k_step_f64")
         if rh:
-            rh["fp64_pipe"] = fp64_pipe_info(e2d, "hll", rh["kernel_ms_avg"], cells)
+            rh["fp64_pipe"] = fp64_pipe_info(e2d, "hll", rh["kernel_ms_avg"], cells, fp64_form(nx))
         line["hll"] = {"config": config(args.problem, nx, "hll", "fp64"),
                        "value": cells * args.steps / (hl["ms"] / 1e3) / 1e9, "unit": METRIC,
                        "ms_per_step": hl["ms"] / args.steps, "roofline": rh}
@@ -884,7 +816,7 @@ def main():
                      barrier, None, with_e2e=False, with_clocks=False)
         rf = roofline(fa["kernels"], "fp64_fast", cells, "k_step_f64")
         if rf:
-            rf["fp64_pipe"] = fp64_pipe_info(e2d, args.riemann, rf["kernel_ms_avg"], cells, fast=True)
+            rf["fp64_pipe"] = fp64_pipe_info(e2d, args.riemann, rf["kernel_ms_avg"], cells, fp64_form(nx), fast=True)
         line["fp64_fast"] = {
             "config": config(args.problem, nx, args.riemann, "fp64_fast"),
             "value": cells * args.steps / (fa["ms"] / 1e3) / 1e9, "unit": METRIC,

@@ -175,7 +175,7 @@ def _solve_alone(params, s, chunk):
 
 def run_one_at_a_time(solves, chunk=256, on_nonfinite="fp64"):
     """Each solve alone: its own simulation handle, the device time loop in
-    graph-replayed chunks until t_end, its result read back.  A FP32C solve
+    chunks of steps until t_end, its result read back.  A FP32C solve
     that stops (E2D_ENUMERIC / E2D_ETIMEOUT) is handled as run_batched
     handles it: re-run in FP64 ("fp64") or recorded as failed ("drop")."""
     stats = RunStats()

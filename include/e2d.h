@@ -231,24 +231,27 @@ int e2d_godunov_unsplit_noalloc(const e2d_params *p, double *u_in, double *u_out
  * t_end - t, runs godunov_unsplit and advances (t, nStep); steps with
  * t >= t_end do nothing.  *t and *nStep are read and updated.  dt_trace
  * (optional, n entries) receives the dt of each step taken.  FP64: one
- * prologue kernel (primitives and CFL maximum of the input state), then one
- * fused kernel per step whose epilogue folds the next step's CFL maximum;
- * launches are replayed from cached CUDA graphs.  Blocks until done.
+ * prologue kernel (primitives and CFL maximum of the input state), then the
+ * fused step, whose epilogue folds the next step's CFL maximum.  Grids whose
+ * tiles or strips are all resident at once run up to 1024 steps per
+ * cooperative launch, with a bounded grid barrier between steps; larger grids
+ * run one launch per step, replayed from cached CUDA graphs.  Blocks until
+ * done.
  * E2D_ENUMERIC: a step saw a non-finite state or dt; E2D_ETIMEOUT: a bounded
- * wait for a TMA copy (FP64 tile staging, FP32C row staging of the TMA
- * variant) gave up (the state of this call is incomplete; the handle stays
- * usable). */
+ * wait gave up: for a TMA copy (FP64 staging, FP32C row staging of the TMA
+ * variants) or at the grid barrier (the state of this call is incomplete; the
+ * handle stays usable). */
 int e2d_step_n(e2d_sim *sim, int n, double t_end, double *t, int *nStep, double *dt_trace);
 
 /* ---------------------------------------------------------------------------
  * Batched solves.  No counterpart in the reference, which runs one grid per
  * process: the serving mode here keeps many independent simulations of
  * uneven size resident in one device memory pool and advances all active
- * ones together, one persistent kernel launch per iteration for the FP32C
- * instances and one for the FP64 ones (the fused step over a tile
- * work-list; each instance with its own dt and t_end), replayed from CUDA
- * graphs.  Arithmetic: each instance's
- * params.precision (FP64 instances end bit for bit where the single FP64
+ * ones together, each instance with its own dt and t_end: one cooperative
+ * launch per run call for the FP64 ones (the fused step over a tile
+ * work-list) and for short lists of FP32C ones, one persistent launch per
+ * iteration (replayed from CUDA graphs) for long lists of FP32C ones.
+ * Arithmetic: each instance's params.precision (FP64 instances end bit for bit where the single FP64
  * path ends).  One Riemann solver per batch.  A handle is used from one host
  * thread.
  * ------------------------------------------------------------------------- */
@@ -270,7 +273,7 @@ int e2d_batch_run(e2d_batch *b, int iterations, int *n_active);
 /* Loop state of an instance as of the last run (t, steps, still active).
  * The outputs are filled in every case; the status is E2D_ENUMERIC or
  * E2D_ETIMEOUT for an instance the batch stopped (a non-finite state or dt;
- * a row-staging wait that gave up), which stays inactive. */
+ * a row-staging wait or a grid barrier that gave up), which stays inactive. */
 int e2d_batch_query(e2d_batch *b, int id, double *t, int *nstep, int *active);
 /* Current state of an instance (hi + lo in FP64, ghosts filled), host copy. */
 int e2d_batch_get_state(e2d_batch *b, int id, double *host, int layout);
@@ -285,9 +288,11 @@ int e2d_batch_stream(e2d_batch *b, void **stream);
  * blocks with rows staged through shared memory by cp.async; 6: 4 blocks,
  * rows staged by TMA copies waited on with mbarriers) and rows per strip (16..512,
  * rounded up to a multiple of 16) for the size classes max(nx, ny) <= 192,
- * <= 512, > 512.  Results do not depend on them.  e2d_batch_autotune times the staged variants (4, 5,
- * 6) and then 16, 32 and 64 rows per size class on the live batch (its iterations advance the
- * instances) and keeps the fastest. */
+ * <= 512, > 512.  Results do not depend on them.  Until a caller sets a
+ * tuning, a short list of FP32C instances runs in strips of 2 to 8 rows
+ * instead.  e2d_batch_autotune times the staged variants (4, 5, 6) and then
+ * 16, 32 and 64 rows per size class on the live batch (its iterations advance
+ * the instances) and keeps the fastest; on a short list it times nothing. */
 int e2d_batch_set_tuning(e2d_batch *b, int variant, const int strip_h[3]);
 int e2d_batch_get_tuning(const e2d_batch *b, int *variant, int strip_h[3]);
 int e2d_batch_autotune(e2d_batch *b, int iters_per_trial);
