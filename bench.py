@@ -635,15 +635,15 @@ def c3_mode(args):
     print(json.dumps(line), flush=True)
 
 
-# The forms of the FP64 step: a march of 32-column segments (the default of large
-# grids; here 208 rows each), tiles of every shape (E2D_F64_TILE = 100 * rows +
+# The forms of the FP64 step: the default (a march of 32-column segments where the
+# grid is large, from 2048^2 on), tiles of every shape (E2D_F64_TILE = 100 * rows +
 # shape) and two launches per step.
-F64_FORMS = [("march", "fp64", {"E2D_F64_MARCH": "208"}),
+F64_FORMS = [("default", "fp64", {}),
              ("tiles 32x13", "fp64", {"E2D_F64_TILE": "1300"}),
              ("tiles 16x16", "fp64", {"E2D_F64_TILE": "1601"}),
              ("tiles 8x8", "fp64", {"E2D_F64_TILE": "802"}),
              ("two launches", "fp64", {"E2D_F64_SPLIT": "1"}),
-             ("fast, march", "fp64_fast", {"E2D_F64_MARCH": "208"}),
+             ("fast, default", "fp64_fast", {}),
              ("fast, tiles 32x16", "fp64_fast", {"E2D_F64_TILE": "1600"})]
 
 
@@ -684,9 +684,9 @@ def f64tiles_mode(args):
                 kt = {k: round(v[0] / v[1], 4) for k, v in m["kernels"].items()}
                 row = {"riemann": rs, "form": label, "ms_per_step": m["ms"] / args.steps,
                        "gcell_per_s": cells * args.steps / (m["ms"] / 1e3) / 1e9, "kernel_ms_avg": kt}
-                if label.endswith("march"):
+                if label.endswith("default"):
                     k = next(k for k in kt if k.startswith("k_step_f64"))
-                    row["fp64_pipe"] = fp64_pipe_info(e2d, rs, kt[k], cells, "march", fast=prec == "fp64_fast")
+                    row["fp64_pipe"] = fp64_pipe_info(e2d, rs, kt[k], cells, fp64_form(nx), fast=prec == "fp64_fast")
                 rows.append(row)
     line = {"metric": METRIC, "mode": "f64tiles", "config": config("blast", nx, "hllc/hll", "fp64"),
             "steps": args.steps, "rows": rows, "clocks": clocks.summary()}
