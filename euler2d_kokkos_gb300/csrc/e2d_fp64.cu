@@ -1536,7 +1536,7 @@ cudaError_t launch_flux_update_f64(const KParams64 &kp, int riemann, const doubl
 
 // Rows of a march's segments (0: tiles).  Grids march from 100 rows a
 // resident block on (two blocks an SM): 1024^2, 108 rows, takes 399 us a step
-// against 408 with tiles, 1531x797 HLL 526 against 547, 2048^2 1445 against
+// against 408 with tiles, 1531x797 HLL 526 against 547 (both before HLL shared its products; now 488), 2048^2 1445 against
 // 1561, 4096^2 5535 against 6143 -- but 700^2, 51 rows, 205 against 197.  The
 // segment is the number of chunks whose waves of blocks take the fewest
 // chunks, a last wave with at most one block an SM counting 0.62 of a full
