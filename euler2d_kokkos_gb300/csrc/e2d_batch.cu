@@ -83,8 +83,9 @@ struct HostInst {
   BatchInst64 mirror64{};  // (FP64)
   double t() const { return fp64 ? mirror64.t : mirror.t; }
   int nstep() const { return fp64 ? mirror64.nstep : mirror.nstep; }
-  int active() const { return fp64 ? mirror64.active : mirror.active; }
   unsigned int status() const { return fp64 ? mirror64.status : mirror.status; }
+  // a wait that gave up sets its bit of the status only
+  int active() const { return (fp64 ? mirror64.active : mirror.active) && !(status() & E2D_FLAG_TIMEOUT); }
 };
 
 // A table entry from a kernel argument: the record is taken at the launch,
@@ -194,7 +195,7 @@ int rebuild_list64(e2d_batch *b) {
   std::vector<int> list, tb, dims;
   for (int k = 0; k < b->max_inst; ++k) {
     HostInst &h = b->slots[k];
-    if (!h.used || !h.fp64 || !h.mirror64.active) continue;
+    if (!h.used || !h.fp64 || !h.active()) continue;
     list.push_back(k);
     dims.push_back(h.p.nx);
     dims.push_back(h.p.ny);
@@ -228,7 +229,7 @@ int rebuild_list(e2d_batch *b) {
   std::vector<int> list, begin;
   long long units = 0;
   for (HostInst &h : b->slots)
-    if (h.used && !h.fp64 && h.mirror.active) units += units_of(h.mirror.kp);
+    if (h.used && !h.fp64 && h.active()) units += units_of(h.mirror.kp);
   b->short_rows = b->tuned_by_caller ? 0 : short_rows_for(units, b->riemann);
   const int per_sm = b->short_rows > 0 ? 1 : batch_blocks_per_sm(b->riemann, b->variant);
   const long long warps = 152LL * per_sm * 4;
@@ -238,7 +239,7 @@ int rebuild_list(e2d_batch *b) {
     bool all_min = true;
     for (int k = 0; k < b->max_inst; ++k) {
       HostInst &h = b->slots[k];
-      if (!h.used || h.fp64 || !h.mirror.active) continue;
+      if (!h.used || h.fp64 || !h.active()) continue;
       KParams32 kp = h.mirror.kp;
       kp.strip_h = std::max(16, ((b->strip_h[h.size_class] >> shift) / 16) * 16);
       all_min &= kp.strip_h == 16;
@@ -249,7 +250,7 @@ int rebuild_list(e2d_batch *b) {
   int total = 0;
   for (int k = 0; k < b->max_inst; ++k) {
     HostInst &h = b->slots[k];
-    if (!h.used || h.fp64 || !h.mirror.active) continue;
+    if (!h.used || h.fp64 || !h.active()) continue;
     list.push_back(k);
     begin.push_back(total);
     if (b->short_rows > 0) {
@@ -287,16 +288,24 @@ int rebuild_list(e2d_batch *b) {
   return E2D_OK;
 }
 
+// Blocks more than there are that the loops' barriers wait for (the test of
+// their bounded wait).
+unsigned int late(const e2d_batch *b) {
+  for (const HostInst &h : b->slots)
+    if (h.used && (h.fp64 ? h.mirror64.kp.wait_test : h.mirror.kp.wait_test) == 2) return 1u;
+  return 0u;
+}
+
 int launch_iterations(e2d_batch *b, int iterations) {
   const int m = b->max_inst;
   if (!b->list64.empty())
     B_CK(b, launch_batch_f64(b->riemann, b->d_insts64, b->d_list64, b->d_list64 + m, (int)b->list64.size(),
-                             b->total_tiles, b->shape64, b->ty64, iterations, b->d_arrived + 1, b->stream),
+                             b->total_tiles, b->shape64, b->ty64, iterations, b->d_arrived + 1, late(b), b->stream),
          "batch launch");
   if (b->list.empty()) return E2D_OK;
   if (b->short_rows > 0) {
     B_CK(b, launch_batch_loop_f32c(b->riemann, b->short_rows, b->d_insts, b->d_list, b->d_list + m,
-                                   (int)b->list.size(), b->total_strips, iterations, b->d_arrived, b->stream),
+                                   (int)b->list.size(), b->total_strips, iterations, b->d_arrived, late(b), b->stream),
          "batch launch");
     return E2D_OK;
   }
@@ -722,7 +731,7 @@ int e2d_batch_autotune(e2d_batch *b, int iters_per_trial) {
   static const int cand[3] = {16, 32, 64};
   for (int c = 0; c < 3 && rc == E2D_OK; ++c) {
     bool present = false;
-    for (auto &h : b->slots) present |= h.used && !h.fp64 && h.mirror.active && h.size_class == c;
+    for (auto &h : b->slots) present |= h.used && !h.fp64 && h.active() && h.size_class == c;
     if (!present) continue;
     int best_h = b->strip_h[c];
     double bm = 1e30;

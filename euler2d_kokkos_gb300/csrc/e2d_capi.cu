@@ -127,7 +127,7 @@ void e2d::make_kparams(const e2d_params &p, KParams64 *kp) {
   const char *mr = std::getenv("E2D_F64_MARCH");  // segment rows; 0: tiles, as with a forced tile
   kp->march_rows = mr ? std::atoi(mr) : tile ? 0 : choose_f64_march(p.nx, p.ny, 0);
   const char *wt = std::getenv("E2D_TEST_WAIT_TIMEOUT");
-  kp->wait_test = (wt && std::atoi(wt) != 0) ? 1 : 0;
+  kp->wait_test = wt ? std::atoi(wt) : 0;
 }
 
 namespace {
@@ -370,7 +370,7 @@ int e2d_create(const e2d_params *pin, e2d_sim **out) {
   if (!(lp && std::atoi(lp) == 0)) {
     if (s->fp32)
       s->loop_blocks = f32c_loop_blocks(s->kp32, p.riemannSolverType);
-    else if (!s->f64_split && s->impl == 0 && !s->kp.wait_test)
+    else if (!s->f64_split && s->impl == 0 && s->kp.wait_test != 1)
       s->loop_blocks = f64_loop_blocks(s->kp, p.riemannSolverType);
   }
   if (cudaMalloc(&s->partial, sizeof(double) * reduce_partial_count(s->kp.g)) != cudaSuccess) return fail(E2D_ENOMEM);

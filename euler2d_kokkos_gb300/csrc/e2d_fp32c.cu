@@ -700,7 +700,7 @@ __device__ __forceinline__ bool march_strip_t(const KParams32 &kp, const float *
   auto stage = [&](int r, int sl) {
     if (bulk && TMA == 1) {
       // wait_test: the first row of strip (1, 0) is never copied
-      if (kp.wait_test && sx == 1 && rb == 2 && r == rb - 2) return;
+      if (kp.wait_test == 1 && sx == 1 && rb == 2 && r == rb - 2) return;
       stage_row_tma(g, map, r, cb - 2, lane, yghost, slot_of(sl), bars + sl);
       pending |= 1u << sl;
     } else {
@@ -1260,7 +1260,7 @@ __device__ __forceinline__ void batch_finalize(BatchInst &I) {
   unsigned int status = __ldcg(&I.status);
   if (!(dt > 0.0) || nonfinite64(dt)) {
     status |= E2D_FLAG_BAD_DT;
-    I.status = status;
+    atomicOr(&I.status, (unsigned)E2D_FLAG_BAD_DT);  // a block whose wait ran out may set its bit meanwhile
   }
   const double t = __ldcg(&I.t) + dt;
   I.t = t;
@@ -1338,13 +1338,20 @@ __global__ void __launch_bounds__(NT, MINB)
 // units, in one cooperative launch: each block takes the same units of the
 // list in every iteration, marches them in short strips (short_unit) with the
 // instance's own dt, and the last unit of an instance advances its loop
-// state; a grid barrier separates iterations.
+// state; a grid barrier separates iterations.  One thread reads what steers a
+// block, and a block whose wait runs out sets a bit of the status only, as in
+// k_batch_loop_f64.
 template <int RS, int SUB, int MINB>
 __global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
     k_batch_loop_f32c(BatchInst *insts, const int *__restrict__ list_slots, const int *__restrict__ unit_begin,
-                      const int n_inst, const int units, const int iterations, unsigned int *arrived) {
+                      const int n_inst, const int units, const int iterations, unsigned int *arrived,
+                      const unsigned int late) {
   constexpr int NTS = 32 * (CFL_UNIT_ROWS / SUB);
   __shared__ KParams32 s_kp;  // of the instance at hand
+  __shared__ struct {
+    int run, par, ns;
+    float dtdx, dtdy;
+  } s_at;  // where it stands
   int held = -1;
   for (int it = 0; it < iterations; ++it) {
     for (int u = blockIdx.x; u < units; u += gridDim.x) {
@@ -1357,19 +1364,24 @@ __global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
           hi = mid;
       }
       BatchInst &I = insts[list_slots[lo]];
-      const int active = __ldcg(&I.active), par = __ldcg(&I.par), ns = __ldcg(&I.nstep);
-      const float dtdx = __ldcg(&I.dtdx), dtdy = __ldcg(&I.dtdy);
-      __syncthreads();  // the previous unit is done with s_kp and the winners' table
+      auto at = decltype(s_at){};
+      if (threadIdx.x == 0) {
+        at = {__ldcg(&I.active), __ldcg(&I.par), __ldcg(&I.nstep), __ldcg(&I.dtdx), __ldcg(&I.dtdy)};
+        if (__ldcg(&I.status) & E2D_FLAG_TIMEOUT) at.run = 0;
+      }
+      __syncthreads();  // the previous unit is done with s_kp, s_at and the winners' table
+      if (threadIdx.x == 0) s_at = at;
       if (lo != held) {
         static_assert(sizeof(KParams32) % 4 == 0, "copied by words");
         for (int j = threadIdx.x; j < (int)(sizeof(KParams32) / 4); j += NTS)
           reinterpret_cast<int *>(&s_kp)[j] = reinterpret_cast<const int *>(&I.kp)[j];
         held = lo;
-        __syncthreads();
       }
-      if (!active) continue;  // block-uniform
-      short_unit<RS, SUB>(s_kp, I.w[par], I.w[par ^ 1], u - unit_begin[lo], &I.acc[(ns + 1) & 1], &I.status,
-                          [&]() { return make_float2(dtdx, dtdy); });
+      __syncthreads();
+      at = s_at;
+      if (!at.run) continue;
+      short_unit<RS, SUB>(s_kp, I.w[at.par], I.w[at.par ^ 1], u - unit_begin[lo], &I.acc[(at.ns + 1) & 1], &I.status,
+                          [&]() { return make_float2(at.dtdx, at.dtdy); });
       if (threadIdx.x == 0) {
         __threadfence();
         const unsigned int ticket = atomicAdd(&I.done, 1u);
@@ -1381,13 +1393,13 @@ __global__ void __launch_bounds__(32 * (CFL_UNIT_ROWS / SUB), MINB)
         }
       }
     }
-    if (!grid_barrier(arrived, (unsigned)(it + 1) * gridDim.x)) {
+    if (it + 1 == iterations) return;
+    if (!grid_barrier(arrived, (unsigned)(it + 1) * gridDim.x + late)) {
       // the states of this block's units are incomplete: their instances stop
       for (int u = blockIdx.x; threadIdx.x == 0 && u < units; u += gridDim.x) {
         int k = 0;
         while (k + 1 < n_inst && unit_begin[k + 1] <= u) ++k;
         atomicOr(&insts[list_slots[k]].status, (unsigned)E2D_FLAG_TIMEOUT);
-        insts[list_slots[k]].active = 0;
       }
       return;
     }
@@ -1583,7 +1595,7 @@ void make_kparams32(const e2d_params &p, KParams32 *kp) {
   choose_strips(p, kp);
   kp->short_rows = default_short_rows(p);
   const char *wt = std::getenv("E2D_TEST_WAIT_TIMEOUT");
-  kp->wait_test = (wt && std::atoi(wt) != 0) ? 1 : 0;
+  kp->wait_test = wt ? std::atoi(wt) : 0;
 }
 
 // Rows of a short strip (see k_step_f32c_short), as template arguments with
@@ -1737,7 +1749,8 @@ int f32c_loop_blocks(const KParams32 &kp, int riemann) {
 
 template <int RS>
 static cudaError_t launch_batch_loop_t(int rows, BatchInst *insts, const int *list_slots, const int *unit_begin,
-                                       int n_inst, int units, int iterations, unsigned int *arrived, cudaStream_t s) {
+                                       int n_inst, int units, int iterations, unsigned int *arrived,
+                                       unsigned int late, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
   with_short(rows, [&](auto sub, auto minb) {
     constexpr int S = decltype(sub)::value, M = decltype(minb)::value, threads = 32 * (CFL_UNIT_ROWS / S);
@@ -1745,7 +1758,7 @@ static cudaError_t launch_batch_loop_t(int rows, BatchInst *insts, const int *li
     const size_t sm = ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / S);
     const int resident = resident_blocks(kernel, threads, sm);
     const int grid = units < resident ? units : resident;
-    void *args[] = {&insts, &list_slots, &unit_begin, &n_inst, &units, &iterations, &arrived};
+    void *args[] = {&insts, &list_slots, &unit_begin, &n_inst, &units, &iterations, &arrived, &late};
     if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;
     if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, sm, s);
   });
@@ -1754,15 +1767,18 @@ static cudaError_t launch_batch_loop_t(int rows, BatchInst *insts, const int *li
 
 cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, const int *list_slots,
                                    const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
-                                   cudaStream_t s) {
+                                   unsigned int late, cudaStream_t s) {
   if (n_inst <= 0 || units <= 0 || iterations <= 0) return cudaSuccess;
   switch (riemann) {
     case E2D_RIEMANN_HLLC:
-      return launch_batch_loop_t<E2D_RIEMANN_HLLC>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived, s);
+      return launch_batch_loop_t<E2D_RIEMANN_HLLC>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived,
+                                                   late, s);
     case E2D_RIEMANN_HLL:
-      return launch_batch_loop_t<E2D_RIEMANN_HLL>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived, s);
+      return launch_batch_loop_t<E2D_RIEMANN_HLL>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived,
+                                                  late, s);
     default:
-      return launch_batch_loop_t<E2D_RIEMANN_APPROX>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived, s);
+      return launch_batch_loop_t<E2D_RIEMANN_APPROX>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived,
+                                                     late, s);
   }
 }
 

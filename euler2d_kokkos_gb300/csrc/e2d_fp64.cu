@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(NT, MINB)
       mbar_init(&s_bar, 1u);
       mbar_init_fence();
       // wait_test: tile (1, 1) never copies, so its bounded wait runs out
-      if (!(kp.wait_test && bx == 1 && by == 1)) {
+      if (!(kp.wait_test == 1 && bx == 1 && by == 1)) {
         mbar_arrive_expect(&s_bar, (unsigned int)(sizeof(double) * 4 * QW) * (unsigned int)(ty + 4));
         tma_load_3d(smem, &tm_q, i0, j0, 0, &s_bar);
       }
@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(MNT, 2)
   auto by_tma = [&](int r0) { return tma_x && r0 - 1 >= 2 && r0 + CHUNK <= g.ny + 1; };
   auto issue = [&](int r0, int b) {
     // wait_test: block (1, 0)'s second chunk is never copied, so its wait runs out
-    if (kp.wait_test && bx == 1 && blockIdx.y == 0 && b == 1) return;
+    if (kp.wait_test == 1 && bx == 1 && blockIdx.y == 0 && b == 1) return;
     fence_proxy_async_smem();
     mbar_arrive_expect(&s_bar[b], (unsigned int)kMarchQ);
     tma_load_3d(sQ[b], &tm_q, i0, r0 - 1, 0, &s_bar[b]);
@@ -1033,7 +1033,8 @@ __global__ void __launch_bounds__(NT, MINB)
     if (blockIdx.x == 0 && tid == 0) loop_record(clk, c, s, dt, dt_trace);
     c.t = c.t + dt;
     c.ns += 1;
-    if (!grid_barrier(&clk->arrived, (unsigned)(s + 1) * gridDim.x)) {
+    // wait_test: a block more than there are, so the bounded wait runs out
+    if (!grid_barrier(&clk->arrived, (unsigned)(s + 1) * gridDim.x + (kp.wait_test ? 1u : 0u))) {
       if (tid == 0) atomicOr(&clk->status, E2D_FLAG_TIMEOUT);
       return;
     }
@@ -1074,14 +1075,21 @@ __global__ void __launch_bounds__(FILL_BX *FILL_BY) k_batch_prime_f64(BatchInst6
 // iteration advances its loop state.  The tile is chosen for the whole list
 // (choose_f64_tile), so the last few solves of a batch still use every SM:
 // 32 x 32 tiles left a lone 256^2 solve on 64 of 152.
+// A block whose barrier wait runs out stops its instances by a bit of their
+// status and leaves; one that arrives after that may go on for a while, so
+// one thread reads what steers a block (another block may be setting the bit
+// meanwhile, and threads that disagree would part at the block's barriers),
+// and nothing but the last tile writes `active`.
+// late: blocks more than there are that the barriers wait for (tests).
 template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL>
 __global__ void __launch_bounds__(NT, MINB)
     k_batch_loop_f64(BatchInst64 *insts, const int *__restrict__ list_slots, const int *__restrict__ tile_begin,
                      const int n_inst, const int total_tiles, const int ty, const int iterations,
-                     unsigned int *arrived) {
+                     unsigned int *arrived, const unsigned int late) {
   extern __shared__ unsigned char smem_raw[];
   double *smem = reinterpret_cast<double *>(smem_raw);
   __shared__ double s_dt[3];
+  __shared__ int s_par;       // of the instance at hand, -1 if it is not to be stepped
   __shared__ KParams64 s_kp;  // of the instance at hand
   const int tid = threadIdx.x;
   const f64x::FpT<XMUL> f;
@@ -1091,16 +1099,22 @@ __global__ void __launch_bounds__(NT, MINB)
     for (int w = blockIdx.x; w < total_tiles; w += gridDim.x) {
       const int k = list_entry(tile_begin, n_inst, w);
       BatchInst64 &I = insts[list_slots[k]];
+      int steer = -1;
+      if (tid == 0) {
+        const int active = __ldcg(&I.active), p = __ldcg(&I.par);
+        if (active && !(__ldcg(&I.status) & E2D_FLAG_TIMEOUT)) steer = p;
+      }
+      __syncthreads();  // the previous tile is done with s_par, s_dt, s_kp and the shared tile
+      if (tid == 0) s_par = steer;
       if (k != held) {
-        __syncthreads();
         static_assert(sizeof(KParams64) % 4 == 0, "copied by words");
         for (int j = tid; j < (int)(sizeof(KParams64) / 4); j += NT)
           reinterpret_cast<int *>(&s_kp)[j] = reinterpret_cast<const int *>(&I.kp)[j];
         held = k;
       }
-      if (!__ldcg(&I.active)) continue;  // block-uniform
-      const int par = __ldcg(&I.par);
       __syncthreads();
+      const int par = s_par;
+      if (par < 0) continue;
       if (tid == 0) {
         const double dt = step_dt(kp.ph, __ldcg(&I.acc[par]), __ldcg(&I.t), __ldcg(&I.t_end));
         s_dt[0] = dt;
@@ -1146,15 +1160,12 @@ __global__ void __launch_bounds__(NT, MINB)
           __threadfence();
         }
       }
-      __syncthreads();  // s_dt and the shared tile are rewritten by the next tile
     }
-    if (!grid_barrier(arrived, (unsigned)(it + 1) * gridDim.x)) {
+    if (it + 1 == iterations) return;
+    if (!grid_barrier(arrived, (unsigned)(it + 1) * gridDim.x + late)) {
       // the states of this block's tiles are incomplete: their instances stop
-      for (int w = blockIdx.x; tid == 0 && w < total_tiles; w += gridDim.x) {
-        BatchInst64 &I = insts[list_slots[list_entry(tile_begin, n_inst, w)]];
-        atomicOr(&I.status, (unsigned)E2D_FLAG_TIMEOUT);
-        I.active = 0;
-      }
+      for (int w = blockIdx.x; tid == 0 && w < total_tiles; w += gridDim.x)
+        atomicOr(&insts[list_slots[list_entry(tile_begin, n_inst, w)]].status, (unsigned)E2D_FLAG_TIMEOUT);
       return;
     }
   }
@@ -1487,7 +1498,7 @@ cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s)
 template <int RS>
 static cudaError_t launch_batch_t(BatchInst64 *insts, const int *list_slots, const int *tile_begin, int n_inst,
                                   int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
-                                  cudaStream_t s) {
+                                  unsigned int late, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
   with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
@@ -1495,7 +1506,7 @@ static cudaError_t launch_batch_t(BatchInst64 *insts, const int *list_slots, con
     constexpr size_t sm = flux_smem_bytes<S::TX, S::TYM>();
     const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), S::NT, sm);
     const int grid = total_tiles < resident ? total_tiles : resident;
-    void *args[] = {&insts, &list_slots, &tile_begin, &n_inst, &total_tiles, &ty, &iterations, &arrived};
+    void *args[] = {&insts, &list_slots, &tile_begin, &n_inst, &total_tiles, &ty, &iterations, &arrived, &late};
     if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;
     if (e == cudaSuccess)
       e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(S::NT), args, sm, s);
@@ -1505,18 +1516,18 @@ static cudaError_t launch_batch_t(BatchInst64 *insts, const int *list_slots, con
 
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
                              int n_inst, int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
-                             cudaStream_t s) {
+                             unsigned int late, cudaStream_t s) {
   if (n_inst <= 0 || total_tiles <= 0 || iterations <= 0) return cudaSuccess;
   switch (riemann) {
     case E2D_RIEMANN_HLLC:
       return launch_batch_t<E2D_RIEMANN_HLLC>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty, iterations,
-                                              arrived, s);
+                                              arrived, late, s);
     case E2D_RIEMANN_HLL:
       return launch_batch_t<E2D_RIEMANN_HLL>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty, iterations,
-                                             arrived, s);
+                                             arrived, late, s);
     default:
       return launch_batch_t<E2D_RIEMANN_APPROX>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty,
-                                                iterations, arrived, s);
+                                                iterations, arrived, late, s);
   }
 }
 

@@ -61,8 +61,9 @@ struct KParams64 {
   int shape, ty;  // tile shape of the step and its rows (choose_f64_tile)
   int march_rows; // rows of the segments a large grid's step marches (choose_f64_march); 0: tiles
   int fast;       // E2D_PRECISION_FP64_FAST: the fused step's fast forms (not bit-identical)
-  int wait_test;  // nonzero: tile (1, 1) of the fused step never stages its primitives,
-                  // so its bounded wait runs out (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
+  int wait_test;  // 1: tile (1, 1) of the fused step never stages its primitives; 2: the barriers of
+                  // multi-step launches wait for a block too many, so that the bounded wait runs
+                  // out (E2D_TEST_WAIT_TIMEOUT; tests the timeout paths)
 };
 
 // FP32 step with FP64 copies of the constants the exact dt recompute uses.
@@ -78,9 +79,9 @@ struct KParams32 {
   int strip_h;       // rows per warp strip of the step kernel
   int tall, tail_h;  // single grids: so many rows of strips of strip_h rows, then strips of tail_h
   int short_rows;    // 2, 4 or 8: the single grid's step runs short strips of so many rows; 0: strip_h
-  int wait_test;     // nonzero: strip (1, 0) never stages its first row, or a multi-step launch's
-                     // barrier waits for a block too many, so that the bounded wait runs out
-                     // (E2D_TEST_WAIT_TIMEOUT=1; tests the timeout path)
+  int wait_test;     // 1: strip (1, 0) never stages its first row; nonzero (batches: 2): the barriers
+                     // of multi-step launches wait for a block too many, so that the bounded wait
+                     // runs out (E2D_TEST_WAIT_TIMEOUT; tests the timeout paths)
 };
 
 // Device-resident loop state of the time loop of src/main.cpp:100-145.
@@ -263,10 +264,10 @@ cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s)
 // `iterations` steps of every listed FP64 instance in one cooperative launch:
 // list entry k is table slot list_slots[k]; tile_begin[k] is its first global
 // tile of that shape (n_inst + 1 entries, the last = total_tiles); arrived: a
-// device word for the launch's barriers.
+// device word for the launch's barriers; late: see k_batch_loop_f64.
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
                              int n_inst, int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
-                             cudaStream_t s);
+                             unsigned int late, cudaStream_t s);
 // Prologue blocks of an FP64 instance.
 void batch_f64_shape(const KParams64 &kp, int *nbx, int *nfill);
 
@@ -280,7 +281,7 @@ cudaError_t launch_batch_f32c(int riemann, int variant, BatchInst *insts, const 
 // strips of `rows` rows, in one cooperative launch (unit_begin as strip_begin).
 cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, const int *list_slots,
                                    const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
-                                   cudaStream_t s);
+                                   unsigned int late, cudaStream_t s);
 int units_of(const KParams32 &kp);
 int short_rows_for(long long units, int riemann);
 // dt, dt/dx, dt/dy and `active` of an instance from acc[nstep & 1].

@@ -1,0 +1,53 @@
+"""The batches' multi-iteration launches (k_batch_loop_f64, k_batch_loop_f32c): a
+wait that runs out, and the same bits whatever the list and its launches are."""
+import numpy as np
+import pytest
+
+import euler2d_kokkos_gb300 as e2d
+
+pytestmark = pytest.mark.gpu
+
+POOL = 1 << 30
+
+
+def implosion(nx, ny, precision, riemann="hllc", **kw):
+    return e2d.make_params(nx, ny, problem="implode", riemann=riemann, gamma0=1.4, cfl=0.8, implode_shape=1,
+                           precision=precision, **kw)
+
+
+@pytest.mark.parametrize("precision", [e2d.PRECISION_FP64, e2d.PRECISION_FP32C])
+def test_batch_barrier_wait_runs_out_with_etimeout(gpu_lib, monkeypatch, precision):
+    """With E2D_TEST_WAIT_TIMEOUT=2 the barrier between two iterations waits for
+    one block more than there are: the wait gives up after its 1 s limit, every
+    instance whose units the blocks had reports E2D_ETIMEOUT, and none is
+    stepped again."""
+    p = [implosion(n, 96, precision) for n in (128, 70)]
+    monkeypatch.setenv("E2D_TEST_WAIT_TIMEOUT", "2")
+    with e2d.Batch(pool_bytes=POOL) as b:
+        ids = [b.admit(q, 10.0) for q in p]
+        assert b.run(3) == 0
+        before = [b.poll(i) for i in ids]
+        for i, (t, ns, active, ok) in zip(ids, before):
+            assert ns == 1 and not active and not ok
+            with pytest.raises(e2d.E2DError) as ei:
+                b.query(i)
+            assert ei.value.status == 4  # E2D_ETIMEOUT
+        assert b.run(3) == 0 and [b.poll(i) for i in ids] == before
+    monkeypatch.delenv("E2D_TEST_WAIT_TIMEOUT")
+    with e2d.Batch(pool_bytes=POOL) as b:
+        ids = [b.admit(q, 10.0) for q in p]
+        assert b.run(3) == 2
+        assert all(b.query(i)[1] == 3 and np.isfinite(b.get_state(i)).all() for i in ids)
+
+
+def test_fp64_loop_barrier_wait_runs_out_with_etimeout(gpu_lib, monkeypatch):
+    p = implosion(128, 96, e2d.PRECISION_FP64)
+    monkeypatch.setenv("E2D_TEST_WAIT_TIMEOUT", "2")
+    with e2d.HydroRun(p) as h:
+        with pytest.raises(e2d.E2DError) as ei:
+            h.step_n(3, 10.0, 0.0, 0)
+        assert ei.value.status == 4  # E2D_ETIMEOUT
+    monkeypatch.delenv("E2D_TEST_WAIT_TIMEOUT")
+    with e2d.HydroRun(p) as h:
+        t, ns, _ = h.step_n(3, 10.0, 0.0, 0)
+        assert ns == 3 and np.isfinite(h.current(ns)).all()
