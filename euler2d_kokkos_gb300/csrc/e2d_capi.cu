@@ -42,6 +42,9 @@ struct e2d_sim {
   // state, and always once its device address has been given out
   int h_ready = -1;
   bool address_out = false;
+  // a godunov_unsplit was captured: replays of its graph change the states
+  // without a call, so nothing is kept of them from one call to the next
+  bool replayed = false;
   DtAcc *dt_acc = nullptr;            // compute_dt: accumulators (zero between calls)
   DtResult *dt_result = nullptr;      // and result (pinned)
   double *impl_scratch = nullptr;     // FP64, implementation 1: stored slopes and fluxes
@@ -553,7 +556,7 @@ int e2d_compute_dt(e2d_sim *s, int useU, double *dt) {
     double *q = s->kp.fast ? nullptr : s->Q[which];
     E2D_CK(s, launch_dt_f64(s->kp, s->U[which], q, s->dt_acc, s->dt_result, s->stream), "compute_dt");
     E2D_CK(s, cudaStreamSynchronize(s->stream), "dt sync");
-    if (q && !s->address_out) s->h_ready = which;
+    if (q && !s->address_out && !s->replayed) s->h_ready = which;
   } else {
     E2D_CK(s, cudaMemsetAsync(s->dt_acc, 0, sizeof(DtAcc), s->stream), "dt reset");
     E2D_CK(s, launch_f32c_dt_to(s->kp32, s->W[which], &s->dt_acc->bits, &s->dt_acc->status, s->stream), "compute_dt");
@@ -574,7 +577,10 @@ int e2d_godunov_unsplit(e2d_sim *s, int nStep, double dt) {
   if (!s) return E2D_EINVAL;
   if (s->kp.fast) return set_err(s, E2D_EINVAL, "fp64_fast runs through the device time loop (e2d_step_n) only");
   const int par = (nStep % 2 == 0) ? 0 : 1;  // src/HydroRun.h:263-270
-  const bool have_q = s->h_ready == par;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  E2D_CK(s, cudaStreamIsCapturing(s->stream, &capture), "capture query");
+  if (capture != cudaStreamCaptureStatusNone) s->replayed = true;
+  const bool have_q = s->h_ready == par && !s->replayed;
   touch(s);
   if (s->fp32) {
     E2D_CK(s, launch_f32c_step(s->kp32, s->p.riemannSolverType, s->W[par], s->W[par ^ 1], s->TM[par], s->clk, 0, dt,
@@ -613,7 +619,7 @@ int e2d_step_n(e2d_sim *s, int n, double t_end, double *t, int *nStep, double *d
   // from the previous call when nothing has changed the state since, else
   // from a prologue fill
   const bool fused = !s->fp32 && !s->f64_split && s->impl == 0;
-  const bool prologue = fused && s->q_ready != par0;
+  const bool prologue = fused && (s->q_ready != par0 || s->replayed);
   if (fused && !prologue) c.acc[par0] = s->q_acc;
   touch(s);
   *s->clk_host = c;

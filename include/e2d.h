@@ -196,7 +196,10 @@ int e2d_make_boundaries(e2d_sim *sim, int which);
  * (useU == 0) or U2; blocks until the value is on the host. */
 int e2d_compute_dt(e2d_sim *sim, int useU, double *dt);
 /* HydroRun::godunov_unsplit (src/HydroRun.h:258-272): U -> U2 for even
- * nStep, U2 -> U for odd, with the caller's dt.  Asynchronous. */
+ * nStep, U2 -> U for odd, with the caller's dt.  Asynchronous, and may be
+ * captured into a graph on the handle's stream (e2d_get_stream); once it has
+ * been, other calls keep nothing of the states between them, since a replay
+ * may have changed them. */
 int e2d_godunov_unsplit(e2d_sim *sim, int nStep, double dt);
 
 /* One FP64 godunov_unsplit step (same kernels and bits as
