@@ -8,6 +8,7 @@
 #include "e2d_internal.h"
 
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <iterator>
 #include <map>
@@ -130,6 +131,7 @@ struct e2d_batch {
   int shape64 = 0, ty64 = 16;  // tile of the current FP64 work list
   int short_rows = 0;          // rows of the FP32C list's short strips (the list counts fold units); 0: strips
   bool tuned_by_caller = false;  // set_tuning named a kernel variant: lists keep to it
+  bool loops = true;  // several iterations per cooperative launch (E2D_LOOP=0: a launch each)
   unsigned int *d_arrived = nullptr;  // barrier words of the multi-iteration launches (FP32C, FP64)
   bool list_dirty = true;
   int grid = 0;
@@ -230,7 +232,8 @@ int rebuild_list(e2d_batch *b) {
   long long units = 0;
   for (HostInst &h : b->slots)
     if (h.used && !h.fp64 && h.active()) units += units_of(h.mirror.kp);
-  b->short_rows = b->tuned_by_caller ? 0 : short_rows_for(units, b->riemann);
+  b->short_rows = b->tuned_by_caller || !b->loops ? 0 : short_rows_for(units, b->riemann);
+  if (b->short_rows > 0 && !batch_loop_f32c_fits(b->riemann, b->short_rows)) b->short_rows = 0;
   const int per_sm = b->short_rows > 0 ? 1 : batch_blocks_per_sm(b->riemann, b->variant);
   const long long warps = 152LL * per_sm * 4;
   int shift = 0;
@@ -300,7 +303,8 @@ int launch_iterations(e2d_batch *b, int iterations) {
   const int m = b->max_inst;
   if (!b->list64.empty())
     B_CK(b, launch_batch_f64(b->riemann, b->d_insts64, b->d_list64, b->d_list64 + m, (int)b->list64.size(),
-                             b->total_tiles, b->shape64, b->ty64, iterations, b->d_arrived + 1, late(b), b->stream),
+                             b->total_tiles, b->shape64, b->ty64, iterations, b->d_arrived + 1, late(b), b->loops,
+                             b->stream),
          "batch launch");
   if (b->list.empty()) return E2D_OK;
   if (b->short_rows > 0) {
@@ -398,6 +402,8 @@ int e2d_batch_create(int riemann, size_t pool_bytes, int max_instances, e2d_batc
   if (!b) return E2D_ENOMEM;
   b->riemann = riemann;
   b->max_inst = max_instances;
+  const char *lp = std::getenv("E2D_LOOP");
+  b->loops = !(lp && std::atoi(lp) == 0);
   b->slots.resize(max_instances);
   auto fail = [&](int st) {
     e2d_batch_destroy(b);

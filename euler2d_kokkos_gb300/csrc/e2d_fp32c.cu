@@ -1747,39 +1747,43 @@ int f32c_loop_blocks(const KParams32 &kp, int riemann) {
   return blocks;
 }
 
-template <int RS>
-static cudaError_t launch_batch_loop_t(int rows, BatchInst *insts, const int *list_slots, const int *unit_begin,
-                                       int n_inst, int units, int iterations, unsigned int *arrived,
-                                       unsigned int late, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
+template <class F>
+static void with_batch_loop(int riemann, int rows, F &&f) {
   with_short(rows, [&](auto sub, auto minb) {
-    constexpr int S = decltype(sub)::value, M = decltype(minb)::value, threads = 32 * (CFL_UNIT_ROWS / S);
-    const void *kernel = reinterpret_cast<const void *>(k_batch_loop_f32c<RS, S, M>);
-    const size_t sm = ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / S);
-    const int resident = resident_blocks(kernel, threads, sm);
-    const int grid = units < resident ? units : resident;
-    void *args[] = {&insts, &list_slots, &unit_begin, &n_inst, &units, &iterations, &arrived, &late};
-    if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;
-    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, sm, s);
+    constexpr int S = decltype(sub)::value, M = decltype(minb)::value;
+    switch (riemann) {
+      case E2D_RIEMANN_HLLC: f(k_batch_loop_f32c<E2D_RIEMANN_HLLC, S, M>, S); break;
+      case E2D_RIEMANN_HLL: f(k_batch_loop_f32c<E2D_RIEMANN_HLL, S, M>, S); break;
+      default: f(k_batch_loop_f32c<E2D_RIEMANN_APPROX, S, M>, S); break;
+    }
   });
-  return e;
+}
+
+bool batch_loop_f32c_fits(int riemann, int rows) {
+  bool fits = false;
+  with_batch_loop(riemann, rows, [&](auto kernel, int sub) {
+    fits = resident_blocks(reinterpret_cast<const void *>(kernel), 32 * (CFL_UNIT_ROWS / sub),
+                           ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / sub)) > 0;
+  });
+  return fits;
 }
 
 cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, const int *list_slots,
                                    const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
                                    unsigned int late, cudaStream_t s) {
   if (n_inst <= 0 || units <= 0 || iterations <= 0) return cudaSuccess;
-  switch (riemann) {
-    case E2D_RIEMANN_HLLC:
-      return launch_batch_loop_t<E2D_RIEMANN_HLLC>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived,
-                                                   late, s);
-    case E2D_RIEMANN_HLL:
-      return launch_batch_loop_t<E2D_RIEMANN_HLL>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived,
-                                                  late, s);
-    default:
-      return launch_batch_loop_t<E2D_RIEMANN_APPROX>(rows, insts, list_slots, unit_begin, n_inst, units, iterations, arrived,
-                                                     late, s);
-  }
+  cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
+  with_batch_loop(riemann, rows, [&](auto kernel, int sub) {
+    const int threads = 32 * (CFL_UNIT_ROWS / sub);
+    const size_t sm = ring_bytes(SHORT_PFD, CFL_UNIT_ROWS / sub);
+    const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), threads, sm);
+    const int grid = units < resident ? units : resident;
+    void *args[] = {&insts, &list_slots, &unit_begin, &n_inst, &units, &iterations, &arrived, &late};
+    if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;  // batch_loop_f32c_fits says so before
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(threads), args, sm, s);
+  });
+  return e;
 }
 
 cudaError_t launch_loop_f32c(const KParams32 &kp, int riemann, int blocks, float *const w[2], DevClock *clk, int steps,

@@ -1081,6 +1081,7 @@ __global__ void __launch_bounds__(FILL_BX *FILL_BY) k_batch_prime_f64(BatchInst6
 // meanwhile, and threads that disagree would part at the block's barriers),
 // and nothing but the last tile writes `active`.
 // late: blocks more than there are that the barriers wait for (tests).
+// A launch of one iteration has no barrier and need not be cooperative.
 template <int RS, int TX, int TYM, int NT, int MINB, bool XMUL>
 __global__ void __launch_bounds__(NT, MINB)
     k_batch_loop_f64(BatchInst64 *insts, const int *__restrict__ list_slots, const int *__restrict__ tile_begin,
@@ -1337,6 +1338,13 @@ struct Shape<2> {
 constexpr int kShapes = 3;
 // Waves of tiles up to which a grid's steps run in one launch.
 constexpr int LOOP_WAVES = 4;
+// Waves of tiles up to which a batch's iterations run in one launch.  A
+// barrier gives up after a second, so what a block does between two has to be
+// bounded: a wave takes 0.25 ms with the slowest solver (the iterative one, a
+// 600x401 grid), this many a quarter of a second, of which a block waits for
+// the part by which others are slower.  A launch for each such iteration
+// costs nothing beside it.
+constexpr int BATCH_WAVES = 1024;
 template <class F>
 static void with_shape(int shape, F &&f) {
   switch (shape) {
@@ -1498,36 +1506,44 @@ cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s)
 template <int RS>
 static cudaError_t launch_batch_t(BatchInst64 *insts, const int *list_slots, const int *tile_begin, int n_inst,
                                   int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
-                                  unsigned int late, cudaStream_t s) {
+                                  unsigned int late, bool loop, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s);
   with_shape(shape, [&](auto sh) {
     using S = decltype(sh);
     auto kernel = k_batch_loop_f64<RS, S::TX, S::TYM, S::NT, S::MINB, S::XMUL>;
     constexpr size_t sm = flux_smem_bytes<S::TX, S::TYM>();
     const int resident = resident_blocks(reinterpret_cast<const void *>(kernel), S::NT, sm);
-    const int grid = total_tiles < resident ? total_tiles : resident;
-    void *args[] = {&insts, &list_slots, &tile_begin, &n_inst, &total_tiles, &ty, &iterations, &arrived, &late};
-    if (e == cudaSuccess && grid == 0) e = cudaErrorNotSupported;
-    if (e == cudaSuccess)
-      e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(S::NT), args, sm, s);
+    if (loop && resident > 0 && total_tiles <= (long long)resident * BATCH_WAVES) {
+      const int grid = total_tiles < resident ? total_tiles : resident;
+      void *args[] = {&insts, &list_slots, &tile_begin, &n_inst, &total_tiles, &ty, &iterations, &arrived, &late};
+      if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(grid), dim3(S::NT), args, sm, s);
+      return;
+    }
+    // as many blocks as are resident take the tiles, where that is known
+    const int grid = resident > 0 && resident < total_tiles ? resident : total_tiles;
+    for (int it = 0; it < iterations && e == cudaSuccess; ++it) {
+      kernel<<<grid, S::NT, sm, s>>>(insts, list_slots, tile_begin, n_inst, total_tiles, ty, 1, arrived, 0u);
+      e = cudaGetLastError();
+    }
   });
   return e;
 }
 
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
                              int n_inst, int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
-                             unsigned int late, cudaStream_t s) {
+                             unsigned int late, bool loop, cudaStream_t s) {
   if (n_inst <= 0 || total_tiles <= 0 || iterations <= 0) return cudaSuccess;
   switch (riemann) {
     case E2D_RIEMANN_HLLC:
       return launch_batch_t<E2D_RIEMANN_HLLC>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty, iterations,
-                                              arrived, late, s);
+                                              arrived, late, loop, s);
     case E2D_RIEMANN_HLL:
       return launch_batch_t<E2D_RIEMANN_HLL>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty, iterations,
-                                             arrived, late, s);
+                                             arrived, late, loop, s);
     default:
       return launch_batch_t<E2D_RIEMANN_APPROX>(insts, list_slots, tile_begin, n_inst, total_tiles, shape, ty,
-                                                iterations, arrived, late, s);
+                                                iterations, arrived, late, loop, s);
   }
 }
 

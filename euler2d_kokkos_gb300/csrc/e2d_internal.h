@@ -261,13 +261,13 @@ struct BatchInst64 {
 
 // The prologue of a newly admitted FP64 instance (q[0], acc[0] from u[0]).
 cudaError_t launch_batch_prime_f64(BatchInst64 *inst, int nfill, cudaStream_t s);
-// `iterations` steps of every listed FP64 instance in one cooperative launch:
-// list entry k is table slot list_slots[k]; tile_begin[k] is its first global
+// `iterations` steps of every listed FP64 instance, in one cooperative launch
+// (loop, where the blocks fit) or a launch each: list entry k is table slot list_slots[k]; tile_begin[k] is its first global
 // tile of that shape (n_inst + 1 entries, the last = total_tiles); arrived: a
 // device word for the launch's barriers; late: see k_batch_loop_f64.
 cudaError_t launch_batch_f64(int riemann, BatchInst64 *insts, const int *list_slots, const int *tile_begin,
                              int n_inst, int total_tiles, int shape, int ty, int iterations, unsigned int *arrived,
-                             unsigned int late, cudaStream_t s);
+                             unsigned int late, bool loop, cudaStream_t s);
 // Prologue blocks of an FP64 instance.
 void batch_f64_shape(const KParams64 &kp, int *nbx, int *nfill);
 
@@ -282,6 +282,8 @@ cudaError_t launch_batch_f32c(int riemann, int variant, BatchInst *insts, const 
 cudaError_t launch_batch_loop_f32c(int riemann, int rows, BatchInst *insts, const int *list_slots,
                                    const int *unit_begin, int n_inst, int units, int iterations, unsigned int *arrived,
                                    unsigned int late, cudaStream_t s);
+// Whether the device can hold that launch at all.
+bool batch_loop_f32c_fits(int riemann, int rows);
 int units_of(const KParams32 &kp);
 int short_rows_for(long long units, int riemann);
 // dt, dt/dx, dt/dy and `active` of an instance from acc[nstep & 1].

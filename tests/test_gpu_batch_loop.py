@@ -51,3 +51,31 @@ def test_fp64_loop_barrier_wait_runs_out_with_etimeout(gpu_lib, monkeypatch):
     with e2d.HydroRun(p) as h:
         t, ns, _ = h.step_n(3, 10.0, 0.0, 0)
         assert ns == 3 and np.isfinite(h.current(ns)).all()
+
+
+def alone(p, steps):
+    with e2d.HydroRun(p) as h:
+        t, ns, _ = h.step_n(steps, 1e9, 0.0, 0)
+        return t, h.current(ns)
+
+
+# lists whose FP64 tiles are chosen 8, 16 and 32 columns wide
+LISTS = [[(96, 80), (40, 33), (2, 2)], [(300, 200), (64, 64)], [(500, 300), (301, 257), (64, 48)]]
+WALLS = [(1, 1, 1, 1), (3, 3, 2, 1), (2, 1, 3, 3)]
+
+
+@pytest.mark.parametrize("loop", ["0", "1"])
+@pytest.mark.parametrize("grids", LISTS)
+@pytest.mark.parametrize("riemann", ["approx", "hll", "hllc"])
+@pytest.mark.parametrize("precision", [e2d.PRECISION_FP64, e2d.PRECISION_FP32C])
+def test_a_list_ends_where_each_grid_alone_does(gpu_lib, monkeypatch, precision, riemann, grids, loop):
+    """Also without cooperative launches (E2D_LOOP=0): a launch per iteration."""
+    monkeypatch.setenv("E2D_LOOP", loop)
+    params = [implosion(nx, ny, precision, riemann, bc=bc) for (nx, ny), bc in zip(grids, WALLS)]
+    with e2d.Batch(riemann, pool_bytes=POOL) as b:
+        ids = [b.admit(p, 1e9) for p in params]
+        assert b.run(4) == len(ids) and b.run(3) == len(ids)
+        got = [(b.query(i)[0], b.get_state(i)) for i in ids]
+    for p, (t, u) in zip(params, got):
+        want = alone(p, 7)
+        assert t == want[0] and np.array_equal(u, want[1])
