@@ -130,7 +130,7 @@ struct e2d_batch {
   int total_tiles = 0;
   int shape64 = 0, ty64 = 16;  // tile of the current FP64 work list
   int short_rows = 0;          // rows of the FP32C list's short strips (the list counts fold units); 0: strips
-  bool tuned_by_caller = false;  // set_tuning named a kernel variant: lists keep to it
+  bool tuned_by_caller = false;  // set_tuning named a variant or a strip height: lists keep to them
   bool loops = true;  // several iterations per cooperative launch (E2D_LOOP=0: a launch each)
   unsigned int *d_arrived = nullptr;  // barrier words of the multi-iteration launches (FP32C, FP64)
   bool list_dirty = true;
@@ -659,7 +659,10 @@ int e2d_batch_set_tuning(e2d_batch *b, int variant, const int strip_h[3]) {
   // strip heights are whole CFL fold units (16 rows)
   if (strip_h)
     for (int c = 0; c < 3; ++c)
-      if (strip_h[c] > 0 && strip_h[c] <= 512) b->strip_h[c] = (strip_h[c] + 15) / 16 * 16;
+      if (strip_h[c] > 0 && strip_h[c] <= 512) {
+        b->strip_h[c] = (strip_h[c] + 15) / 16 * 16;
+        b->tuned_by_caller = true;
+      }
   b->list_dirty = true;
   return E2D_OK;
 }
@@ -678,12 +681,18 @@ int e2d_batch_get_tuning(const e2d_batch *b, int *variant, int strip_h[3]) {
 // timing candidates are ordinary progress of the batch.
 int e2d_batch_autotune(e2d_batch *b, int iters_per_trial) {
   if (!b || iters_per_trial <= 0) return E2D_EINVAL;
-  b->tuned_by_caller = false;
   {
-    // a list in short strips leaves nothing to choose
+    // a list that runs in short strips leaves nothing to choose, and what a
+    // caller has set stays
+    const bool tuned = b->tuned_by_caller;
+    b->tuned_by_caller = false;
     int rc = rebuild_list(b);
+    if (rc == E2D_OK && (b->list.empty() || b->short_rows > 0)) {
+      b->tuned_by_caller = tuned;
+      b->list_dirty = tuned;
+      return E2D_OK;
+    }
     if (rc != E2D_OK) return rc;
-    if (b->list.empty() || b->short_rows > 0) return E2D_OK;
   }
   cudaEvent_t e0, e1;
   B_CK(b, cudaEventCreate(&e0), "event");

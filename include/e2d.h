@@ -292,10 +292,11 @@ int e2d_batch_stream(e2d_batch *b, void **stream);
  * rows staged by TMA copies waited on with mbarriers) and rows per strip (16..512,
  * rounded up to a multiple of 16) for the size classes max(nx, ny) <= 192,
  * <= 512, > 512.  Results do not depend on them.  Until a caller sets a
- * tuning, a short list of FP32C instances runs in strips of 2 to 8 rows
- * instead.  e2d_batch_autotune times the staged variants (4, 5, 6) and then
+ * variant or a height, a short list of FP32C instances runs in strips of 2 to
+ * 8 rows instead.  e2d_batch_autotune times the staged variants (4, 5, 6) and then
  * 16, 32 and 64 rows per size class on the live batch (its iterations advance
- * the instances) and keeps the fastest; on a short list it times nothing. */
+ * the instances) and keeps the fastest; on a list short enough for those
+ * strips it times nothing and leaves what a caller has set. */
 int e2d_batch_set_tuning(e2d_batch *b, int variant, const int strip_h[3]);
 int e2d_batch_get_tuning(const e2d_batch *b, int *variant, int strip_h[3]);
 int e2d_batch_autotune(e2d_batch *b, int iters_per_trial);

@@ -53,6 +53,22 @@ def test_fp64_loop_barrier_wait_runs_out_with_etimeout(gpu_lib, monkeypatch):
         assert ns == 3 and np.isfinite(h.current(ns)).all()
 
 
+def test_strip_heights_alone_are_a_tuning(gpu_lib, monkeypatch):
+    """Heights without a variant keep a short list in strips of them, and an
+    autotune that has nothing to time leaves them: strips have no grid barrier,
+    so E2D_TEST_WAIT_TIMEOUT=2 does not stop the solve."""
+    p = implosion(128, 96, e2d.PRECISION_FP32C)
+    monkeypatch.setenv("E2D_TEST_WAIT_TIMEOUT", "2")
+    for autotune in (False, True):
+        with e2d.Batch(pool_bytes=POOL) as b:
+            b.set_tuning(strip_h=[32, 48, 64])
+            i = b.admit(p, 10.0)
+            if autotune:
+                b.autotune(2)
+            assert b.run(3) == 1 and b.query(i)[1] == 3
+            assert b.get_tuning()[1] == [32, 48, 64]
+
+
 def alone(p, steps):
     with e2d.HydroRun(p) as h:
         t, ns, _ = h.step_n(steps, 1e9, 0.0, 0)
