@@ -95,6 +95,8 @@ E2D_HD uint32_t low(double x) {
   return (uint32_t)bits(x);
 #endif
 }
+// x > 0.0 (a NaN of either sign gives false)
+E2D_HD bool positive(double x) { return bits(x) - 1u < 0x7ff0000000000000ull; }
 // FP32 seeds: bit patterns of 1 / f and 1 / sqrt(f), relative error < 2^-21
 // (the hardware estimates are within 2^-22.9).
 E2D_HD uint32_t seed_rcp(uint32_t f) {

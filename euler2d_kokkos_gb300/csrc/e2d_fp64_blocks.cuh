@@ -337,7 +337,7 @@ __device__ __forceinline__ double cfl_term(const F &f, const KPhys<double> &ph, 
 __device__ __forceinline__ unsigned int state_flags(double rho, double e, double mx, double my) {
   unsigned int f = 0;
   if (nonfinite(rho) || nonfinite(e) || nonfinite(mx) || nonfinite(my)) f |= E2D_FLAG_NONFINITE;
-  if (!gt0(rho)) f |= E2D_FLAG_DENSITY;
+  if (!f64i::positive(rho)) f |= E2D_FLAG_DENSITY;
   return f;
 }
 
