@@ -6,6 +6,7 @@
 // per-instance dt; admission by free pool bytes; strip height per size class and
 // the kernel's register budget set by a measured autotuner.
 #include "e2d_internal.h"
+#include "e2d_tma.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -96,6 +97,7 @@ __global__ void k_put_record(T *dst, const __grid_constant__ T rec) {
   static_assert(sizeof(T) % 4 == 0, "copied by words");
   const int *src = reinterpret_cast<const int *>(&rec);
   for (int k = threadIdx.x; k < (int)(sizeof(T) / 4); k += blockDim.x) reinterpret_cast<int *>(dst)[k] = src[k];
+  tensormap_release();  // an FP32C instance's maps
 }
 template <class T>
 cudaError_t put_record(T *dst, const T &rec, cudaStream_t s) {

@@ -1292,6 +1292,7 @@ __global__ void __launch_bounds__(NT, MINB)
   unsigned long long *bars = s_bars + (TMA ? (threadIdx.x >> 5) * kMaxSlots : 0);
   unsigned int phase = 0u;  // carried across the warp's strips
   bool ring_ok = true;      // false after a TMA wait gave up with a copy maybe in flight
+  int mapped = -1;          // list entry whose tensor map the warp has acquired
   if (TMA && PFD > 0) ring_bars_init(bars, PFD + 3, lane);
   for (int w = blockIdx.x * WPB + (threadIdx.x >> 5); w < total_strips; w += nwarps) {
     // instance k with strip_begin[k] <= w < strip_begin[k + 1]
@@ -1309,6 +1310,10 @@ __global__ void __launch_bounds__(NT, MINB)
     const int par = I.par;
     const int strip = w - strip_begin[lo];
     const int rb = 2 + strip / I.nsx * kp.strip_h;
+    if (TMA && lo != mapped) {
+      if (lane == 0) tensormap_acquire(&I.tm[par]);  // the lane that copies
+      mapped = lo;
+    }
     if (ring_ok) {
       // the general march only: a persistent warp takes strips of many
       // instances, mostly boundary strips of small grids, and a second

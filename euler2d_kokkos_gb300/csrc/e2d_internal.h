@@ -227,8 +227,8 @@ cudaError_t launch_loop_f32c(const KParams32 &kp, int riemann, int blocks, float
 // One instance of a batch (device table entry): its grid, its two
 // compensated states and its own time loop.  The loop state is advanced by
 // the last strip of the instance to finish each iteration.
-struct BatchInst {
-  CUtensorMap tm[2];  // TMA maps of w[0], w[1] (64-byte aligned: first member)
+struct alignas(128) BatchInst {
+  CUtensorMap tm[2];  // TMA maps of w[0], w[1] (128 bytes each)
   KParams32 kp;
   float *w[2];
   double t, t_end, dt;          // dt: of the pending step

@@ -95,3 +95,17 @@ def test_a_list_ends_where_each_grid_alone_does(gpu_lib, monkeypatch, precision,
     for p, (t, u) in zip(params, got):
         want = alone(p, 7)
         assert t == want[0] and np.array_equal(u, want[1])
+
+
+def test_a_reused_slot_copies_by_its_own_tensor_map(gpu_lib):
+    """Instances of other sizes one after another in the same table slot, rows
+    staged by TMA (variant 6): each ends where the grid alone does."""
+    with e2d.Batch(pool_bytes=POOL) as b:
+        b.set_tuning(6, [32, 32, 32])
+        for k, (nx, ny) in enumerate([(300, 96), (421, 130), (200, 64), (700, 200), (301, 97)]):
+            p = implosion(nx, ny, e2d.PRECISION_FP32C, bc=WALLS[k % 3])
+            i = b.admit(p, 1e9)
+            assert i == 0 and b.run(5) == 1
+            want = alone(p, 5)
+            assert b.query(i)[0] == want[0] and np.array_equal(b.get_state(i), want[1])
+            b.release(i)
