@@ -109,3 +109,24 @@ def test_a_reused_slot_copies_by_its_own_tensor_map(gpu_lib):
             want = alone(p, 5)
             assert b.query(i)[0] == want[0] and np.array_equal(b.get_state(i), want[1])
             b.release(i)
+
+
+@pytest.mark.parametrize("autotune", [False, True])
+@pytest.mark.parametrize("riemann", ["hllc", "approx"])
+def test_a_long_list_that_gets_short(gpu_lib, riemann, autotune):
+    """More than 1100 fold units (strips, one launch an iteration, timed by an
+    autotune), then 449 and 65 as the larger solves end (short strips, many
+    iterations a launch): each solve ends where its grid alone does."""
+    params = [implosion(nx, ny, e2d.PRECISION_FP32C, riemann, bc=bc)
+              for (nx, ny), bc in zip([(1100, 700), (700, 500), (300, 200)], WALLS)]
+    want = [alone(p, 50 + 10 * k) for k, p in enumerate(params)]
+    with e2d.Batch(riemann, pool_bytes=POOL) as b:
+        ids = [b.admit(p, t) for p, (t, _) in zip(params, want)]
+        if autotune:
+            b.autotune(2)
+            assert 0 < b.query(ids[0])[1] < 50 and b.get_tuning()[0] in (4, 5, 6)
+        while b.run(7) > 0:
+            pass
+        got = [(b.query(i), b.get_state(i)) for i in ids]
+    for k, ((t, ns, active), u) in enumerate(got):
+        assert not active and ns == 50 + 10 * k and t == want[k][0] and np.array_equal(u, want[k][1])
