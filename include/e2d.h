@@ -157,7 +157,10 @@ int e2d_save_vtk(e2d_sim *sim, int which, const char *filename);
  * LayoutRight FP64, ghosts included) into `filename`.  No device work. */
 int e2d_write_vtk(const e2d_params *p, const double *host, int layout, const char *filename);
 /* Device address of U (which = 0) or U2 (1), LayoutLeft FP64, for zero-copy
- * use.  FP32C handles return a converted copy (hi + lo, ghosts filled) in a
+ * use: it holds for the life of the handle, and a state may be written through
+ * it between any two calls (the write finished, or ordered before the next call
+ * on the handle's stream).  So once an address has been given out, the handle
+ * keeps nothing of its states from one call to the next.  FP32C handles return a converted copy (hi + lo, ghosts filled) in a
  * staging array that the next call on the handle may overwrite. */
 int e2d_device_state(e2d_sim *sim, int which, double **dptr);
 /* Conservation audit: FP64 sums over the interior cells of rho, E, mx, my of
