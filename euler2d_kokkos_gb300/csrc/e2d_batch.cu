@@ -2,7 +2,8 @@
 // size resident in one device memory pool, advanced together by one kernel
 // launch per iteration for the FP32C instances (k_batch_f32c, replayed from
 // CUDA graphs), or one per run call when they are few (k_batch_loop_f32c),
-// and one per run call for the FP64 ones (k_batch_loop_f64), with
+// and one per run call for the FP64 ones (k_batch_loop_f64; one per iteration
+// where a cooperative launch is not to be had), with
 // per-instance dt; admission by free pool bytes; strip height per size class and
 // the kernel's register budget set by a measured autotuner.
 #include "e2d_internal.h"
@@ -577,7 +578,7 @@ int e2d_batch_query(e2d_batch *b, int id, double *t, int *nstep, int *active) {
   if (t) *t = m.t();
   if (nstep) *nstep = m.nstep();
   if (active) *active = m.active();
-  if (m.status() & E2D_FLAG_TIMEOUT) return berr(b, E2D_ETIMEOUT, "instance stopped: a row-staging wait gave up");
+  if (m.status() & E2D_FLAG_TIMEOUT) return berr(b, E2D_ETIMEOUT, "instance stopped: a bounded device wait gave up");
   if (m.status() & (E2D_FLAG_NONFINITE | E2D_FLAG_BAD_DT)) return berr(b, E2D_ENUMERIC, "instance hit NaN/Inf or a bad dt");
   return E2D_OK;
 }

@@ -1363,7 +1363,7 @@ static void with_shape(int shape, F &&f) {
 // the two add with exponent 1.3; tiles beyond what is resident make further
 // waves, which average out once there are four.  The constants are fitted to
 // 300 timings (16 grids from 32x20 to 2048^2, every shape, 3 to 16 rows; 4 %
-// rms), on which the model's choice is the fastest tile of every grid.
+// rms), on which the model's choice is within a few percent of the fastest.
 // What it buys (us a step, HLLC; before: 32 x 32 tiles for every grid):
 // 64x48 71 -> 10.9 (8 x 3), 128^2 71 -> 15.1 (8 x 7), 256^2 72 -> 33.4
 // (32 x 7), 500x300 128 -> 61 (32 x 16), 2048^2 1832 -> 1553 (32 x 13: the

@@ -148,7 +148,8 @@ cudaError_t launch_fill_f64(const KParams64 &kp, double *u_in, double *u_out, do
 cudaError_t launch_step_f64(const KParams64 &kp, int riemann, const CUtensorMap &tm_q, int use_tma,
                             const double *q_in, double *q_out, double *u_in, double *u_out, DevClock *clk,
                             double *dt_trace, cudaStream_t s);
-// Blocks of a multi-step launch of the fused step, all resident at once
+// Blocks of a multi-step launch of the fused step, all resident at once, each
+// with up to LOOP_WAVES tiles
 // (0: the grid is too large for it), and that launch: up to `steps` steps
 // with a grid barrier between them, from states u[0], u[1] and their
 // primitives, beginning at clk's t and nstep.

@@ -13,8 +13,8 @@ serve            -- continuous batching under open-loop Poisson arrivals:
                     request's latency (arrival to completion) is recorded.
 
 A FP32C solve whose state turns non-finite is stopped by the batch
-(E2D_ENUMERIC; E2D_ETIMEOUT for a row-staging wait of the TMA variant that
-gave up) without affecting the others.  With on_nonfinite="fp64" (the
+(E2D_ENUMERIC; E2D_ETIMEOUT for a bounded device wait that gave up: row
+staging of the TMA variant, grid barrier) without affecting the others.  With on_nonfinite="fp64" (the
 default) it is admitted again from its initial state as an FP64 instance --
 the bit-exact FP64 kernels, in the same batch -- and its latency runs from the
 original arrival; "drop" records it in RunStats.failed instead.  FP32 arithmetic

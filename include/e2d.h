@@ -238,11 +238,14 @@ int e2d_godunov_unsplit_noalloc(const e2d_params *p, double *u_in, double *u_out
  * t >= t_end do nothing.  *t and *nStep are read and updated.  dt_trace
  * (optional, n entries) receives the dt of each step taken.  FP64: one
  * prologue kernel (primitives and CFL maximum of the input state), then the
- * fused step, whose epilogue folds the next step's CFL maximum.  Grids whose
- * tiles or strips are all resident at once run up to 1024 steps per
- * cooperative launch, with a bounded grid barrier between steps; larger grids
- * run one launch per step, replayed from cached CUDA graphs.  Blocks until
- * done.
+ * fused step, whose epilogue folds the next step's CFL maximum.  Small grids
+ * (FP64: up to four waves of tiles, FP32C: up to two of short strips) run up
+ * to 1024 steps per cooperative launch, with a bounded grid barrier between
+ * steps; larger grids run one launch per step, replayed from cached CUDA
+ * graphs.  Blocks until done.  A cooperative launch starts once all its blocks
+ * fit the GPU beside what else runs there, so it waits for a kernel that
+ * occupies a part of it for long; programs that keep such a kernel set
+ * E2D_LOOP=0 (one launch per step) before they create the handle or batch.
  * E2D_ENUMERIC: a step saw a non-finite state or dt; E2D_ETIMEOUT: a bounded
  * wait gave up: for a TMA copy (FP64 staging, FP32C row staging of the TMA
  * variants) or at the grid barrier (the state of this call is incomplete; the
@@ -279,7 +282,8 @@ int e2d_batch_run(e2d_batch *b, int iterations, int *n_active);
 /* Loop state of an instance as of the last run (t, steps, still active).
  * The outputs are filled in every case; the status is E2D_ENUMERIC or
  * E2D_ETIMEOUT for an instance the batch stopped (a non-finite state or dt;
- * a row-staging wait or a grid barrier that gave up), which stays inactive. */
+ * a bounded device wait -- row staging, grid barrier -- that gave up), which
+ * stays inactive. */
 int e2d_batch_query(e2d_batch *b, int id, double *t, int *nstep, int *active);
 /* Current state of an instance (hi + lo in FP64, ghosts filled), host copy. */
 int e2d_batch_get_state(e2d_batch *b, int id, double *host, int layout);

@@ -248,7 +248,7 @@ class Batch {
   }
   // like active() without throwing for a solve the batch stopped: returns
   // E2D_OK, E2D_ENUMERIC (non-finite state or dt) or E2D_ETIMEOUT (a
-  // row-staging wait gave up); *active, *t, *nstep are filled in every case
+  // bounded device wait gave up); *active, *t, *nstep are filled in every case
   int poll(int id, bool *active, double *t = nullptr, int *nstep = nullptr) {
     int a = 0;
     const int rc = e2d_batch_query(b_, id, t, nstep, &a);
