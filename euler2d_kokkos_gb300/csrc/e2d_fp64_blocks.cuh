@@ -268,8 +268,11 @@ __device__ __forceinline__ void riemann_hll(const F &f, const KPhys<double> &ph,
   const double pr = floor_pressure(f, ph, qr[E2D_IP], rr);
   const double ur = qr[E2D_IU], vr = qr[E2D_IV];
   // r u, r v and r u u serve the state, the flux and the energy, whose factor
-  // 0.5 is exact wherever it is applied (barring underflow, and the energy's
-  // pressure term absorbs that): 12 products a cell fewer, 523 -> 495 us a
+  // 0.5 is exact wherever it is applied, barring underflow, which the energy's
+  // pressure term absorbs, and kinetic energies within a factor of two of the
+  // largest double, whose r u u overflows: the step reports such a state as
+  // non-finite (forming it again there cost 1.8 to 4 % of every HLL step in
+  // five forms): 12 products a cell fewer, 523 -> 495 us a
   // 1531x797 step, 488 with the last product on the integer pipes in the
   // room this leaves there (another 4 or 8 of a flux's: 492, 500).
   const double mxl = f.mul(rl, ul), myl = f.mul(rl, vl), mxul = f.mul(mxl, ul);
